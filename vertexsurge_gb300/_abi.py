@@ -546,7 +546,7 @@ class ExpandPlan:
         check(lib().vs_expand_plan_set_row_limits_device(self.h, _ptr(row_kmax), int(n), _stream(stream)))
 
     def set_pull_kernel(self, kind: int):
-        """PULL kernel variant 0..3 (bit 0: 8 blocks/SM, bit 1: L2 cache policies)."""
+        """PULL kernel variant 0..7 (bit 2: short mode without preloading)."""
         check(lib().vs_expand_plan_set_pull_kernel(self.h, int(kind)))
 
     def set_row_limits(self, row_kmax):

@@ -27,7 +27,7 @@
 //           visited AND-NOT, the [k_min,k_max] accumulation and the popcounts
 //           (dedup_and_update_visit_and_count, bitmap.cpp:1054-1096, and
 //           merge_to_MT's union, vexpand.cpp:298-354, folded into the hop).
-//           Vertices above the hub threshold get a whole CTA.
+//           Vertices above the hub threshold are cut into pieces.
 //   PUSH    active rows OR-ed into their out-neighbours with 64-bit atomics,
 //           followed by a fused dedup/accumulate pass over the touched rows.
 #include <algorithm>
@@ -690,11 +690,10 @@ template <int H> struct L2Pol {
 };
 
 // ---------------------------------------------------------------------------
-// PULL.  A warp owns one target vertex; its lanes form G = 32/L groups of L
-// lanes, each group ORs one whole active in-neighbour row (Q uint4 = L * UPL
-// per lane at most) at a time.  In-neighbour ids are read 32 at a time,
-// filtered by the frontier flags with a ballot and compacted through shared
-// memory, so inactive rows cost one flag load and no gather.
+// Short-mode PULL.  A warp owns one target vertex; its lanes form G = 32/L
+// groups of L lanes, each group ORs one whole active in-neighbour row (Q uint4 =
+// L * UPL per lane at most) at a time.  In-neighbour ids are read 32 at a time,
+// filtered with a ballot and compacted through shared memory.
 //
 // Short rows.  In the later hops of a many-source expand over a power-law
 // graph most frontier rows hold a handful of sources, and a whole-row gather
@@ -965,6 +964,16 @@ __device__ __forceinline__ bool write_short(const PullArgs &a, uint32_t v, const
 // flag, counters.
 // PRE: the visited words of the row (vpre, lanes 0..L-1) and the row's
 // next-layer flag (oldf_pre) were loaded ahead by the caller.
+// the union is read first: it is complete after a few rows and then costs no atomic
+__device__ __forceinline__ void add_union(uint4 *u, uint4 x) {
+  const uint4 n = andnot4(x, __ldcg(u));
+  unsigned *w = reinterpret_cast<unsigned *>(u);
+  if (n.x) atomicOr(w, n.x);
+  if (n.y) atomicOr(w + 1, n.y);
+  if (n.z) atomicOr(w + 2, n.z);
+  if (n.w) atomicOr(w + 3, n.w);
+}
+
 template <int L, int UPL, int H, bool PRE = false>
 __device__ __forceinline__ void pull_epilogue(const PullArgs &a, const L2Pol<H> &pol, uint32_t v,
                                               const uint32_t q0, const uint32_t qn, uint4 (&acc)[UPL],
@@ -1061,33 +1070,469 @@ __device__ __forceinline__ void pull_counters(const PullArgs &a, unsigned long l
   if (a.tiny_in) block_add(se, &a.ctr->hop[a.h].short_edges);
 }
 
-template <int L, int UPL, int H>
-__device__ __forceinline__ void pull_vertices(const PullArgs &a) {
-  const L2Pol<H> pol;
-  __shared__ uint32_t s_u[8][32];
-  const int wib = threadIdx.x >> 5;
-  const uint32_t q0 = blockIdx.y * a.qslice;
-  const uint32_t qn = min(a.qslice, a.Q - q0);
-  unsigned long long nb = 0, nv = 0, ns = 0, se = 0;
-  for (uint32_t v = blockIdx.x * 8 + wib; v < a.V; v += gridDim.x * 8) {
-    if (a.hub_threshold) {
-      int64_t d = 0;
-      _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n) d += a.in.off[l][v + 1] - a.in.off[l][v];
-      if (d > (int64_t)a.hub_threshold) continue;  // handled by k_pull_hub
-    }
-    uint4 acc[UPL];
+// ---------------------------------------------------------------------------
+// Dense PULL.  L lanes hold a row (UPL uint4 per lane; L < 32 when the row is
+// narrower than a warp), and a warp's G = 32 / L groups each own a target of
+// their own: a group walks its target's in-list 8 or more entries a round with
+// every row load in flight at once, so neither a reduction across groups nor a
+// shuffle tree is paid per target.  What bounds it: row loads from L2 (rows of
+// 256 bytes and more), else instructions and the latency of the chain offset ->
+// neighbour -> flag -> row, which the groups of a warp overlap.
+//
+// Scheduling.  Warps take tasks of `tile` consecutive targets from a counter
+// (in-degrees of R-MAT graphs follow the bits of the vertex id, so any fixed
+// stride gives some warps a multiple of the mean work).  Targets above the
+// heavy threshold are cut into pieces that come first
+// in the same queue: a warp ORs a piece with all its groups, adds it to the
+// target's union in HBM, and the warp that adds the last piece runs the
+// epilogue.
+//
+// Early exit.  A row can only gain sources that some row of layer h-1 holds
+// (their union, kept per layer by the PULL epilogues) and that the target has
+// not visited: a target with nothing left to gain is skipped, and a list is
+// left as soon as the row holds everything it could gain.  In the saturated
+// hops of a small-world graph most targets stop within a few neighbours.
+//
+// Measured on GB300 against a warp per target at a fixed stride with a CTA per
+// hub: R-MAT scale 16, 512 sources, hops 2 and 3 172 + 27 us -> 36 us each;
+// 1M-vertex power law, 64 sources, hop 4 465 -> 151 us; R-MAT scale 20 both
+// ways, 1,001 sources, hop 2 3.36 -> 0.63 ms; R-MAT scale 18, 3,000 sources, hops
+// 3 to 5 1.38 ms -> 0.31, 0.20 and 0.17 ms; 4,096 sources on the 1M-vertex power
+// law, hop 4 (no row saturates) 1.58 -> 1.43 ms at 10.7 TB/s of row loads.
+constexpr uint32_t NONE = 0xffffffffu;
+template <int L> constexpr int kChunk = L == 1 ? 8 : 32;
+
+// Entries per piece and default heavy threshold: a piece of a narrow row is one
+// or two rounds of a warp's groups, and the groups of a warp wait for its
+// longest list, so narrow rows (many groups) cut earlier.
+inline uint32_t piece_edges(int L) { return L <= 8 ? 512 : 256; }
+inline uint32_t heavy_default(int L) { return L <= 8 ? 64 : 256; }
+
+// Whether `p` holds on every lane of this lane's group.
+template <int L> __device__ __forceinline__ bool group_all(bool p) {
+  if (L == 1) return p;
+  if (L == 32) return __all_sync(FULL, p);
+  const unsigned gm = ((1u << (L & 31)) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+  return (__ballot_sync(FULL, p) & gm) == gm;
+}
+
+// Bits of uint4 q of a row that exist (sources below S).
+__device__ __forceinline__ uint4 row_bits(uint32_t q, uint32_t S) {
+  uint32_t w[4];
 #pragma unroll
-    for (int k = 0; k < UPL; k++) acc[k] = make_uint4(0, 0, 0, 0);
-    _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n)
-      gather_rows<L, UPL, H, false>(a, pol, s_u[wib], nullptr, q0, qn, acc, a.in.adj[l],
-                                    pol.ld_stream(a.in.off[l] + v), pol.ld_stream(a.in.off[l] + v + 1), 0, 32, se);
-#pragma unroll
-    for (int o = L; o < 32; o <<= 1)
-#pragma unroll
-      for (int k = 0; k < UPL; k++) acc[k] = or4(acc[k], shfl_xor4(acc[k], o));
-    pull_epilogue<L, UPL, H>(a, pol, v, q0, qn, acc, nb, nv, ns);
+  for (int i = 0; i < 4; i++) {
+    const uint32_t b = q * 128 + i * 32;
+    w[i] = b + 32 <= S ? 0xffffffffu : b < S ? (1u << (S - b)) - 1u : 0u;
   }
-  pull_counters(a, nb, nv, ns, se);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__device__ __forceinline__ uint4 and4(uint4 a, uint4 b) {
+  return make_uint4(a.x & b.x, a.y & b.y, a.z & b.z, a.w & b.w);
+}
+
+// Nothing left to gain: every bit of um is in vv or acc.
+template <int L, int UPL>
+__device__ __forceinline__ bool covered(const uint4 *s_um, uint32_t qn, const uint4 (&vv)[UPL], const uint4 (&acc)[UPL]) {
+  const uint32_t gl = threadIdx.x & (L - 1);
+  bool c = true;
+#pragma unroll
+  for (int k = 0; k < UPL; k++) {
+    const uint32_t q = gl + k * L;
+    if (q < qn) c = c && !nz4(andnot4(s_um[q], or4(vv[k], acc[k])));
+  }
+  return c;
+}
+
+// OR the rows of list entries j, j + 1, ... (a group's rounds are `step` apart)
+// below n into acc, until the row is covered.  Every lane of the warp calls it;
+// a group with sat set only takes part in the votes.
+template <int L, int UPL>
+__device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__restrict__ F, const uint32_t *__restrict__ flag,
+                                            const uint4 *s_um, uint32_t qn, const uint32_t *__restrict__ adj,
+                                            uint32_t n, uint32_t j, uint32_t step, const uint4 (&vv)[UPL],
+                                            uint4 (&acc)[UPL], bool &sat) {
+  const uint32_t lane = threadIdx.x & 31, gl = lane & (L - 1);
+  if constexpr (L < 32) {
+    constexpr int CH = kChunk<L>;  // entries per group and round, all requested at once
+    constexpr int K = CH / L;         // ... per lane
+    for (;;) {
+      const bool more = !sat && j < n;
+      if (!__any_sync(FULL, more)) break;
+      uint32_t id[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const uint32_t i = j + k * L + gl;
+        id[k] = NONE;
+        if (more && i < n) id[k] = __ldg(adj + i);
+      }
+      if (flag) {  // few rows of a round are non-empty: walk those
+#pragma unroll
+        for (int k = 0; k < K; k++)
+          if (id[k] != NONE && !__ldg(flag + id[k])) id[k] = NONE;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          unsigned m = __ballot_sync(FULL, id[k] != NONE) >> (lane & ~(L - 1)) & ((1u << L) - 1u);
+          while (__any_sync(FULL, m)) {
+            uint4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const uint32_t u = __shfl_sync(FULL, id[k], m ? __ffs(m) - 1 : 0, L);
+              x[i] = make_uint4(0, 0, 0, 0);
+              if (m && gl < qn) x[i] = __ldg(F + (size_t)u * a.Q + gl);
+              m &= m - 1;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[0] = or4(acc[0], x[i]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i0 = 0; i0 < CH; i0 += 8) {
+          if (i0 && !__any_sync(FULL, !sat && j + i0 < n)) break;
+          uint4 x[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const uint32_t u = L == 1 ? id[(i0 + i) / L] : __shfl_sync(FULL, id[(i0 + i) / L], (i0 + i) % L, L);
+            x[i] = make_uint4(0, 0, 0, 0);
+            if (u != NONE && gl < qn) x[i] = __ldg(F + (size_t)u * a.Q + gl);
+          }
+#pragma unroll
+          for (int i = 0; i < 8; i++) acc[0] = or4(acc[0], x[i]);
+        }
+      }
+      j += step;
+      const bool c = group_all<L>(covered<L, UPL>(s_um, qn, vv, acc));
+      sat = sat || c;
+    }
+  } else {
+    constexpr int R = UPL == 1 ? 8 : UPL == 2 ? 4 : 2;  // rows in flight
+    for (; j < n && !sat; j += step) {
+      uint32_t id = NONE;
+      if (j + lane < n) id = __ldg(adj + j + lane);
+      if (flag && id != NONE && !__ldg(flag + id)) id = NONE;
+      unsigned m = __ballot_sync(FULL, id != NONE);
+      while (m) {
+        uint32_t u[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {  // m is the same on every lane
+          const uint32_t t = __shfl_sync(FULL, id, m ? __ffs(m) - 1 : 0);
+          u[k] = m ? t : NONE;
+          m &= m - 1;
+        }
+#pragma unroll
+        for (int t = 0; t < UPL; t++) {
+          const uint32_t q = lane + t * 32;
+          uint4 x[R];
+#pragma unroll
+          for (int k = 0; k < R; k++) {
+            x[k] = make_uint4(0, 0, 0, 0);
+            if (u[k] != NONE && q < qn) x[k] = __ldg(F + (size_t)u[k] * a.Q + q);
+          }
+#pragma unroll
+          for (int k = 0; k < R; k++) acc[t] = or4(acc[t], x[k]);
+        }
+        if (group_all<32>(covered<L, UPL>(s_um, qn, vv, acc))) {
+          sat = true;
+          break;
+        }
+      }
+    }
+  }
+}
+
+// Group form of write_short for every group of the warp at once: the tiny
+// word and slot of the group's row x (valid: the group has a target, nz: its
+// row is not empty), c the lane's bit count.  Returns whether the row is short.
+template <int L, int UPL>
+__device__ __forceinline__ bool write_short_group(const PullArgs &a, uint32_t v, bool valid, bool nz,
+                                                  const uint4 (&x)[UPL], uint32_t qn, uint32_t c,
+                                                  unsigned long long &ns) {
+  constexpr int G = 32 / L, SQ = G * 2 > 8 ? G * 2 : 8;
+  // slots of up to 64 entries where a warp holds one row (L == 32), of 16 below
+  __shared__ uint4 s_stage[8][SQ];
+  const uint32_t lane = threadIdx.x & 31, gl = lane & (L - 1), g = lane / L;
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < L; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, incl, o, L);
+    if (gl >= (uint32_t)o) incl += y;
+  }
+  const uint32_t total = L == 1 ? c : __shfl_sync(FULL, incl, L - 1, L);
+  const bool fits = valid && nz && total < a.slot_n;
+  uint4 *stage4 = &s_stage[threadIdx.x >> 5][L == 32 ? 0 : g * 2];
+  uint16_t *stage = reinterpret_cast<uint16_t *>(stage4);
+  uint4 *slot = reinterpret_cast<uint4 *>(a.slot_out + (size_t)v * a.slot_n);
+  if (fits && c) {
+    uint32_t pos = 1 + incl - c;
+#pragma unroll
+    for (int k = 0; k < UPL; k++) {
+      const uint32_t q = gl + k * L;
+      if (q < qn) {
+        const uint32_t w[4] = {x[k].x, x[k].y, x[k].z, x[k].w};
+#pragma unroll
+        for (int wi = 0; wi < 4; wi++) {
+          uint32_t bits = w[wi];
+          while (bits) {
+            stage[pos++] = (uint16_t)(q * 128 + wi * 32 + __ffs(bits) - 1);
+            bits &= bits - 1;
+          }
+        }
+      }
+    }
+  }
+  if (fits && gl == 0) stage[0] = (uint16_t)total;
+  __syncwarp();
+  if (fits)
+    for (uint32_t i = gl; i < a.slot_n / 8; i += L) slot[i] = stage4[i];
+  if (valid && gl == 0) {
+    if (!nz) {
+      a.tiny_out[v] = 0;
+      a.slot_out[(size_t)v * a.slot_n] = 0;
+    } else if (!fits) {  // a long row: its count alone
+      a.tiny_out[v] = tiny_word(total, 0);
+      a.slot_out[(size_t)v * a.slot_n] = (uint16_t)(total < 0xFFFFu ? total : 0xFFFFu);
+    } else {
+      a.tiny_out[v] = tiny_word(total, total <= TINY_MAX ? stage[1] | (total > 1 ? (uint32_t)stage[2] << 15 : 0u) : 0u);
+      ns += 1ull + (total <= TINY_MAX ? 1ull << 32 : 0ull);
+    }
+  }
+  __syncwarp();  // the staging slots are free for the warp's next round
+  return fits;
+}
+
+// Epilogue of a round: every group's target v (valid per group), its ORed rows
+// acc and visited words vv: visited update, accumulator OR, layer union,
+// next-layer row (with its tiny word and slot), flag, counters.
+template <int L, int UPL>
+__device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bool valid, uint32_t q0, uint32_t qn,
+                                               const uint4 *s_um, uint4 *s_un, const uint4 (&vv)[UPL], uint4 (&acc)[UPL],
+                                               unsigned long long &nb, unsigned long long &nv, unsigned long long &ns) {
+  const uint32_t lane = threadIdx.x & 31, gl = lane & (L - 1);
+  bool any = false;
+  uint32_t bits = 0;
+#pragma unroll
+  for (int k = 0; k < UPL; k++) {
+    const uint32_t q = gl + k * L;
+    uint4 x = make_uint4(0, 0, 0, 0);
+    if (valid && q < qn) {
+      x = and4(andnot4(acc[k], vv[k]), s_um[q]);
+      if (nz4(x)) {
+        const size_t idx = (size_t)v * a.Q + q0 + q;
+        any = true;
+        bits += popc4(x);
+        if (a.shortest) a.vis[idx] = or4(vv[k], x);
+        if (a.acc_on) {
+          const uint4 o = a.acc[idx];
+          if (nz4(andnot4(x, o))) a.acc[idx] = or4(o, x);
+        }
+        if (!a.last) {
+          const uint4 n = andnot4(x, s_un[q]);
+          unsigned *w = reinterpret_cast<unsigned *>(s_un + q);
+          if (n.x) atomicOr(w, n.x);
+          if (n.y) atomicOr(w + 1, n.y);
+          if (n.z) atomicOr(w + 2, n.z);
+          if (n.w) atomicOr(w + 3, n.w);
+        }
+      }
+    }
+    acc[k] = x;
+  }
+  nb += bits;
+  const bool rownz = !group_all<L>(!any);
+  if (valid && gl == 0 && rownz && (a.res_vis || a.acc_on)) a.resflag[v] = 1;
+  if (a.multislice) {
+    if (valid && rownz) {
+#pragma unroll
+      for (int k = 0; k < UPL; k++) {
+        const uint32_t q = gl + k * L;
+        if (q < qn && nz4(acc[k])) a.N[(size_t)v * a.Q + q0 + q] = acc[k];
+      }
+      if (gl == 0 && atomicOr(&a.flagN[v], 1u) == 0) nv++;
+    }
+    return;
+  }
+  const uint32_t oldf = valid ? a.flagN[v] : 0u;  // 1: the buffer row holds an older layer's bits
+  if (a.last) {
+    // layer k_max is not kept: clear the rows an earlier layer left in this
+    // buffer, so the next run finds it clean (a flag-2 row is zero already)
+    if (oldf == 1) {
+#pragma unroll
+      for (int k = 0; k < UPL; k++) {
+        const uint32_t q = gl + k * L;
+        if (q < qn) a.N[(size_t)v * a.Q + q0 + q] = make_uint4(0, 0, 0, 0);
+      }
+    }
+    __syncwarp();  // every lane of a group read its flag
+    if (valid && gl == 0) {
+      if (oldf) a.flagN[v] = 0;
+      nv += rownz;
+    }
+    return;
+  }
+  bool virt = false;  // the row is left in its slot only (flag 2)
+  if (a.tiny_out) virt = write_short_group<L, UPL>(a, v, valid, rownz, acc, qn, bits, ns) && a.virt_out;
+  if (valid && ((rownz && !virt) || oldf == 1)) {
+#pragma unroll
+    for (int k = 0; k < UPL; k++) {
+      const uint32_t q = gl + k * L;
+      if (q < qn) a.N[(size_t)v * a.Q + q0 + q] = virt ? make_uint4(0, 0, 0, 0) : acc[k];
+    }
+  }
+  __syncwarp();
+  if (valid && gl == 0) {
+    const uint32_t nf = rownz ? (virt ? 2u : 1u) : 0u;
+    if (nf != oldf) a.flagN[v] = nf;
+    nv += rownz;
+  }
+}
+
+template <int L, int UPL>
+__global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 2 : 1) k_pull(PullArgs a) {
+  HopCtr &hc = a.ctr->hop[a.h];
+  if (hc.strategy != ST_PULL || hc.short_pull) return;
+  constexpr uint32_t G = 32 / L, CH = kChunk<L>;
+  __shared__ uint4 s_um[L * UPL];  // what a row can gain: the union of layer h-1, rows still growing
+  __shared__ uint4 s_un[L * UPL];  // union of the rows this block wrote
+  const uint32_t lane = threadIdx.x & 31, g = lane / L, gl = lane & (L - 1);
+  const uint32_t q0 = blockIdx.y * a.qslice, qn = min(a.qslice, a.Q - q0);
+  const HopCtr &pc = a.ctr->hop[a.h - 1];
+  for (uint32_t q = threadIdx.x; q < qn; q += blockDim.x) {
+    uint4 m = pc.strategy == ST_PULL && !pc.short_pull ? a.Uin[q0 + q] : row_bits(q0 + q, a.S);
+    if (a.hmask) m = and4(m, a.hmask[q0 + q]);
+    s_um[q] = m;
+    s_un[q] = make_uint4(0, 0, 0, 0);
+  }
+  __syncthreads();
+  // a row of one sector is loaded as fast as its flag, and a nearly full layer has few rows to skip
+  const bool useflag = a.Q > 2 && pc.active_vertices * 10 < 9ull * a.V;
+  const uint32_t *flag = useflag ? a.flagF : nullptr;
+  const uint4 *F = a.F + q0;
+  const bool known = a.res_vis && a.Q >= 8;  // resflag 0: the visited row is zero, without reading it
+  // rows are often complete only once a good part of all bits is visited; before
+  // that the visited words arrive while the first neighbours are fetched
+  unsigned long long seen = 0;
+  if (a.shortest)
+    for (int i = 0; i < a.h; i++) seen += a.ctr->hop[i].new_bits;
+  const bool precheck = seen > (unsigned long long)a.V * a.S / 8;
+  const uint32_t ntasks = a.npieces + (a.V + a.tile - 1) / a.tile;
+  unsigned long long nb = 0, nv = 0, ns = 0;
+  auto fetch = [&]() {
+    uint32_t t = 0;
+    if (lane == 0) t = atomicAdd(a.queue + blockIdx.y, 1u);
+    return t;  // lane 0's; broadcast when used
+  };
+  auto visited = [&](uint32_t v, bool valid, uint4(&vv)[UPL]) {
+    const bool look = valid && a.shortest && (!known || a.resflag[v]);
+#pragma unroll
+    for (int k = 0; k < UPL; k++) {
+      vv[k] = make_uint4(0, 0, 0, 0);
+      const uint32_t q = gl + k * L;
+      if (look && q < qn) vv[k] = a.vis[(size_t)v * a.Q + q0 + q];
+    }
+  };
+  uint32_t task = __shfl_sync(FULL, fetch(), 0);
+  while (task < ntasks) {
+    const uint32_t nexttask = fetch();  // in flight during this task
+    uint4 vv[UPL], acc[UPL];
+    if (task < a.npieces) {
+      const uint4 pc4 = __ldg(a.pieces + task);
+      const uint32_t v = pc4.x, np = pc4.y == NONE ? 1u : a.heavy_np[pc4.y];
+      uint4 *sum = a.heavy_rows + (np > 1 ? (size_t)pc4.y * a.Q + q0 : 0);
+      visited(v, true, vv);
+      uint4 cov[UPL];
+#pragma unroll
+      for (int k = 0; k < UPL; k++) {
+        acc[k] = make_uint4(0, 0, 0, 0);
+        cov[k] = vv[k];
+        const uint32_t q = gl + k * L;
+        if (np > 1 && q < qn) cov[k] = or4(cov[k], __ldcg(sum + q));  // what other pieces found already
+      }
+      bool sat = group_all<L>(covered<L, UPL>(s_um, qn, cov, acc));
+      const int64_t beg = a.in.off[pc4.z][v], end = a.in.off[pc4.z][v + 1];
+      const uint32_t n = (uint32_t)min((int64_t)pc4.w + a.piece_edges, end - beg);
+      gather_list<L, UPL>(a, F, flag, s_um, qn, a.in.adj[pc4.z] + beg, n, pc4.w + (L < 32 ? g * CH : 0),
+                          L < 32 ? G * CH : 32, cov, acc, sat);
+#pragma unroll
+      for (int o = L; o < 32; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < UPL; k++) acc[k] = or4(acc[k], shfl_xor4(acc[k], o));
+      bool mine = true;
+      if (np > 1) {
+        if (g == 0) {
+#pragma unroll
+          for (int k = 0; k < UPL; k++) {
+            const uint32_t q = gl + k * L;
+            if (q < qn) add_union(sum + q, acc[k]);
+          }
+          __threadfence();
+        }
+        __syncwarp();
+        uint32_t left = 0;
+        uint32_t *cnt = a.heavy_left + (size_t)pc4.y * gridDim.y + blockIdx.y;
+        if (lane == 0) left = atomicSub(cnt, 1u);
+        left = __shfl_sync(FULL, left, 0);
+        mine = left == 1;
+        if (mine) {  // the last piece: the whole union, and both left as they were found
+          __threadfence();
+#pragma unroll
+          for (int k = 0; k < UPL; k++) {
+            const uint32_t q = gl + k * L;
+            acc[k] = make_uint4(0, 0, 0, 0);
+            if (q < qn) acc[k] = __ldcg(sum + q);
+          }
+          __syncwarp();
+          if (g == 0) {
+#pragma unroll
+            for (int k = 0; k < UPL; k++) {
+              const uint32_t q = gl + k * L;
+              if (q < qn) sum[q] = make_uint4(0, 0, 0, 0);
+            }
+          }
+          if (lane == 0) *cnt = np;
+        }
+      }
+      if (mine) group_epilogue<L, UPL>(a, v, g == 0, q0, qn, s_um, s_un, vv, acc, nb, nv, ns);
+    } else {
+      // the tile's list starts at once: lane i holds those of target v0 + i (a tile of
+      // L > 1 has at most 16 targets, so lane i + 1 holds the end too)
+      const uint32_t v0 = (task - a.npieces) * a.tile;
+      int64_t off[2] = {0, 0}, oend[2] = {0, 0};
+      _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n) {
+        off[l] = __ldg(a.in.off[l] + min(v0 + lane, a.V));
+        if (L == 1) oend[l] = __ldg(a.in.off[l] + min(v0 + lane + 1, a.V));
+      }
+      for (uint32_t r = 0; r < a.tile && v0 + r < a.V; r += G) {
+        const uint32_t v = v0 + r + g;
+        bool valid = v < a.V;
+        int64_t beg[2] = {0, 0};
+        uint32_t n[2] = {0, 0};
+        uint64_t d = 0;
+        _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n) {
+          beg[l] = L == 1 ? off[l] : __shfl_sync(FULL, off[l], r + g);
+          n[l] = (uint32_t)((L == 1 ? oend[l] : __shfl_sync(FULL, off[l], r + g + 1)) - beg[l]);
+          d += n[l];
+        }
+        if (a.heavy_threshold && d > a.heavy_threshold) valid = false;  // comes in pieces
+        visited(v, valid, vv);
+#pragma unroll
+        for (int k = 0; k < UPL; k++) acc[k] = make_uint4(0, 0, 0, 0);
+        bool sat = !valid;
+        if (precheck) {
+          const bool c = group_all<L>(covered<L, UPL>(s_um, qn, vv, acc));
+          sat = sat || c;
+        }
+        _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n)
+          gather_list<L, UPL>(a, F, flag, s_um, qn, a.in.adj[l] + beg[l], n[l], 0, L < 32 ? CH : 32, vv, acc, sat);
+        group_epilogue<L, UPL>(a, v, valid, q0, qn, s_um, s_un, vv, acc, nb, nv, ns);
+      }
+    }
+    task = __shfl_sync(FULL, nexttask, 0);
+  }
+  pull_counters(a, nb, nv, ns, 0);
+  __syncthreads();
+  if (!a.last)
+    for (uint32_t q = threadIdx.x; q < qn; q += blockDim.x) add_union(a.Uout + q0 + q, s_un[q]);
 }
 
 // Short mode (one slice).  Software-pipelined over the warp's targets: while
@@ -1247,12 +1692,6 @@ __device__ __forceinline__ void pull_vertices_short(const PullArgs &a) {
   pull_counters(a, nb, nv, ns, se);
 }
 
-template <int L, int UPL, int MINB, int H>
-__global__ void __launch_bounds__(256, MINB) k_pull(PullArgs a) {
-  if (a.ctr->hop[a.h].strategy != ST_PULL || a.ctr->hop[a.h].short_pull) return;
-  pull_vertices<L, UPL, H>(a);
-}
-
 // the same in short mode (its own kernel: the slot path's registers stay out
 // of the dense kernels' budget)
 template <int L, int UPL>
@@ -1324,12 +1763,6 @@ __device__ __forceinline__ void pull_hubs(const PullArgs &a) {
     }
   }
   pull_counters(a, nb, nv, ns, se);
-}
-
-template <int L, int UPL>
-__global__ void __launch_bounds__(512) k_pull_hub(PullArgs a) {
-  if (a.ctr->hop[a.h].strategy != ST_PULL || a.ctr->hop[a.h].short_pull || a.nhubs == 0) return;
-  pull_hubs<L, UPL, false>(a);
 }
 
 template <int L, int UPL>
@@ -1681,12 +2114,41 @@ __global__ void k_clear_diag(uint64_t *__restrict__ vis, const uint32_t *__restr
     if (src[i] < V) atomicAnd((unsigned long long *)&vis[(size_t)src[i] * W + (i >> 6)], ~(1ull << (i & 63)));
 }
 
-// Hub list of a direction set (degree above the threshold).
-__global__ void k_hubs(Lists in, uint32_t V, uint32_t thr, uint32_t *list, unsigned *n) {
+// Targets of a direction set whose in-degree is above the threshold: their list
+// (n[0]), the pieces the dense PULL cuts them into (n[1]) and how many have more
+// than one (n[2]).
+__device__ __forceinline__ uint32_t pieces_of(const Lists &in, uint32_t v, int l, uint32_t piece) {
+  return l < in.n ? (uint32_t)((in.off[l][v + 1] - in.off[l][v] + piece - 1) / piece) : 0u;
+}
+
+__global__ void k_hubs(Lists in, uint32_t V, uint32_t thr, uint32_t piece, uint32_t *list, unsigned *n) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
     int64_t d = 0;
     _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < in.n) d += in.off[l][v + 1] - in.off[l][v];
-    if (d > (int64_t)thr) list[atomicAdd(n, 1u)] = v;
+    if (d <= (int64_t)thr) continue;
+    list[atomicAdd(n, 1u)] = v;
+    const uint32_t np = pieces_of(in, v, 0, piece) + pieces_of(in, v, 1, piece);
+    atomicAdd(n + 1, np);
+    if (np > 1) atomicAdd(n + 2, 1u);
+  }
+}
+
+// n[0] pieces and n[1] targets of several pieces written so far
+__global__ void k_hub_pieces(Lists in, const uint32_t *__restrict__ heavy, uint32_t nheavy, uint32_t piece,
+                             uint4 *__restrict__ pieces, unsigned *n, uint32_t *__restrict__ np_of,
+                             uint32_t *__restrict__ left, uint32_t nslices) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nheavy; i += gridDim.x * blockDim.x) {
+    const uint32_t v = heavy[i];
+    const uint32_t np[2] = {pieces_of(in, v, 0, piece), pieces_of(in, v, 1, piece)};
+    uint32_t row = NONE;
+    if (np[0] + np[1] > 1) {
+      row = atomicAdd(n + 1, 1u);
+      np_of[row] = np[0] + np[1];
+      for (uint32_t y = 0; y < nslices; y++) left[(size_t)row * nslices + y] = np[0] + np[1];
+    }
+    uint32_t at = atomicAdd(n, np[0] + np[1]);
+    for (uint32_t l = 0; l < 2; l++)
+      for (uint32_t k = 0; k < np[l]; k++) pieces[at++] = make_uint4(v, row, l, k * piece);
   }
 }
 
@@ -1733,19 +2195,15 @@ using PullFn = void (*)(PullArgs);
 
 struct PullVariant {
   int L, UPL;
-  PullFn pull[4], hub;  // pull[k]: bit 0 = 8 blocks per SM, bit 1 = L2 cache policies
-  PullFn pull_short, hub_short, pull_short_pre;
+  PullFn pull, pull_short, hub_short, pull_short_pre;
 };
 
-#define VS_PULLS(L, U) {k_pull<L, U, 1, 0>, k_pull<L, U, 8, 0>, k_pull<L, U, 1, 1>, k_pull<L, U, 8, 1>}
-#define VS_VARIANT(L, U) \
-  {L, U, VS_PULLS(L, U), k_pull_hub<L, U>, k_pull_short<L, U>, k_pull_hub_short<L, U>, k_pull_short_pre<L, U>}
+#define VS_VARIANT(L, U) {L, U, k_pull<L, U>, k_pull_short<L, U>, k_pull_hub_short<L, U>, k_pull_short_pre<L, U>}
 const PullVariant kVariants[] = {
     VS_VARIANT(1, 1),  VS_VARIANT(2, 1),  VS_VARIANT(4, 1),  VS_VARIANT(8, 1), VS_VARIANT(16, 1),
     VS_VARIANT(32, 1), VS_VARIANT(32, 2), VS_VARIANT(32, 4), VS_VARIANT(32, 8),
 };
 #undef VS_VARIANT
-#undef VS_PULLS
 
 const PullVariant &pick_variant(uint32_t qslice) {
   for (const auto &v : kVariants)
@@ -1776,6 +2234,13 @@ struct vs_expand_plan {
   Ctr *ctr = nullptr;
   uint32_t *hubs = nullptr;
   uint32_t nhubs = 0, hub_threshold = 0;
+  // dense PULL: targets above heavy_threshold are cut into pieces
+  uint32_t heavy_threshold = 0, nheavy = 0, npieces = 0, tile = 32;
+  uint4 *pieces = nullptr, *heavy_rows = nullptr;
+  uint32_t *heavy_np = nullptr, *heavy_left = nullptr;
+  uint4 *un = nullptr;         // (k_max + 1) x Q uint4: union of the rows of every layer a PULL hop wrote
+  uint32_t *queue = nullptr;   // (k_max + 1) x nslices task counters of the PULL hops
+  size_t ctr_bytes = 0;        // ctr, un and queue are one allocation, zeroed at every run start
   bool use_vis = false, use_acc = false, clear_diag = false;
   bool collect_stats = false;
   int grid_pull = 0, grid_hub = 0, grid_sparse = 0, grid_v = 0, grid_push = 0, grid_short = 0, grid_short_pre = 0;
@@ -1835,7 +2300,7 @@ int plan_free(vs_expand_plan *pl) {
   void *ptrs[] = {pl->tiny[0], pl->tiny[1], pl->slot[0], pl->slot[1], pl->resflag, pl->pdeg[0], pl->pdeg[1], pl->doff,
                   pl->bsum, pl->hmask, pl->rowk, pl->buf[0], pl->buf[1], pl->flag[0], pl->flag[1], pl->vis, pl->acc,
                   pl->pairs[0], pl->pairs[1], pl->push_list, pl->touched, pl->d_src,
-                  pl->d_tgt, pl->d_dist, pl->ctr, pl->hubs};
+                  pl->d_tgt, pl->d_dist, pl->ctr, pl->hubs, pl->pieces, pl->heavy_rows, pl->heavy_np, pl->heavy_left};
   for (void *p : ptrs)  // stream-ordered after the plan's last run
     if (p) dfree(p, st);
   for (cudaEvent_t e : pl->ev)
@@ -2027,7 +2492,15 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     PL_ALLOC(pl->d_tgt, S);
     PL_ALLOC(pl->d_dist, S);
   }
-  PL_ALLOC(pl->ctr, 1);
+  {  // counters, layer unions and task queues in one block: one memset clears them
+    const size_t c = (sizeof(Ctr) + 15) / 16 * 16, u = (size_t)(p->k_max + 1) * pl->Q * 16;
+    pl->ctr_bytes = c + u + (size_t)(p->k_max + 1) * pl->nslices * 4;
+    char *base = nullptr;
+    PL_ALLOC(base, pl->ctr_bytes);
+    pl->ctr = reinterpret_cast<Ctr *>(base);
+    pl->un = reinterpret_cast<uint4 *>(base + c);
+    pl->queue = reinterpret_cast<uint32_t *>(base + c + u);
+  }
   PL_ALLOC(pl->hmask, (size_t)(p->k_max + 1) * pl->W);
   PL_ALLOC(pl->rowk, 2);
   pl->short_min = p->short_share == 0 ? 0.1 : p->short_share;
@@ -2053,37 +2526,69 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     plan_free(pl);
     return cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
   }
-  // hub list for the pull direction set
+  // heavy targets of the pull direction set: a list for short mode, pieces for the dense PULL
+  const PullVariant &var = pick_variant(pl->qslice);
   pl->hub_threshold = p->hub_threshold ? p->hub_threshold : 2048;
+  pl->heavy_threshold = p->hub_threshold ? p->hub_threshold : heavy_default(var.L);
   {
     Lists in = pull_lists(g, p->direction);
     unsigned *dn = nullptr;
-    if ((rc = dalloc_n(&pl->hubs, V, st)) != VS_OK || (rc = dalloc_n(&dn, 1, st)) != VS_OK) {
+    uint32_t *heavy = nullptr;
+    if ((rc = dalloc_n(&pl->hubs, V, st)) != VS_OK || (rc = dalloc_n(&heavy, V, st)) != VS_OK ||
+        (rc = dalloc_n(&dn, 8, st)) != VS_OK) {
+      dfree(heavy, st);
       plan_free(pl);
       return rc;
     }
-    cudaMemsetAsync(dn, 0, sizeof(unsigned), st);
-    { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->hub_threshold, pl->hubs, dn); vs::note_launch(); }
-    unsigned hn = 0;
-    cudaMemcpyAsync(&hn, dn, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    cudaMemsetAsync(dn, 0, 8 * sizeof(unsigned), st);
+    const uint32_t pe = piece_edges(var.L);
+    { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->hub_threshold, pe, pl->hubs, dn); vs::note_launch(); }
+    { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->heavy_threshold, pe, heavy, dn + 3); vs::note_launch(); }
+    unsigned hn[6] = {0, 0, 0, 0, 0, 0};
+    cudaMemcpyAsync(hn, dn, sizeof(hn), cudaMemcpyDeviceToHost, st);
     e = cudaStreamSynchronize(st);
+    pl->nhubs = hn[0];
+    pl->nheavy = hn[3];
+    pl->npieces = hn[4];
+    const size_t nmulti = hn[5];
+    if (e == cudaSuccess && pl->nheavy) {
+      if ((rc = dalloc_n(&pl->pieces, pl->npieces, st)) != VS_OK ||
+          (rc = dalloc_n(&pl->heavy_rows, nmulti * pl->Q, st)) != VS_OK ||
+          (rc = dalloc_n(&pl->heavy_np, nmulti, st)) != VS_OK ||
+          (rc = dalloc_n(&pl->heavy_left, nmulti * pl->nslices, st)) != VS_OK) {
+        dfree(heavy, st);
+        dfree(dn, st);
+        plan_free(pl);
+        return rc;
+      }
+      e = cudaMemsetAsync(pl->heavy_rows, 0, nmulti * pl->Q * 16, st);
+      { k_hub_pieces<<<sm_count() * 4, 256, 0, st>>>(in, heavy, pl->nheavy, pe, pl->pieces, dn + 6, pl->heavy_np,
+                                                     pl->heavy_left, pl->nslices); vs::note_launch(); }
+      if (e == cudaSuccess) e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // runs may be on any stream
+    }
+    dfree(heavy, st);
     dfree(dn, st);
     if (e != cudaSuccess) {
       plan_free(pl);
       return cuda_fail(e, "hub list", __FILE__, __LINE__);
     }
-    pl->nhubs = hn;
   }
   pl->pull_kind = p->pull_kernel;
   if (p->sparse_frac > 0) pl->sparse_frac = p->sparse_frac;
-  const PullVariant &var = pick_variant(pl->qslice);
   const int hub_smem = 16 * 32 * 16 * var.UPL;
-  if (hub_smem > 48 * 1024) cudaFuncSetAttribute(var.hub, cudaFuncAttributeMaxDynamicSharedMemorySize, hub_smem);
-  pl->grid_pull = occupancy_grid(var.pull[pl->pull_kind & 3], 256, 0, 8);
-  pl->grid_hub = std::max(1, std::min((int)pl->nhubs, occupancy_grid(var.hub, 512, hub_smem, 2)));
+  // a task is `tile` consecutive targets: a round of the warp's groups on small
+  // graphs (more tasks than warps), up to 16 targets on large ones
+  const uint32_t G = 32 / var.L;
+  const int occ = occupancy_grid(var.pull, 256, 0, 8);
+  pl->tile = G;
+  while (pl->tile < 16 && (uint64_t)V / pl->tile > 64ull * occ) pl->tile *= 2;
+  const uint64_t tasks = pl->npieces + ((uint64_t)V + pl->tile - 1) / pl->tile;
+  pl->grid_pull = (int)std::max<uint64_t>(1, std::min<uint64_t>(occ, (tasks + 7) / 8));
   if (pl->slot[0]) {  // short mode: a row of Q uint4 per warp (PULL) or per CTA (hubs)
     const int hs = hub_smem + (int)pl->Q * 16;
     if (hs > 48 * 1024) cudaFuncSetAttribute(var.hub_short, cudaFuncAttributeMaxDynamicSharedMemorySize, hs);
+    pl->grid_hub = std::max(1, std::min((int)pl->nhubs, occupancy_grid(var.hub_short, 512, hs, 2)));
     pl->grid_short = occupancy_grid(var.pull_short, 256, 8 * (size_t)pl->Q * 16, 8);
     pl->grid_short_pre = occupancy_grid(var.pull_short_pre, 256, 8 * (size_t)pl->Q * 16, 8);
   }
@@ -2149,7 +2654,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     { k_clear_flagged<<<pl->grid_v, 256, 0, st>>>(reinterpret_cast<uint4 *>(pl->acc ? pl->acc : pl->vis),
                                                 pl->resflag, V, Q, pl->ctr, 0, 0); vs::note_launch(); }
   if (pl->acc && pl->vis) VS_CK(cudaMemsetAsync(pl->vis, 0, rowbytes, st));
-  VS_CK(cudaMemsetAsync(pl->ctr, 0, sizeof(Ctr), st));
+  VS_CK(cudaMemsetAsync(pl->ctr, 0, pl->ctr_bytes, st));
   const Lists in = pull_lists(g, p.direction), outl = push_lists(g, p.direction);
   SeedArgs sa;
   sa.sources = pl->d_src;
@@ -2322,6 +2827,18 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     a.hub_threshold = pl->nhubs ? pl->hub_threshold : 0;
     a.hubs = pl->hubs;
     a.nhubs = pl->nhubs;
+    a.heavy_threshold = pl->nheavy ? pl->heavy_threshold : 0;
+    a.pieces = pl->pieces;
+    a.npieces = pl->npieces;
+    a.piece_edges = piece_edges(var.L);
+    a.heavy_np = pl->heavy_np;
+    a.heavy_left = pl->heavy_left;
+    a.heavy_rows = pl->heavy_rows;
+    a.tile = pl->tile;
+    a.queue = pl->queue + (size_t)h * pl->nslices;
+    a.Uin = pl->un + (size_t)(h - 1) * Q;
+    a.Uout = pl->un + (size_t)h * Q;
+    a.S = S_;
     a.ctr = pl->ctr;
     a.h = h;
     const bool keep_short = pl->slot[0] && h < p.k_max && !a.last;  // the next hop may read this layer's words
@@ -2346,9 +2863,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
       { k_slot_build<<<pl->grid_v, 256, 0, st>>>(pl->flag[fb], reinterpret_cast<const uint4 *>(pl->buf[fb]), V, Q,
                                                pl->tiny[fb], pl->slot[fb], pl->slot_n, pl->ctr, h); vs::note_launch(); }
     }
-    { var.pull[pl->pull_kind & 3]<<<dim3(pl->grid_pull, pl->nslices), 256, 0, st>>>(a); vs::note_launch(); }
-    if (pl->nhubs)
-      { var.hub<<<dim3(pl->grid_hub, pl->nslices), 512, 16 * 32 * 16 * var.UPL, st>>>(a); vs::note_launch(); }
+    { var.pull<<<dim3(pl->grid_pull, pl->nslices), 256, 0, st>>>(a); vs::note_launch(); }
     if (pl->slot[0]) {
       if (a.pre)
         { var.pull_short_pre<<<pl->grid_short_pre, 256, 8 * (size_t)Q * 16, st>>>(a); vs::note_launch(); }
@@ -2516,16 +3031,13 @@ int vs_expand_plan_set_row_limits_device(vs_expand_plan *pl, const uint8_t *row_
   return VS_OK;
 }
 
-// Kernel shape of the PULL hops (chosen by the autotuner): bit 0 asks for 8
-// resident 256-thread blocks per SM (32 registers), bit 1 adds L2 cache
-// policies (streams evict-first, frontier rows evict-last), bit 2 runs
-// short-mode hops without loading the next target's visited words and flag
-// ahead.
+// Kernel shape of the PULL hops: bit 2 runs short-mode hops without loading the
+// next target's visited words and flag ahead.  Bits 0 and 1 chose shapes of the
+// dense kernel that are gone (its groups run one shape per row width); they are
+// still taken, so saved settings stay valid.
 int vs_expand_plan_set_pull_kernel(vs_expand_plan *pl, int kind) {
   if (!pl || kind < 0 || kind > 7) return fail(VS_ERR_ARG, "pull kernel variant must be 0..7");
   pl->pull_kind = kind;
-  const PullVariant &var = pick_variant(pl->qslice);
-  pl->grid_pull = occupancy_grid(var.pull[kind & 3], 256, 0, 8);
   return VS_OK;
 }
 

@@ -134,6 +134,18 @@ struct PullArgs {
   uint32_t hub_threshold;
   const uint32_t *hubs;
   uint32_t nhubs;
+  // dense PULL: targets above heavy_threshold (0: none) come in pieces
+  uint32_t heavy_threshold;
+  const uint4 *pieces;       // (target, its row of heavy_rows or ~0 when this is its only piece, list, first entry)
+  uint32_t npieces, piece_edges;
+  const uint32_t *heavy_np;  // pieces of a heavy target
+  uint32_t *heavy_left;      // ... still to come, per slice (back at heavy_np after every hop)
+  uint4 *heavy_rows;         // union of the pieces done (zero between hops)
+  uint32_t tile;             // targets per task
+  uint32_t *queue;           // next task, per slice
+  const uint4 *Uin;          // union of layer h-1's rows (when a PULL hop wrote it)
+  uint4 *Uout;               // union of layer h's rows
+  uint32_t S;
   Ctr *ctr;
   int h;
 };
