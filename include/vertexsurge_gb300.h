@@ -179,10 +179,11 @@ typedef struct vs_expand_params {
   double short_share;      /* short-mode PULL: rows of the frontier with few bits (at most 15, or 31
                               / 63 for rows of 128 / more words) are read from a slot of their
                               source ids instead of whole, on hops where at least this share of
-                              the frontier's rows are short and the frontier exceeds half of L2
+                              the frontier's rows are short and the planner finds it faster
                               (0 = 0.1; < 0 = never; > 1 = every PULL hop); needs S <= 32768 and
                               whole-row passes, and keeps 36 to 132 B per vertex, except in plans
-                              whose V x S matrix fits in half of L2 (short mode never runs there) */
+                              whose V x S matrix fits in half of L2 or whose rows are below 32
+                              words (short mode never runs there unless it is forced) */
 } vs_expand_params;
 
 #define VS_MAX_HOPS 64
@@ -461,10 +462,8 @@ int vs_expand_plan_set_row_limits(vs_expand_plan *plan, const uint8_t *row_kmax,
  * row limit. */
 int vs_expand_plan_set_row_limits_device(vs_expand_plan *plan, const uint8_t *row_kmax, uint32_t n,
                                          vs_stream_t stream);
-/* Kernel shape of PULL hops (the autotuner's knob): kind 0..7, bit 2 =
- * short-mode hops without loading the next target's visited words and flag
- * ahead; bits 0 and 1 are taken and have no effect.  Results never depend on
- * it. */
+/* Kernel shape of PULL hops: kind 0..7 is taken and has no effect (the kernels
+ * run one shape per row width). */
 int vs_expand_plan_set_pull_kernel(vs_expand_plan *plan, int kind);
 /* Feature logging: when on, every run records the 32 features of each hop;
  * vs_expand_plan_features copies (VS_MAX_HOPS + 1) x 32 floats (row h = hop h). */

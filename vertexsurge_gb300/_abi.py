@@ -546,7 +546,7 @@ class ExpandPlan:
         check(lib().vs_expand_plan_set_row_limits_device(self.h, _ptr(row_kmax), int(n), _stream(stream)))
 
     def set_pull_kernel(self, kind: int):
-        """PULL kernel variant 0..7 (bit 2: short mode without preloading)."""
+        """PULL kernel variant 0..7: taken, without effect (one shape per row width)."""
         check(lib().vs_expand_plan_set_pull_kernel(self.h, int(kind)))
 
     def set_row_limits(self, row_kmax):

@@ -314,22 +314,41 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
   }
   if (t == 0) {
     cur.strategy = s_choice;
-    // short mode: enough short rows in a frontier that L2 does not already
-    // hold (a layer from a PULL hop counted them; from SPARSE or PUSH, a few
-    // bits per row on average stand in for the count)
+    // short mode where the hop costs less, in ps measured on GB300 over 1M- and
+    // 4M-vertex power-law and R-MAT graphs with 512 to 8,192 sources: a dense hop
+    // pays 7 to 18 per edge for neighbour and flag (with the row's lanes) and 0.8
+    // per word of every active row from L2; short mode 12.5 per edge, 21 per id read
+    // from words (10 on a last hop, which keeps no lists), 1.5 per id read from
+    // slots and 350 per target row then searched for bits (none on a last hop),
+    // and about twice the dense price for a row too long for a slot.
     bool sp = false;
+    const bool counted = prev.strategy == ST_PULL;  // ... its layer's words, slots and degrees
+    const double act = (double)prev.active_vertices, V = (double)a.V, E = (double)a.E * (a.both ? 2 : 1);
+    const double ids = prev.strategy == ST_PUSH ? E * (double)prev.new_bits / V : (double)prev.pair_edges;
+    double rows, longs = 0;  // edges leaving non-empty rows, and rows too long for a slot
+    if (counted) {
+      rows = (double)prev.row_out;
+      longs = rows - (double)prev.short_out;
+    } else {
+      rows = ids * act / fmax(1.0, (double)prev.new_bits);
+    }
+    const double t_long = 1.6 * a.W * longs;
+    const double t_words = 12.5 * E + (a.last ? 10.0 : 21.0) * ids + t_long;
+    const double t_slots = 12.5 * E + 1.5 * fmin(ids, 15.0 * (double)prev.short_out) +
+                           (a.last ? 0.0 : 350.0 * fmin(V, ids)) + t_long;
+    const bool slots = counted && t_slots < t_words;
     if (s_choice == ST_PULL && a.short_min > 0 && !c->multislice) {
-      const double act = (double)prev.active_vertices;
-      if (a.short_min > 1.0)
+      if (a.short_min > 1.0) {
         sp = true;
-      else if (act * 8.0 * (double)a.W > (double)a.l2_half)
-        sp = prev.strategy == ST_PULL ? (double)(prev.short_rows & 0xFFFFFFFFull) >= a.short_min * act
-                                      : (double)prev.new_bits <= 4.0 * act;
+      } else if (!counted || (double)(prev.short_rows & 0xFFFFFFFFull) >= a.short_min * act) {
+        const double flag = act >= 0.9 * V ? 6.0 : a.W <= 8 ? 7.0 : a.W <= 16 ? 8.0 : a.W <= 32 ? 12.0 : 18.0;
+        sp = (slots ? t_slots : t_words) < 0.9 * (flag * E + 0.8 * a.W * rows);
+      }
     }
     cur.short_pull = sp;
-    // a frontier of mostly 4..15-bit rows reads slots instead of words
-    cur.short_slots = sp && prev.strategy == ST_PULL &&
-                      (double)(prev.short_rows >> 32) < 0.5 * (double)(prev.short_rows & 0xFFFFFFFFull);
+    cur.short_slots = sp && slots;
+    // more than half a slot of ids per target: its new row will often be long
+    cur.short_long = ids > 1.2 * V * (a.W <= 64 ? 16 : a.W <= 128 ? 32 : 64);
   }
 }
 
@@ -641,60 +660,6 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// L2 cache policies for the PULL kernels (variant H = 1): adjacency lists,
-// offsets and the visited / next-layer streams are read or written once per
-// hop and marked evict-first, so L2 keeps the frontier rows, which power-law
-// hubs make the only reused data (marked evict-last).
-template <int H> struct L2Pol {
-  uint64_t first = 0, last = 0;
-  __device__ __forceinline__ L2Pol() {
-    if (H) {
-      asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
-      asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(last));
-    }
-  }
-  __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) const {
-    if (!H) return __ldg(p);
-    uint32_t r;
-    asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(first));
-    return r;
-  }
-  __device__ __forceinline__ int64_t ld_stream(const int64_t *p) const {
-    if (!H) return __ldg(p);
-    int64_t r;
-    asm("ld.global.nc.L2::cache_hint.s64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(first));
-    return r;
-  }
-  __device__ __forceinline__ uint4 ld_row(const uint4 *p) const {
-    if (!H) return __ldg(p);
-    uint4 r;
-    asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-        : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p), "l"(last));
-    return r;
-  }
-  __device__ __forceinline__ uint4 ld_rw(const uint4 *p) const {
-    if (!H) return *p;
-    uint4 r;
-    asm volatile("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p), "l"(first) : "memory");
-    return r;
-  }
-  __device__ __forceinline__ void st(uint4 *p, uint4 v) const {
-    if (!H) {
-      *p = v;
-      return;
-    }
-    asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;"
-                 :: "l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(first) : "memory");
-  }
-};
-
-// ---------------------------------------------------------------------------
-// Short-mode PULL.  A warp owns one target vertex; its lanes form G = 32/L
-// groups of L lanes, each group ORs one whole active in-neighbour row (Q uint4 =
-// L * UPL per lane at most) at a time.  In-neighbour ids are read 32 at a time,
-// filtered with a ballot and compacted through shared memory.
-//
 // Short rows.  In the later hops of a many-source expand over a power-law
 // graph most frontier rows hold a handful of sources, and a whole-row gather
 // then moves mostly zero words.  Every PULL hop with a successor therefore
@@ -708,7 +673,7 @@ template <int H> struct L2Pol {
 // bits) or its slot alone (slot mode, for frontiers of mostly longer rows):
 // count 0 is an empty row, short rows OR their ids into a per-warp
 // shared-memory row with 32-bit atomics, and only longer rows are gathered
-// whole.  Short rows of a layer with a successor stay in their slots only
+// whole (see the kernel).  Short rows of a layer with a successor stay in their slots only
 // (flag 2, buffer row zero) unless the layer's rows are read directly;
 // k_materialize writes them out before a hop that reads rows.  Layers
 // written by SPARSE or the seed get their words and slots from the hop's
@@ -737,234 +702,17 @@ __device__ __forceinline__ uint32_t tiny_count(Tiny t) {
   return cls < 3 ? cls : (t & 0xFFFFu);
 }
 
-// Bulk prefetch of `bytes` (a multiple of 16, 16-byte aligned) into L2.
-__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(p), "r"(bytes) : "memory");
-}
-
 // Read-only tiny-word load that asks L2 to keep the line (evict-last).
 __device__ __forceinline__ Tiny ld_keep(const Tiny *p) {
   uint64_t pol;
   asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  if constexpr (sizeof(Tiny) == 8) {
-    uint64_t r;
-    asm("ld.global.nc.L2::cache_hint.b64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(pol));
-    return (Tiny)r;
-  } else {
-    uint32_t r;
-    asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
-    return (Tiny)r;
-  }
+  Tiny r;
+  asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
+  return r;
 }
 
-// OR the ids of a tiny word (count in [1, TINY_MAX]) into a shared row
-__device__ __forceinline__ void or_tiny_ids(uint32_t *row32, Tiny t, uint32_t cnt) {
-  const uint32_t id0 = t & 0x7FFFu;
-  atomicOr(row32 + (id0 >> 5), 1u << (id0 & 31));
-  if (cnt > 1) {
-    const uint32_t id1 = (t >> 15) & 0x7FFFu;
-    atomicOr(row32 + (id1 >> 5), 1u << (id1 & 31));
-  }
-}
-
-// OR entries first..last (last < CHUNK_IDS) of one 32-byte slot chunk into
-// a shared row; the loop leaves at the warp's longest list
-__device__ __forceinline__ void or_chunk_ids(uint32_t *row32, const uint4 s0, const uint4 s1, uint32_t first,
-                                             uint32_t last) {
-  const uint32_t w[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-  for (uint32_t i = 0; i < CHUNK_IDS; i++) {
-    if (i > last) break;
-    if (i < first) continue;
-    const uint32_t id = (w[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu;
-    atomicOr(row32 + (id >> 5), 1u << (id & 31));
-  }
-}
-
-// OR the ids of a slot (count in [1, slot_n - 1]) whose first chunk is s0/s1
-__device__ __forceinline__ void or_slot_ids(uint32_t *row32, const uint4 *sp, const uint4 s0, const uint4 s1,
-                                            uint32_t cnt) {
-  or_chunk_ids(row32, s0, s1, 1, cnt < CHUNK_IDS - 1 ? cnt : CHUNK_IDS - 1);
-  for (uint32_t c0 = CHUNK_IDS; c0 <= cnt; c0 += CHUNK_IDS) {
-    const uint32_t left = cnt - c0;  // entries c0..cnt remain
-    or_chunk_ids(row32, __ldg(sp + c0 / 8), __ldg(sp + c0 / 8 + 1), 0, left < CHUNK_IDS - 1 ? left : CHUNK_IDS - 1);
-  }
-}
-
-// One chunk of up to 32 in-neighbours, u / act per lane.  Dense mode: act =
-// the row is non-zero (flag).  Short mode: act = the lane holds an
-// in-neighbour and tv is its tiny word; short rows OR their ids into row32,
-// the others are gathered whole.
-template <int L, int UPL, int H, bool SHORT>
-__device__ __forceinline__ void gather_chunk(const PullArgs &a, const L2Pol<H> &pol, uint32_t *s_u, uint32_t *row32,
-                                             const uint32_t q0, const uint32_t qn, uint4 (&acc)[UPL], uint32_t u,
-                                             bool act, Tiny tv, bool slotmode, unsigned long long &se,
-                                             const uint4 *pre = nullptr) {
-  constexpr int G = 32 / L;
-  const int lane = threadIdx.x & 31, g = lane / L, gl = lane % L;
-  if (SHORT && act) {
-    // slot mode (frontiers of mostly 4..15-bit rows): the slot alone, its
-    // entry 0 holds the count (pre: its first chunk, loaded ahead); word
-    // mode: the word, then the slot when the row has more ids than the word
-    // holds
-    const uint4 *sp = a.slot_in + (size_t)u * (a.slot_n / 8);
-    uint4 s0 = make_uint4(0, 0, 0, 0), s1 = s0;
-    uint32_t cnt;
-    if (slotmode) {
-      if (pre) {
-        s0 = pre[0];
-        s1 = pre[1];
-      } else {
-        s0 = __ldg(sp);
-        s1 = __ldg(sp + 1);
-      }
-      cnt = s0.x & 0xFFFFu;
-    } else {
-      cnt = tiny_count(tv);
-    }
-    if (cnt == 0) {
-      act = false;
-    } else if (!slotmode && cnt <= TINY_MAX) {
-      or_tiny_ids(row32, tv, cnt);
-      act = false;
-      se++;
-    } else if (cnt < a.slot_n) {
-      if (!slotmode) {
-        s0 = __ldg(sp);
-        s1 = __ldg(sp + 1);
-      }
-      or_slot_ids(row32, sp, s0, s1, cnt);
-      act = false;
-      se++;
-    }
-  }
-  const unsigned m = __ballot_sync(FULL, act);
-  if (!m) return;
-  if (act) s_u[__popc(m & lanemask_lt())] = u;
-  __syncwarp();
-  const int n = __popc(m);
-  int t = g;
-  for (; t + 3 * G < n; t += 4 * G) {
-    const uint4 *r0 = a.F + (size_t)s_u[t] * a.Q + q0;
-    const uint4 *r1 = a.F + (size_t)s_u[t + G] * a.Q + q0;
-    const uint4 *r2 = a.F + (size_t)s_u[t + 2 * G] * a.Q + q0;
-    const uint4 *r3 = a.F + (size_t)s_u[t + 3 * G] * a.Q + q0;
-#pragma unroll
-    for (int k = 0; k < UPL; k++) {
-      const uint32_t q = gl + k * L;
-      if (q < qn) {
-        uint4 x0 = pol.ld_row(r0 + q), x1 = pol.ld_row(r1 + q), x2 = pol.ld_row(r2 + q), x3 = pol.ld_row(r3 + q);
-        acc[k] = or4(acc[k], or4(or4(x0, x1), or4(x2, x3)));
-      }
-    }
-  }
-  for (; t < n; t += G) {
-    const uint4 *r0 = a.F + (size_t)s_u[t] * a.Q + q0;
-#pragma unroll
-    for (int k = 0; k < UPL; k++) {
-      const uint32_t q = gl + k * L;
-      if (q < qn) acc[k] = or4(acc[k], pol.ld_row(r0 + q));
-    }
-  }
-  __syncwarp();
-}
-
-template <int L, int UPL, int H, bool SHORT>
-__device__ __forceinline__ void gather_rows(const PullArgs &a, const L2Pol<H> &pol, uint32_t *s_u, uint32_t *row32,
-                                            const uint32_t q0, const uint32_t qn, uint4 (&acc)[UPL],
-                                            const uint32_t *adj, int64_t beg, int64_t end,
-                                            int64_t step_start, int64_t step, unsigned long long &se,
-                                            bool slotmode = false) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = beg + step_start; base < end; base += step) {
-    const int64_t j = base + lane;
-    uint32_t u = 0;
-    bool act = false;
-    Tiny tv = 0;
-    if (j < end) {
-      u = pol.ld_stream(adj + j);
-      if (SHORT) {
-        if (!slotmode) tv = ld_keep(a.tiny_in + u);
-        act = true;
-      } else {
-        act = __ldg(a.flagF + u) != 0;
-      }
-    }
-    gather_chunk<L, UPL, H, SHORT>(a, pol, s_u, row32, q0, qn, acc, u, act, tv, slotmode, se);
-  }
-}
-
-// The tiny word and the slot (ids for up to slot_n - 1 bits) of the
-// non-zero row of v held by lanes 0..L-1 (uint4 q = lane + k * L).  A short
-// row's ids are gathered in the warp's staging slot in shared memory and
-// stored with one 16-byte store per lane of the slot; stale entries past the
-// count are never read.
-template <int L, int UPL>
-// c: this lane's bit count of the row (0 past the row's lanes), counted by the caller
-__device__ __forceinline__ bool write_short(const PullArgs &a, uint32_t v, const uint4 (&acc)[UPL], uint32_t qn,
-                                            uint32_t c, unsigned long long &ns) {
-  __shared__ uint4 s_stage[16][8];  // a slot per warp (at most 64 entries, 16 warps)
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint32_t total = __reduce_add_sync(FULL, c);
-  uint16_t *slot = a.slot_out + (size_t)v * a.slot_n;
-  if (total >= a.slot_n) {  // a long row: its count alone
-    if (lane == 0) {
-      a.tiny_out[v] = tiny_word(total, 0);
-      slot[0] = (uint16_t)(total < 0xFFFFu ? total : 0xFFFFu);
-    }
-    return false;
-  }
-  // position of this lane's first id: exclusive prefix of the bit counts
-  uint32_t excl;
-  if (__ballot_sync(FULL, c > 1) == 0) {
-    excl = __popc(__ballot_sync(FULL, c != 0) & lanemask_lt());
-  } else {
-    uint32_t incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += y;
-    }
-    excl = incl - c;
-  }
-  uint16_t *stage = reinterpret_cast<uint16_t *>(s_stage[wib]);
-  if (c) {
-    uint32_t pos = 1 + excl;
-#pragma unroll
-    for (int k = 0; k < UPL; k++) {
-      const uint32_t q = lane + k * L;
-      if (q < qn) {
-        const uint32_t w[4] = {acc[k].x, acc[k].y, acc[k].z, acc[k].w};
-#pragma unroll
-        for (int wi = 0; wi < 4; wi++) {
-          uint32_t bits = w[wi];
-          while (bits) {
-            stage[pos++] = (uint16_t)(q * 128 + wi * 32 + __ffs(bits) - 1);
-            bits &= bits - 1;
-          }
-        }
-      }
-    }
-  }
-  if (lane == 0) stage[0] = (uint16_t)total;
-  __syncwarp();
-  if ((uint32_t)lane < a.slot_n / 8) reinterpret_cast<uint4 *>(slot)[lane] = s_stage[wib][lane];
-  if (lane == 0) {
-    // up to two ids ride in the word, more stay in the slot
-    a.tiny_out[v] = tiny_word(total, total <= TINY_MAX ? stage[1] | (total > 1 ? (uint32_t)stage[2] << 15 : 0u) : 0u);
-    // short rows in the low half, rows of at most TINY_MAX bits in the high half
-    ns += 1ull + (total <= TINY_MAX ? 1ull << 32 : 0ull);
-  }
-  __syncwarp();  // the staging slot is free for the warp's next row
-  return true;
-}
-
-// Fused epilogue for the row of v held by lanes 0..L-1 after the group reduction:
-// visited AND-NOT + update, accumulator OR, next-layer write (and its slot),
-// flag, counters.
-// PRE: the visited words of the row (vpre, lanes 0..L-1) and the row's
-// next-layer flag (oldf_pre) were loaded ahead by the caller.
-// the union is read first: it is complete after a few rows and then costs no atomic
+// OR x into a union in global memory; it is read first: it is complete after a
+// few rows and then costs no atomic.
 __device__ __forceinline__ void add_union(uint4 *u, uint4 x) {
   const uint4 n = andnot4(x, __ldcg(u));
   unsigned *w = reinterpret_cast<unsigned *>(u);
@@ -974,99 +722,18 @@ __device__ __forceinline__ void add_union(uint4 *u, uint4 x) {
   if (n.w) atomicOr(w + 3, n.w);
 }
 
-template <int L, int UPL, int H, bool PRE = false>
-__device__ __forceinline__ void pull_epilogue(const PullArgs &a, const L2Pol<H> &pol, uint32_t v,
-                                              const uint32_t q0, const uint32_t qn, uint4 (&acc)[UPL],
-                                              unsigned long long &nb, unsigned long long &nv,
-                                              unsigned long long &ns, const uint4 *vpre = nullptr,
-                                              uint32_t oldf_pre = 0) {
-  const int lane = threadIdx.x & 31;
-  const bool leader_group = lane < L;
-  bool any = false;
-  uint32_t bits = 0;  // this lane's new bits of the row
-  if (leader_group) {
-#pragma unroll
-    for (int k = 0; k < UPL; k++) {
-      const uint32_t q = lane + k * L;
-      if (q < qn) {
-        const size_t idx = (size_t)v * a.Q + q0 + q;
-        uint4 x = acc[k];
-        if (a.hmask) {
-          const uint4 m = __ldg(a.hmask + q0 + q);
-          x = make_uint4(x.x & m.x, x.y & m.y, x.z & m.z, x.w & m.w);
-        }
-        if (a.shortest && nz4(x)) {
-          const uint4 vv = PRE ? vpre[k] : pol.ld_rw(a.vis + idx);
-          x = andnot4(x, vv);
-          if (nz4(x)) pol.st(a.vis + idx, or4(vv, x));
-        }
-        if (nz4(x)) {
-          any = true;
-          bits += popc4(x);
-          if (a.acc_on) a.acc[idx] = or4(a.acc[idx], x);
-        }
-        acc[k] = x;
-      }
-    }
-  }
-  nb += bits;
-  const bool rownz = __any_sync(FULL, any);
-  if (lane == 0 && rownz && (a.res_vis || a.acc_on)) a.resflag[v] = 1;
-  if (!a.multislice && a.last) {
-    // layer k_max is not kept: clear the rows an earlier layer left in this
-    // buffer, so the next run finds it clean (a flag-2 row is zero already)
-    const uint32_t oldf = PRE ? oldf_pre : a.flagN[v];
-    if (leader_group && oldf == 1) {
-#pragma unroll
-      for (int k = 0; k < UPL; k++) {
-        const uint32_t q = lane + k * L;
-        if (q < qn) pol.st(a.N + (size_t)v * a.Q + q0 + q, make_uint4(0, 0, 0, 0));
-      }
-    }
-    if (lane == 0) {
-      if (oldf) a.flagN[v] = 0;
-      if (rownz) nv++;
-    }
-  } else if (!a.multislice) {
-    const uint32_t oldf = PRE ? oldf_pre : a.flagN[v];  // 1: the buffer row holds an older layer's bits
-    bool virt = false;                 // the row is left in its slot only (flag 2)
-    if (a.tiny_out) {  // every vertex gets a tiny word: the count is 0 for an empty row
-      if (rownz)
-        virt = write_short<L, UPL>(a, v, acc, qn, bits, ns) && a.virt_out;
-      else if (lane == 0) {
-        a.tiny_out[v] = 0;
-        a.slot_out[(size_t)v * a.slot_n] = 0;
-      }
-    }
-    if (leader_group && ((rownz && !virt) || oldf == 1)) {
-#pragma unroll
-      for (int k = 0; k < UPL; k++) {
-        const uint32_t q = lane + k * L;
-        if (q < qn) pol.st(a.N + (size_t)v * a.Q + q0 + q, virt ? make_uint4(0, 0, 0, 0) : acc[k]);
-      }
-    }
-    if (lane == 0) {
-      const uint32_t nf = rownz ? (virt ? 2u : 1u) : 0u;
-      if (nf != oldf) a.flagN[v] = nf;
-      if (rownz) nv++;
-    }
-  } else if (rownz) {
-    if (leader_group) {
-#pragma unroll
-      for (int k = 0; k < UPL; k++) {
-        const uint32_t q = lane + k * L;
-        if (q < qn && nz4(acc[k])) a.N[(size_t)v * a.Q + q0 + q] = acc[k];
-      }
-    }
-    if (lane == 0 && atomicOr(&a.flagN[v], 1u) == 0) nv++;
-  }
-}
-
+// ro, so, po: out-degrees of the layer's non-empty rows, of its short rows, and per bit
 __device__ __forceinline__ void pull_counters(const PullArgs &a, unsigned long long nb, unsigned long long nv,
-                                              unsigned long long ns, unsigned long long se) {
+                                              unsigned long long ns, unsigned long long se, unsigned long long ro,
+                                              unsigned long long so, unsigned long long po) {
   block_add(nb, &a.ctr->hop[a.h].new_bits);
   block_add(nv, &a.ctr->hop[a.h].active_vertices);
-  if (a.tiny_out) block_add(ns, &a.ctr->hop[a.h].short_rows);
+  if (a.tiny_out) {
+    block_add(ns, &a.ctr->hop[a.h].short_rows);
+    block_add(ro, &a.ctr->hop[a.h].row_out);
+    block_add(so, &a.ctr->hop[a.h].short_out);
+    block_add(po, &a.ctr->hop[a.h].pair_edges);
+  }
   if (a.tiny_in) block_add(se, &a.ctr->hop[a.h].short_edges);
 }
 
@@ -1307,7 +974,9 @@ __device__ __forceinline__ bool write_short_group(const PullArgs &a, uint32_t v,
 template <int L, int UPL>
 __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bool valid, uint32_t q0, uint32_t qn,
                                                const uint4 *s_um, uint4 *s_un, const uint4 (&vv)[UPL], uint4 (&acc)[UPL],
-                                               unsigned long long &nb, unsigned long long &nv, unsigned long long &ns) {
+                                               unsigned long long &nb, unsigned long long &nv, unsigned long long &ns,
+                                               unsigned long long &ro, unsigned long long &so,
+                                               unsigned long long &po) {
   const uint32_t lane = threadIdx.x & 31, gl = lane & (L - 1);
   bool any = false;
   uint32_t bits = 0;
@@ -1371,7 +1040,16 @@ __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bo
     return;
   }
   bool virt = false;  // the row is left in its slot only (flag 2)
-  if (a.tiny_out) virt = write_short_group<L, UPL>(a, v, valid, rownz, acc, qn, bits, ns) && a.virt_out;
+  if (a.tiny_out) {
+    const bool fits = write_short_group<L, UPL>(a, v, valid, rownz, acc, qn, bits, ns);
+    virt = fits && a.virt_out;
+    if (valid && rownz && (bits || gl == 0)) {
+      const unsigned long long d = out_degree(a.out, v);
+      po += d * bits;
+      if (gl == 0) ro += d;
+      if (gl == 0 && fits) so += d;
+    }
+  }
   if (valid && ((rownz && !virt) || oldf == 1)) {
 #pragma unroll
     for (int k = 0; k < UPL; k++) {
@@ -1398,7 +1076,7 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
   const uint32_t q0 = blockIdx.y * a.qslice, qn = min(a.qslice, a.Q - q0);
   const HopCtr &pc = a.ctr->hop[a.h - 1];
   for (uint32_t q = threadIdx.x; q < qn; q += blockDim.x) {
-    uint4 m = pc.strategy == ST_PULL && !pc.short_pull ? a.Uin[q0 + q] : row_bits(q0 + q, a.S);
+    uint4 m = pc.strategy == ST_PULL ? a.Uin[q0 + q] : row_bits(q0 + q, a.S);
     if (a.hmask) m = and4(m, a.hmask[q0 + q]);
     s_um[q] = m;
     s_un[q] = make_uint4(0, 0, 0, 0);
@@ -1416,7 +1094,7 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
     for (int i = 0; i < a.h; i++) seen += a.ctr->hop[i].new_bits;
   const bool precheck = seen > (unsigned long long)a.V * a.S / 8;
   const uint32_t ntasks = a.npieces + (a.V + a.tile - 1) / a.tile;
-  unsigned long long nb = 0, nv = 0, ns = 0;
+  unsigned long long nb = 0, nv = 0, ns = 0, ro = 0, so = 0, po = 0;
   auto fetch = [&]() {
     uint32_t t = 0;
     if (lane == 0) t = atomicAdd(a.queue + blockIdx.y, 1u);
@@ -1492,7 +1170,7 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
           if (lane == 0) *cnt = np;
         }
       }
-      if (mine) group_epilogue<L, UPL>(a, v, g == 0, q0, qn, s_um, s_un, vv, acc, nb, nv, ns);
+      if (mine) group_epilogue<L, UPL>(a, v, g == 0, q0, qn, s_um, s_un, vv, acc, nb, nv, ns, ro, so, po);
     } else {
       // the tile's list starts at once: lane i holds those of target v0 + i (a tile of
       // L > 1 has at most 16 targets, so lane i + 1 holds the end too)
@@ -1524,251 +1202,625 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
         }
         _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n)
           gather_list<L, UPL>(a, F, flag, s_um, qn, a.in.adj[l] + beg[l], n[l], 0, L < 32 ? CH : 32, vv, acc, sat);
-        group_epilogue<L, UPL>(a, v, valid, q0, qn, s_um, s_un, vv, acc, nb, nv, ns);
+        group_epilogue<L, UPL>(a, v, valid, q0, qn, s_um, s_un, vv, acc, nb, nv, ns, ro, so, po);
       }
     }
     task = __shfl_sync(FULL, nexttask, 0);
   }
-  pull_counters(a, nb, nv, ns, 0);
+  pull_counters(a, nb, nv, ns, 0, ro, so, po);
   __syncthreads();
   if (!a.last)
     for (uint32_t q = threadIdx.x; q < qn; q += blockDim.x) add_union(a.Uout + q0 + q, s_un[q]);
 }
 
-// Short mode (one slice).  Software-pipelined over the warp's targets: while
-// target v is processed, the next target's list bounds, first 32
-// in-neighbours and their tiny words are already in flight.  PRE: so are the
-// next target's visited words (in registers of lanes 0..L-1) and its
-// next-layer flag, which the epilogue would otherwise wait for, and the list
-// bounds run one target further ahead, so the next target's in-neighbours
-// are requested when v starts.
-template <int L, int UPL, bool PRE = false>
-__device__ __forceinline__ void pull_vertices_short(const PullArgs &a) {
-  const L2Pol<0> pol;
-  __shared__ uint32_t s_u[8][32];
-  extern __shared__ uint4 s_short[];  // [8 warps][Q], the ids of short in-neighbour rows
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint32_t qn = a.Q;
-  uint4 *srow = s_short + (size_t)wib * a.Q;
-  uint32_t *row32 = reinterpret_cast<uint32_t *>(srow);
-  for (uint32_t q = lane; q < a.Q; q += 32) srow[q] = make_uint4(0, 0, 0, 0);
+// ---------------------------------------------------------------------------
+// Short-mode PULL (one slice).  A warp takes T consecutive targets and keeps
+// their rows as bitmaps in shared memory.  Their in-lists lie end to end in the
+// CSR and are read as one range, 32 edges at a time whatever the degrees, a lane
+// per edge, the loads of several such rounds in flight at once:
+//   words  most edges of such a layer come from empty rows, so the ids of the
+//          others are queued and OR-ed into the bitmaps 32 at a time, a full
+//          warp whatever target they belong to;
+//   slots  a lane per edge ORs its slot's ids.
+// In-neighbours with 16 ids or more are put aside: those with a slot are done by
+// all lanes, an id each, the others are rows gathered whole.
+//
+// Three ways to finish a tile:
+//   LIST  (word hops) the bitmaps start as the visited rows, so the atomic's old
+//         word tells a new id, which is appended to the target's list at once: the
+//         list is the slot of the next layer and no row is searched for bits.
+//         Long rows, and targets that got a whole row, are done from the bitmap.
+//   LAST  nothing follows the layer: the bitmaps start as the visited rows and
+//         are written back; popcounts before and after give the new bits.
+//   GEN   any other hop (accumulator, kept layer, long new rows): the bitmaps
+//         start empty and finish_row does every touched target.
+//
+// What bounds it: instructions and latency (about 170 warp instructions a target at
+// 28 edges, IPC 1.5 of 4 with 32 warps on the SM), not DRAM (15 to 25% of the copy
+// rate).  So no call in a kernel's loops (around one, 40 registers went to local
+// memory that L1 could not hold: 2.2 times slower), words and slots in kernels of
+// their own (together they spill), four targets a tile (eight halve what is left of
+// L1: 7.85 -> 12.2 ms on the 10M-vertex slot hop).  Against a warp per target with
+// its row in registers, 4,096 sources: 1M-vertex power law, the hop after SPARSE 545
+// (a dense hop; short mode did not pay) -> 345 us; backward lists, 2,048 sources 645 +
+// a CTA per hub 409 -> 755 us; 10M vertices, third hop 5.56 -> 5.01 ms, last hop 7.88
+// -> 7.85 ms.
+enum { SH_LIST = 0, SH_LAST = 1, SH_GEN = 2 };
+constexpr int SH_WARPS = 8;
+
+// Shared memory of a block, in uint4: the union of the rows it wrote [Q], the
+// rows that may still grow [Q] (with row limits), then per warp, from wb on:
+// bitmap rows [T][Q], lists of slot_n entries (entry 0: the count) [T] from
+// sh_list, counts of the lists and queue of ids from sh_queue, in-neighbours put
+// aside (id, target | count << 8) from sh_aside.
+extern __shared__ uint4 s_short[];
+
+// A slot's first 32 bytes (32-byte aligned) in one load that leaves L1 to the lists.
+__device__ __forceinline__ void ld_slot(const uint4 *p, uint4 &x, uint4 &y) {
+  asm("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w), "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w)
+      : "l"(p));
+}
+
+// A lane's id into a target's bitmap, the old word unused.
+__device__ __forceinline__ void or_id(uint32_t *row, uint32_t id) { atomicOr(row + (id >> 5), 1u << (id & 31)); }
+
+// Whether an id's row may still grow.
+__device__ __forceinline__ bool may_grow(const PullArgs &a, uint32_t id) {
+  return !a.hmask || (reinterpret_cast<const uint32_t *>(s_short + a.Q)[id >> 5] >> (id & 31) & 1u);
+}
+
+// Every lane with act ORs its id into target own's bitmap; LIST: new ids are
+// appended to the targets' lists.
+template <int MODE>
+__device__ __forceinline__ void put_ids(const PullArgs &a, uint32_t wb, bool act, uint32_t own, uint32_t id) {
+  act = act && may_grow(a, id);
+  const uint32_t w = id >> 5, bit = 1u << (id & 31);
+  uint32_t *row = reinterpret_cast<uint32_t *>(s_short + wb + own * a.Q);
+  if (MODE != SH_LIST) {
+    if (act) atomicOr(row + w, bit);
+    return;
+  }
+  const bool fresh = act && !(atomicOr(row + w, bit) & bit);
+  const unsigned m = __ballot_sync(FULL, fresh);
+  if (!m) return;
+  const unsigned peers = __match_any_sync(FULL, fresh ? own : 32u);
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(s_short + wb + a.sh_queue) + own;
+  if (fresh) {
+    const uint32_t base = *cnt, at = 1 + base + __popc(peers & lanemask_lt());
+    if (at < a.slot_n) reinterpret_cast<uint16_t *>(s_short + wb + a.sh_list)[own * a.slot_n + at] = (uint16_t)id;
+    uint32_t *un = reinterpret_cast<uint32_t *>(s_short) + w;
+    if (!(*un & bit)) atomicOr(un, bit);
+  }
   __syncwarp();
-  const bool slotmode = a.ctr->hop[a.h].short_slots;
-  const int64_t *off0 = a.in.off[0];
-  const uint32_t *adj0 = a.in.adj[0];
-  const uint32_t stride = gridDim.x * 8;
-  unsigned long long nb = 0, nv = 0, ns = 0, se = 0;
-  uint32_t v = blockIdx.x * 8 + wib;
-  int64_t beg = 0, end = 0;  // list 0 of target v
-  uint32_t pu = 0;           // this lane's in-neighbour in v's first chunk
-  Tiny pt = 0;               // ... and its tiny word (word mode)
-  uint4 ps[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};  // ... or its slot's first chunk (slot mode)
-  bool pact = false;
-  const uint32_t sq = a.slot_n / 8;  // uint4 per slot
-  uint4 vpre[UPL];       // PRE: visited words of v held by lanes 0..L-1
-  uint32_t oldf = 0;     // PRE: next-layer flag of v
+  if (fresh && (peers & lanemask_lt()) == 0) *cnt += __popc(peers);
+  __syncwarp();
+}
+
+// The n in-neighbours put aside, two at a time: rows with a slot an id per lane,
+// others whole.  Returns the targets that got a whole row.
+template <int MODE> __device__ __forceinline__ unsigned do_aside(const PullArgs &a, uint32_t wb, uint32_t naside) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint2 *aside = reinterpret_cast<const uint2 *>(s_short + wb + a.sh_aside);
+  const uint16_t *slots = reinterpret_cast<const uint16_t *>(a.slot_in);
+  unsigned whole = 0;
+  for (uint32_t k = 0; k < naside; k += 2) {
+    uint2 e[2];
+    uint32_t id[2];
 #pragma unroll
-  for (int k = 0; k < UPL; k++) vpre[k] = make_uint4(0, 0, 0, 0);
-  if (PRE && v < a.V) {
-    oldf = a.flagN[v];
-    if (a.shortest && lane < L)
-#pragma unroll
-      for (int k = 0; k < UPL; k++)
-        if (lane + k * L < qn) vpre[k] = pol.ld_rw(a.vis + (size_t)v * a.Q + lane + k * L);
-  }
-  int64_t b1 = 0, e1 = 0;  // PRE: list 0 of the next target, loaded one target ahead
-  if (PRE && (uint64_t)v + stride < a.V) {
-    b1 = __ldg(off0 + v + stride);
-    e1 = __ldg(off0 + v + stride + 1);
-  }
-  if (v < a.V) {
-    beg = __ldg(off0 + v);
-    end = __ldg(off0 + v + 1);
-    if (beg + lane < end) {
-      pu = __ldg(adj0 + beg + lane);
-      if (slotmode) {
-        ps[0] = __ldg(a.slot_in + (size_t)pu * sq);
-        ps[1] = __ldg(a.slot_in + (size_t)pu * sq + 1);
-      } else {
-        pt = ld_keep(a.tiny_in + pu);
-      }
-      pact = true;
+    for (int i = 0; i < 2; i++) {
+      e[i] = k + i < naside ? aside[k + i] : make_uint2(0, 0);
+      const uint32_t c = e[i].y >> 8;
+      id[i] = c < a.slot_n && lane < c ? __ldg(slots + (size_t)e[i].x * a.slot_n + 1 + lane) : 0u;
     }
-  }
-  for (; v < a.V; v += stride) {
-    const uint32_t vn = v + stride;
-    int64_t nbeg = 0, nend = 0, b2 = 0, e2 = 0;
-    if (PRE) {  // the next target's bounds arrived during v - stride; fetch those of vn + stride
-      nbeg = b1;
-      nend = e1;
-      const uint64_t v2 = (uint64_t)vn + stride;
-      if (v2 < a.V) {
-        b2 = __ldg(off0 + v2);
-        e2 = __ldg(off0 + v2 + 1);
+    if ((e[0].y >> 8) >= a.slot_n || (e[1].y >> 8) >= a.slot_n) {
+      for (uint32_t q = lane; q < a.Q; q += 32) {
+        uint4 x[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          x[i] = make_uint4(0, 0, 0, 0);
+          if ((e[i].y >> 8) >= a.slot_n) x[i] = __ldg(a.F + (size_t)e[i].x * a.Q + q);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+          if ((e[i].y >> 8) >= a.slot_n) {
+            uint4 *p = s_short + wb + (e[i].y & 255u) * a.Q + q;
+            if (a.hmask) x[i] = and4(x[i], s_short[a.Q + q]);
+            *p = or4(*p, x[i]);
+          }
       }
-    } else if (vn < a.V) {
-      nbeg = __ldg(off0 + vn);
-      nend = __ldg(off0 + vn + 1);
-    }
-    int64_t d = end - beg;
-    if (a.in.n > 1) d += a.in.off[1][v + 1] - a.in.off[1][v];
-    uint32_t pun = 0;
-    Tiny ptn = 0;
-    uint4 psn[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-    const bool pactn = nbeg + lane < nend;
-    if (PRE && pactn) pun = __ldg(adj0 + nbeg + lane);  // in flight during all of v
-    uint4 vpren[UPL];
-    uint32_t oldfn = 0;
-#pragma unroll
-    for (int k = 0; k < UPL; k++) vpren[k] = make_uint4(0, 0, 0, 0);
-    if (PRE && vn < a.V) {  // the next target's visited words and flag, in flight during v
-      oldfn = a.flagN[vn];
-      if (a.shortest && lane < L)
-#pragma unroll
-        for (int k = 0; k < UPL; k++)
-          if (lane + k * L < qn) vpren[k] = pol.ld_rw(a.vis + (size_t)vn * a.Q + lane + k * L);
-    }
-    if (!(a.hub_threshold && d > (int64_t)a.hub_threshold)) {  // hubs: k_pull_hub_short
-      if (lane == 0) {  // the epilogue's read-modify-write rows, fetched while the gather runs
-        if (a.shortest && !PRE) prefetch_l2(a.vis + (size_t)v * a.Q, qn * 16);
-        if (a.acc_on) prefetch_l2(a.acc + (size_t)v * a.Q, qn * 16);
-      }
-      uint4 acc[UPL];
-#pragma unroll
-      for (int k = 0; k < UPL; k++) acc[k] = make_uint4(0, 0, 0, 0);
-      gather_chunk<L, UPL, 0, true>(a, pol, s_u[wib], row32, 0, qn, acc, pu, pact, pt, slotmode, se, ps);
-      if (!PRE && pactn) pun = __ldg(adj0 + nbeg + lane);  // in flight during the rest of v
-      gather_rows<L, UPL, 0, true>(a, pol, s_u[wib], row32, 0, qn, acc, adj0, beg + 32, end, 0, 32, se, slotmode);
-      if (a.in.n > 1)
-        gather_rows<L, UPL, 0, true>(a, pol, s_u[wib], row32, 0, qn, acc, a.in.adj[1], a.in.off[1][v],
-                                     a.in.off[1][v + 1], 0, 32, se, slotmode);
-#pragma unroll
-      for (int o = L; o < 32; o <<= 1)
-#pragma unroll
-        for (int k = 0; k < UPL; k++) acc[k] = or4(acc[k], shfl_xor4(acc[k], o));
       __syncwarp();
-      if (lane < L) {
+    }
 #pragma unroll
-        for (int k = 0; k < UPL; k++) {
-          const uint32_t q = lane + k * L;
-          if (q < qn) {
-            acc[k] = or4(acc[k], srow[q]);
-            srow[q] = make_uint4(0, 0, 0, 0);
+    for (int i = 0; i < 2; i++) {
+      const uint32_t c = e[i].y >> 8, own = e[i].y & 255u;
+      if (c >= a.slot_n) {
+        whole |= 1u << own;
+      } else {
+        for (uint32_t i0 = 0; i0 < c; i0 += 32) {
+          const bool act = i0 + lane < c;
+          const uint32_t x = !i0 ? id[i] : act ? __ldg(slots + (size_t)e[i].x * a.slot_n + 1 + i0 + lane) : 0u;
+          put_ids<MODE>(a, wb, act, own, x);
+        }
+      }
+    }
+  }
+  return whole;
+}
+
+// A target from its bitmap row (raw unions, or unions and visited bits): new bits
+// = row & ~visited; visited, accumulator, union, next-layer row, word, slot,
+// flag.  The row is overwritten with the new bits; returns their number.
+__device__ __forceinline__ uint32_t finish_row(const PullArgs &a, uint32_t wb, uint32_t t, uint32_t v) {
+  uint4 *row = s_short + wb + t * a.Q, *s_un = s_short;
+  const uint4 *hm = a.hmask ? s_short + a.Q : nullptr;
+  uint16_t *list = reinterpret_cast<uint16_t *>(s_short + wb + a.sh_list) + t * a.slot_n;
+  const uint32_t lane = threadIdx.x & 31;
+  __syncwarp();
+  const uint32_t oldf = a.flagN[v];
+  uint32_t bits = 0;
+  for (uint32_t q = lane; q < a.Q; q += 32) {
+    const size_t idx = (size_t)v * a.Q + q;
+    uint4 x = row[q];
+    if (hm) x = and4(x, hm[q]);
+    if (nz4(x) && a.shortest) {
+      const uint4 vv = a.vis[idx];
+      x = andnot4(x, vv);
+      if (nz4(x)) a.vis[idx] = or4(vv, x);
+    }
+    if (nz4(x)) {
+      bits += popc4(x);
+      if (a.acc_on) {
+        const uint4 o = a.acc[idx];
+        if (nz4(andnot4(x, o))) a.acc[idx] = or4(o, x);
+      }
+      if (!a.last) {
+        const uint4 n = andnot4(x, s_un[q]);
+        unsigned *w = reinterpret_cast<unsigned *>(s_un + q);
+        if (n.x) atomicOr(w, n.x);
+        if (n.y) atomicOr(w + 1, n.y);
+        if (n.z) atomicOr(w + 2, n.z);
+        if (n.w) atomicOr(w + 3, n.w);
+      }
+    }
+    row[q] = x;
+  }
+  const uint32_t total = __reduce_add_sync(FULL, bits);
+  if (lane == 0 && total && (a.res_vis || a.acc_on)) a.resflag[v] = 1;
+  if (a.last) {  // layer k_max is not kept: leave the buffer row and its flag clean
+    if (oldf == 1)
+      for (uint32_t q = lane; q < a.Q; q += 32) a.N[(size_t)v * a.Q + q] = make_uint4(0, 0, 0, 0);
+    if (lane == 0 && oldf) a.flagN[v] = 0;
+    return total;
+  }
+  bool virt = false;
+  if (a.tiny_out) {
+    uint4 *slot = reinterpret_cast<uint4 *>(a.slot_out + (size_t)v * a.slot_n);
+    if (total && total < a.slot_n) {
+      uint32_t pos = 1;
+      for (uint32_t q0 = 0; q0 < a.Q; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        const uint4 x = q < a.Q ? row[q] : make_uint4(0, 0, 0, 0);
+        const uint32_t n = popc4(x);
+        uint32_t incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(FULL, incl, o);
+          if (lane >= (uint32_t)o) incl += y;
+        }
+        uint32_t at = pos + incl - n;
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int wi = 0; wi < 4; wi++)
+          for (uint32_t b = w[wi]; b; b &= b - 1) list[at++] = (uint16_t)(q * 128 + wi * 32 + __ffs(b) - 1);
+        pos += __shfl_sync(FULL, incl, 31);
+      }
+      if (lane == 0) list[0] = (uint16_t)total;
+      __syncwarp();
+      if (lane < a.slot_n / 8) slot[lane] = reinterpret_cast<const uint4 *>(list)[lane];
+      if (lane == 0)
+        a.tiny_out[v] = tiny_word(total, total <= TINY_MAX ? list[1] | (total > 1 ? (uint32_t)list[2] << 15 : 0u) : 0u);
+      virt = a.virt_out;
+      __syncwarp();
+    } else if (lane == 0) {
+      a.tiny_out[v] = tiny_word(total, 0);
+      a.slot_out[(size_t)v * a.slot_n] = (uint16_t)(total < 0xFFFFu ? total : 0xFFFFu);
+    }
+  }
+  if ((total && !virt) || oldf == 1)
+    for (uint32_t q = lane; q < a.Q; q += 32)
+      a.N[(size_t)v * a.Q + q] = virt ? make_uint4(0, 0, 0, 0) : row[q];
+  if (lane == 0) {
+    const uint32_t nf = total ? (virt ? 2u : 1u) : 0u;
+    if (nf != oldf) a.flagN[v] = nf;
+  }
+  return total;
+}
+
+// What a warp carries over the edges of its tile.
+struct ShortEdges {
+  uint32_t wb, nq, naside, se;  // shared memory; ids queued, in-neighbours put aside, edges served (this lane)
+  unsigned whole, touched;      // targets that got a whole row; any id
+};
+
+constexpr uint32_t SH_GROUP = 2;                    // word hops: 32-edge items per round
+constexpr uint32_t SH_IDS = 32 + SH_GROUP * 64;     // queued ids at most
+constexpr uint32_t SH_ASIDE = 32 + SH_GROUP * 32;   // in-neighbours put aside at most
+
+// Lanes with act queue an id for their target.
+__device__ __forceinline__ void queue_id(const PullArgs &a, ShortEdges &s, bool act, uint32_t own, uint32_t id) {
+  const unsigned m = __ballot_sync(FULL, act);
+  uint32_t *q = reinterpret_cast<uint32_t *>(s_short + s.wb + a.sh_queue) + 8;  // past the counts
+  if (act) q[s.nq + __popc(m & lanemask_lt())] = id | own << 16;
+  s.nq += __popc(m);
+}
+
+__device__ __forceinline__ void put_aside(const PullArgs &a, ShortEdges &s, bool act, uint32_t own, uint32_t u,
+                                          uint32_t n) {
+  const unsigned m = __ballot_sync(FULL, act);
+  if (!m) return;
+  if (act)
+    reinterpret_cast<uint2 *>(s_short + s.wb + a.sh_aside)[s.naside + __popc(m & lanemask_lt())] =
+        make_uint2(u, own | n << 8);
+  s.naside += __popc(m);
+}
+
+// OR the queued ids into the bitmaps, 32 at a time; all: the last ones too.
+template <int MODE> __device__ __forceinline__ void drain(const PullArgs &a, ShortEdges &s, bool all) {
+  const uint32_t lane = threadIdx.x & 31;
+  if (s.nq >= 32 || (all && s.nq)) {
+    uint32_t *q = reinterpret_cast<uint32_t *>(s_short + s.wb + a.sh_queue) + 8;
+    __syncwarp();
+    uint32_t at = 0;
+    for (; at + 32 <= s.nq || (all && at < s.nq); at += 32) {
+      const bool act = at + lane < s.nq;
+      const uint32_t e = act ? q[at + lane] : 0u;
+      put_ids<MODE>(a, s.wb, act, e >> 16, e & 0x7FFFu);
+    }
+    const uint32_t left = at < s.nq ? s.nq - at : 0u, e = lane < left ? q[at + lane] : 0u;
+    __syncwarp();
+    if (lane < left) q[lane] = e;
+    s.nq = left;
+  }
+  if (s.naside >= 32 || (all && s.naside)) {
+    __syncwarp();
+    s.whole |= do_aside<MODE>(a, s.wb, s.naside);
+    s.naside = 0;
+    __syncwarp();
+  }
+}
+
+// 32 edges of a word hop: u the neighbour (NONE: no edge), t its word, own the target.
+template <int MODE>
+__device__ __forceinline__ void word_edges(const PullArgs &a, ShortEdges &s, uint32_t own, uint32_t u, Tiny t) {
+  if (!__any_sync(FULL, t)) return;
+  const uint32_t cls = t >> 30;
+  if (MODE == SH_GEN) s.touched |= __reduce_or_sync(FULL, t ? 1u << own : 0u);
+  queue_id(a, s, cls == 1 || cls == 2, own, t & 0x7FFFu);
+  uint32_t n = cls;
+  if (__any_sync(FULL, cls > 1)) {
+    queue_id(a, s, cls == 2, own, t >> 15 & 0x7FFFu);
+    if (cls == 3) n = t & 0xFFFFu;
+    put_aside(a, s, cls == 3, own, u, n);  // 3 to 15 ids: an id per lane too
+  }
+  s.se += n && n < a.slot_n;
+}
+
+// 32 edges of a slot hop: u the neighbour, its slot's first 32 bytes.
+template <int MODE>
+__device__ __forceinline__ void slot_edges(const PullArgs &a, ShortEdges &s, uint32_t own, uint32_t u,
+                                           const uint4 first, const uint4 second) {
+  uint32_t n = first.x & 0xFFFFu;
+  if (!__any_sync(FULL, n)) return;
+  if (MODE == SH_GEN) s.touched |= __reduce_or_sync(FULL, n ? 1u << own : 0u);
+  s.se += n && n < a.slot_n;
+  const bool far = n >= CHUNK_IDS || n >= a.slot_n;
+  put_aside(a, s, far, own, u, n);
+  if (far) n = 0;
+  const uint32_t mx = __reduce_max_sync(FULL, n);
+  uint32_t *row = reinterpret_cast<uint32_t *>(s_short + s.wb + own * a.Q);
+  const uint32_t w[8] = {first.x, first.y, first.z, first.w, second.x, second.y, second.z, second.w};
+#pragma unroll
+  for (uint32_t i = 1; i < CHUNK_IDS; i++) {
+    if (i > mx) break;
+    const uint32_t id = i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu;
+    if (i <= n && may_grow(a, id)) or_id(row, id);
+  }
+}
+
+// The in-lists of the tile's targets, end to end (lane t: length deg of target t,
+// which starts at entry `at` of adj; consecutive lists are consecutive there, a
+// gap is a target that comes in pieces).  Rounds of G x 32 edges with their loads
+// in flight at once; the warps of the SM cover the waits.
+template <int MODE, bool SLOTS, int T>
+__device__ __forceinline__ void short_edges(const PullArgs &a, ShortEdges &s, const uint32_t *__restrict__ adj,
+                                            int64_t at, uint32_t deg, bool gaps) {
+  constexpr int G = SLOTS ? 2 : SH_GROUP;
+  const uint32_t lane = threadIdx.x & 31, sq = a.slot_n / 8;
+  // lane t: first edge of target t in the tile; lanes from T on: the number of edges
+  uint32_t pre = deg;
+#pragma unroll
+  for (int o = 1; o < T; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, pre, o);
+    if (lane >= o) pre += y;
+  }
+  const uint32_t total = __shfl_sync(FULL, pre, T - 1);
+  pre = lane < T ? pre - deg : total;
+  if (gaps) at -= pre;  // where target t's edges are, less their number in the tile
+  else at = __shfl_sync(FULL, at, 0);
+  for (uint32_t c = 0; c < total; c += 32 * G) {
+    uint32_t u[G], own[G];
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      const uint32_t e = c + k * 32 + lane;
+      own[k] = 0;
+#pragma unroll
+      for (int step = T >> 1; step; step >>= 1)
+        if (__shfl_sync(FULL, pre, own[k] + step) <= e) own[k] += step;
+      const int64_t d = gaps ? __shfl_sync(FULL, at, own[k]) : at;
+      u[k] = e < total ? __ldg(adj + d + e) : NONE;
+    }
+    if constexpr (!SLOTS) {
+      Tiny w[G];
+#pragma unroll
+      for (int k = 0; k < G; k++) w[k] = u[k] != NONE ? ld_keep(a.tiny_in + u[k]) : 0u;
+#pragma unroll
+      for (int k = 0; k < G; k++) word_edges<MODE>(a, s, own[k], u[k], w[k]);
+    } else {
+      uint4 x[G], y[G];
+#pragma unroll
+      for (int k = 0; k < G; k++) {
+        x[k] = y[k] = make_uint4(0, 0, 0, 0);
+        if (u[k] != NONE) ld_slot(a.slot_in + (size_t)u[k] * sq, x[k], y[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < G; k++) slot_edges<MODE>(a, s, own[k], u[k], x[k], y[k]);
+    }
+    drain<MODE>(a, s, c + 32 * G >= total);
+  }
+}
+
+template <int MODE, bool SLOTS, int T>
+__device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
+  const uint32_t lane = threadIdx.x & 31, Q = a.Q;
+  uint4 *bm = s_short + wb;
+  uint16_t *list = reinterpret_cast<uint16_t *>(bm + a.sh_list);
+  uint8_t *before = reinterpret_cast<uint8_t *>(list);  // LAST: the cells' popcounts (at most 128)
+  uint32_t *counts = reinterpret_cast<uint32_t *>(bm + a.sh_queue);
+  const uint32_t ntasks = a.npieces + (a.V + T - 1) / T;
+  // per thread: a warp's share of the rows, bits and edges stays far below 2^32
+  unsigned long long po = 0;
+  uint32_t nb = 0, nv = 0, nshort = 0, ntiny = 0, ro = 0, so = 0;
+  ShortEdges s{wb, 0, 0, 0, 0, 0};
+  auto fetch_task = [&]() { return lane == 0 ? atomicAdd(a.queue, 1u) : 0u; };
+  uint32_t task = __shfl_sync(FULL, fetch_task(), 0);
+  while (task < ntasks) {
+    const uint32_t nexttask = fetch_task();  // in flight during this task
+    s.whole = s.touched = 0;
+    uint32_t v0;
+    unsigned fm = 0;  // targets from v0 on to be done from their bitmaps
+    if (task < a.npieces) {  // part of one long list
+      const uint4 pc = __ldg(a.pieces + task);
+      const uint32_t np = pc.y == NONE ? 1u : a.heavy_np[pc.y];
+      for (uint32_t q = lane; q < Q; q += 32) bm[q] = make_uint4(0, 0, 0, 0);
+      __syncwarp();
+      const int64_t beg = a.in.off[pc.z][pc.x] + pc.w, end = a.in.off[pc.z][pc.x + 1];
+      const uint32_t n = (uint32_t)min((int64_t)a.piece_edges, end - beg);
+      short_edges<SH_GEN, SLOTS, 1>(a, s, a.in.adj[pc.z], beg, lane ? 0u : n, false);
+      bool mine = true;
+      if (np > 1) {
+        uint4 *sum = a.heavy_rows + (size_t)pc.y * Q;
+        for (uint32_t q = lane; q < Q; q += 32) add_union(sum + q, bm[q]);
+        __threadfence();
+        __syncwarp();
+        uint32_t left = lane == 0 ? atomicSub(a.heavy_left + pc.y, 1u) : 0u;
+        left = __shfl_sync(FULL, left, 0);
+        mine = left == 1;
+        if (mine) {  // the last piece: the whole union, and both left as they were found
+          __threadfence();
+          for (uint32_t q = lane; q < Q; q += 32) {
+            bm[q] = __ldcg(sum + q);
+            sum[q] = make_uint4(0, 0, 0, 0);
+          }
+          if (lane == 0) a.heavy_left[pc.y] = np;
+        }
+      }
+      v0 = pc.x;
+      fm = mine;
+    } else {
+      v0 = (task - a.npieces) * T;
+      const uint32_t v = v0 + lane;
+      bool valid = lane < T && v < a.V, gaps = false;
+      int64_t beg = 0;
+      uint32_t deg = 0, rf = 0;
+      if (valid) {
+        beg = __ldg(a.in.off[0] + v);
+        deg = (uint32_t)(__ldg(a.in.off[0] + v + 1) - beg);
+        if (MODE != SH_GEN && a.shortest) rf = a.res_vis ? a.resflag[v] : 1u;
+      }
+      if (a.heavy_threshold) {
+        uint64_t d = deg;
+        if (valid && a.in.n > 1) d += (uint64_t)(__ldg(a.in.off[1] + v + 1) - __ldg(a.in.off[1] + v));
+        const bool heavy = d > a.heavy_threshold;  // comes in pieces
+        gaps = __any_sync(FULL, heavy);
+        if (heavy) {
+          valid = false;
+          deg = rf = 0;
+        }
+      }
+      if (MODE == SH_LIST && lane < T) counts[lane] = 0;
+      {  // the bitmaps; resflag 0: the visited row is zero, without reading it
+        const unsigned known = __ballot_sync(FULL, rf != 0);
+        for (uint32_t q = lane; q < Q; q += 32) {
+#pragma unroll
+          for (int t0 = 0; t0 < T; t0 += T < 4 ? T : 4) {
+            constexpr int B = T < 4 ? T : 4;  // rows with their loads in flight at once
+            uint4 x[B];
+#pragma unroll
+            for (int t = 0; t < B; t++) {
+              x[t] = make_uint4(0, 0, 0, 0);
+              if (MODE != SH_GEN && (known >> (t0 + t) & 1u)) x[t] = a.vis[(size_t)(v0 + t0 + t) * Q + q];
+            }
+#pragma unroll
+            for (int t = 0; t < B; t++) {
+              bm[(t0 + t) * Q + q] = x[t];
+              if (MODE == SH_LAST) before[(t0 + t) * Q + q] = (uint8_t)popc4(x[t]);
+            }
           }
         }
       }
       __syncwarp();
-      if (pactn) {  // in flight during the epilogue
-        if (slotmode) {
-          psn[0] = __ldg(a.slot_in + (size_t)pun * sq);
-          psn[1] = __ldg(a.slot_in + (size_t)pun * sq + 1);
-        } else {
-          ptn = ld_keep(a.tiny_in + pun);
+#pragma unroll 1
+      for (int l = 0; l < a.in.n; l++) {
+        if (l) {
+          if (lane < T && v < a.V) beg = __ldg(a.in.off[1] + v);
+          if (valid) deg = (uint32_t)(__ldg(a.in.off[1] + v + 1) - beg);
         }
+        short_edges<MODE, SLOTS, T>(a, s, l ? a.in.adj[1] : a.in.adj[0], beg, deg, gaps);
       }
-      pull_epilogue<L, UPL, 0, PRE>(a, pol, v, 0, qn, acc, nb, nv, ns, vpre, oldf);
-    } else if (pactn) {
-      if (!PRE) pun = __ldg(adj0 + nbeg + lane);
-      if (slotmode) {
-        psn[0] = __ldg(a.slot_in + (size_t)pun * sq);
-        psn[1] = __ldg(a.slot_in + (size_t)pun * sq + 1);
+      __syncwarp();
+      const uint32_t oldf = valid ? a.flagN[v] : 0u;  // 1: the buffer row holds an older layer's bits
+      bool clean = valid && oldf == 1;                // ... and nothing will be written there
+      if (MODE == SH_LAST) {
+        const unsigned vm = __ballot_sync(FULL, valid);
+        bool grew = false;
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+          if (!(vm >> t & 1u)) continue;
+          bool any = false;
+          for (uint32_t q0 = 0; q0 < Q; q0 += 32) {
+            const uint32_t q = q0 + lane;
+            uint4 x = make_uint4(0, 0, 0, 0);
+            uint32_t more = 0;
+            if (q < Q) {
+              x = bm[t * Q + q];
+              more = popc4(x) - before[t * Q + q];
+            }
+            nb += more;
+            if (!__any_sync(FULL, more)) continue;
+            if (q < Q) a.vis[(size_t)(v0 + t) * Q + q] = x;
+            any = true;
+          }
+          if (lane == t) grew = any;
+        }
+        if (valid) {
+          nv += grew;
+          if (grew && a.res_vis) a.resflag[v] = 1;
+          if (oldf) a.flagN[v] = 0;
+        }
       } else {
-        ptn = ld_keep(a.tiny_in + pun);
-      }
-    }
-    beg = nbeg;
-    end = nend;
-    pu = pun;
-    pt = ptn;
-    ps[0] = psn[0];
-    ps[1] = psn[1];
-    pact = pactn;
-    b1 = b2;
-    e1 = e2;
-    oldf = oldfn;
+        const uint32_t cnt = MODE == SH_LIST && lane < T ? counts[lane] : 0u;
+        const bool from_row =
+            valid && ((s.whole >> lane & 1u) || (MODE == SH_GEN ? (s.touched >> lane & 1u) : cnt >= a.slot_n));
+        const bool listed = valid && !from_row;
+        clean = clean && listed;
+        fm = __ballot_sync(FULL, from_row);
+        if (listed) {
+          Tiny word = 0;
+          if (MODE == SH_LIST && cnt) {
+            uint16_t *li = list + lane * a.slot_n;
+            li[0] = (uint16_t)cnt;
+            word = tiny_word(cnt, cnt <= TINY_MAX ? li[1] | (cnt > 1 ? (uint32_t)li[2] << 15 : 0u) : 0u);
+            if (a.res_vis) a.resflag[v] = 1;
+            const uint32_t d = (uint32_t)out_degree(a.out, v);
+            nb += cnt;
+            nv++;
+            nshort++;
+            ntiny += cnt <= TINY_MAX;
+            ro += d;
+            so += d;
+            po += d * cnt;
+          }
+          if (a.tiny_out) {
+            a.tiny_out[v] = word;
+            if (!cnt) a.slot_out[(size_t)v * a.slot_n] = 0;
+          }
+          const uint32_t nf = cnt ? 2u : 0u;
+          if (nf != oldf) a.flagN[v] = nf;
+        }
+        if (MODE == SH_LIST) {
+          const unsigned nm = __ballot_sync(FULL, listed && cnt);
+          __syncwarp();
+          const uint32_t sq = a.slot_n / 8, sh = 31 - __clz(sq);
+          for (uint32_t i = lane; i < T * sq; i += 32)
+            if (nm >> (i >> sh) & 1u)
+              reinterpret_cast<uint4 *>(a.slot_out)[(size_t)v0 * sq + i] = reinterpret_cast<const uint4 *>(list)[i];
+          if (a.shortest) {
 #pragma unroll
-    for (int k = 0; k < UPL; k++) vpre[k] = vpren[k];
-  }
-  pull_counters(a, nb, nv, ns, se);
-}
-
-// the same in short mode (its own kernel: the slot path's registers stay out
-// of the dense kernels' budget)
-template <int L, int UPL>
-__global__ void __launch_bounds__(256, UPL >= 4 ? 2 : 5) k_pull_short(PullArgs a) {
-  if (a.ctr->hop[a.h].strategy != ST_PULL || !a.ctr->hop[a.h].short_pull || !a.tiny_in || a.pre) return;
-  pull_vertices_short<L, UPL>(a);
-}
-
-// ... with the visited words and flag of the next target loaded ahead
-template <int L, int UPL>
-__global__ void __launch_bounds__(256, UPL >= 4 ? 2 : UPL == 2 ? 3 : 4) k_pull_short_pre(PullArgs a) {
-  if (a.ctr->hop[a.h].strategy != ST_PULL || !a.ctr->hop[a.h].short_pull || !a.tiny_in || !a.pre) return;
-  pull_vertices_short<L, UPL, true>(a);
-}
-
-// Hub vertices (in-degree above the threshold): one 512-thread CTA per vertex,
-// warps stride over the in-list, rows reduced through shared memory (short
-// rows through one shared row of the CTA).
-template <int L, int UPL, bool SHORT>
-__device__ __forceinline__ void pull_hubs(const PullArgs &a) {
-  extern __shared__ uint4 s_red[];  // [16 warps][32 lanes][UPL], then SHORT: one row of Q
-  const L2Pol<0> pol;
-  __shared__ uint32_t s_u[16][32];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t q0 = blockIdx.y * a.qslice;
-  const uint32_t qn = min(a.qslice, a.Q - q0);
-  uint4 *srow = s_red + 16 * 32 * UPL;
-  if (SHORT) {
-    for (uint32_t q = threadIdx.x; q < a.Q; q += blockDim.x) srow[q] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-  }
-  unsigned long long nb = 0, nv = 0, ns = 0, se = 0;
-  for (uint32_t hi = blockIdx.x; hi < a.nhubs; hi += gridDim.x) {
-    const uint32_t v = a.hubs[hi];
-    uint4 acc[UPL];
-#pragma unroll
-    for (int k = 0; k < UPL; k++) acc[k] = make_uint4(0, 0, 0, 0);
-    _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n)
-      gather_rows<L, UPL, 0, SHORT>(a, pol, s_u[wib], reinterpret_cast<uint32_t *>(srow), q0, qn, acc,
-                                    a.in.adj[l], a.in.off[l][v], a.in.off[l][v + 1], (int64_t)wib * 32,
-                                    (int64_t)nw * 32, se, SHORT && a.ctr->hop[a.h].short_slots);
-#pragma unroll
-    for (int o = L; o < 32; o <<= 1)
-#pragma unroll
-      for (int k = 0; k < UPL; k++) acc[k] = or4(acc[k], shfl_xor4(acc[k], o));
-    if (lane < L)
-#pragma unroll
-      for (int k = 0; k < UPL; k++) s_red[(wib * 32 + lane) * UPL + k] = acc[k];
-    __syncthreads();
-    if (wib == 0) {
-      if (lane < L) {
-        for (int w = 1; w < nw; w++)
-#pragma unroll
-          for (int k = 0; k < UPL; k++) acc[k] = or4(acc[k], s_red[(w * 32 + lane) * UPL + k]);
-        if (SHORT) {
-#pragma unroll
-          for (int k = 0; k < UPL; k++) {
-            const uint32_t q = lane + k * L;
-            if (q < qn) acc[k] = or4(acc[k], srow[q]);
+            for (int t = 0; t < T; t++)
+              if (nm >> t & 1u)
+                for (uint32_t q = lane; q < Q; q += 32) a.vis[(size_t)(v0 + t) * Q + q] = bm[t * Q + q];
           }
         }
       }
-      pull_epilogue<L, UPL, 0>(a, pol, v, q0, qn, acc, nb, nv, ns);
+      unsigned z = __ballot_sync(FULL, clean);
+      while (z) {
+        const uint32_t t = __ffs(z) - 1;
+        z &= z - 1;
+        for (uint32_t q = lane; q < Q; q += 32) a.N[(size_t)(v0 + t) * Q + q] = make_uint4(0, 0, 0, 0);
+      }
     }
-    __syncthreads();
-    if (SHORT) {
-      for (uint32_t q = threadIdx.x; q < a.Q; q += blockDim.x) srow[q] = make_uint4(0, 0, 0, 0);
-      __syncthreads();
+    while (fm) {
+      const uint32_t t = __ffs(fm) - 1;
+      fm &= fm - 1;
+      const uint32_t c = finish_row(a, wb, t, v0 + t);
+      if (lane == 0 && c) {
+        nb += c;
+        nv++;
+        if (a.tiny_out) {
+          const uint32_t d = (uint32_t)out_degree(a.out, v0 + t);
+          ro += d;
+          po += (unsigned long long)d * c;
+          if (c < a.slot_n) {
+            nshort++;
+            ntiny += c <= TINY_MAX;
+            so += d;
+          }
+        }
+      }
     }
+    __syncwarp();
+    task = __shfl_sync(FULL, nexttask, 0);
   }
-  pull_counters(a, nb, nv, ns, se);
+  pull_counters(a, nb, nv, nshort + ((unsigned long long)ntiny << 32), s.se, ro, so, po);
 }
 
-template <int L, int UPL>
-__global__ void __launch_bounds__(512) k_pull_hub_short(PullArgs a) {
-  if (a.ctr->hop[a.h].strategy != ST_PULL || !a.ctr->hop[a.h].short_pull || !a.tiny_in || a.nhubs == 0) return;
-  pull_hubs<L, UPL, true>(a);
+// Layout of a warp's shared memory (uint4), and bytes of a block's.
+inline void short_layout(PullArgs &a, uint32_t T) {
+  a.sh_list = T * a.Q;
+  a.sh_queue = a.sh_list + std::max(T * a.slot_n / 8, (T * a.Q + 15) / 16);  // lists, or a byte per cell
+  a.sh_aside = a.sh_queue + (8 + SH_IDS) / 4;
+  a.sh_warp = a.sh_aside + SH_ASIDE / 2;
+}
+// Targets per tile: rows up to 512 bytes eight, wider ones two.
+inline uint32_t short_tile(uint32_t Q) { return Q <= 64 ? 4 : 2; }
+inline size_t short_smem(uint32_t Q, uint32_t slot_n) {
+  PullArgs a;
+  a.Q = Q;
+  a.slot_n = slot_n;
+  short_layout(a, short_tile(Q));
+  return 16 * (2 * (size_t)Q + SH_WARPS * (size_t)a.sh_warp);
+}
+
+// The mode is the host's choice (short_kernel) except that a hop whose new rows
+// will mostly be long finishes LIST as GEN; whether it reads words or slots is the
+// device's: of the two kernels of a hop one returns at once (one kernel for both
+// would need the registers of both).
+template <int MODE, bool SLOTS, int T>
+__global__ void __launch_bounds__(SH_WARPS * 32, 4) k_pull_short(const __grid_constant__ PullArgs a) {
+  const HopCtr &hc = a.ctr->hop[a.h];
+  if (hc.strategy != ST_PULL || !hc.short_pull || !a.tiny_in || (hc.short_slots != 0) != SLOTS ||
+      (MODE == SH_LIST && hc.short_long) || (MODE == SH_GEN && a.list_too && !hc.short_long))
+    return;
+  for (uint32_t q = threadIdx.x; q < a.Q; q += blockDim.x) {
+    s_short[q] = make_uint4(0, 0, 0, 0);
+    if (a.hmask) s_short[a.Q + q] = a.hmask[q];
+  }
+  __syncthreads();
+  pull_short_run<MODE, SLOTS, T>(a, 2 * a.Q + (threadIdx.x >> 5) * a.sh_warp);
+  __syncthreads();
+  if (!a.last)
+    for (uint32_t q = threadIdx.x; q < a.Q; q += blockDim.x) add_union(a.Uout + q, s_short[q]);
 }
 
 // Rows of layer h-1 left in their slots (flag 2), written out whole when hop
@@ -2193,12 +2245,24 @@ Lists push_lists(const vs_graph *g, int dir) {
 
 using PullFn = void (*)(PullArgs);
 
+// Short-mode kernels of a tile size: words and slots by mode (a slot hop has no LIST).
+struct ShortVariant {
+  uint32_t T;
+  PullFn words[3], slots[3];
+};
+#define VS_SHORT(T) \
+  {T, {k_pull_short<SH_LIST, false, T>, k_pull_short<SH_LAST, false, T>, k_pull_short<SH_GEN, false, T>}, \
+   {nullptr, k_pull_short<SH_LAST, true, T>, k_pull_short<SH_GEN, true, T>}}
+const ShortVariant kShort[2] = {VS_SHORT(4), VS_SHORT(2)};
+#undef VS_SHORT
+const ShortVariant &pick_short(uint32_t Q) { return kShort[short_tile(Q) == 4 ? 0 : 1]; }
+
 struct PullVariant {
   int L, UPL;
-  PullFn pull, pull_short, hub_short, pull_short_pre;
+  PullFn pull;
 };
 
-#define VS_VARIANT(L, U) {L, U, k_pull<L, U>, k_pull_short<L, U>, k_pull_hub_short<L, U>, k_pull_short_pre<L, U>}
+#define VS_VARIANT(L, U) {L, U, k_pull<L, U>}
 const PullVariant kVariants[] = {
     VS_VARIANT(1, 1),  VS_VARIANT(2, 1),  VS_VARIANT(4, 1),  VS_VARIANT(8, 1), VS_VARIANT(16, 1),
     VS_VARIANT(32, 1), VS_VARIANT(32, 2), VS_VARIANT(32, 4), VS_VARIANT(32, 8),
@@ -2232,9 +2296,7 @@ struct vs_expand_plan {
   uint32_t *d_src = nullptr, *d_tgt = nullptr;
   int32_t *d_dist = nullptr;
   Ctr *ctr = nullptr;
-  uint32_t *hubs = nullptr;
-  uint32_t nhubs = 0, hub_threshold = 0;
-  // dense PULL: targets above heavy_threshold are cut into pieces
+  // PULL: targets above heavy_threshold are cut into pieces
   uint32_t heavy_threshold = 0, nheavy = 0, npieces = 0, tile = 32;
   uint4 *pieces = nullptr, *heavy_rows = nullptr;
   uint32_t *heavy_np = nullptr, *heavy_left = nullptr;
@@ -2243,14 +2305,13 @@ struct vs_expand_plan {
   size_t ctr_bytes = 0;        // ctr, un and queue are one allocation, zeroed at every run start
   bool use_vis = false, use_acc = false, clear_diag = false;
   bool collect_stats = false;
-  int grid_pull = 0, grid_hub = 0, grid_sparse = 0, grid_v = 0, grid_push = 0, grid_short = 0, grid_short_pre = 0;
+  int grid_pull = 0, grid_sparse = 0, grid_v = 0, grid_push = 0, grid_short = 0;
   vs_bitmat result{};
   bool has_result = false;
   // tuning knobs of the fixed planner
   double sparse_frac = 0.02, push_frac = 0.0;
   const void *picker = nullptr;
   bool log_features = false;
-  int pull_kind = 0;  // PULL kernel variant (bit 0: 8 blocks/SM bound, bit 1: L2 policies)
   uint64_t *hmask = nullptr;  // (k_max + 1) x W words: rows allowed to grow at hop h
   uint32_t *rowk = nullptr;   // [0] largest row limit, [1] a limit exceeded k_max (device-set limits)
   uint64_t *layer_out[VS_MAX_HOPS + 1] = {};  // with_distance: layer h is copied here (zeroed, V x W words)
@@ -2287,11 +2348,12 @@ inline bool needs_acc(const vs_expand_params &p) {
 // the row's bytes at 64 and 128 words, 128 bytes beyond.
 inline uint32_t slot_entries(uint32_t W) { return W <= 64 ? 16 : W <= 128 ? 32 : 64; }
 
-// Short-row words and slots (15-bit ids: S <= 32768) need rows in one slice, and short
-// mode runs only on frontiers larger than half of L2 (unless forced: share >
-// 1): a graph whose whole V x W matrix fits there never uses them.
+// Short-row words and slots (15-bit ids: S <= 32768) need rows in one slice.
+// Short mode is not worth them on a graph whose whole V x W matrix fits in half
+// of L2, nor for rows below 32 words: a dense hop of 16-word rows took 0.25 ms on
+// the 1M-vertex power law where a short one took 0.38 (unless forced: share > 1).
 inline bool short_slots_ok(uint32_t S, uint32_t nslices, double share, uint64_t V, uint32_t W) {
-  return share >= 0 && S <= 32768 && nslices == 1 && (share > 1.0 || V * 8ull * W > l2_bytes() / 2);
+  return share >= 0 && S <= 32768 && nslices == 1 && (share > 1.0 || (W >= 32 && V * 8ull * W > l2_bytes() / 2));
 }
 
 int plan_free(vs_expand_plan *pl) {
@@ -2300,7 +2362,7 @@ int plan_free(vs_expand_plan *pl) {
   void *ptrs[] = {pl->tiny[0], pl->tiny[1], pl->slot[0], pl->slot[1], pl->resflag, pl->pdeg[0], pl->pdeg[1], pl->doff,
                   pl->bsum, pl->hmask, pl->rowk, pl->buf[0], pl->buf[1], pl->flag[0], pl->flag[1], pl->vis, pl->acc,
                   pl->pairs[0], pl->pairs[1], pl->push_list, pl->touched, pl->d_src,
-                  pl->d_tgt, pl->d_dist, pl->ctr, pl->hubs, pl->pieces, pl->heavy_rows, pl->heavy_np, pl->heavy_left};
+                  pl->d_tgt, pl->d_dist, pl->ctr, pl->pieces, pl->heavy_rows, pl->heavy_np, pl->heavy_left};
   for (void *p : ptrs)  // stream-ordered after the plan's last run
     if (p) dfree(p, st);
   for (cudaEvent_t e : pl->ev)
@@ -2526,31 +2588,27 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     plan_free(pl);
     return cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
   }
-  // heavy targets of the pull direction set: a list for short mode, pieces for the dense PULL
+  // heavy targets of the pull direction set and their pieces
   const PullVariant &var = pick_variant(pl->qslice);
-  pl->hub_threshold = p->hub_threshold ? p->hub_threshold : 2048;
-  pl->heavy_threshold = p->hub_threshold ? p->hub_threshold : heavy_default(var.L);
+  pl->heavy_threshold = p->hub_threshold ? std::min(p->hub_threshold, 1u << 16) : heavy_default(var.L);
   {
     Lists in = pull_lists(g, p->direction);
     unsigned *dn = nullptr;
     uint32_t *heavy = nullptr;
-    if ((rc = dalloc_n(&pl->hubs, V, st)) != VS_OK || (rc = dalloc_n(&heavy, V, st)) != VS_OK ||
-        (rc = dalloc_n(&dn, 8, st)) != VS_OK) {
+    if ((rc = dalloc_n(&heavy, V, st)) != VS_OK || (rc = dalloc_n(&dn, 8, st)) != VS_OK) {
       dfree(heavy, st);
       plan_free(pl);
       return rc;
     }
     cudaMemsetAsync(dn, 0, 8 * sizeof(unsigned), st);
     const uint32_t pe = piece_edges(var.L);
-    { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->hub_threshold, pe, pl->hubs, dn); vs::note_launch(); }
-    { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->heavy_threshold, pe, heavy, dn + 3); vs::note_launch(); }
-    unsigned hn[6] = {0, 0, 0, 0, 0, 0};
+    { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->heavy_threshold, pe, heavy, dn); vs::note_launch(); }
+    unsigned hn[3] = {0, 0, 0};
     cudaMemcpyAsync(hn, dn, sizeof(hn), cudaMemcpyDeviceToHost, st);
     e = cudaStreamSynchronize(st);
-    pl->nhubs = hn[0];
-    pl->nheavy = hn[3];
-    pl->npieces = hn[4];
-    const size_t nmulti = hn[5];
+    pl->nheavy = hn[0];
+    pl->npieces = hn[1];
+    const size_t nmulti = hn[2];
     if (e == cudaSuccess && pl->nheavy) {
       if ((rc = dalloc_n(&pl->pieces, pl->npieces, st)) != VS_OK ||
           (rc = dalloc_n(&pl->heavy_rows, nmulti * pl->Q, st)) != VS_OK ||
@@ -2562,7 +2620,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
         return rc;
       }
       e = cudaMemsetAsync(pl->heavy_rows, 0, nmulti * pl->Q * 16, st);
-      { k_hub_pieces<<<sm_count() * 4, 256, 0, st>>>(in, heavy, pl->nheavy, pe, pl->pieces, dn + 6, pl->heavy_np,
+      { k_hub_pieces<<<sm_count() * 4, 256, 0, st>>>(in, heavy, pl->nheavy, pe, pl->pieces, dn + 3, pl->heavy_np,
                                                      pl->heavy_left, pl->nslices); vs::note_launch(); }
       if (e == cudaSuccess) e = cudaGetLastError();
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // runs may be on any stream
@@ -2574,9 +2632,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
       return cuda_fail(e, "hub list", __FILE__, __LINE__);
     }
   }
-  pl->pull_kind = p->pull_kernel;
   if (p->sparse_frac > 0) pl->sparse_frac = p->sparse_frac;
-  const int hub_smem = 16 * 32 * 16 * var.UPL;
   // a task is `tile` consecutive targets: a round of the warp's groups on small
   // graphs (more tasks than warps), up to 16 targets on large ones
   const uint32_t G = 32 / var.L;
@@ -2585,12 +2641,16 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   while (pl->tile < 16 && (uint64_t)V / pl->tile > 64ull * occ) pl->tile *= 2;
   const uint64_t tasks = pl->npieces + ((uint64_t)V + pl->tile - 1) / pl->tile;
   pl->grid_pull = (int)std::max<uint64_t>(1, std::min<uint64_t>(occ, (tasks + 7) / 8));
-  if (pl->slot[0]) {  // short mode: a row of Q uint4 per warp (PULL) or per CTA (hubs)
-    const int hs = hub_smem + (int)pl->Q * 16;
-    if (hs > 48 * 1024) cudaFuncSetAttribute(var.hub_short, cudaFuncAttributeMaxDynamicSharedMemorySize, hs);
-    pl->grid_hub = std::max(1, std::min((int)pl->nhubs, occupancy_grid(var.hub_short, 512, hs, 2)));
-    pl->grid_short = occupancy_grid(var.pull_short, 256, 8 * (size_t)pl->Q * 16, 8);
-    pl->grid_short_pre = occupancy_grid(var.pull_short_pre, 256, 8 * (size_t)pl->Q * 16, 8);
+  if (pl->slot[0]) {
+    const size_t sm = short_smem(pl->Q, pl->slot_n);
+    int occ_short = 0;
+    const ShortVariant &sv = pick_short(pl->Q);
+    for (PullFn f : {sv.words[0], sv.words[1], sv.words[2], sv.slots[1], sv.slots[2]}) {
+      if (sm > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      occ_short = std::max(occ_short, occupancy_grid(f, SH_WARPS * 32, sm, 8));
+    }
+    const uint64_t stasks = pl->npieces + ((uint64_t)V + short_tile(pl->Q) - 1) / short_tile(pl->Q);
+    pl->grid_short = (int)std::max<uint64_t>(1, std::min<uint64_t>(occ_short, (stasks + SH_WARPS - 1) / SH_WARPS));
   }
   pl->grid_sparse = occupancy_grid(k_sparse, 256, 0, 8);
   pl->grid_push = occupancy_grid(k_push, 256, 0, 8);
@@ -2610,12 +2670,19 @@ int vs_expand_plan_footprint(const vs_graph *g, uint32_t S, const vs_expand_para
                                   : std::max<uint64_t>(1u << 20, std::min<uint64_t>((uint64_t)S * V / 8, 1ull << 25));
   cap = std::max<uint64_t>(cap, S);
   uint64_t b = (2 + use_vis + use_acc) * V * W * 8;             // frontier pair, visited, accumulator
-  b += 6 * V * 4;                                                 // flags x2, resflag, push list, touched, hubs
+  b += 5 * V * 4;                                                 // flags x2, resflag, push list, touched
+  // heavy targets: at most a piece per piece_edges entries and one per target, a row per two pieces
+  const uint64_t list_edges = (p->direction == VS_DIR_BOTH && g->directed ? 2 : 1) * g->E;
   b += cap * (2 * 8 + 2 * 8 + 8) + ((cap + 1023) / 1024 + 1) * 8;  // pair lists, degrees, offsets, block sums
   b += (uint64_t)S * 4 * 3 + sizeof(Ctr) + (uint64_t)(p->k_max + 1) * W * 8;
   uint32_t qs = p->slice_words ? (p->slice_words + 1) / 2 : (uint32_t)(W / 2);
   qs = std::max<uint32_t>(1, std::min<uint32_t>(qs, 256));
   const uint32_t nslices = (uint32_t)((W / 2 + qs - 1) / qs);
+  const int L = pick_variant(qs).L;
+  const uint64_t thr = p->hub_threshold ? std::min(p->hub_threshold, 1u << 16) : heavy_default(L);
+  const uint64_t multi = std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, std::max<uint64_t>(thr, piece_edges(L))));
+  b += 16 * (list_edges / piece_edges(L) + 2 * std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, thr)));
+  b += multi * (W * 8 + 4 + 4 * nslices) + (uint64_t)(p->k_max + 1) * (W * 8 + 4 * nslices);
   if (short_slots_ok(S, nslices, p->short_share, V, (uint32_t)W))
     b += 2 * V * (2 * slot_entries((uint32_t)W) + sizeof(Tiny));  // short-row words and slots of both buffers
   *bytes = b;
@@ -2730,7 +2797,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     da.push_ok = can_push;
     da.rowk = pl->use_hmask ? pl->rowk : nullptr;
     da.short_min = pl->short_min;
-    da.l2_half = l2_bytes() / 2;
+    da.last = h == p.k_max && pl->use_vis && !pl->use_acc && p.path_type != VS_PATH_FIND_SHORTEST && !pl->layer_out[h];
     da.W = W;
     da.k_min = p.k_min;
     da.k_max = p.k_max;
@@ -2824,9 +2891,6 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     // matrix or the accumulator (FindShortest checks every layer's targets)
     a.last = h == p.k_max && (pl->use_vis || pl->use_acc) && p.path_type != VS_PATH_FIND_SHORTEST &&
              !pl->layer_out[h];
-    a.hub_threshold = pl->nhubs ? pl->hub_threshold : 0;
-    a.hubs = pl->hubs;
-    a.nhubs = pl->nhubs;
     a.heavy_threshold = pl->nheavy ? pl->heavy_threshold : 0;
     a.pieces = pl->pieces;
     a.npieces = pl->npieces;
@@ -2848,7 +2912,8 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     a.tiny_out = keep_short ? pl->tiny[nbuf] : nullptr;
     a.slot_out = keep_short ? pl->slot[nbuf] : nullptr;
     a.slot_n = pl->slot_n;
-    a.pre = (pl->pull_kind & 4) == 0;
+    a.out = outl;
+    short_layout(a, short_tile(Q));
     if (timing) cudaEventRecord(pl->ev[3 * h + 1], st);
     if (pl->slot[0]) {  // words and slots of a layer SPARSE, PUSH or the seed wrote, when this hop reads them
       { k_pairs_zero<<<pl->grid_v, 256, 0, st>>>(pl->touched, V, pl->ctr, h); vs::note_launch(); }
@@ -2865,12 +2930,14 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     }
     { var.pull<<<dim3(pl->grid_pull, pl->nslices), 256, 0, st>>>(a); vs::note_launch(); }
     if (pl->slot[0]) {
-      if (a.pre)
-        { var.pull_short_pre<<<pl->grid_short_pre, 256, 8 * (size_t)Q * 16, st>>>(a); vs::note_launch(); }
-      else
-        { var.pull_short<<<pl->grid_short, 256, 8 * (size_t)Q * 16, st>>>(a); vs::note_launch(); }
-      if (pl->nhubs)
-        { var.hub_short<<<pl->grid_hub, 512, 16 * 32 * 16 * var.UPL + (size_t)Q * 16, st>>>(a); vs::note_launch(); }
+      const ShortVariant &sv = pick_short(Q);
+      const size_t sm = short_smem(Q, pl->slot_n);
+      const bool last = a.last && a.shortest && !a.acc_on;
+      a.list_too = !last && a.tiny_out && a.virt_out && !a.acc_on;
+      if (a.list_too) { sv.words[SH_LIST]<<<pl->grid_short, SH_WARPS * 32, sm, st>>>(a); vs::note_launch(); }
+      { sv.words[last ? SH_LAST : SH_GEN]<<<pl->grid_short, SH_WARPS * 32, sm, st>>>(a); vs::note_launch(); }
+      a.list_too = 0;
+      { sv.slots[last ? SH_LAST : SH_GEN]<<<pl->grid_short, SH_WARPS * 32, sm, st>>>(a); vs::note_launch(); }
     }
     if (p.path_type == VS_PATH_FIND_SHORTEST)
       { k_find_check<<<std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st>>>(
@@ -3031,13 +3098,11 @@ int vs_expand_plan_set_row_limits_device(vs_expand_plan *pl, const uint8_t *row_
   return VS_OK;
 }
 
-// Kernel shape of the PULL hops: bit 2 runs short-mode hops without loading the
-// next target's visited words and flag ahead.  Bits 0 and 1 chose shapes of the
-// dense kernel that are gone (its groups run one shape per row width); they are
-// still taken, so saved settings stay valid.
+// Kernel shape of the PULL hops: the shapes it chose from are gone (the kernels
+// run one shape per row width); the kind is still taken, so saved settings stay
+// valid.
 int vs_expand_plan_set_pull_kernel(vs_expand_plan *pl, int kind) {
   if (!pl || kind < 0 || kind > 7) return fail(VS_ERR_ARG, "pull kernel variant must be 0..7");
-  pl->pull_kind = kind;
   return VS_OK;
 }
 

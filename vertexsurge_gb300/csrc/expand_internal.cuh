@@ -15,16 +15,19 @@ struct HopCtr {
   unsigned long long active_vertices;  // non-zero rows of layer h
   unsigned long long active_edges;     // edges leaving non-zero rows of layer h-1 (stats pass)
   unsigned long long pairs;            // SPARSE: (vertex, source) pairs of layer h
-  unsigned long long pair_edges;       // SPARSE: sum of out-degrees over those pairs
+  unsigned long long pair_edges;       // sum of out-degrees over the layer's (vertex, source) pairs (SPARSE, and PULL
+                                       // when it keeps words)
   unsigned long long work_edges;       // SPARSE: edges scanned by the hop
   unsigned long long hist[16];         // log2(out-degree + 1) histogram of layer h-1's active rows
   int overflow;                        // SPARSE: pair list overflowed
   int strategy;                        // strategy run at hop h (0 = not run)
   int short_pull;                      // PULL reads the short rows of layer h-1 through their slots
+  int short_long;                      // ... and most of its new rows will be too long for a slot
   int short_slots;                     // ... reading slots (count in entry 0) instead of tiny words
   unsigned long long short_rows;       // rows of layer h with 1..slot_n-1 bits (low 32 bits) and with at most
                                        // TINY_MAX bits (high 32 bits), counted when its words are written
   unsigned long long short_edges;      // active in-edges of a short-mode PULL served from a slot
+  unsigned long long row_out, short_out;  // out-degrees of layer h's non-empty rows and of its short rows (likewise)
 };
 
 struct Ctr {
@@ -71,8 +74,8 @@ struct DecideArgs {
   double sparse_frac, push_frac;
   const void *picker;  // bf16 weights of a vs_picker (NULL = fixed planner)
   const uint32_t *rowk;  // [0] largest row hop limit (NULL: no row limits)
-  double short_min;      // short-mode PULL when at least this share of the frontier's rows are short (0: off; > 1: always)
-  uint64_t l2_half;       // ... and the frontier's rows exceed this many bytes (smaller ones stay in L2)
+  int last;              // nothing reads layer h and the result is the visited matrix
+  double short_min;      // short-mode PULL needs at least this share of the frontier's rows short (0: off; > 1: always)
 };
 
 struct SparseArgs {
@@ -130,11 +133,10 @@ struct PullArgs {
   uint16_t *slot_out;       // slots of layer h (count, then the ids of a row of < slot_n bits)
   uint32_t slot_n;          // uint16 entries per slot (16, 32 or 64)
   int virt_out;             // short rows of layer h may stay in their slots (flag 2, buffer row zero)
-  int pre;                  // short mode: the next target's visited words and flag are loaded ahead
-  uint32_t hub_threshold;
-  const uint32_t *hubs;
-  uint32_t nhubs;
-  // dense PULL: targets above heavy_threshold (0: none) come in pieces
+  int list_too;             // short mode: the LIST kernel runs beside this GEN one (one of them returns at once)
+  uint32_t sh_list, sh_queue, sh_aside, sh_warp;  // short mode: a warp's shared memory, in uint4
+  Lists out;                // out-lists (degrees of the layer's rows)
+  // targets above heavy_threshold (0: none) come in pieces
   uint32_t heavy_threshold;
   const uint4 *pieces;       // (target, its row of heavy_rows or ~0 when this is its only piece, list, first entry)
   uint32_t npieces, piece_edges;
