@@ -100,7 +100,7 @@ int flat_alloc(uint32_t ncols, const int32_t *types, uint64_t nrows, cudaStream_
   return VS_OK;
 }
 
-int bitmat_alloc(uint32_t rows, uint32_t cols, int kind, cudaStream_t st, vs_bitmat **out) {
+int bitmat_alloc(uint32_t rows, uint32_t cols, int kind, cudaStream_t st, vs_bitmat **out, bool clear) {
   if (kind != VS_KIND_VARROW && kind != VS_KIND_COLMAIN)
     return fail(VS_ERR_ARG, "unknown matrix kind %d", kind);
   vs_bitmat *m = new vs_bitmat();
@@ -116,7 +116,7 @@ int bitmat_alloc(uint32_t rows, uint32_t cols, int kind, cudaStream_t st, vs_bit
     delete m;
     return rc;
   }
-  cudaError_t e = cudaMemsetAsync(m->words, 0, sizeof(uint64_t) * (n ? n : 1), st);
+  cudaError_t e = clear ? cudaMemsetAsync(m->words, 0, sizeof(uint64_t) * (n ? n : 1), st) : cudaSuccess;
   if (e != cudaSuccess) {
     dfree(m->words, st);
     delete m;
@@ -150,10 +150,12 @@ __global__ void mask_last_word_kernel(uint64_t *w, uint32_t cols, uint32_t wpc, 
     w[(size_t)c * wpc + last] &= mask;
 }
 
-// popcount of the columns whose colnz flag is set: a warp loads 32 flags at
-// once and walks only the flagged columns (16-byte loads).
-__global__ void popcount_cols_kernel(const uint4 *__restrict__ w, uint32_t cols, uint32_t q_per_col,
-                                     const uint32_t *__restrict__ colnz, unsigned long long *__restrict__ out) {
+// popcount of the columns whose colnz flag is set: a warp loads 32 flags at once
+// and walks only the flagged columns, four at a time (16-byte loads; the bytes of
+// the flagged columns bound it).
+__global__ void __launch_bounds__(256) popcount_cols_kernel(const uint4 *__restrict__ w, uint32_t cols, uint32_t q_per_col,
+                                                            const uint32_t *__restrict__ colnz,
+                                                            unsigned long long *__restrict__ out) {
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   unsigned long long s = 0;
@@ -161,11 +163,19 @@ __global__ void popcount_cols_kernel(const uint4 *__restrict__ w, uint32_t cols,
     const uint32_t c = c0 + lane;
     unsigned m = __ballot_sync(0xffffffffu, c < cols && colnz[c]);
     while (m) {
-      const uint32_t cc = c0 + __ffs(m) - 1;
-      m &= m - 1;
+      uint32_t cc[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        cc[k] = m ? c0 + __ffs(m) - 1 : 0xffffffffu;
+        m &= m - 1;
+      }
       for (uint32_t q = lane; q < q_per_col; q += 32) {
-        const uint4 x = __ldg(w + (size_t)cc * q_per_col + q);
-        s += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+        uint4 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          x[k] = cc[k] != 0xffffffffu ? __ldg(w + (size_t)cc[k] * q_per_col + q) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) s += popc4(x[k]);
       }
     }
   }

@@ -2,7 +2,7 @@
 // SemiJoin<N> (src/objects/operator/matrix_column_count.cpp:6-87,
 // matrix_row_or_sum.cpp:7-54, semi_join.cpp:7-262) re-designed for sm_103a.
 //
-// Column counts: G = min(32, pow2 >= words per column) lanes per column
+// Column counts: G = min(32, pow2 >= uint4 per column) lanes per column
 // popcount its words.  The ordered form sorts the 64-bit keys
 // (count << 32 | column value) — bit-complemented for descending order, which
 // reproduces std::greater on the (count, value) pair — with a stable LSD radix
@@ -47,19 +47,39 @@ struct Scratch {
 };
 
 // ---- column popcounts --------------------------------------------------------
-__global__ void k_col_counts(const uint64_t *__restrict__ w, uint32_t wpc, uint32_t cols, uint32_t G,
-                             const uint32_t *__restrict__ colnz, uint32_t *__restrict__ cnt) {
-  const uint32_t lane = threadIdx.x & 31, gl = lane % G, gpw = 32 / G;
+// G = min(32, pow2 >= uint4 per column) lanes per column, 4 columns per group in
+// flight at once: bound by reading the matrix.
+__global__ void __launch_bounds__(256) k_col_counts(const uint4 *__restrict__ w, uint32_t Q, uint32_t cols, uint32_t G,
+                                                    const uint32_t *__restrict__ colnz, uint32_t *__restrict__ cnt) {
+  const uint32_t lane = threadIdx.x & 31, gl = lane & (G - 1), g = lane / G, gpw = 32 / G;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const uint64_t warps = (uint64_t)gridDim.x * blockDim.x / 32;
   // warp-uniform loop: every lane reaches the group shuffles
-  for (uint64_t base = warp * gpw; base < cols; base += warps * gpw) {
-    const uint64_t c = base + lane / G;
-    uint32_t s = 0;
-    if (c < cols && (!colnz || colnz[c]))
-      for (uint32_t q = gl; q < wpc; q += G) s += __popcll(__ldg(w + c * wpc + q));
-    for (uint32_t o = G >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-    if (gl == 0 && c < cols) cnt[c] = s;
+  for (uint64_t base = warp * gpw * 4; base < cols; base += warps * gpw * 4) {
+    uint32_t s[4];
+    bool look[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint64_t c = base + k * gpw + g;
+      look[k] = c < cols && (!colnz || __ldg(colnz + c));
+      s[k] = 0;
+    }
+    for (uint32_t q = gl; q < Q; q += G) {
+      uint4 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = look[k] ? __ldg(w + (base + k * gpw + g) * Q + q) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int k = 0; k < 4; k++) s[k] += popc4(x[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (G == 32)
+        s[k] = __reduce_add_sync(0xffffffffu, s[k]);
+      else
+        for (uint32_t o = G >> 1; o; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o, G);
+      const uint64_t c = base + k * gpw + g;
+      if (gl == 0 && c < cols) cnt[c] = s[k];
+    }
   }
 }
 
@@ -67,7 +87,9 @@ __global__ void k_cc_keys(const uint32_t *__restrict__ cnt, const uint32_t *__re
                           int desc, unsigned long long *__restrict__ keys) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x) {
     const unsigned long long k = ((unsigned long long)cnt[c] << 32) | (col_map ? col_map[c] : c);
-    keys[c] = desc ? ~k : k;
+    // without a map the keys are laid down in the order of their low halves, so
+    // that a stable sort needs the counts' bytes alone
+    keys[desc && !col_map ? cols - 1 - c : c] = desc ? ~k : k;
   }
 }
 
@@ -175,10 +197,10 @@ __global__ void k_compact_cols(const uint32_t *__restrict__ cnt, const unsigned 
 int column_counts(const vs_bitmat *m, Scratch &sc, uint32_t **cnt) {
   VS_TRY(sc.get(cnt, m->cols));
   uint32_t G = 1;
-  while (G < 32 && G < m->wpc) G <<= 1;
+  while (G < 32 && G < m->wpc / 2) G <<= 1;
   if (m->cols)
-    { k_col_counts<<<grid_for((uint64_t)m->cols * G), 256, 0, sc.st>>>(m->words, m->wpc, m->cols, G, m->colnz,
-                                                                      *cnt); vs::note_launch(); }
+    { k_col_counts<<<grid_for(((uint64_t)m->cols * G + 3) / 4), 256, 0, sc.st>>>(
+          reinterpret_cast<const uint4 *>(m->words), m->wpc / 2, m->cols, G, m->colnz, *cnt); vs::note_launch(); }
   VS_CK(cudaGetLastError());
   return VS_OK;
 }
@@ -407,11 +429,12 @@ int vs_matrix_column_count(const vs_bitmat *m, int order, vs_flat **out, vs_stre
   if (order && m->cols) {
     VS_TRY(sc.get(&keys, m->cols));
     { k_cc_keys<<<grid_for(m->cols), 256, 0, st>>>(cnt, m->col_map, m->cols, desc, keys); vs::note_launch(); }
-    // the bytes that can differ: the 32-bit column value, then the count (at most rows)
+    // the bytes that can differ: the 32-bit column value (of a mapped matrix; k_cc_keys
+    // orders the others), then the count (at most rows)
     int cbits = 0;
     while (cbits < 32 && (1ull << cbits) <= m->rows) cbits++;
     const int hi = 32 + ((cbits + 7) / 8) * 8;
-    int rc = radix_sort_u64(sc, keys, m->cols, 0, hi, &sorted);
+    int rc = radix_sort_u64(sc, keys, m->cols, m->col_map ? 0 : 32, hi, &sorted);
     if (rc != VS_OK) {
       vs_flat_free(f);
       return rc;

@@ -31,33 +31,72 @@ __global__ void k_count_invalid(const uint32_t *__restrict__ ids, uint32_t n, ui
     if (ids[i] >= bound) atomicAdd(bad, 1u);
 }
 
-// 64x64 bit-block transpose.  Block (bw, bc) covers input rows 64*bw..+63 and
-// input columns 64*bc..+63; lane l holds input columns bc*64+l and bc*64+32+l.
-// Output column r = 64*bw + j receives word bc: bit c = input (r, 64*bc + c).
-__global__ void k_transpose(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
-                            uint32_t in_rows, uint32_t in_cols, uint32_t wpc_in,
-                            uint32_t wpc_out, uint32_t tiles_r, uint32_t tiles_c) {
-  const int lane = threadIdx.x & 31;
+// Bit transpose in tiles of 512 rows x 512 columns.  Bound by memory: a tile reads
+// 64 contiguous bytes of each of its columns and writes 64 of each of its output
+// columns (whole sectors, 16 bytes per lane), and is turned in shared memory, a
+// 32 x 32 block per warp by five shuffle steps (a ballot per bit took 64 votes and
+// 8-byte accesses at the column stride).  Output words past the last input column
+// are written as zeros.  4,096 x 200,000: 305 -> 70 us (floor 31).
+constexpr int TP = 512, TPW = TP / 32;             // rows (columns) of a tile, 32-bit words of them
+constexpr int TP_IN = TP + 1, TP_OUT = TPW + 1;    // padded strides: odd, a warp's column falls on all banks
+constexpr size_t TP_SMEM = 4 * ((size_t)TPW * TP_IN + 3) / 16 * 16 + 4 * (size_t)TP * TP_OUT + 16;
+
+__global__ void __launch_bounds__(256) k_transpose(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
+                                                   uint32_t in_rows, uint32_t in_cols, uint32_t wpc_in,
+                                                   uint32_t wpc_out, uint32_t tiles_r, uint32_t tiles_c) {
+  extern __shared__ uint4 s_tp[];
+  uint32_t *s_in = reinterpret_cast<uint32_t *>(s_tp);                                 // [TPW][TP_IN]: word, column
+  uint32_t *s_out = s_in + ((size_t)TPW * TP_IN + 3) / 4 * 4;                          // [TP][TP_OUT]: row, word
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t ntiles = (uint64_t)tiles_r * tiles_c;
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  for (uint64_t t = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < ntiles;
-       t += warps) {
-    const uint32_t bw = (uint32_t)(t % tiles_r), bc = (uint32_t)(t / tiles_r);
-    const uint32_t c_lo = bc * 64 + lane, c_hi = c_lo + 32;
-    const uint64_t a = c_lo < in_cols ? in[(size_t)c_lo * wpc_in + bw] : 0ull;
-    const uint64_t b = c_hi < in_cols ? in[(size_t)c_hi * wpc_in + bw] : 0ull;
-    uint64_t mine_lo = 0, mine_hi = 0;  // output rows 64bw+lane and 64bw+32+lane
-#pragma unroll 8
-    for (int j = 0; j < 64; j++) {
-      const unsigned lo = __ballot_sync(FULL, (a >> j) & 1ull);
-      const unsigned hi = __ballot_sync(FULL, (b >> j) & 1ull);
-      const uint64_t w = (uint64_t)lo | ((uint64_t)hi << 32);
-      if (j == lane) mine_lo = w;
-      if (j == lane + 32) mine_hi = w;
+  // a step swaps the off-diagonal halves of ever smaller blocks between lanes k
+  // apart: bytes by a permutation, smaller pieces by a rotation and a select
+  const uint32_t sel16 = lane & 16 ? 0x3276u : 0x5410u, sel8 = lane & 8 ? 0x3715u : 0x6240u;
+  uint32_t keep[3], rot[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const uint32_t k = 4 >> i, m = i == 0 ? 0x0f0f0f0fu : i == 1 ? 0x33333333u : 0x55555555u;
+    keep[i] = lane & k ? ~m : m;
+    rot[i] = lane & k ? 32 - k : k;
+  }
+  for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const uint32_t tr = (uint32_t)(t % tiles_r), tc = (uint32_t)(t / tiles_r);
+#pragma unroll
+    for (int k = 0; k < TP * 4 / 256; k++) {
+      const uint32_t i = k * 256 + threadIdx.x, c = i >> 2, q = i & 3;
+      const uint32_t col = tc * TP + c, qi = tr * 4 + q;
+      uint4 x = make_uint4(0, 0, 0, 0);
+      if (col < in_cols && qi < wpc_in / 2) x = __ldg(reinterpret_cast<const uint4 *>(in + (size_t)col * wpc_in) + qi);
+      s_in[(q * 4 + 0) * TP_IN + c] = x.x;
+      s_in[(q * 4 + 1) * TP_IN + c] = x.y;
+      s_in[(q * 4 + 2) * TP_IN + c] = x.z;
+      s_in[(q * 4 + 3) * TP_IN + c] = x.w;
     }
-    const uint32_t r_lo = bw * 64 + lane, r_hi = r_lo + 32;
-    if (r_lo < in_rows) out[(size_t)r_lo * wpc_out + bc] = mine_lo;
-    if (r_hi < in_rows) out[(size_t)r_hi * wpc_out + bc] = mine_hi;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t b = warp; b < TPW * TPW; b += 8) {  // 32 x 32 blocks: word w of columns 32g..32g+31
+      const uint32_t w = b / TPW, g = b % TPW;
+      uint32_t x = s_in[w * TP_IN + g * 32 + lane];
+      x = __byte_perm(x, __shfl_xor_sync(FULL, x, 16), sel16);
+      x = __byte_perm(x, __shfl_xor_sync(FULL, x, 8), sel8);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const uint32_t y = __shfl_xor_sync(FULL, x, 4 >> i);
+        x = (x & keep[i]) | (__funnelshift_l(y, y, rot[i]) & ~keep[i]);
+      }
+      s_out[(w * 32 + lane) * TP_OUT + g] = x;  // row 32w + lane
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < TP * 4 / 256; k++) {
+      const uint32_t i = k * 256 + threadIdx.x, r = i >> 2, q = i & 3;
+      const uint32_t row = tr * TP + r, qo = tc * 4 + q;
+      if (row < in_rows && qo < wpc_out / 2)
+        reinterpret_cast<uint4 *>(out + (size_t)row * wpc_out)[qo] =
+            make_uint4(s_out[r * TP_OUT + q * 4], s_out[r * TP_OUT + q * 4 + 1], s_out[r * TP_OUT + q * 4 + 2],
+                       s_out[r * TP_OUT + q * 4 + 3]);
+    }
+    __syncthreads();
   }
 }
 
@@ -280,7 +319,7 @@ int vs_matrix_select(const vs_bitmat *m, const uint32_t *targets, uint32_t T, vs
     return fail(VS_ERR_UNSUPPORTED, "MatrixTableSelect on a matrix that already has a col_map");
   cudaStream_t st = S(stream);
   vs_bitmat *r = nullptr;
-  VS_TRY(bitmat_alloc(m->rows, T, m->kind, st, &r));
+  VS_TRY(bitmat_alloc(m->rows, T, m->kind, st, &r, false));  // every column is written
   int rc = VS_OK;
   if (T) {
     if ((rc = dalloc_n(&r->col_map, T, st)) != VS_OK || (rc = copy_in(r->col_map, targets, T, st)) != VS_OK) {
@@ -321,17 +360,23 @@ int vs_table_convert(const vs_bitmat *m, int transpose, vs_bitmat **out, vs_stre
   cudaStream_t st = S(stream);
   vs_bitmat *r = nullptr;
   const uint32_t rows = transpose ? m->cols : m->rows, cols = transpose ? m->rows : m->cols;
-  VS_TRY(bitmat_alloc(rows, cols, VS_KIND_COLMAIN, st, &r));
+  // every word is written, unless there are none
+  VS_TRY(bitmat_alloc(rows, cols, VS_KIND_COLMAIN, st, &r, !(m->rows && m->cols)));
   int rc = VS_OK;
   if (!transpose) {
     if (m->rows && m->cols)
       cudaMemcpyAsync(r->words, m->words, 8ull * m->wpc * m->cols, cudaMemcpyDeviceToDevice, st);
   } else if (m->rows && m->cols) {
-    const uint32_t tiles_r = (m->rows + 63) / 64, tiles_c = (m->cols + 63) / 64;
-    uint64_t tiles = (uint64_t)tiles_r * tiles_c;
-    int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((tiles + 7) / 8, (uint64_t)sm_count() * 16));
-    { mx::k_transpose<<<blocks, 256, 0, st>>>(m->words, r->words, m->rows, m->cols, m->wpc, r->wpc,
-                                            tiles_r, tiles_c); vs::note_launch(); }
+    const uint32_t tiles_r = (m->rows + mx::TP - 1) / mx::TP, tiles_c = (m->cols + mx::TP - 1) / mx::TP;
+    const uint64_t tiles = (uint64_t)tiles_r * tiles_c;
+    const cudaError_t ea = cudaFuncSetAttribute(mx::k_transpose, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::TP_SMEM);
+    if (ea != cudaSuccess) {
+      vs_bitmat_free(r);
+      return cuda_fail(ea, "vs_table_convert", __FILE__, __LINE__);
+    }
+    const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)sm_count() * 3));
+    { mx::k_transpose<<<blocks, 256, mx::TP_SMEM, st>>>(m->words, r->words, m->rows, m->cols, m->wpc, r->wpc,
+                                                      tiles_r, tiles_c); vs::note_launch(); }
   }
   const uint32_t *rm = transpose ? m->col_map : m->row_map;
   const uint32_t *cm = transpose ? m->row_map : m->col_map;

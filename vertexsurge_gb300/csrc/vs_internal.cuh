@@ -117,7 +117,8 @@ int bitmat_to_flat(const vs_bitmat *m, cudaStream_t st, vs_flat **out);
 int validate_ids(const uint32_t *d_ids, uint32_t n, uint32_t bound, cudaStream_t st, bool *ok);
 extern "C" const void *vs_picker_device_weights(const vs_picker *p);
 int flat_alloc(uint32_t ncols, const int32_t *types, uint64_t nrows, cudaStream_t st, vs_flat **out);
-int bitmat_alloc(uint32_t rows, uint32_t cols, int kind, cudaStream_t st, vs_bitmat **out);
+// clear: zero the words (a caller that writes every one leaves it out)
+int bitmat_alloc(uint32_t rows, uint32_t cols, int kind, cudaStream_t st, vs_bitmat **out, bool clear = true);
 
 // Device-side helpers -------------------------------------------------------
 __device__ __forceinline__ uint4 or4(uint4 a, uint4 b) {
