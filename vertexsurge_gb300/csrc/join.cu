@@ -32,6 +32,16 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned long long EMPTY = HT_EMPTY;
 using Table = HashTable;
 
+// Arrays indexed by vertex-id keys (below, at k_key_max).
+struct Direct {
+  uint32_t *cnt;   // rows per key
+  uint32_t *row;   // a build row of the key (NULL: counts only)
+  uint32_t bound;  // entries of the arrays
+  uint32_t *ctl;   // [0] largest build key, [1] some key has several rows
+};
+
+__device__ __forceinline__ bool direct_ok(const Direct &d) { return d.ctl[0] < d.bound; }
+
 __device__ __forceinline__ unsigned long long load_key(const void *col, int type, uint64_t i) {
   return type == VS_T_I64 ? (unsigned long long)((const long long *)col)[i]
                           : (unsigned long long)((const uint32_t *)col)[i];
@@ -67,7 +77,9 @@ __global__ void k_build(Table t, const void *keycol, int ktype, uint64_t n, uint
 // Keys that find no shared slot within a few probes go to the global table
 // directly.
 constexpr int LOC_SLOTS = 4096;
-__global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol, int ktype, uint64_t n) {
+__global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol, int ktype, uint64_t n,
+                                                      Direct d) {
+  if (d.ctl && direct_ok(d)) return;
   __shared__ unsigned long long s_key[LOC_SLOTS];
   __shared__ uint32_t s_cnt[LOC_SLOTS];
   for (int i = threadIdx.x; i < LOC_SLOTS; i += blockDim.x) {
@@ -104,6 +116,143 @@ __global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol
     }
 }
 
+// ---------------------------------------------------------------------------
+// Vertex-id keys below a bound of a few times the build rows need no hash: an
+// array indexed by the key holds each key's count (and build row), in L2 where the
+// hash table of 10M keys is 537 MB of HBM.  The largest build key is found on the
+// device and every kernel checks it against the bound, so the host waits for
+// nothing; above the bound the kernels return and the hash kernels run.  Count of
+// 10M x 10M Zipf-skewed keys below 10M: 432 -> 117 us, of which counting the build
+// keys (shared-memory atomics) 71.
+__global__ void __launch_bounds__(256) k_key_max(const uint32_t *__restrict__ keys, uint64_t n, uint32_t *ctl) {
+  uint32_t m = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint4 *k4 = reinterpret_cast<const uint4 *>(keys);  // a column starts on an allocation
+  for (uint64_t i = i0; i < n / 4; i += stride) {
+    const uint4 k = __ldg(k4 + i);
+    m = max(max(max(m, k.x), max(k.y, k.z)), k.w);
+  }
+  if (i0 < (n & 3)) m = max(m, keys[(n & ~3ull) + i0]);
+  m = __reduce_max_sync(FULL, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(ctl, m);
+}
+
+__global__ void __launch_bounds__(256) k_direct_clear(Direct d) {
+  if (!direct_ok(d)) return;
+  const uint32_t n4 = d.ctl[0] / 4 + 1;  // the bound is a multiple of four
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x)
+    reinterpret_cast<uint4 *>(d.cnt)[i] = make_uint4(0, 0, 0, 0);
+}
+
+// The hash table's clear, when it is needed after all.
+__global__ void __launch_bounds__(256) k_hash_clear(Table t, Direct d) {
+  if (direct_ok(d)) return;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= t.cap; i += (uint64_t)gridDim.x * blockDim.x) {
+    t.keys[i] = EMPTY;
+    t.cnt[i] = 0;
+  }
+}
+
+// Counts per key.  As in k_build_count a block first counts in a table of its own
+// in shared memory (Zipf-skewed columns send an eighth of the rows to one key), with
+// one probe: a key that finds the slot taken adds to the array in L2.
+constexpr int DIRECT_SLOTS = 4096;
+__global__ void __launch_bounds__(512) k_direct_count(Direct d, const uint32_t *__restrict__ keys, uint64_t n) {
+  if (!direct_ok(d)) return;
+  __shared__ uint32_t s_key[DIRECT_SLOTS], s_cnt[DIRECT_SLOTS];
+  for (int i = threadIdx.x; i < DIRECT_SLOTS; i += blockDim.x) {
+    s_key[i] = 0xffffffffu;  // not a key below the bound
+    s_cnt[i] = 0;
+  }
+  __syncthreads();
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto add = [&](uint32_t k) {
+    const uint32_t h = (k * 2654435761u) >> 20;  // 12 bits
+    uint32_t old = s_key[h];
+    if (old == 0xffffffffu) old = atomicCAS(&s_key[h], 0xffffffffu, k);
+    if (old == 0xffffffffu || old == k)
+      atomicAdd(&s_cnt[h], 1u);
+    else
+      atomicAdd(&d.cnt[k], 1u);
+  };
+  const uint4 *k4 = reinterpret_cast<const uint4 *>(keys);
+  for (uint64_t i = i0; i < n / 4; i += stride) {
+    const uint4 k = __ldg(k4 + i);
+    add(k.x);
+    add(k.y);
+    add(k.z);
+    add(k.w);
+  }
+  if (i0 < (n & 3)) add(keys[(n & ~3ull) + i0]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < DIRECT_SLOTS; i += blockDim.x)
+    if (s_cnt[i]) atomicAdd(&d.cnt[s_key[i]], s_cnt[i]);
+}
+
+// Sum of the counts of the probe keys.
+__global__ void __launch_bounds__(256) k_direct_probe(Direct d, const uint32_t *__restrict__ keys, uint64_t n,
+                                                      unsigned long long *total) {
+  if (!direct_ok(d)) return;
+  const uint32_t top = d.ctl[0];
+  unsigned long long s = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint4 *k4 = reinterpret_cast<const uint4 *>(keys);
+  for (uint64_t i = i0; i < n / 4; i += stride) {
+    const uint4 k = __ldg(k4 + i);
+    const uint32_t a = k.x <= top ? __ldg(d.cnt + k.x) : 0u, b = k.y <= top ? __ldg(d.cnt + k.y) : 0u;
+    const uint32_t c = k.z <= top ? __ldg(d.cnt + k.z) : 0u, e = k.w <= top ? __ldg(d.cnt + k.w) : 0u;
+    s += (unsigned long long)a + b + c + e;
+  }
+  if (i0 < (n & 3)) {
+    const uint32_t k = keys[(n & ~3ull) + i0];
+    if (k <= top) s += d.cnt[k];
+  }
+  block_add(s, total);
+}
+
+// Materialising joins whose build keys are unique (a property table): the key's row.
+__global__ void __launch_bounds__(256) k_direct_rows(Direct d, const uint32_t *__restrict__ keys, uint64_t n) {
+  if (!direct_ok(d)) return;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    if (__ldcg(d.ctl + 1)) return;  // a repeated key: the general join will run
+    const uint32_t k = __ldg(keys + i);
+    if (atomicAdd(&d.cnt[k], 1u) == 0)
+      d.row[k] = (uint32_t)i;
+    else
+      d.ctl[1] = 1;
+  }
+}
+
+// Matching probe rows per tile of FK_ROWS (sums[tile]) and in all.
+constexpr int FK_ROWS = 1024;
+__global__ void __launch_bounds__(256) k_fk_count(Direct d, const uint32_t *__restrict__ keys, uint64_t n,
+                                                  unsigned long long *__restrict__ sums, unsigned long long *total) {
+  if (!direct_ok(d) || d.ctl[1]) return;
+  const uint32_t top = d.ctl[0];
+  __shared__ uint32_t part[8];
+  unsigned long long all = 0;
+  for (uint64_t b = blockIdx.x; b * FK_ROWS < n; b += gridDim.x) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < FK_ROWS / 256; k++) {
+      const uint64_t i = b * FK_ROWS + k * 256 + threadIdx.x;
+      const uint32_t x = i < n ? __ldg(keys + i) : 0xffffffffu;
+      c += x <= top && __ldg(d.cnt + x);
+    }
+    c = __reduce_add_sync(FULL, c);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t t = 0;
+      for (int w = 0; w < 8; w++) t += part[w];
+      sums[b] = t;
+      all += t;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && all) atomicAdd(total, all);
+}
+
 // Build over matrix columns: key = col_map[c] (or c) -> first column index.
 __global__ void k_build_cols(Table t, const uint32_t *col_map, uint32_t cols) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x) {
@@ -124,7 +273,8 @@ __global__ void k_scatter(Table t, const uint32_t *slot_of, uint64_t n, uint32_t
 
 // Probe: matches per probe row (and the slot), total into *total.
 __global__ void k_probe(Table t, const void *keycol, int ktype, uint64_t n,
-                        unsigned long long *pcnt, uint32_t *pslot, unsigned long long *total) {
+                        unsigned long long *pcnt, uint32_t *pslot, unsigned long long *total, Direct d) {
+  if (d.ctl && direct_ok(d)) return;
   unsigned long long s = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -287,9 +437,60 @@ __global__ void __launch_bounds__(256) k_emit(EmitArgs a) {
   }
 }
 
+// Output rows of the matching probe rows of each tile, in probe order: one build
+// row each, so a row's place is the tile's offset plus its rank among the tile's
+// matches and no per-row counts, offsets or slots go through memory.
+__global__ void __launch_bounds__(256) k_fk_emit(EmitArgs a, Direct d, const uint32_t *__restrict__ keys,
+                                                 const unsigned long long *__restrict__ tile_off) {
+  const uint32_t top = d.ctl[0];
+  __shared__ uint32_t part[FK_ROWS / 32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint64_t b = blockIdx.x; b * FK_ROWS < a.n_probe; b += gridDim.x) {
+    const unsigned long long o0 = tile_off[b];
+    if (o0 >= a.out_rows) return;  // later tiles lie past the caller's bound too
+    uint32_t row[FK_ROWS / 256];
+    unsigned hit[FK_ROWS / 256];
+#pragma unroll
+    for (int k = 0; k < FK_ROWS / 256; k++) {
+      const uint64_t i = b * FK_ROWS + k * 256 + threadIdx.x;
+      const uint32_t x = i < a.n_probe ? __ldg(keys + i) : 0xffffffffu;
+      const bool h = x <= top && __ldg(d.cnt + x);
+      row[k] = h ? __ldg(d.row + x) : 0u;
+      hit[k] = __ballot_sync(FULL, h);
+      if (lane == 0) part[k * 8 + warp] = __popc(hit[k]);
+    }
+    __syncthreads();
+    if (warp == 0) {  // FK_ROWS / 32 == 32: a lane per warp-row
+      const uint32_t x = part[lane];
+      uint32_t incl = x;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      part[lane] = incl - x;
+    }
+    __syncthreads();
+    for (int c = 0; c < a.ncols; c++) {
+      const OutCol oc = a.col[c];
+#pragma unroll
+      for (int k = 0; k < FK_ROWS / 256; k++) {
+        const uint64_t i = b * FK_ROWS + k * 256 + threadIdx.x;
+        const unsigned long long o = o0 + part[k * 8 + warp] + __popc(hit[k] & lanemask_lt());
+        if (!(hit[k] >> lane & 1u) || o >= a.out_rows) continue;
+        const uint64_t r = oc.side ? (uint64_t)row[k] : i;
+        if (oc.type == VS_T_I64)
+          ((long long *)oc.dst)[o] = __ldg((const long long *)oc.src + r);
+        else
+          ((uint32_t *)oc.dst)[o] = __ldg((const uint32_t *)oc.src + r);
+      }
+    }
+    __syncthreads();
+  }
+}
+
 struct Scratch {
   cudaStream_t st;
-  void *p[12] = {};
+  void *p[16] = {};
   int n = 0;
   template <typename T> int get(T **out, size_t count) {
     int rc = dalloc_n(out, count, st);
@@ -301,12 +502,14 @@ struct Scratch {
   }
 };
 
-int table_alloc(Scratch &sc, uint64_t n_keys, bool with_val, bool with_off, Table *t) {
+int table_alloc(Scratch &sc, uint64_t n_keys, bool with_val, bool with_off, Table *t, bool clear = true) {
   t->cap = ht_capacity(std::max<uint64_t>(n_keys, 1));
   VS_TRY(sc.get(&t->keys, t->cap + 1));
   VS_TRY(sc.get(&t->cnt, t->cap + 1));
-  VS_CK(cudaMemsetAsync(t->keys, 0xff, 8 * (t->cap + 1), sc.st));
-  VS_CK(cudaMemsetAsync(t->cnt, 0, 8 * (t->cap + 1), sc.st));
+  if (clear) {
+    VS_CK(cudaMemsetAsync(t->keys, 0xff, 8 * (t->cap + 1), sc.st));
+    VS_CK(cudaMemsetAsync(t->cnt, 0, 8 * (t->cap + 1), sc.st));
+  }
   t->val = nullptr;
   t->off = t->cur = nullptr;
   if (with_val) {
@@ -340,6 +543,101 @@ struct FlatSide {
   uint32_t key;
 };
 
+// Key bound up to which the direct arrays are used.  They take 4 bytes an entry
+// (8 with rows) where a hash table takes 32 to 64 a row, so up to four entries a
+// row they are the smaller of the two; below 4M entries (16 MB, cleared in 5 us, in
+// L2) they win whatever the rows.
+uint32_t direct_bound(uint64_t n_build) {
+  return n_build > (1ull << 28) ? 0u : (uint32_t)std::max<uint64_t>(1u << 22, (4 * n_build + 3) / 4 * 4);
+}
+
+// The direct arrays of the build keys, and a total before their control words (one
+// 16-byte block, read back at once).  VS_ERR_OOM leaves nothing behind.
+int direct_alloc(Scratch &sc, const uint32_t *keys, uint64_t n, uint32_t bound, bool rows, Direct *d,
+                 unsigned long long **total) {
+  d->bound = bound;
+  d->row = nullptr;
+  VS_TRY(sc.get(total, 2));
+  d->ctl = reinterpret_cast<uint32_t *>(*total + 1);
+  VS_TRY(sc.get(&d->cnt, bound));
+  if (rows) VS_TRY(sc.get(&d->row, bound));
+  VS_CK(cudaMemsetAsync(*total, 0, 16, sc.st));
+  { k_key_max<<<std::min(grid_for((n + 3) / 4), 4 * sm_count()), 256, 0, sc.st>>>(keys, n, d->ctl); vs::note_launch(); }
+  { k_direct_clear<<<std::min(grid_for((bound + 3) / 4), 8 * sm_count()), 256, 0, sc.st>>>(*d); vs::note_launch(); }
+  return VS_OK;
+}
+
+// Result schema: a's columns, then b's non-key columns.
+int join_columns(FlatSide a, FlatSide b, bool build_a, int32_t *types, EmitArgs *ea) {
+  int nc = 0;
+  for (uint32_t i = 0; i < a.f->ncols; i++) {
+    types[nc] = a.f->types[i];
+    ea->col[nc].src = a.f->cols[i];
+    ea->col[nc].type = a.f->types[i];
+    ea->col[nc].side = build_a ? 1 : 0;
+    nc++;
+  }
+  for (uint32_t i = 0; i < b.f->ncols; i++) {
+    if (i == b.key) continue;
+    if (nc >= 16) return fail(VS_ERR_UNSUPPORTED, "join result wider than 16 columns");
+    types[nc] = b.f->types[i];
+    ea->col[nc].src = b.f->cols[i];
+    ea->col[nc].type = b.f->types[i];
+    ea->col[nc].side = build_a ? 0 : 1;
+    nc++;
+  }
+  ea->ncols = nc;
+  return VS_OK;
+}
+
+// The rows of a join whose build keys fit the direct arrays and are unique (a
+// property table): no slots, scatter or per-row offsets.  *done stays false when
+// they are not; the general join then runs.  4M probe rows x 1M build rows, five
+// columns: 376 -> 179 us.
+int join_unique(Scratch &sc, FlatSide a, FlatSide b, bool build_a, Direct d, const uint32_t *bkeys, uint64_t nb,
+                const uint32_t *pkeys, uint64_t np, unsigned long long *d_total, uint64_t max_rows, vs_flat **out,
+                uint64_t *count, bool *done) {
+  cudaStream_t st = sc.st;
+  const uint64_t tiles = (np + FK_ROWS - 1) / FK_ROWS;
+  unsigned long long *sums, *offs;
+  VS_TRY(sc.get(&sums, tiles));
+  VS_TRY(sc.get(&offs, tiles + 1));
+  const int grid = (int)std::min<uint64_t>(tiles, (uint64_t)sm_count() * 8);
+  { k_direct_rows<<<grid_for(nb), 256, 0, st>>>(d, bkeys, nb); vs::note_launch(); }
+  { k_fk_count<<<grid, 256, 0, st>>>(d, pkeys, np, sums, d_total); vs::note_launch(); }
+  VS_CK(cudaGetLastError());
+  struct {
+    unsigned long long total;
+    uint32_t top, dup;
+  } h;
+  VS_CK(cudaMemcpyAsync(&h, d_total, 16, cudaMemcpyDeviceToHost, st));
+  VS_CK(cudaStreamSynchronize(st));
+  if (h.top >= d.bound || h.dup) return VS_OK;
+  *done = true;
+  *count = h.total;
+  const uint64_t rows = std::min<uint64_t>(h.total, max_rows);
+  int32_t types[16];
+  EmitArgs ea{};
+  VS_TRY(join_columns(a, b, build_a, types, &ea));
+  vs_flat *f = nullptr;
+  VS_TRY(flat_alloc(ea.ncols, types, rows, st, &f));
+  for (int i = 0; i < ea.ncols; i++) ea.col[i].dst = f->cols[i];
+  ea.n_probe = np;
+  ea.out_rows = rows;
+  const int rc = rows ? exclusive_scan_u64(sums, offs, tiles, st) : VS_OK;
+  if (rc == VS_OK && rows) { k_fk_emit<<<grid, 256, 0, st>>>(ea, d, pkeys, offs); vs::note_launch(); }
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (rc != VS_OK || e != cudaSuccess) {
+    vs_flat_free(f);
+    return rc != VS_OK ? rc : cuda_fail(e, "hash join", __FILE__, __LINE__);
+  }
+  *out = f;
+  return h.total > max_rows ? fail(VS_ERR_CAPACITY, "join produced %llu rows, bound %llu", h.total,
+                                   (unsigned long long)max_rows)
+                            : VS_OK;
+}
+
 // Flat x Flat join.  a = deps[0], b = deps[1]; result = a cols + b non-key cols.
 int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, vs_flat **out,
                    uint64_t *count, cudaStream_t st) {
@@ -351,12 +649,44 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   const FlatSide &bd = build_a ? a : b, &pr = build_a ? b : a;
   Scratch sc{st};
   Table t;
-  VS_TRY(table_alloc(sc, bd.f->nrows, false, !only_count, &t));
+  const uint64_t nb = bd.f->nrows, np = pr.f->nrows;
+  const bool vid = bd.f->types[bd.key] == VS_T_VID;
+  const uint32_t *bkeys = (const uint32_t *)bd.f->cols[bd.key], *pkeys = (const uint32_t *)pr.f->cols[pr.key];
+  const uint32_t bound = vid && nb && np ? direct_bound(nb) : 0u;
+  if (bound) {
+    Scratch dsc{st};
+    Direct d;
+    unsigned long long *d_total = nullptr;
+    const int rc = only_count ? table_alloc(sc, nb, false, false, &t, false) : VS_OK;
+    if (rc != VS_OK) return rc;
+    const int dc = direct_alloc(dsc, bkeys, nb, bound, !only_count, &d, &d_total);
+    if (dc != VS_OK && dc != VS_ERR_OOM) return dc;
+    if (dc == VS_OK && only_count) {  // the arrays, or the hash table in their place
+      { k_direct_count<<<std::min(grid_for((nb + 3) / 4, 512), 2 * sm_count()), 512, 0, st>>>(d, bkeys, nb); vs::note_launch(); }
+      { k_direct_probe<<<grid_for((np + 3) / 4), 256, 0, st>>>(d, pkeys, np, d_total); vs::note_launch(); }
+      { k_hash_clear<<<grid_for(t.cap), 256, 0, st>>>(t, d); vs::note_launch(); }
+      { k_build_count<<<std::min(grid_for(nb), 4 * sm_count()), 256, 0, st>>>(t, bkeys, VS_T_VID, nb, d); vs::note_launch(); }
+      { k_probe<<<grid_for(np), 256, 0, st>>>(t, pkeys, VS_T_VID, np, nullptr, nullptr, d_total, d); vs::note_launch(); }
+      VS_CK(cudaGetLastError());
+      return read_total(d_total, count, st);
+    }
+    if (dc == VS_OK) {
+      bool done = false;
+      const int rr = join_unique(dsc, a, b, build_a, d, bkeys, nb, pkeys, np, d_total, max_rows, out, count, &done);
+      if (rr != VS_OK || done) return rr;
+    }
+  }
+  if (bound && only_count) {  // the table is there; no room for the arrays beside it
+    VS_CK(cudaMemsetAsync(t.keys, 0xff, 8 * (t.cap + 1), st));
+    VS_CK(cudaMemsetAsync(t.cnt, 0, 8 * (t.cap + 1), st));
+  } else {
+    VS_TRY(table_alloc(sc, bd.f->nrows, false, !only_count, &t));
+  }
   uint32_t *slot_of = nullptr;
   if (!only_count) VS_TRY(sc.get(&slot_of, bd.f->nrows));
   if (bd.f->nrows && only_count)
     { k_build_count<<<std::min(grid_for(bd.f->nrows), 4 * sm_count()), 256, 0, st>>>(
-          t, bd.f->cols[bd.key], bd.f->types[bd.key], bd.f->nrows); vs::note_launch(); }
+          t, bd.f->cols[bd.key], bd.f->types[bd.key], bd.f->nrows, Direct{}); vs::note_launch(); }
   else if (bd.f->nrows)
     { k_build<<<grid_for(bd.f->nrows), 256, 0, st>>>(t, bd.f->cols[bd.key], bd.f->types[bd.key],
                                                    bd.f->nrows, slot_of); vs::note_launch(); }
@@ -366,7 +696,7 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   if (only_count) {
     if (pr.f->nrows)
       { k_probe<<<grid_for(pr.f->nrows), 256, 0, st>>>(t, pr.f->cols[pr.key], pr.f->types[pr.key],
-                                                     pr.f->nrows, nullptr, nullptr, d_total); vs::note_launch(); }
+                                                     pr.f->nrows, nullptr, nullptr, d_total, Direct{}); vs::note_launch(); }
     VS_CK(cudaGetLastError());
     return read_total(d_total, count, st);
   }
@@ -382,36 +712,19 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   VS_TRY(sc.get(&pslot, pr.f->nrows));
   if (pr.f->nrows)
     { k_probe<<<grid_for(pr.f->nrows), 256, 0, st>>>(t, pr.f->cols[pr.key], pr.f->types[pr.key],
-                                                   pr.f->nrows, pcnt, pslot, d_total); vs::note_launch(); }
+                                                   pr.f->nrows, pcnt, pslot, d_total, Direct{}); vs::note_launch(); }
   VS_TRY(exclusive_scan_u64(pcnt, poff, pr.f->nrows, st));
   uint64_t total = 0;
   VS_TRY(read_total(d_total, &total, st));
   *count = total;
   const uint64_t rows = std::min<uint64_t>(total, max_rows);
-  // result schema: a's columns, then b's non-key columns
   int32_t types[16];
   EmitArgs ea{};
-  int nc = 0;
-  for (uint32_t i = 0; i < a.f->ncols; i++) {
-    types[nc] = a.f->types[i];
-    ea.col[nc].src = a.f->cols[i];
-    ea.col[nc].type = a.f->types[i];
-    ea.col[nc].side = build_a ? 1 : 0;
-    nc++;
-  }
-  for (uint32_t i = 0; i < b.f->ncols; i++) {
-    if (i == b.key) continue;
-    if (nc >= 16) return fail(VS_ERR_UNSUPPORTED, "join result wider than 16 columns");
-    types[nc] = b.f->types[i];
-    ea.col[nc].src = b.f->cols[i];
-    ea.col[nc].type = b.f->types[i];
-    ea.col[nc].side = build_a ? 0 : 1;
-    nc++;
-  }
+  VS_TRY(join_columns(a, b, build_a, types, &ea));
+  const int nc = ea.ncols;
   vs_flat *f = nullptr;
   VS_TRY(flat_alloc(nc, types, rows, st, &f));
   for (int i = 0; i < nc; i++) ea.col[i].dst = f->cols[i];
-  ea.ncols = nc;
   ea.poff = poff;
   ea.pslot = pslot;
   ea.rows_by_key = rows_by_key;
@@ -661,7 +974,7 @@ int vs_hash_join_count_noalloc(const void *keys_a, uint64_t na, const void *keys
   unsigned long long *total = base + 2 * (NOALLOC_SLOTS + 1);
   { k_noalloc_clear<<<grid_for(t.cap + 1), 256, 0, st>>>(t.keys, t.cnt, total, t.cap); vs::note_launch(); }
   if (nbld) { k_build<<<grid_for(nbld), 256, 0, st>>>(t, bk, key_type, nbld, nullptr); vs::note_launch(); }
-  if (nprb) { k_probe<<<grid_for(nprb), 256, 0, st>>>(t, pk, key_type, nprb, nullptr, nullptr, total); vs::note_launch(); }
+  if (nprb) { k_probe<<<grid_for(nprb), 256, 0, st>>>(t, pk, key_type, nprb, nullptr, nullptr, total, Direct{}); vs::note_launch(); }
   VS_CK(cudaGetLastError());
   VS_CK(cudaMemcpyAsync(count, total, sizeof(unsigned long long), cudaMemcpyDefault, st));
   VS_CK(cudaStreamSynchronize(st));
