@@ -77,11 +77,8 @@ __global__ void k_build(Table t, const void *keycol, int ktype, uint64_t n, uint
 // Keys that find no shared slot within a few probes go to the global table
 // directly.
 constexpr int LOC_SLOTS = 4096;
-__global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol, int ktype, uint64_t n,
-                                                      Direct d) {
-  if (d.ctl && direct_ok(d)) return;
-  __shared__ unsigned long long s_key[LOC_SLOTS];
-  __shared__ uint32_t s_cnt[LOC_SLOTS];
+__device__ __forceinline__ void build_count(const Table &t, const void *keycol, int ktype, uint64_t n,
+                                            unsigned long long *s_key, uint32_t *s_cnt) {
   for (int i = threadIdx.x; i < LOC_SLOTS; i += blockDim.x) {
     s_key[i] = EMPTY;
     s_cnt[i] = 0;
@@ -116,12 +113,18 @@ __global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol
     }
 }
 
+__global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol, int ktype, uint64_t n) {
+  __shared__ unsigned long long s_key[LOC_SLOTS];
+  __shared__ uint32_t s_cnt[LOC_SLOTS];
+  build_count(t, keycol, ktype, n, s_key, s_cnt);
+}
+
 // ---------------------------------------------------------------------------
 // Vertex-id keys below a bound of a few times the build rows need no hash: an
 // array indexed by the key holds each key's count (and build row), in L2 where the
 // hash table of 10M keys is 537 MB of HBM.  The largest build key is found on the
 // device and every kernel checks it against the bound, so the host waits for
-// nothing; above the bound the kernels return and the hash kernels run.  Count of
+// nothing; above the bound the count's kernels use the hash table instead.  Count of
 // 10M x 10M Zipf-skewed keys below 10M: 432 -> 117 us, of which counting the build
 // keys (shared-memory atomics) 71.
 __global__ void __launch_bounds__(256) k_key_max(const uint32_t *__restrict__ keys, uint64_t n, uint32_t *ctl) {
@@ -137,29 +140,33 @@ __global__ void __launch_bounds__(256) k_key_max(const uint32_t *__restrict__ ke
   if ((threadIdx.x & 31) == 0) atomicMax(ctl, m);
 }
 
-__global__ void __launch_bounds__(256) k_direct_clear(Direct d) {
-  if (!direct_ok(d)) return;
-  const uint32_t n4 = d.ctl[0] / 4 + 1;  // the bound is a multiple of four
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x)
-    reinterpret_cast<uint4 *>(d.cnt)[i] = make_uint4(0, 0, 0, 0);
-}
-
-// The hash table's clear, when it is needed after all.
-__global__ void __launch_bounds__(256) k_hash_clear(Table t, Direct d) {
-  if (direct_ok(d)) return;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= t.cap; i += (uint64_t)gridDim.x * blockDim.x) {
-    t.keys[i] = EMPTY;
-    t.cnt[i] = 0;
+// Clears the part of the arrays that the keys use, or the hash table that takes
+// their place (when there is one).
+__global__ void __launch_bounds__(256) k_direct_clear(Direct d, Table t) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (direct_ok(d)) {
+    const uint32_t n4 = d.ctl[0] / 4 + 1;  // the bound is a multiple of four
+    for (uint64_t i = i0; i < n4; i += stride) reinterpret_cast<uint4 *>(d.cnt)[i] = make_uint4(0, 0, 0, 0);
+  } else if (t.keys) {
+    for (uint64_t i = i0; i <= t.cap; i += stride) {
+      t.keys[i] = EMPTY;
+      t.cnt[i] = 0;
+    }
   }
 }
 
 // Counts per key.  As in k_build_count a block first counts in a table of its own
 // in shared memory (Zipf-skewed columns send an eighth of the rows to one key), with
 // one probe: a key that finds the slot taken adds to the array in L2.
-constexpr int DIRECT_SLOTS = 4096;
-__global__ void __launch_bounds__(512) k_direct_count(Direct d, const uint32_t *__restrict__ keys, uint64_t n) {
-  if (!direct_ok(d)) return;
-  __shared__ uint32_t s_key[DIRECT_SLOTS], s_cnt[DIRECT_SLOTS];
+constexpr int DIRECT_SLOTS = LOC_SLOTS;
+__global__ void __launch_bounds__(512) k_direct_count(Direct d, Table t, const uint32_t *__restrict__ keys, uint64_t n) {
+  __shared__ unsigned long long s_wide[LOC_SLOTS];
+  __shared__ uint32_t s_cnt[LOC_SLOTS];
+  if (!direct_ok(d)) {
+    build_count(t, keys, VS_T_VID, n, s_wide, s_cnt);
+    return;
+  }
+  uint32_t *s_key = reinterpret_cast<uint32_t *>(s_wide);
   for (int i = threadIdx.x; i < DIRECT_SLOTS; i += blockDim.x) {
     s_key[i] = 0xffffffffu;  // not a key below the bound
     s_cnt[i] = 0;
@@ -190,12 +197,19 @@ __global__ void __launch_bounds__(512) k_direct_count(Direct d, const uint32_t *
 }
 
 // Sum of the counts of the probe keys.
-__global__ void __launch_bounds__(256) k_direct_probe(Direct d, const uint32_t *__restrict__ keys, uint64_t n,
-                                                      unsigned long long *total) {
-  if (!direct_ok(d)) return;
+__global__ void __launch_bounds__(256) k_direct_probe(Direct d, Table t, const uint32_t *__restrict__ keys,
+                                                      uint64_t n, unsigned long long *total) {
   const uint32_t top = d.ctl[0];
   unsigned long long s = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (!direct_ok(d)) {
+    for (uint64_t i = i0; i < n; i += stride) {
+      const uint64_t slot = ht_find(t, keys[i]);
+      if (slot != ~0ull) s += t.cnt[slot];
+    }
+    block_add(s, total);
+    return;
+  }
   const uint4 *k4 = reinterpret_cast<const uint4 *>(keys);
   for (uint64_t i = i0; i < n / 4; i += stride) {
     const uint4 k = __ldg(k4 + i);
@@ -273,8 +287,7 @@ __global__ void k_scatter(Table t, const uint32_t *slot_of, uint64_t n, uint32_t
 
 // Probe: matches per probe row (and the slot), total into *total.
 __global__ void k_probe(Table t, const void *keycol, int ktype, uint64_t n,
-                        unsigned long long *pcnt, uint32_t *pslot, unsigned long long *total, Direct d) {
-  if (d.ctl && direct_ok(d)) return;
+                        unsigned long long *pcnt, uint32_t *pslot, unsigned long long *total) {
   unsigned long long s = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -553,7 +566,7 @@ uint32_t direct_bound(uint64_t n_build) {
 
 // The direct arrays of the build keys, and a total before their control words (one
 // 16-byte block, read back at once).  VS_ERR_OOM leaves nothing behind.
-int direct_alloc(Scratch &sc, const uint32_t *keys, uint64_t n, uint32_t bound, bool rows, Direct *d,
+int direct_alloc(Scratch &sc, const uint32_t *keys, uint64_t n, uint32_t bound, bool rows, const Table &t, Direct *d,
                  unsigned long long **total) {
   d->bound = bound;
   d->row = nullptr;
@@ -563,7 +576,7 @@ int direct_alloc(Scratch &sc, const uint32_t *keys, uint64_t n, uint32_t bound, 
   if (rows) VS_TRY(sc.get(&d->row, bound));
   VS_CK(cudaMemsetAsync(*total, 0, 16, sc.st));
   { k_key_max<<<std::min(grid_for((n + 3) / 4), 4 * sm_count()), 256, 0, sc.st>>>(keys, n, d->ctl); vs::note_launch(); }
-  { k_direct_clear<<<std::min(grid_for((bound + 3) / 4), 8 * sm_count()), 256, 0, sc.st>>>(*d); vs::note_launch(); }
+  { k_direct_clear<<<std::min(grid_for((bound + 3) / 4), 8 * sm_count()), 256, 0, sc.st>>>(*d, t); vs::note_launch(); }
   return VS_OK;
 }
 
@@ -648,7 +661,7 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   const bool build_a = a.f->nrows < b.f->nrows;
   const FlatSide &bd = build_a ? a : b, &pr = build_a ? b : a;
   Scratch sc{st};
-  Table t;
+  Table t{};
   const uint64_t nb = bd.f->nrows, np = pr.f->nrows;
   const bool vid = bd.f->types[bd.key] == VS_T_VID;
   const uint32_t *bkeys = (const uint32_t *)bd.f->cols[bd.key], *pkeys = (const uint32_t *)pr.f->cols[pr.key];
@@ -659,14 +672,11 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
     unsigned long long *d_total = nullptr;
     const int rc = only_count ? table_alloc(sc, nb, false, false, &t, false) : VS_OK;
     if (rc != VS_OK) return rc;
-    const int dc = direct_alloc(dsc, bkeys, nb, bound, !only_count, &d, &d_total);
+    const int dc = direct_alloc(dsc, bkeys, nb, bound, !only_count, t, &d, &d_total);
     if (dc != VS_OK && dc != VS_ERR_OOM) return dc;
     if (dc == VS_OK && only_count) {  // the arrays, or the hash table in their place
-      { k_direct_count<<<std::min(grid_for((nb + 3) / 4, 512), 2 * sm_count()), 512, 0, st>>>(d, bkeys, nb); vs::note_launch(); }
-      { k_direct_probe<<<grid_for((np + 3) / 4), 256, 0, st>>>(d, pkeys, np, d_total); vs::note_launch(); }
-      { k_hash_clear<<<grid_for(t.cap), 256, 0, st>>>(t, d); vs::note_launch(); }
-      { k_build_count<<<std::min(grid_for(nb), 4 * sm_count()), 256, 0, st>>>(t, bkeys, VS_T_VID, nb, d); vs::note_launch(); }
-      { k_probe<<<grid_for(np), 256, 0, st>>>(t, pkeys, VS_T_VID, np, nullptr, nullptr, d_total, d); vs::note_launch(); }
+      { k_direct_count<<<std::min(grid_for((nb + 3) / 4, 512), 2 * sm_count()), 512, 0, st>>>(d, t, bkeys, nb); vs::note_launch(); }
+      { k_direct_probe<<<grid_for((np + 3) / 4), 256, 0, st>>>(d, t, pkeys, np, d_total); vs::note_launch(); }
       VS_CK(cudaGetLastError());
       return read_total(d_total, count, st);
     }
@@ -686,7 +696,7 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   if (!only_count) VS_TRY(sc.get(&slot_of, bd.f->nrows));
   if (bd.f->nrows && only_count)
     { k_build_count<<<std::min(grid_for(bd.f->nrows), 4 * sm_count()), 256, 0, st>>>(
-          t, bd.f->cols[bd.key], bd.f->types[bd.key], bd.f->nrows, Direct{}); vs::note_launch(); }
+          t, bd.f->cols[bd.key], bd.f->types[bd.key], bd.f->nrows); vs::note_launch(); }
   else if (bd.f->nrows)
     { k_build<<<grid_for(bd.f->nrows), 256, 0, st>>>(t, bd.f->cols[bd.key], bd.f->types[bd.key],
                                                    bd.f->nrows, slot_of); vs::note_launch(); }
@@ -696,7 +706,7 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   if (only_count) {
     if (pr.f->nrows)
       { k_probe<<<grid_for(pr.f->nrows), 256, 0, st>>>(t, pr.f->cols[pr.key], pr.f->types[pr.key],
-                                                     pr.f->nrows, nullptr, nullptr, d_total, Direct{}); vs::note_launch(); }
+                                                     pr.f->nrows, nullptr, nullptr, d_total); vs::note_launch(); }
     VS_CK(cudaGetLastError());
     return read_total(d_total, count, st);
   }
@@ -712,7 +722,7 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   VS_TRY(sc.get(&pslot, pr.f->nrows));
   if (pr.f->nrows)
     { k_probe<<<grid_for(pr.f->nrows), 256, 0, st>>>(t, pr.f->cols[pr.key], pr.f->types[pr.key],
-                                                   pr.f->nrows, pcnt, pslot, d_total, Direct{}); vs::note_launch(); }
+                                                   pr.f->nrows, pcnt, pslot, d_total); vs::note_launch(); }
   VS_TRY(exclusive_scan_u64(pcnt, poff, pr.f->nrows, st));
   uint64_t total = 0;
   VS_TRY(read_total(d_total, &total, st));
@@ -974,7 +984,7 @@ int vs_hash_join_count_noalloc(const void *keys_a, uint64_t na, const void *keys
   unsigned long long *total = base + 2 * (NOALLOC_SLOTS + 1);
   { k_noalloc_clear<<<grid_for(t.cap + 1), 256, 0, st>>>(t.keys, t.cnt, total, t.cap); vs::note_launch(); }
   if (nbld) { k_build<<<grid_for(nbld), 256, 0, st>>>(t, bk, key_type, nbld, nullptr); vs::note_launch(); }
-  if (nprb) { k_probe<<<grid_for(nprb), 256, 0, st>>>(t, pk, key_type, nprb, nullptr, nullptr, total, Direct{}); vs::note_launch(); }
+  if (nprb) { k_probe<<<grid_for(nprb), 256, 0, st>>>(t, pk, key_type, nprb, nullptr, nullptr, total); vs::note_launch(); }
   VS_CK(cudaGetLastError());
   VS_CK(cudaMemcpyAsync(count, total, sizeof(unsigned long long), cudaMemcpyDefault, st));
   VS_CK(cudaStreamSynchronize(st));
