@@ -92,6 +92,28 @@ __global__ void k_clear_flagged(uint4 *__restrict__ buf, uint32_t *__restrict__ 
     const uint4 f = g < nq ? flag4[g] : make_uint4(0, 0, 0, 0);
     if (f.x | f.y | f.z | f.w) flag4[g] = make_uint4(0, 0, 0, 0);
     const uint32_t fv[4] = {f.x, f.y, f.z, f.w};
+    if (Q <= 8) {
+      // narrow rows: the 128 rows are one range, its flagged cells stored by all
+      // lanes (a row at a time left most lanes idle: 1M rows of 16 bytes 43 -> 6 us)
+      unsigned m[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) m[k] = __ballot_sync(FULL, fv[k] == 1);
+      if (!(m[0] | m[1] | m[2] | m[3])) continue;
+      uint4 *rows = buf + (size_t)base * 4 * Q;
+      uint32_t r = lane / Q, q = lane % Q;  // cell lane + 32 i: row r, uint4 q
+      const uint32_t dr = 32 / Q, dq = 32 % Q;
+      for (uint32_t i = lane; i < 128 * Q; i += 32) {
+        const unsigned mk = (r & 2) ? (r & 1 ? m[3] : m[2]) : (r & 1 ? m[1] : m[0]);
+        if (mk >> (r >> 2) & 1u) rows[i] = make_uint4(0, 0, 0, 0);
+        r += dr;
+        q += dq;
+        if (q >= Q) {
+          q -= Q;
+          r++;
+        }
+      }
+      continue;
+    }
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       unsigned m = __ballot_sync(FULL, fv[k] == 1);
@@ -199,27 +221,20 @@ __global__ void k_copy_layer(const uint4 *__restrict__ buf, const uint32_t *__re
 
 // Per-hop row masks of batched queries from per-row hop limits: word w of
 // hop h has bit r set when row 64w+r may still grow at hop h.
-__global__ void k_row_mask(const uint8_t *__restrict__ lim, uint32_t n, uint32_t K, uint32_t W,
-                           uint64_t *__restrict__ hmask, uint32_t *rowk) {
-  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= W) return;
-  uint32_t kmax = 0, over = 0;
-  for (uint32_t r = 0; r < 64; r++) {
-    const uint32_t i = w * 64 + r;
-    const uint32_t l = i < n ? lim[i] : 0u;
-    over |= l > K;
-    kmax = max(kmax, min(l, K));
-  }
+__global__ void __launch_bounds__(256) k_row_mask(const uint8_t *__restrict__ lim, uint32_t n, uint32_t K, uint32_t W,
+                                                  uint64_t *__restrict__ hmask, uint32_t *rowk) {
+  const uint32_t lane = threadIdx.x & 31, w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= W) return;  // a warp per word: a lane's two rows, a ballot per hop
+  const uint32_t i = w * 64 + lane, j = i + 32;
+  const uint32_t a = i < n ? lim[i] : 0u, b = j < n ? lim[j] : 0u, top = __reduce_max_sync(FULL, max(a, b));
   for (uint32_t h = 0; h <= K; h++) {
-    uint64_t m = 0;
-    for (uint32_t r = 0; h > 0 && r < 64; r++) {
-      const uint32_t i = w * 64 + r;
-      if (i < n && min((uint32_t)lim[i], K) >= h) m |= 1ull << r;
-    }
-    hmask[(size_t)h * W + w] = m;
+    const unsigned lo = __ballot_sync(FULL, h && a >= h), hi = __ballot_sync(FULL, h && b >= h);
+    if (lane == 0) hmask[(size_t)h * W + w] = (uint64_t)lo | (uint64_t)hi << 32;
   }
-  if (kmax) atomicMax(&rowk[0], kmax);
-  if (over) rowk[1] = 1;
+  if (lane == 0) {
+    if (top) atomicMax(&rowk[0], min(top, K));
+    if (top > K) rowk[1] = 1;
+  }
 }
 
 // One block of 256 threads: early-stop checks of hop h-1 (VExpand::after_child,
@@ -391,7 +406,7 @@ __global__ void k_hop_stats(const uint32_t *__restrict__ flagF, Lists out, uint3
 // out-degrees (k_pscan*) lays all their out-lists end to end, and each warp
 // takes fixed chunks of that edge range, so a pair on a 50k-degree hub is
 // spread over many warps instead of serialising one.
-constexpr int SPARSE_CHUNK = 256;  // edges per warp task
+constexpr int SPARSE_CHUNK = 256;  // edges per warp task at most
 constexpr int SPARSE_K = 2;        // edges per lane per round
 
 // Pairs the SPARSE hop h scans (0 when the hop runs another strategy).
@@ -520,11 +535,14 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
   const unsigned long long T = a.doff[np];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t nchunks = (T + SPARSE_CHUNK - 1) / SPARSE_CHUNK;
+  // one round of edges per task while that leaves warps idle (a task's rounds are
+  // one dependent chain of misses after the other: 10k edges 30 -> 15 us)
+  const uint32_t chunk = T < warps * 32 * SPARSE_K * 2 ? 32 * SPARSE_K : SPARSE_CHUNK;
+  const uint64_t nchunks = (T + chunk - 1) / chunk;
   unsigned long long nb = 0, nv = 0, pe = 0, ae = 0;
   for (uint64_t ck = (uint64_t)blockIdx.x * (blockDim.x >> 5) + wib; ck < nchunks; ck += warps) {
-    const unsigned long long e0 = ck * SPARSE_CHUNK;
-    const unsigned long long e1 = min(e0 + SPARSE_CHUNK, T);
+    const unsigned long long e0 = ck * chunk;
+    const unsigned long long e1 = min(e0 + chunk, T);
     // pairs owning the chunk's first and last edge: largest p with doff[p] <= e,
     // both found at once by a 16-way search per half-warp
     uint64_t plo, phi;
@@ -3092,7 +3110,7 @@ int vs_expand_plan_set_row_limits_device(vs_expand_plan *pl, const uint8_t *row_
   }
   VS_CK(cudaMemsetAsync(pl->rowk, 0, 2 * sizeof(uint32_t), st));
   const uint32_t W = pl->W;
-  { k_row_mask<<<(W + 255) / 256, 256, 0, st>>>(row_kmax, n, pl->p.k_max, W, pl->hmask, pl->rowk); vs::note_launch(); }
+  { k_row_mask<<<(W + 7) / 8, 256, 0, st>>>(row_kmax, n, pl->p.k_max, W, pl->hmask, pl->rowk); vs::note_launch(); }
   VS_CK(cudaGetLastError());
   pl->use_hmask = true;
   return VS_OK;
