@@ -71,15 +71,9 @@ __device__ __forceinline__ void block_add(unsigned long long v, unsigned long lo
 }
 
 // ---------------------------------------------------------------------------
-// Run start: clear both frontier buffers (flagged rows only) and the counters.
-__global__ void k_clear_flagged(uint4 *__restrict__ buf, uint32_t *__restrict__ flag, uint32_t V,
-                                uint32_t Q, const Ctr *ctr, int h, int mode) {
-  // mode 0: unconditional; mode 1: only when hop h runs SPARSE or PUSH, or a
-  // multi-slice PULL (those write with atomics / partially and need clean rows)
-  if (mode == 1) {
-    int s = ctr->hop[h].strategy;
-    if (!(s == ST_SPARSE || s == ST_PUSH || (s == ST_PULL && ctr->multislice))) return;
-  }
+// Zero the flagged rows of a buffer and their flags.
+__device__ __forceinline__ void clear_flagged(uint4 *__restrict__ buf, uint32_t *__restrict__ flag, uint32_t V,
+                                              uint32_t Q) {
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   // four flags per lane (16-byte loads of the 16-byte aligned flag array):
@@ -134,6 +128,17 @@ __global__ void k_clear_flagged(uint4 *__restrict__ buf, uint32_t *__restrict__ 
       if (lane == 0 && f) flag[v] = 0;
     }
   }
+}
+
+// Run start: the rows the previous run left in both frontier buffers and in the
+// result (NULL: none), and the counter block (n 16-byte words).
+__global__ void __launch_bounds__(256) k_run_start(uint4 *buf0, uint32_t *flag0, uint4 *buf1, uint32_t *flag1, uint4 *res,
+                                                   uint32_t *resflag, uint32_t V, uint32_t Q, uint4 *ctr, uint32_t n) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    ctr[i] = make_uint4(0, 0, 0, 0);
+  clear_flagged(buf0, flag0, V, Q);
+  clear_flagged(buf1, flag1, V, Q);
+  if (res) clear_flagged(res, resflag, V, Q);
 }
 
 // Layer 0 (ExpandStatus::init_first_m_layer, expand_impl.hh:252-277).
@@ -336,34 +341,35 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
     // from words (10 on a last hop, which keeps no lists), 1.5 per id read from
     // slots and 350 per target row then searched for bits (none on a last hop),
     // and about twice the dense price for a row too long for a slot.
-    bool sp = false;
-    const bool counted = prev.strategy == ST_PULL;  // ... its layer's words, slots and degrees
-    const double act = (double)prev.active_vertices, V = (double)a.V, E = (double)a.E * (a.both ? 2 : 1);
-    const double ids = prev.strategy == ST_PUSH ? E * (double)prev.new_bits / V : (double)prev.pair_edges;
-    double rows, longs = 0;  // edges leaving non-empty rows, and rows too long for a slot
-    if (counted) {
-      rows = (double)prev.row_out;
-      longs = rows - (double)prev.short_out;
-    } else {
-      rows = ids * act / fmax(1.0, (double)prev.new_bits);
-    }
-    const double t_long = 1.6 * a.W * longs;
-    const double t_words = 12.5 * E + (a.last ? 10.0 : 21.0) * ids + t_long;
-    const double t_slots = 12.5 * E + 1.5 * fmin(ids, 15.0 * (double)prev.short_out) +
-                           (a.last ? 0.0 : 350.0 * fmin(V, ids)) + t_long;
-    const bool slots = counted && t_slots < t_words;
+    bool sp = false, slots = false, lng = false;
     if (s_choice == ST_PULL && a.short_min > 0 && !c->multislice) {
+      const bool counted = prev.strategy == ST_PULL;  // ... its layer's words, slots and degrees
+      const float act = (float)prev.active_vertices, V = (float)a.V, E = (float)a.E * (a.both ? 2 : 1), W = (float)a.W;
+      const float ids = prev.strategy == ST_PUSH ? E * ((float)prev.new_bits / V) : (float)prev.pair_edges;
+      float rows, longs = 0, so = 0;  // edges leaving non-empty rows, rows too long for a slot, and rows within one
+      if (counted) {
+        rows = (float)prev.row_out;
+        so = (float)prev.short_out;
+        longs = (float)(prev.row_out - prev.short_out);
+      } else {
+        rows = ids * (act / fmaxf(1.f, (float)prev.new_bits));
+      }
+      const float t_long = 1.6f * W * longs;
+      const float t_words = 12.5f * E + (a.last ? 10.f : 21.f) * ids + t_long;
+      const float t_slots = 12.5f * E + 1.5f * fminf(ids, 15.f * so) + (a.last ? 0.f : 350.f * fminf(V, ids)) + t_long;
+      slots = counted && t_slots < t_words;
       if (a.short_min > 1.0) {
         sp = true;
-      } else if (!counted || (double)(prev.short_rows & 0xFFFFFFFFull) >= a.short_min * act) {
-        const double flag = act >= 0.9 * V ? 6.0 : a.W <= 8 ? 7.0 : a.W <= 16 ? 8.0 : a.W <= 32 ? 12.0 : 18.0;
-        sp = (slots ? t_slots : t_words) < 0.9 * (flag * E + 0.8 * a.W * rows);
+      } else if (!counted || (float)(prev.short_rows & 0xFFFFFFFFull) >= (float)a.short_min * act) {
+        const float flag = act >= 0.9f * V ? 6.f : a.W <= 8 ? 7.f : a.W <= 16 ? 8.f : a.W <= 32 ? 12.f : 18.f;
+        sp = (slots ? t_slots : t_words) < 0.9f * (flag * E + 0.8f * W * rows);
       }
+      // more than half a slot of ids per target: its new row will often be long
+      lng = ids > 1.2f * V * (a.W <= 64 ? 16 : a.W <= 128 ? 32 : 64);
     }
     cur.short_pull = sp;
     cur.short_slots = sp && slots;
-    // more than half a slot of ids per target: its new row will often be long
-    cur.short_long = ids > 1.2 * V * (a.W <= 64 ? 16 : a.W <= 128 ? 32 : 64);
+    cur.short_long = sp && lng;
   }
 }
 
@@ -403,7 +409,7 @@ __global__ void k_hop_stats(const uint32_t *__restrict__ flagF, Lists out, uint3
 // bit i.  Shortest dedups through the visited bit (atomicOr returns the old
 // word), Any through the next-layer bit.  New pairs form layer h's list.
 // The work is balanced over edges, not pairs: a prefix sum of the pairs'
-// out-degrees (k_pscan*) lays all their out-lists end to end, and each warp
+// out-degrees (k_pscan) lays all their out-lists end to end, and each warp
 // takes fixed chunks of that edge range, so a pair on a 50k-degree hub is
 // spread over many warps instead of serialising one.
 constexpr int SPARSE_CHUNK = 256;  // edges per warp task at most
@@ -416,77 +422,81 @@ __device__ __forceinline__ uint64_t scan_len(const Ctr *ctr, int h, uint64_t cap
   return npr < cap ? npr : cap;
 }
 
-__global__ void k_pscan1(const unsigned long long *__restrict__ pdeg, unsigned long long *__restrict__ doff,
-                         unsigned long long *__restrict__ bsum, const Ctr *ctr, int h, uint64_t cap) {
-  const uint64_t np = scan_len(ctr, h, cap);
-  if (!np) return;
-  __shared__ unsigned long long wt[8];
+// Exclusive prefix of the pairs' out-degrees in two levels, in one launch: doff
+// within tiles of 1,024 pairs, and by the block that finishes last the tiles' starts
+// (bsum, the total after them).  A reader adds the two, which costs a load beside
+// the one it waits for anyway and saves a pass and two launches.
+__device__ __forceinline__ unsigned long long block_scan4(unsigned long long (&v)[4], unsigned long long *wt) {
+  // v becomes the exclusive prefix over the block's 1,024 values; returns their sum
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  for (uint64_t b = blockIdx.x; b * 1024 < np; b += gridDim.x) {
-    const uint64_t base = b * 1024;
-    unsigned long long v[4], run = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const uint64_t i = base + (uint64_t)t * 4 + k;
-      v[k] = i < np ? pdeg[i] : 0ull;
-      run += v[k];
-    }
-    unsigned long long incl = run;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long y = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) wt[w] = incl;
-    __syncthreads();
-    unsigned long long pre = 0;
-    for (int k = 0; k < w; k++) pre += wt[k];
-    pre += incl - run;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const uint64_t i = base + (uint64_t)t * 4 + k;
-      if (i < np) doff[i] = pre;
-      pre += v[k];
-    }
-    if (t == 255) bsum[b] = pre;  // block total (pre ends at the block's inclusive sum)
-    __syncthreads();
+  unsigned long long run = v[0] + v[1] + v[2] + v[3], incl = run;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
   }
-}
-
-__global__ void k_pscan2(unsigned long long *__restrict__ bsum, unsigned long long *__restrict__ doff,
-                         const Ctr *ctr, int h, uint64_t cap) {
-  const uint64_t np = scan_len(ctr, h, cap);
-  if (!np) return;
-  const uint64_t nb = (np + 1023) / 1024;
-  __shared__ unsigned long long carry, wt[32];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  if (t == 0) carry = 0;
+  if (lane == 31) wt[w] = incl;
   __syncthreads();
-  for (uint64_t b0 = 0; b0 < nb; b0 += blockDim.x) {
-    const uint64_t i = b0 + t;
-    const unsigned long long x = i < nb ? bsum[i] : 0ull;
-    unsigned long long xi = x;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long y = __shfl_up_sync(FULL, xi, o);
-      if (lane >= o) xi += y;
-    }
-    if (lane == 31) wt[w] = xi;
-    __syncthreads();
-    unsigned long long pre = carry;
-    for (int k = 0; k < w; k++) pre += wt[k];
-    if (i < nb) bsum[i] = pre + xi - x;
-    __syncthreads();
-    if (t == blockDim.x - 1) carry = pre + xi;
-    __syncthreads();
+  unsigned long long pre = 0, sum = 0;
+  for (int k = 0; k < 8; k++) {
+    if (k < w) pre += wt[k];
+    sum += wt[k];
   }
-  if (t == 0) doff[np] = carry;
+  pre += incl - run;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const unsigned long long x = v[k];
+    v[k] = pre;
+    pre += x;
+  }
+  __syncthreads();
+  return sum;
 }
 
-__global__ void k_pscan3(unsigned long long *__restrict__ doff, const unsigned long long *__restrict__ bsum,
-                         const Ctr *ctr, int h, uint64_t cap) {
+__global__ void __launch_bounds__(256) k_pscan(const unsigned long long *__restrict__ pdeg,
+                                               unsigned long long *__restrict__ doff,
+                                               unsigned long long *__restrict__ bsum, Ctr *ctr, int h, uint64_t cap) {
   const uint64_t np = scan_len(ctr, h, cap);
-  if (!np) return;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < np; i += (uint64_t)gridDim.x * blockDim.x)
-    doff[i] += bsum[i / 1024];
+  const uint64_t nb = (np + 1023) / 1024;
+  if (blockIdx.x >= nb) return;
+  __shared__ unsigned long long wt[8];
+  __shared__ bool s_last;
+  const int t = threadIdx.x;
+  unsigned long long v[4];
+  for (uint64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    const uint64_t base = b * 1024 + (uint64_t)t * 4;
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = base + k < np ? pdeg[base + k] : 0ull;
+    const unsigned long long sum = block_scan4(v, wt);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (base + k < np) doff[base + k] = v[k];
+    if (t == 0) bsum[b] = sum;
+  }
+  __threadfence();
+  __syncthreads();
+  const uint64_t blocks = nb < gridDim.x ? nb : gridDim.x;
+  if (t == 0) s_last = atomicAdd(&ctr->hop[h].scan_done, 1u) == blocks - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  unsigned long long carry = 0;
+  for (uint64_t b0 = 0; b0 < nb; b0 += 1024) {
+    const uint64_t base = b0 + (uint64_t)t * 4;
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = base + k < nb ? __ldcg(bsum + base + k) : 0ull;
+    const unsigned long long sum = block_scan4(v, wt);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (base + k < nb) bsum[base + k] = carry + v[k];
+    carry += sum;
+  }
+  if (t == 0) bsum[nb] = carry;
+}
+
+// First edge of pair p in the layer's edge range.
+__device__ __forceinline__ unsigned long long pair_start(const unsigned long long *__restrict__ doff,
+                                                         const unsigned long long *__restrict__ bsum, uint64_t p) {
+  return doff[p] + bsum[p >> 10];
 }
 
 __device__ __forceinline__ unsigned long long out_degree(const Lists &L, uint32_t v) {
@@ -495,12 +505,13 @@ __device__ __forceinline__ unsigned long long out_degree(const Lists &L, uint32_
   return d;
 }
 
-// Largest p in [0, np) with doff[p] <= x for x0 (lanes 0-15) and x1 (lanes
-// 16-31), doff ascending with doff[0] = 0 <= x: each step a half-warp probes
+// Largest p in [0, np) with pair_start(p) <= x for x0 (lanes 0-15) and x1 (lanes
+// 16-31), starts ascending from 0 <= x: each step a half-warp probes
 // 15 positions spread over its range at once and keeps the part between the
 // last probe at or below x and the next, so a range shrinks 16-fold per
 // dependent load instead of 2-fold.  Every lane receives both answers.
-__device__ __forceinline__ void owner_pairs(const unsigned long long *__restrict__ doff, uint64_t np,
+__device__ __forceinline__ void owner_pairs(const unsigned long long *__restrict__ doff,
+                                            const unsigned long long *__restrict__ bsum, uint64_t np,
                                             unsigned long long x0, unsigned long long x1, int lane, uint64_t &p0,
                                             uint64_t &p1) {
   const int hl = lane & 15;
@@ -509,7 +520,7 @@ __device__ __forceinline__ void owner_pairs(const unsigned long long *__restrict
   while (__any_sync(FULL, hi - lo > 1)) {
     const uint64_t span = hi - lo;
     const uint64_t pos = lo + (span * (uint64_t)hl + 15) / 16;  // probe hl; probe 0 is lo itself
-    const bool ok = span > 1 && (hl == 0 || (pos < hi && doff[pos] <= x));
+    const bool ok = span > 1 && (hl == 0 || (pos < hi && pair_start(doff, bsum, pos) <= x));
     const unsigned b = __ballot_sync(FULL, ok);
     const unsigned half = lane < 16 ? (b & 0xFFFFu) : (b >> 16);
     if (span > 1) {
@@ -532,7 +543,7 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
   __syncthreads();
   const unsigned long long np_raw = c->hop[a.h - 1].pairs;
   const uint64_t np = np_raw < a.cap ? np_raw : a.cap;
-  const unsigned long long T = a.doff[np];
+  const unsigned long long T = np ? a.bsum[(np + 1023) / 1024] : 0ull;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   // one round of edges per task while that leaves warps idle (a task's rounds are
@@ -546,7 +557,7 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
     // pairs owning the chunk's first and last edge: largest p with doff[p] <= e,
     // both found at once by a 16-way search per half-warp
     uint64_t plo, phi;
-    owner_pairs(a.doff, np, e0, e1 - 1, lane, plo, phi);
+    owner_pairs(a.doff, a.bsum, np, e0, e1 - 1, lane, plo, phi);
     uint32_t nloc = 0;  // new pairs of this chunk so far (s_new)
     // the chunk's pairs 32 at a time: lane j holds pair g0 + j (its first
     // edge, source id, and its vertex's list starts and first-list length),
@@ -557,7 +568,7 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
       uint32_t pi = 0;
       int64_t pb0 = 0, pd0 = 0, pb1 = 0;
       if (g0 + lane <= phi) {
-        dj = a.doff[g0 + lane];
+        dj = pair_start(a.doff, a.bsum, g0 + lane);
         const uint2 pr = a.pin[g0 + lane];
         pi = pr.y;
         pb0 = a.out.off[0][pr.x];
@@ -569,7 +580,7 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
       const unsigned long long gs = d0j > e0 ? d0j : e0;
       unsigned long long ge = e1;
       if (g0 + 32 <= phi) {
-        const unsigned long long nx = a.doff[g0 + 32];
+        const unsigned long long nx = pair_start(a.doff, a.bsum, g0 + 32);
         ge = nx < e1 ? nx : e1;
       }
       // SPARSE_K edges per lane per round, each phase issued for all of them
@@ -1844,7 +1855,7 @@ __global__ void __launch_bounds__(SH_WARPS * 32, 4) k_pull_short(const __grid_co
 // Rows of layer h-1 left in their slots (flag 2), written out whole when hop
 // h reads rows: a dense PULL or a PUSH (a short-mode PULL reads the slots).
 // prev_virt: the PULL of hop h-1 was allowed to leave rows in their slots.
-__global__ void k_materialize(uint32_t *__restrict__ flagF, uint4 *__restrict__ F, uint32_t V, uint32_t Q,
+__device__ __forceinline__ void materialize(uint32_t *__restrict__ flagF, uint4 *__restrict__ F, uint32_t V, uint32_t Q,
                               const uint16_t *__restrict__ slots, uint32_t slot_n, const Ctr *ctr, int h,
                               int prev_virt) {
   const HopCtr &p = ctr->hop[h - 1], &c = ctr->hop[h];
@@ -1927,7 +1938,7 @@ __device__ __forceinline__ bool pairs_build(const Ctr *c, int h) {
 // short-row index from rows (the list overflowed); mode 1, after the index
 // was built from the pairs: the pairs of rows too long for a slot, which a
 // short-mode PULL gathers whole.  SPARSE reads only pairs.
-__global__ void k_pairs_rows(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ cnt,
+__device__ __forceinline__ void pairs_rows(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ cnt,
                              unsigned long long *__restrict__ N, uint32_t W, uint32_t slot_n, uint64_t cap,
                              const Ctr *ctr, int h, int mode) {
   if (ctr->hop[h - 1].strategy != ST_SPARSE) return;
@@ -1941,11 +1952,6 @@ __global__ void k_pairs_rows(const uint2 *__restrict__ pairs, const uint32_t *__
     if (mode == 1 && cnt[pr.x] < slot_n) continue;
     atomicOr(&N[(size_t)pr.x * W + (pr.y >> 6)], 1ull << (pr.y & 63));
   }
-}
-
-__global__ void k_pairs_zero(uint32_t *__restrict__ cnt, uint32_t V, const Ctr *ctr, int h) {
-  if (!pairs_build(ctr, h)) return;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) cnt[v] = 0;
 }
 
 // every pair's source id into its vertex's slot (entries 1.., in any order)
@@ -1962,7 +1968,7 @@ __global__ void k_pairs_slots(const uint2 *__restrict__ pairs, uint32_t *__restr
 }
 
 // the tiny word of every vertex from its pair count (0 for an empty row)
-__global__ void k_pairs_words(const uint32_t *__restrict__ flagF, const uint32_t *__restrict__ cnt,
+__device__ __forceinline__ void pairs_words(const uint32_t *__restrict__ flagF, const uint32_t *__restrict__ cnt,
                               Tiny *__restrict__ tiny, uint16_t *__restrict__ slots, uint32_t slot_n, uint32_t V,
                               const Ctr *ctr, int h) {
   if (!pairs_build(ctr, h)) return;
@@ -1982,7 +1988,7 @@ __global__ void k_pairs_words(const uint32_t *__restrict__ flagF, const uint32_t
 // layer was written by PUSH or by a SPARSE hop whose pair list overflowed: a warp per
 // flagged row counts its bits and writes its word (and slot); every other
 // vertex gets the count 0.
-__global__ void k_slot_build(const uint32_t *__restrict__ flagF, const uint4 *__restrict__ F, uint32_t V,
+__device__ __forceinline__ void slot_build(const uint32_t *__restrict__ flagF, const uint4 *__restrict__ F, uint32_t V,
                              uint32_t Q, Tiny *__restrict__ tiny, uint16_t *__restrict__ slots, uint32_t slot_n,
                              const Ctr *ctr, int h) {
   if (ctr->hop[h].strategy != ST_PULL || !ctr->hop[h].short_pull || ctr->hop[h - 1].strategy == ST_PULL ||
@@ -2065,6 +2071,46 @@ __global__ void k_slot_build(const uint32_t *__restrict__ flagF, const uint4 *__
       }
     }
   }
+}
+
+// Before hop h runs, in one launch: the rows of layer h-1 that its hop left in its
+// pair list (deferred) or in their slots (virt), if hop h reads rows; the rows of
+// layer h's buffer that an older layer left, if hop h needs them clean (SPARSE and
+// PUSH write with atomics, a multi-slice PULL in parts; any PULL at hop 1 and later
+// overwrites them itself); the pair counts of the short-row index.
+struct PrepArgs {
+  const uint2 *pairs;
+  uint32_t *cnt;
+  unsigned long long *F;
+  uint32_t *flagF;
+  uint4 *N;
+  uint32_t *flagN;
+  Tiny *tiny;
+  uint16_t *slots;
+  uint32_t V, W, Q, slot_n;
+  uint64_t cap;
+  const Ctr *ctr;
+  int h, deferred, virt, clear;
+};
+
+__global__ void __launch_bounds__(256) k_hop_prep(PrepArgs a) {
+  if (a.deferred) pairs_rows(a.pairs, a.cnt, a.F, a.W, a.slot_n, a.cap, a.ctr, a.h, 0);
+  if (a.virt)
+    materialize(a.flagF, reinterpret_cast<uint4 *>(a.F), a.V, a.Q, a.slots, a.slot_n, a.ctr, a.h, 1);
+  const int s = a.ctr->hop[a.h].strategy;
+  if (a.clear && (s == ST_SPARSE || s == ST_PUSH || (s == ST_PULL && a.ctr->multislice)))
+    clear_flagged(a.N, a.flagN, a.V, a.Q);
+  if (a.slots && pairs_build(a.ctr, a.h))
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x) a.cnt[v] = 0;
+}
+
+// Short-row words of a layer SPARSE, PUSH or the seed wrote, from the pairs placed in
+// the slots or from the rows, and the rows too long for a slot, which a short-mode
+// PULL gathers whole.
+__global__ void __launch_bounds__(256) k_short_index(PrepArgs a) {
+  pairs_words(a.flagF, a.cnt, a.tiny, a.slots, a.slot_n, a.V, a.ctr, a.h);
+  if (a.deferred) pairs_rows(a.pairs, a.cnt, a.F, a.W, a.slot_n, a.cap, a.ctr, a.h, 1);
+  slot_build(a.flagF, reinterpret_cast<const uint4 *>(a.F), a.V, a.Q, a.tiny, a.slots, a.slot_n, a.ctr, a.h);
 }
 
 // ---------------------------------------------------------------------------
@@ -2574,7 +2620,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   }
   {  // counters, layer unions and task queues in one block: one memset clears them
     const size_t c = (sizeof(Ctr) + 15) / 16 * 16, u = (size_t)(p->k_max + 1) * pl->Q * 16;
-    pl->ctr_bytes = c + u + (size_t)(p->k_max + 1) * pl->nslices * 4;
+    pl->ctr_bytes = (c + u + (size_t)(p->k_max + 1) * pl->nslices * 4 + 15) / 16 * 16;
     char *base = nullptr;
     PL_ALLOC(base, pl->ctr_bytes);
     pl->ctr = reinterpret_cast<Ctr *>(base);
@@ -2728,18 +2774,14 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
   const bool timing = pl->timing && cap == cudaStreamCaptureStatusNone;  // events are not captured
   VS_TRY(copy_in(pl->d_src, sources, S_, st));
   if (pl->d_tgt) VS_TRY(copy_in(pl->d_tgt, targets, S_, st));
-  // run start: clean frontier buffers, zero visited/accumulator/counters
-  for (int b = 0; b < 2; b++)
-    { k_clear_flagged<<<pl->grid_v, 256, 0, st>>>(reinterpret_cast<uint4 *>(pl->buf[b]), pl->flag[b],
-                                                V, Q, pl->ctr, 0, 0); vs::note_launch(); }
-  // the result matrix (visited or accumulator): clear the rows the previous
-  // run marked in resflag, which also zeroes resflag; a visited matrix beside
-  // an accumulator has no row marks and is cleared whole
-  if (pl->acc || pl->vis)
-    { k_clear_flagged<<<pl->grid_v, 256, 0, st>>>(reinterpret_cast<uint4 *>(pl->acc ? pl->acc : pl->vis),
-                                                pl->resflag, V, Q, pl->ctr, 0, 0); vs::note_launch(); }
+  // run start: clean frontier buffers, zero counters, and the rows of the result
+  // matrix (visited or accumulator) that the previous run marked in resflag; a
+  // visited matrix beside an accumulator has no row marks and is cleared whole
+  { k_run_start<<<pl->grid_v, 256, 0, st>>>(
+        reinterpret_cast<uint4 *>(pl->buf[0]), pl->flag[0], reinterpret_cast<uint4 *>(pl->buf[1]), pl->flag[1],
+        reinterpret_cast<uint4 *>(pl->acc ? pl->acc : pl->vis), pl->resflag, V, Q, reinterpret_cast<uint4 *>(pl->ctr),
+        (uint32_t)(pl->ctr_bytes / 16)); vs::note_launch(); }
   if (pl->acc && pl->vis) VS_CK(cudaMemsetAsync(pl->vis, 0, rowbytes, st));
-  VS_CK(cudaMemsetAsync(pl->ctr, 0, pl->ctr_bytes, st));
   const Lists in = pull_lists(g, p.direction), outl = push_lists(g, p.direction);
   SeedArgs sa;
   sa.sources = pl->d_src;
@@ -2828,16 +2870,26 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     { k_decide<<<1, 256, 0, st>>>(da); vs::note_launch(); }
     // hop_ms covers what the chosen strategy costs, not the statistics and decision before it
     if (timing) cudaEventRecord(pl->ev[3 * h], st);
-    if (defer_rows(h - 1))  // rows a SPARSE hop h-1 left in its pair list, when hop h reads rows
-      { k_pairs_rows<<<pl->grid_v, 256, 0, st>>>(pl->pairs[fb], pl->touched, reinterpret_cast<unsigned long long *>(pl->buf[fb]),
-                                               W, pl->slot_n, pl->pair_cap, pl->ctr, h, 0); vs::note_launch(); }
-    if (pl->slot[0] && leave_in_slots(h - 1))  // whole rows back for a hop that reads rows
-      { k_materialize<<<pl->grid_v, 256, 0, st>>>(pl->flag[fb], reinterpret_cast<uint4 *>(pl->buf[fb]), V, Q,
-                                                pl->slot[fb], pl->slot_n, pl->ctr, h, 1); vs::note_launch(); }
-
-    if (h > 1)  // hop 1 writes a buffer the run start cleared
-      { k_clear_flagged<<<pl->grid_v, 256, 0, st>>>(reinterpret_cast<uint4 *>(pl->buf[nbuf]),
-                                                  pl->flag[nbuf], V, Q, pl->ctr, h, 1); vs::note_launch(); }
+    PrepArgs prep;
+    prep.pairs = pl->pairs[fb];
+    prep.cnt = pl->touched;
+    prep.F = reinterpret_cast<unsigned long long *>(pl->buf[fb]);
+    prep.flagF = pl->flag[fb];
+    prep.N = reinterpret_cast<uint4 *>(pl->buf[nbuf]);
+    prep.flagN = pl->flag[nbuf];
+    prep.tiny = pl->tiny[fb];
+    prep.slots = pl->slot[fb];
+    prep.V = V;
+    prep.W = W;
+    prep.Q = Q;
+    prep.slot_n = pl->slot_n;
+    prep.cap = pl->pair_cap;
+    prep.ctr = pl->ctr;
+    prep.h = h;
+    prep.deferred = defer_rows(h - 1);
+    prep.virt = pl->slot[0] && leave_in_slots(h - 1);
+    prep.clear = h > 1;  // hop 1 writes a buffer the run start cleared
+    if (h > 1 || pl->slot[0]) { k_hop_prep<<<pl->grid_v, 256, 0, st>>>(prep); vs::note_launch(); }
     const bool acc_on = pl->use_acc && h >= p.k_min && h <= p.k_max;
     SparseArgs sp;
     sp.ctr = pl->ctr;
@@ -2861,9 +2913,8 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     sp.stats = stats && h < p.k_max;
     sp.last = h == p.k_max && pl->use_vis && p.path_type != VS_PATH_FIND_SHORTEST && !pl->layer_out[h];
     sp.defer = defer_rows(h);
-    { k_pscan1<<<pl->grid_v, 256, 0, st>>>(pl->pdeg[fb], pl->doff, pl->bsum, pl->ctr, h, pl->pair_cap); vs::note_launch(); }
-    { k_pscan2<<<1, 1024, 0, st>>>(pl->bsum, pl->doff, pl->ctr, h, pl->pair_cap); vs::note_launch(); }
-    { k_pscan3<<<pl->grid_v, 256, 0, st>>>(pl->doff, pl->bsum, pl->ctr, h, pl->pair_cap); vs::note_launch(); }
+    sp.bsum = pl->bsum;
+    { k_pscan<<<pl->grid_v, 256, 0, st>>>(pl->pdeg[fb], pl->doff, pl->bsum, pl->ctr, h, pl->pair_cap); vs::note_launch(); }
     { k_sparse<<<pl->grid_sparse, 256, 0, st>>>(sp); vs::note_launch(); }
     PushArgs pa;
     pa.ctr = pl->ctr;
@@ -2934,17 +2985,9 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     short_layout(a, short_tile(Q));
     if (timing) cudaEventRecord(pl->ev[3 * h + 1], st);
     if (pl->slot[0]) {  // words and slots of a layer SPARSE, PUSH or the seed wrote, when this hop reads them
-      { k_pairs_zero<<<pl->grid_v, 256, 0, st>>>(pl->touched, V, pl->ctr, h); vs::note_launch(); }
       { k_pairs_slots<<<pl->grid_v, 256, 0, st>>>(pl->pairs[fb], pl->touched, pl->slot[fb], pl->slot_n, pl->pair_cap,
                                                 pl->ctr, h); vs::note_launch(); }
-      { k_pairs_words<<<pl->grid_v, 256, 0, st>>>(pl->flag[fb], pl->touched, pl->tiny[fb], pl->slot[fb], pl->slot_n, V,
-                                                pl->ctr, h); vs::note_launch(); }
-      if (defer_rows(h - 1))  // the rows too long for a slot, which the short-mode PULL gathers whole
-        { k_pairs_rows<<<pl->grid_v, 256, 0, st>>>(pl->pairs[fb], pl->touched,
-                                                 reinterpret_cast<unsigned long long *>(pl->buf[fb]), W, pl->slot_n,
-                                                 pl->pair_cap, pl->ctr, h, 1); vs::note_launch(); }
-      { k_slot_build<<<pl->grid_v, 256, 0, st>>>(pl->flag[fb], reinterpret_cast<const uint4 *>(pl->buf[fb]), V, Q,
-                                               pl->tiny[fb], pl->slot[fb], pl->slot_n, pl->ctr, h); vs::note_launch(); }
+      { k_short_index<<<pl->grid_v, 256, 0, st>>>(prep); vs::note_launch(); }
     }
     { var.pull<<<dim3(pl->grid_pull, pl->nslices), 256, 0, st>>>(a); vs::note_launch(); }
     if (pl->slot[0]) {

@@ -19,6 +19,7 @@ struct HopCtr {
                                        // when it keeps words)
   unsigned long long work_edges;       // SPARSE: edges scanned by the hop
   unsigned long long hist[16];         // log2(out-degree + 1) histogram of layer h-1's active rows
+  unsigned scan_done;                  // SPARSE: blocks of its degree scan that have finished
   int overflow;                        // SPARSE: pair list overflowed
   int strategy;                        // strategy run at hop h (0 = not run)
   int short_pull;                      // PULL reads the short rows of layer h-1 through their slots
@@ -86,7 +87,8 @@ struct SparseArgs {
   const unsigned long long *hmask;  // rows that may still grow at hop h (NULL = all)
   const uint2 *pin;
   uint2 *pout;
-  const unsigned long long *doff;  // exclusive prefix of the input pairs' out-degrees (+ total)
+  const unsigned long long *doff, *bsum;  // exclusive prefix of the input pairs' out-degrees in tiles of 1,024, tile
+                                          // starts (+ total)
   unsigned long long *pdeg_out;    // out-degree of every output pair's vertex
   uint64_t cap;
   Lists out;
