@@ -134,6 +134,7 @@ __device__ __forceinline__ void clear_flagged(uint4 *__restrict__ buf, uint32_t 
 // result (NULL: none), and the counter block (n 16-byte words).
 __global__ void __launch_bounds__(256) k_run_start(uint4 *buf0, uint32_t *flag0, uint4 *buf1, uint32_t *flag1, uint4 *res,
                                                    uint32_t *resflag, uint32_t V, uint32_t Q, uint4 *ctr, uint32_t n) {
+  vs::grid_wait();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     ctr[i] = make_uint4(0, 0, 0, 0);
   clear_flagged(buf0, flag0, V, Q);
@@ -147,6 +148,7 @@ __device__ __forceinline__ int degree_bin(unsigned long long d) {
 }
 
 __global__ void k_seed(SeedArgs a) {
+  vs::grid_wait();
   __shared__ unsigned s_hist[pk::NHIST];  // hop 1's frontier statistics (a.stats)
   if (threadIdx.x < pk::NHIST) s_hist[threadIdx.x] = 0;
   __syncthreads();
@@ -195,6 +197,7 @@ __global__ void k_seed(SeedArgs a) {
 // FindShortest bookkeeping before hop 1 (VExpand::before_execution, vexpand.cpp:179-195).
 __global__ void k_dist_init(const uint32_t *__restrict__ src, const uint32_t *__restrict__ tgt,
                             int32_t *__restrict__ dist, uint32_t S, uint32_t V, Ctr *ctr) {
+  vs::grid_wait();
   unsigned long long f = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < S; i += gridDim.x * blockDim.x) {
     if (tgt[i] >= V) ctr->error = 1;
@@ -209,6 +212,7 @@ __global__ void k_dist_init(const uint32_t *__restrict__ src, const uint32_t *__
 // own zeroed matrix, flagged rows only; a hop that did not run copies nothing.
 __global__ void k_copy_layer(const uint4 *__restrict__ buf, const uint32_t *__restrict__ flag, uint4 *__restrict__ out,
                              uint32_t V, uint32_t Q, const Ctr *ctr, int h) {
+  vs::grid_wait();
   if (h > 0 && ctr->hop[h].strategy == 0) return;
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -256,6 +260,7 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
   const bool use_picker = a.picker && a.picker_on && a.forced == 0;
   // the network's parameters load while thread 0 reads the counters
   const __nv_bfloat16 *w = use_picker ? pk::mlp_stage(a.picker) : nullptr;
+  vs::grid_wait();
   if (t == 0) {
     if (!c->done && a.rowk && (uint32_t)a.h > a.rowk[0]) c->done = 1;  // every row is past its last hop
     if (!c->done && a.h >= 2) {
@@ -381,6 +386,7 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
 // choice: no pair list after a PULL or PUSH hop, and no PUSH in the plan.
 __global__ void k_hop_stats(const uint32_t *__restrict__ flagF, Lists out, uint32_t V, Ctr *ctr, int h,
                             int picker_only, int push_ok) {
+  vs::grid_wait();
   if (ctr->done || h == 1 || ctr->hop[h - 1].strategy == ST_SPARSE) return;
   if (picker_only && !push_ok) return;
   __shared__ unsigned long long hist[pk::NHIST];
@@ -455,6 +461,7 @@ __device__ __forceinline__ unsigned long long block_scan4(unsigned long long (&v
 __global__ void __launch_bounds__(256) k_pscan(const unsigned long long *__restrict__ pdeg,
                                                unsigned long long *__restrict__ doff,
                                                unsigned long long *__restrict__ bsum, Ctr *ctr, int h, uint64_t cap) {
+  vs::grid_wait();
   const uint64_t np = scan_len(ctr, h, cap);
   const uint64_t nb = (np + 1023) / 1024;
   if (blockIdx.x >= nb) return;
@@ -535,6 +542,7 @@ __device__ __forceinline__ void owner_pairs(const unsigned long long *__restrict
 }
 
 __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
+  vs::grid_wait();
   Ctr *c = a.ctr;
   if (c->hop[a.h].strategy != ST_SPARSE) return;
   __shared__ uint2 s_new[8][SPARSE_CHUNK];  // a warp's new pairs of its current chunk
@@ -1096,6 +1104,7 @@ __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bo
 
 template <int L, int UPL>
 __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 2 : 1) k_pull(PullArgs a) {
+  vs::grid_wait();
   HopCtr &hc = a.ctr->hop[a.h];
   if (hc.strategy != ST_PULL || hc.short_pull) return;
   constexpr uint32_t G = 32 / L, CH = kChunk<L>;
@@ -1837,6 +1846,7 @@ inline size_t short_smem(uint32_t Q, uint32_t slot_n) {
 // would need the registers of both).
 template <int MODE, bool SLOTS, int T>
 __global__ void __launch_bounds__(SH_WARPS * 32, 4) k_pull_short(const __grid_constant__ PullArgs a) {
+  vs::grid_wait();
   const HopCtr &hc = a.ctr->hop[a.h];
   if (hc.strategy != ST_PULL || !hc.short_pull || !a.tiny_in || (hc.short_slots != 0) != SLOTS ||
       (MODE == SH_LIST && hc.short_long) || (MODE == SH_GEN && a.list_too && !hc.short_long))
@@ -1957,6 +1967,7 @@ __device__ __forceinline__ void pairs_rows(const uint2 *__restrict__ pairs, cons
 // every pair's source id into its vertex's slot (entries 1.., in any order)
 __global__ void k_pairs_slots(const uint2 *__restrict__ pairs, uint32_t *__restrict__ cnt, uint16_t *__restrict__ slots,
                               uint32_t slot_n, uint64_t cap, const Ctr *ctr, int h) {
+  vs::grid_wait();
   if (!pairs_build(ctr, h)) return;
   const unsigned long long np_raw = ctr->hop[h - 1].pairs;
   const uint64_t np = np_raw < cap ? np_raw : cap;
@@ -2094,6 +2105,7 @@ struct PrepArgs {
 };
 
 __global__ void __launch_bounds__(256) k_hop_prep(PrepArgs a) {
+  vs::grid_wait();
   if (a.deferred) pairs_rows(a.pairs, a.cnt, a.F, a.W, a.slot_n, a.cap, a.ctr, a.h, 0);
   if (a.virt)
     materialize(a.flagF, reinterpret_cast<uint4 *>(a.F), a.V, a.Q, a.slots, a.slot_n, a.ctr, a.h, 1);
@@ -2108,6 +2120,7 @@ __global__ void __launch_bounds__(256) k_hop_prep(PrepArgs a) {
 // the slots or from the rows, and the rows too long for a slot, which a short-mode
 // PULL gathers whole.
 __global__ void __launch_bounds__(256) k_short_index(PrepArgs a) {
+  vs::grid_wait();
   pairs_words(a.flagF, a.cnt, a.tiny, a.slots, a.slot_n, a.V, a.ctr, a.h);
   if (a.deferred) pairs_rows(a.pairs, a.cnt, a.F, a.W, a.slot_n, a.cap, a.ctr, a.h, 1);
   slot_build(a.flagF, reinterpret_cast<const uint4 *>(a.F), a.V, a.Q, a.tiny, a.slots, a.slot_n, a.ctr, a.h);
@@ -2120,6 +2133,7 @@ __global__ void __launch_bounds__(256) k_short_index(PrepArgs a) {
 // list applies the visited AND-NOT and the accumulator (Shortest/Any rules).
 __global__ void k_push_compact(const uint32_t *__restrict__ flagF, uint32_t V, uint32_t *list,
                                Ctr *ctr, int h) {
+  vs::grid_wait();
   if (ctr->hop[h].strategy != ST_PUSH) return;
   const int lane = threadIdx.x & 31;
   for (uint32_t v0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; v0 < V;
@@ -2136,6 +2150,7 @@ __global__ void k_push_compact(const uint32_t *__restrict__ flagF, uint32_t V, u
 }
 
 __global__ void __launch_bounds__(256) k_push(PushArgs a) {
+  vs::grid_wait();
   Ctr *c = a.ctr;
   if (c->hop[a.h].strategy != ST_PUSH) return;
   const uint32_t n = c->push_active;
@@ -2163,6 +2178,7 @@ __global__ void __launch_bounds__(256) k_push(PushArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_push_epilogue(PushArgs a) {
+  vs::grid_wait();
   Ctr *c = a.ctr;
   if (c->hop[a.h].strategy != ST_PUSH) return;
   const uint32_t n = c->push_touched;
@@ -2203,6 +2219,7 @@ __global__ void __launch_bounds__(256) k_push_epilogue(PushArgs a) {
 }
 
 __global__ void k_push_reset(Ctr *c) {
+  vs::grid_wait();
   c->push_active = 0;
   c->push_touched = 0;
 }
@@ -2211,6 +2228,7 @@ __global__ void k_push_reset(Ctr *c) {
 __global__ void k_find_check(const uint64_t *__restrict__ N, const uint32_t *__restrict__ tgt,
                              int32_t *__restrict__ dist, uint32_t S, uint32_t W, uint32_t V,
                              Ctr *ctr, int h) {
+  vs::grid_wait();
   if (ctr->hop[h].strategy == 0) return;
   unsigned long long f = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < S; i += gridDim.x * blockDim.x) {
@@ -2226,6 +2244,7 @@ __global__ void k_find_check(const uint64_t *__restrict__ N, const uint32_t *__r
 // source bits (i, s_i) cleared (a source is never re-reached once visited).
 __global__ void k_clear_diag(uint64_t *__restrict__ vis, const uint32_t *__restrict__ src,
                              uint32_t S, uint32_t W, uint32_t V) {
+  vs::grid_wait();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < S; i += gridDim.x * blockDim.x)
     if (src[i] < V) atomicAnd((unsigned long long *)&vis[(size_t)src[i] * W + (i >> 6)], ~(1ull << (i & 63)));
 }
@@ -2774,14 +2793,13 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
   const bool timing = pl->timing && cap == cudaStreamCaptureStatusNone;  // events are not captured
   VS_TRY(copy_in(pl->d_src, sources, S_, st));
   if (pl->d_tgt) VS_TRY(copy_in(pl->d_tgt, targets, S_, st));
+  if (pl->acc && pl->vis) VS_CK(cudaMemsetAsync(pl->vis, 0, rowbytes, st));  // no row marks
   // run start: clean frontier buffers, zero counters, and the rows of the result
-  // matrix (visited or accumulator) that the previous run marked in resflag; a
-  // visited matrix beside an accumulator has no row marks and is cleared whole
+  // matrix (visited or accumulator) that the previous run marked in resflag
   { k_run_start<<<pl->grid_v, 256, 0, st>>>(
         reinterpret_cast<uint4 *>(pl->buf[0]), pl->flag[0], reinterpret_cast<uint4 *>(pl->buf[1]), pl->flag[1],
         reinterpret_cast<uint4 *>(pl->acc ? pl->acc : pl->vis), pl->resflag, V, Q, reinterpret_cast<uint4 *>(pl->ctr),
         (uint32_t)(pl->ctr_bytes / 16)); vs::note_launch(); }
-  if (pl->acc && pl->vis) VS_CK(cudaMemsetAsync(pl->vis, 0, rowbytes, st));
   const Lists in = pull_lists(g, p.direction), outl = push_lists(g, p.direction);
   SeedArgs sa;
   sa.sources = pl->d_src;
@@ -2801,14 +2819,14 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
   sa.multislice = pl->nslices > 1;
   sa.rowk = pl->use_hmask ? pl->rowk : nullptr;
   sa.stats = pl->collect_stats || pl->log_features || (pl->picker && p.use_picker);
-  { k_seed<<<std::max(1u, std::min((S_ + 255) / 256, (uint32_t)sm_count() * 4)), 256, 0, st>>>(sa); vs::note_launch(); }
+  vs::launch_next(k_seed, std::max(1u, std::min((S_ + 255) / 256, (uint32_t)sm_count() * 4)), 256, 0, st, sa);
   VS_CK(cudaGetLastError());
   if (pl->layer_out[0])
-    { k_copy_layer<<<pl->grid_v, 256, 0, st>>>(reinterpret_cast<const uint4 *>(pl->buf[0]), pl->flag[0],
-                                             reinterpret_cast<uint4 *>(pl->layer_out[0]), V, Q, pl->ctr, 0); vs::note_launch(); }
+    vs::launch_next(k_copy_layer, pl->grid_v, 256, 0, st, reinterpret_cast<const uint4 *>(pl->buf[0]), pl->flag[0],
+                                             reinterpret_cast<uint4 *>(pl->layer_out[0]), V, Q, pl->ctr, 0);
   if (p.path_type == VS_PATH_FIND_SHORTEST)
-    { k_dist_init<<<std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st>>>(pl->d_src, pl->d_tgt,
-                                                                              pl->d_dist, S_, V, pl->ctr); vs::note_launch(); }
+    vs::launch_next(k_dist_init, std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st, pl->d_src, pl->d_tgt,
+                                                                              pl->d_dist, S_, V, pl->ctr);
   const PullVariant &var = pick_variant(pl->qslice);
   const int forced = p.strategy == VS_STRAT_PULL ? ST_PULL
                      : p.strategy == VS_STRAT_PUSH ? ST_PUSH
@@ -2865,9 +2883,8 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     // PUSH hop only a picker that may choose PUSH (or logging) needs the pass
     const bool picker_only = !pl->collect_stats && !pl->log_features;
     if (stats && h > 1 && !(picker_only && !can_push))
-      { k_hop_stats<<<pl->grid_v, 256, 0, st>>>(pl->flag[fb], outl, V, pl->ctr, h, picker_only, can_push);
-        vs::note_launch(); }
-    { k_decide<<<1, 256, 0, st>>>(da); vs::note_launch(); }
+      vs::launch_next(k_hop_stats, pl->grid_v, 256, 0, st, pl->flag[fb], outl, V, pl->ctr, h, picker_only, can_push);
+    vs::launch_next(k_decide, 1, 256, 0, st, da);
     // hop_ms covers what the chosen strategy costs, not the statistics and decision before it
     if (timing) cudaEventRecord(pl->ev[3 * h], st);
     PrepArgs prep;
@@ -2889,7 +2906,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     prep.deferred = defer_rows(h - 1);
     prep.virt = pl->slot[0] && leave_in_slots(h - 1);
     prep.clear = h > 1;  // hop 1 writes a buffer the run start cleared
-    if (h > 1 || pl->slot[0]) { k_hop_prep<<<pl->grid_v, 256, 0, st>>>(prep); vs::note_launch(); }
+    if (h > 1 || pl->slot[0]) vs::launch_next(k_hop_prep, pl->grid_v, 256, 0, st, prep);
     const bool acc_on = pl->use_acc && h >= p.k_min && h <= p.k_max;
     SparseArgs sp;
     sp.ctr = pl->ctr;
@@ -2914,8 +2931,8 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     sp.last = h == p.k_max && pl->use_vis && p.path_type != VS_PATH_FIND_SHORTEST && !pl->layer_out[h];
     sp.defer = defer_rows(h);
     sp.bsum = pl->bsum;
-    { k_pscan<<<pl->grid_v, 256, 0, st>>>(pl->pdeg[fb], pl->doff, pl->bsum, pl->ctr, h, pl->pair_cap); vs::note_launch(); }
-    { k_sparse<<<pl->grid_sparse, 256, 0, st>>>(sp); vs::note_launch(); }
+    vs::launch_next(k_pscan, pl->grid_v, 256, 0, st, pl->pdeg[fb], pl->doff, pl->bsum, pl->ctr, h, pl->pair_cap);
+    vs::launch_next(k_sparse, pl->grid_sparse, 256, 0, st, sp);
     PushArgs pa;
     pa.ctr = pl->ctr;
     pa.h = h;
@@ -2934,10 +2951,10 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     pa.shortest = pl->use_vis;
     pa.acc_on = acc_on;
     if (can_push) {  // PUSH kernels only when the hop can run PUSH
-      { k_push_reset<<<1, 1, 0, st>>>(pl->ctr); vs::note_launch(); }
-      { k_push_compact<<<pl->grid_v, 256, 0, st>>>(pl->flag[fb], V, pl->push_list, pl->ctr, h); vs::note_launch(); }
-      { k_push<<<pl->grid_push, 256, 0, st>>>(pa); vs::note_launch(); }
-      { k_push_epilogue<<<pl->grid_push, 256, 0, st>>>(pa); vs::note_launch(); }
+      vs::launch_next(k_push_reset, 1, 1, 0, st, pl->ctr);
+      vs::launch_next(k_push_compact, pl->grid_v, 256, 0, st, pl->flag[fb], V, pl->push_list, pl->ctr, h);
+      vs::launch_next(k_push, pl->grid_push, 256, 0, st, pa);
+      vs::launch_next(k_push_epilogue, pl->grid_push, 256, 0, st, pa);
     }
     PullArgs a;
     a.resflag = pl->resflag;
@@ -2985,34 +3002,34 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     short_layout(a, short_tile(Q));
     if (timing) cudaEventRecord(pl->ev[3 * h + 1], st);
     if (pl->slot[0]) {  // words and slots of a layer SPARSE, PUSH or the seed wrote, when this hop reads them
-      { k_pairs_slots<<<pl->grid_v, 256, 0, st>>>(pl->pairs[fb], pl->touched, pl->slot[fb], pl->slot_n, pl->pair_cap,
-                                                pl->ctr, h); vs::note_launch(); }
-      { k_short_index<<<pl->grid_v, 256, 0, st>>>(prep); vs::note_launch(); }
+      vs::launch_next(k_pairs_slots, pl->grid_v, 256, 0, st, pl->pairs[fb], pl->touched, pl->slot[fb], pl->slot_n, pl->pair_cap,
+                                                pl->ctr, h);
+      vs::launch_next(k_short_index, pl->grid_v, 256, 0, st, prep);
     }
-    { var.pull<<<dim3(pl->grid_pull, pl->nslices), 256, 0, st>>>(a); vs::note_launch(); }
+    vs::launch_next(var.pull, dim3(pl->grid_pull, pl->nslices), 256, 0, st, a);
     if (pl->slot[0]) {
       const ShortVariant &sv = pick_short(Q);
       const size_t sm = short_smem(Q, pl->slot_n);
       const bool last = a.last && a.shortest && !a.acc_on;
       a.list_too = !last && a.tiny_out && a.virt_out && !a.acc_on;
-      if (a.list_too) { sv.words[SH_LIST]<<<pl->grid_short, SH_WARPS * 32, sm, st>>>(a); vs::note_launch(); }
-      { sv.words[last ? SH_LAST : SH_GEN]<<<pl->grid_short, SH_WARPS * 32, sm, st>>>(a); vs::note_launch(); }
+      if (a.list_too) vs::launch_next(sv.words[SH_LIST], pl->grid_short, SH_WARPS * 32, sm, st, a);
+      vs::launch_next(sv.words[last ? SH_LAST : SH_GEN], pl->grid_short, SH_WARPS * 32, sm, st, a);
       a.list_too = 0;
-      { sv.slots[last ? SH_LAST : SH_GEN]<<<pl->grid_short, SH_WARPS * 32, sm, st>>>(a); vs::note_launch(); }
+      vs::launch_next(sv.slots[last ? SH_LAST : SH_GEN], pl->grid_short, SH_WARPS * 32, sm, st, a);
     }
     if (p.path_type == VS_PATH_FIND_SHORTEST)
-      { k_find_check<<<std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st>>>(
-          pl->buf[nbuf], pl->d_tgt, pl->d_dist, S_, W, V, pl->ctr, h); vs::note_launch(); }
+      vs::launch_next(k_find_check, std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st,
+          pl->buf[nbuf], pl->d_tgt, pl->d_dist, S_, W, V, pl->ctr, h);
     if (pl->layer_out[h])
-      { k_copy_layer<<<pl->grid_v, 256, 0, st>>>(reinterpret_cast<const uint4 *>(pl->buf[nbuf]), pl->flag[nbuf],
-                                               reinterpret_cast<uint4 *>(pl->layer_out[h]), V, Q, pl->ctr, h); vs::note_launch(); }
+      vs::launch_next(k_copy_layer, pl->grid_v, 256, 0, st, reinterpret_cast<const uint4 *>(pl->buf[nbuf]), pl->flag[nbuf],
+                                               reinterpret_cast<uint4 *>(pl->layer_out[h]), V, Q, pl->ctr, h);
     if (timing) cudaEventRecord(pl->ev[3 * h + 2], st);
     VS_CK(cudaGetLastError());
   }
   pl->timed_hops = timing ? p.k_max : 0;
   if (pl->clear_diag)
-    { k_clear_diag<<<std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st>>>(pl->vis, pl->d_src,
-                                                                                S_, W, V); vs::note_launch(); }
+    vs::launch_next(k_clear_diag, std::max(1u, std::min((S_ + 255) / 256, 1024u)), 256, 0, st, pl->vis, pl->d_src,
+                                                                                S_, W, V);
   if (p.path_type == VS_PATH_FIND_SHORTEST)
     VS_TRY(copy_in(distances, (const int32_t *)pl->d_dist, S_, st));
   VS_CK(cudaGetLastError());

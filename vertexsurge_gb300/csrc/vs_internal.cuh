@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
@@ -16,6 +17,34 @@ namespace vs {
 // Kernels launched by this library since load (vs_kernel_launches).
 extern std::atomic<unsigned long long> g_launches;
 inline void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+
+#ifdef __CUDACC__
+// A launch whose blocks may be placed while the stream's previous kernel still runs
+// (once all of that kernel's blocks have called grid_wait or ended): the kernel
+// waits for that one, and for what it wrote, in grid_wait().  Only for kernels
+// that call grid_wait() before they touch memory, after a kernel of this library.
+// Saves 1 to 1.5 us between two kernels, which is what a short kernel takes: an
+// expand of 3 hops and some 30 launches 180 -> 147 us.
+template <class... P, class... A>
+inline void launch_next(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, std::forward<A>(args)...);
+  note_launch();
+}
+__device__ __forceinline__ void grid_wait() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+#endif
 
 void set_error(const char *fmt, ...);
 int fail(int code, const char *fmt, ...);
