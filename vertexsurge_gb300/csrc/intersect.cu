@@ -83,6 +83,11 @@ struct Args {
   uint32_t *out_new;
   const int *method;  // learned method for AUTO adjacency deps (VS_ISECT_*), or NULL
   unsigned long long *next;  // work queue head: next base tuple to hand out (zeroed per launch)
+  // pair rows: a bit per walked candidate, kept between the counting and the emitting pass
+  uint32_t *mask;                // mask_cap words (NULL: none kept)
+  uint64_t mask_cap;             // below 2^32 - 1
+  unsigned long long *mask_n;    // words the tasks need, kept or not
+  uint32_t *mask_at;             // a task's first word
 };
 
 constexpr int ISECT_CHUNK = 4;  // base tuples a warp takes from the queue at a time
@@ -408,14 +413,29 @@ __global__ void __launch_bounds__(256) k_isect_pair_pieces(Args a, const ulonglo
 }
 
 // Rows of a two-adjacency intersection (triangle listing): counts per tuple, then,
-// with the prefix sums, the rows.  A warp takes PAIR_TUPLES tuples, lane j loading
-// tuple j's lists, so their dependent loads overlap, and walks each shorter list 64
-// candidates at a time (two membership loads per lane in flight).  Bound by the
-// latency of those loads; tuples without a match are skipped when emitting.
-// 955k edges of an R-MAT 16 graph, 20M rows: count 1379 -> 378 us, emit 1635 ->
-// 638 us against the general kernel, most of it from bitmaps of shorter lists
-// (hub_index).
+// with the prefix sums, the rows.  A warp takes PAIR_TUPLES tuples (a task), lane j
+// loading tuple j's lists, so their dependent loads overlap, and walks each shorter
+// list 64 candidates at a time (two membership loads per lane in flight).  Bound by
+// the latency of those loads.  The counting pass keeps a bit per candidate, from
+// which k_isect_pair_emit writes the rows; where the bits do not fit their scratch,
+// this kernel tests every candidate again and emits (tuples without a match skipped).
+// 955k edges of an R-MAT 16 graph, 20M rows: count 1379 -> 406 us, emit 1635 ->
+// 210 us against the general kernel (count 378, emit 638 when it tests again),
+// most of the count's from bitmaps of shorter lists (hub_index).
 constexpr int PAIR_TUPLES = 8;
+
+// A tuple's words of the mask: two per 64 candidates.
+__device__ __forceinline__ uint32_t pair_words(int64_t wn) { return (uint32_t)((wn + 63) / 64 * 2); }
+
+// Inclusive sum over the first PAIR_TUPLES lanes; the lanes after them get the total.
+__device__ __forceinline__ unsigned long long pair_scan(unsigned long long v, int lane) {
+  for (int o = 1; o < PAIR_TUPLES; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(FULLMASK, v, o);
+    if (lane >= o) v += y;
+  }
+  const unsigned long long sum = __shfl_sync(FULLMASK, v, PAIR_TUPLES - 1);
+  return lane < PAIR_TUPLES ? v : sum;
+}
 
 template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Args a) {
   const int lane = threadIdx.x & 31;
@@ -438,6 +458,17 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
       }
       if (look) p = pair_tuple(a, t, learned);
     }
+    uint32_t mo = 0xffffffffu;  // the tuple's words of the mask, if its task's fit
+    if (!EMIT && a.mask) {
+      const unsigned long long nw = pair_words(p.wn), end = pair_scan(nw, lane);
+      unsigned long long at = 0;
+      if (lane == PAIR_TUPLES - 1 && end) at = atomicAdd(a.mask_n, end);
+      at = __shfl_sync(FULLMASK, at, PAIR_TUPLES - 1);
+      if (at + __shfl_sync(FULLMASK, end, PAIR_TUPLES - 1) <= a.mask_cap) {
+        mo = (uint32_t)(at + end - nw);
+        if (lane == 0) a.mask_at[t0 / PAIR_TUPLES] = (uint32_t)at;
+      }
+    }
     unsigned long long found = 0;  // lane j: matches of tuple j
     unsigned todo = __ballot_sync(FULLMASK, p.wn > 0);
     while (todo) {
@@ -447,6 +478,7 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
       const int64_t olo = __shfl_sync(FULLMASK, p.olo, j), ohi = __shfl_sync(FULLMASK, p.ohi, j);
       const int w1 = __shfl_sync(FULLMASK, p.w1, j), hs = __shfl_sync(FULLMASK, p.hs, j);
       const unsigned long long at = EMIT ? __shfl_sync(FULLMASK, pos, j) : 0ull;
+      const uint32_t mat = EMIT ? 0xffffffffu : __shfl_sync(FULLMASK, mo, j);
       const uint32_t *walk = (w1 ? a.dep[1] : a.dep[0]).adj + wlo;
       unsigned long long count = 0;
       for (int64_t k = lane; k - lane < wn; k += 64) {
@@ -458,6 +490,8 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
           if (h0) emit_row(a, t0 + j, at + count + __popc(m0 & lanemask_lt()), x0);
           if (h1) emit_row(a, t0 + j, at + count + __popc(m0) + __popc(m1 & lanemask_lt()), x1);
         }
+        if (!EMIT && mat != 0xffffffffu && lane == 0)
+          *reinterpret_cast<uint2 *>(a.mask + mat + ((k - lane) >> 5)) = make_uint2(m0, m1);
         count += __popc(m0) + __popc(m1);
       }
       if (lane == j) found = count;
@@ -470,6 +504,76 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
   if (!EMIT) {
     for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(FULLMASK, tot, o);
     if (lane == 0 && tot) atomicAdd(a.total, tot);
+  }
+}
+
+// k-th set bit of m, k < popc(m).
+__device__ __forceinline__ int kth_bit(uint32_t m, int k) {
+  int b = 0;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const int c = __popc(m & ((1u << o) - 1));
+    if (k >= c) {
+      k -= c;
+      b += o;
+      m >>= o;
+    }
+  }
+  return b;
+}
+
+// The rows of every task from the candidates' bits.  A task's words and its output
+// rows are both contiguous, so a lane takes a word of any of the tuples and then the
+// warp writes 32 rows at a time, each lane finding its row's word and bit: full
+// stores whatever the tuples' sizes, and no dependent loads but the candidate's.
+__global__ void __launch_bounds__(256) k_isect_pair_emit(Args a) {
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    unsigned long long t0 = 0;
+    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)PAIR_TUPLES);
+    t0 = __shfl_sync(FULLMASK, t0, 0);
+    if (t0 >= a.nbase) break;
+    const uint64_t tn = t0 + PAIR_TUPLES < a.nbase ? t0 + PAIR_TUPLES : a.nbase;
+    unsigned long long out = a.toff[t0];
+    const unsigned long long out_end = a.toff[tn] < a.max_rows ? a.toff[tn] : a.max_rows;
+    if (out >= out_end) continue;
+    PairTuple p{0, 0, 0, 0, 0, -1};
+    if (t0 + lane < tn) p = pair_tuple(a, t0 + lane, VS_ISECT_BINARY);
+    const uint32_t nw = pair_words(p.wn), end = (uint32_t)pair_scan(nw, lane);
+    const uint32_t start = lane < PAIR_TUPLES ? end - nw : end;
+    const uint32_t words = __shfl_sync(FULLMASK, end, PAIR_TUPLES - 1);
+    const uint32_t *walk = (p.w1 ? a.dep[1] : a.dep[0]).adj + p.wlo - (int64_t)start * 32;
+    const uint32_t *mask = a.mask + a.mask_at[t0 / PAIR_TUPLES];
+    for (uint32_t w0 = 0; w0 < words && out < out_end; w0 += 32) {
+      const uint32_t w = w0 + lane, m = w < words ? __ldg(mask + w) : 0u;
+      int own = 0;  // the last tuple whose words start at or before w
+#pragma unroll
+      for (int step = PAIR_TUPLES / 2; step; step >>= 1)
+        if (__shfl_sync(FULLMASK, start, own + step) <= w) own += step;
+      const unsigned long long from =
+          __shfl_sync(FULLMASK, (unsigned long long)walk, own) + (unsigned long long)w * 32 * sizeof(uint32_t);
+      const uint32_t c = __popc(m);
+      uint32_t first = c;  // exclusive prefix of the words' rows
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULLMASK, first, o);
+        if (lane >= o) first += y;
+      }
+      const uint32_t rows = __shfl_sync(FULLMASK, first, 31);
+      first -= c;
+      for (uint32_t r0 = 0; r0 < rows; r0 += 32) {
+        const uint32_t r = r0 + lane;
+        int i = 0;  // the last word whose rows start at or before r
+#pragma unroll
+        for (int step = 16; step; step >>= 1)
+          if (__shfl_sync(FULLMASK, first, i + step) <= r) i += step;
+        const uint32_t mi = __shfl_sync(FULLMASK, m, i), k = r - __shfl_sync(FULLMASK, first, i);
+        const uint32_t *f = reinterpret_cast<const uint32_t *>(__shfl_sync(FULLMASK, from, i));
+        const uint64_t t = t0 + __shfl_sync(FULLMASK, own, i);
+        if (r < rows) emit_row(a, t, out + r, __ldg(f + kth_bit(mi, (int)k)));
+      }
+      out += rows;
+    }
   }
 }
 
@@ -986,8 +1090,17 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
       piece_cap = res[1];
     }
   } else if (a.nbase) {
-    if (pair)
+    if (pair) {
+      // bits of the candidates for the emitting pass: room for 512 a tuple (64 bytes of
+      // scratch, 256 MB in all), none when memory is short
+      a.mask_cap = std::min<uint64_t>(16 * a.nbase, 1ull << 26);
+      if (sc.get(&a.mask, a.mask_cap) != VS_OK || sc.get(&a.mask_at, a.nbase / PAIR_TUPLES + 1) != VS_OK) {
+        cudaGetLastError();
+        a.mask = nullptr;
+      }
+      a.mask_n = d_total + 1;
       { k_isect_pair_rows<false><<<grid, 256, 0, st>>>(a); vs::note_launch(); }
+    }
     else
       { k_isect<<<grid, 256, 0, st>>>(a); vs::note_launch(); }
     VS_CK(cudaGetLastError());
@@ -1003,6 +1116,7 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
     VS_CK(cudaStreamSynchronize(st));
   }
   unsigned long long total = res[0];
+  const uint64_t masked = res[1];
   *count = total;
   if (only_count) return VS_OK;
   VS_TRY(exclusive_scan_u64(tcnt, toff, a.nbase, st));
@@ -1024,7 +1138,10 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
   a.max_rows = rows;
   a.emit = 1;
   VS_CK(cudaMemsetAsync(a.next, 0, 8, st));
-  if (a.nbase && rows && pair) { k_isect_pair_rows<true><<<grid, 256, 0, st>>>(a); vs::note_launch(); }
+  if (a.nbase && rows && pair && a.mask && masked <= a.mask_cap)
+    { k_isect_pair_emit<<<grid, 256, 0, st>>>(a); vs::note_launch(); }
+  else if (a.nbase && rows && pair)
+    { k_isect_pair_rows<true><<<grid, 256, 0, st>>>(a); vs::note_launch(); }
   if (a.nbase && rows && !pair) { k_isect<<<grid, 256, 0, st>>>(a); vs::note_launch(); }
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
