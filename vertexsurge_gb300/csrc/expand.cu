@@ -246,6 +246,13 @@ __global__ void __launch_bounds__(256) k_row_mask(const uint8_t *__restrict__ li
   }
 }
 
+// Row flags as bits in a block's shared memory: up to BITS_MAX_V vertices (160 KB; the
+// rest of the SM's 228 KB stays L1).
+constexpr uint32_t BITS_MAX_V = 160 * 1024 * 8;
+constexpr uint32_t BITS_MIN_V = 128 * 1024;
+constexpr uint64_t BITS_MIN_EDGES = 16ull << 20;
+inline size_t bits_smem(uint32_t V) { return (size_t)((V + 127) / 128) * 16; }
+
 // One block of 256 threads: early-stop checks of hop h-1 (VExpand::after_child,
 // vexpand.cpp:222-284), the fixed planner's choice for hop h, and — when a
 // picker is loaded or features are logged — the feature vector of hop h and
@@ -373,6 +380,22 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
       lng = ids > 1.2f * V * (a.W <= 64 ? 16 : a.W <= 128 ? 32 : 64);
     }
     cur.short_pull = sp;
+    // row flags as bits where they save loads: below 9 in 10 active vertices for rows of
+    // more than a sector.  A narrower row is loaded as fast as its flag, so only with
+    // under half of the list entries active: counted after SPARSE; after PULL a fifth
+    // of the vertices (30% of an R-MAT's vertices hold 90% of the entries: 7% slower).
+    // Never at hop 1, whose layer is the sources.
+    bool bits = s_choice == ST_PULL && !sp && a.bits_ok && a.h > 1;
+    if (bits) {
+      const float act = (float)prev.active_vertices, V = (float)a.V;
+      if (a.W > 2)
+        bits = act < 0.9f * V;
+      else if (prev.strategy == ST_SPARSE)
+        bits = (float)prev.pair_edges * act < 0.5f * (float)a.E * (a.both ? 2 : 1) * (float)prev.new_bits;
+      else
+        bits = act < 0.2f * V;
+    }
+    cur.bits = bits;
     cur.short_slots = sp && slots;
     cur.short_long = sp && lng;
   }
@@ -800,7 +823,7 @@ __device__ __forceinline__ void pull_counters(const PullArgs &a, unsigned long l
 // Measured on GB300 against a warp per target at a fixed stride with a CTA per
 // hub: R-MAT scale 16, 512 sources, hops 2 and 3 172 + 27 us -> 36 us each;
 // 1M-vertex power law, 64 sources, hop 4 465 -> 151 us; R-MAT scale 20 both
-// ways, 1,001 sources, hop 2 3.36 -> 0.63 ms; R-MAT scale 18, 3,000 sources, hops
+// ways, 1,001 sources, hop 2 3.36 -> 0.55 ms; R-MAT scale 18, 3,000 sources, hops
 // 3 to 5 1.38 ms -> 0.31, 0.20 and 0.17 ms; 4,096 sources on the 1M-vertex power
 // law, hop 4 (no row saturates) 1.58 -> 1.43 ms at 10.7 TB/s of row loads.
 constexpr uint32_t NONE = 0xffffffffu;
@@ -848,11 +871,16 @@ __device__ __forceinline__ bool covered(const uint4 *s_um, uint32_t qn, const ui
   return c;
 }
 
+// Whether vertex u has a row: its bit in shared memory (BITS) or its flag.
+template <bool BITS> __device__ __forceinline__ bool has_row(const uint32_t *flag, uint32_t u) {
+  return BITS ? flag[u >> 5] >> (u & 31) & 1u : __ldg(flag + u) != 0;
+}
+
 // OR the rows of list entries j, j + 1, ... (a group's rounds are `step` apart)
 // below n into acc, until the row is covered.  Every lane of the warp calls it;
 // a group with sat set only takes part in the votes.
-template <int L, int UPL>
-__device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__restrict__ F, const uint32_t *__restrict__ flag,
+template <int L, int UPL, bool BITS>
+__device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__restrict__ F, const uint32_t *flag,
                                             const uint4 *s_um, uint32_t qn, const uint32_t *__restrict__ adj,
                                             uint32_t n, uint32_t j, uint32_t step, const uint4 (&vv)[UPL],
                                             uint4 (&acc)[UPL], bool &sat) {
@@ -870,10 +898,15 @@ __device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__re
         id[k] = NONE;
         if (more && i < n) id[k] = __ldg(adj + i);
       }
-      if (flag) {  // few rows of a round are non-empty: walk those
+      if (BITS && L <= 2) {  // rows of one sector: only the loads of the non-empty ones, in place
 #pragma unroll
         for (int k = 0; k < K; k++)
-          if (id[k] != NONE && !__ldg(flag + id[k])) id[k] = NONE;
+          if (id[k] != NONE && !has_row<BITS>(flag, id[k])) id[k] = NONE;
+      }
+      if (!(BITS && L <= 2) && (BITS || flag)) {  // few rows of a round are non-empty: walk those
+#pragma unroll
+        for (int k = 0; k < K; k++)
+          if (id[k] != NONE && !has_row<BITS>(flag, id[k])) id[k] = NONE;
 #pragma unroll
         for (int k = 0; k < K; k++) {
           unsigned m = __ballot_sync(FULL, id[k] != NONE) >> (lane & ~(L - 1)) & ((1u << L) - 1u);
@@ -914,7 +947,7 @@ __device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__re
     for (; j < n && !sat; j += step) {
       uint32_t id = NONE;
       if (j + lane < n) id = __ldg(adj + j + lane);
-      if (flag && id != NONE && !__ldg(flag + id)) id = NONE;
+      if ((BITS || flag) && id != NONE && !has_row<BITS>(flag, id)) id = NONE;
       unsigned m = __ballot_sync(FULL, id != NONE);
       while (m) {
         uint32_t u[R];
@@ -948,13 +981,13 @@ __device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__re
 // Group form of write_short for every group of the warp at once: the tiny
 // word and slot of the group's row x (valid: the group has a target, nz: its
 // row is not empty), c the lane's bit count.  Returns whether the row is short.
-template <int L, int UPL>
+template <int L, int UPL, int NW>
 __device__ __forceinline__ bool write_short_group(const PullArgs &a, uint32_t v, bool valid, bool nz,
                                                   const uint4 (&x)[UPL], uint32_t qn, uint32_t c,
                                                   unsigned long long &ns) {
   constexpr int G = 32 / L, SQ = G * 2 > 8 ? G * 2 : 8;
   // slots of up to 64 entries where a warp holds one row (L == 32), of 16 below
-  __shared__ uint4 s_stage[8][SQ];
+  __shared__ uint4 s_stage[NW][SQ];
   const uint32_t lane = threadIdx.x & 31, gl = lane & (L - 1), g = lane / L;
   uint32_t incl = c;
 #pragma unroll
@@ -1008,7 +1041,7 @@ __device__ __forceinline__ bool write_short_group(const PullArgs &a, uint32_t v,
 // Epilogue of a round: every group's target v (valid per group), its ORed rows
 // acc and visited words vv: visited update, accumulator OR, layer union,
 // next-layer row (with its tiny word and slot), flag, counters.
-template <int L, int UPL>
+template <int L, int UPL, int NW>
 __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bool valid, uint32_t q0, uint32_t qn,
                                                const uint4 *s_um, uint4 *s_un, const uint4 (&vv)[UPL], uint4 (&acc)[UPL],
                                                unsigned long long &nb, unsigned long long &nv, unsigned long long &ns,
@@ -1077,8 +1110,8 @@ __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bo
     return;
   }
   bool virt = false;  // the row is left in its slot only (flag 2)
-  if (a.tiny_out) {
-    const bool fits = write_short_group<L, UPL>(a, v, valid, rownz, acc, qn, bits, ns);
+  if (!(NW > 8 && L < 16) && a.tiny_out) {
+    const bool fits = write_short_group<L, UPL, NW>(a, v, valid, rownz, acc, qn, bits, ns);
     virt = fits && a.virt_out;
     if (valid && rownz && (bits || gl == 0)) {
       const unsigned long long d = out_degree(a.out, v);
@@ -1102,11 +1135,23 @@ __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bo
   }
 }
 
-template <int L, int UPL>
-__global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 2 : 1) k_pull(PullArgs a) {
+// BITS: the flags of layer h-1 as bits in shared memory, one block of 32 warps an SM.
+// A flag in global memory costs an L1 tag and mostly an L2 sector per list entry (5 ps
+// on the whole chip, as much as a row of one uint4); its bit costs a shared-memory word.
+// 64 sources on the 1M-vertex power law, hop 3 (5% of the rows active) 149 -> 94 us;
+// 1,001 sources both ways on R-MAT 20, hops 2 to 5 2.25 -> 2.06 ms; 2,048 sources on the
+// power law, two hops 1.20 -> 1.09 ms.
+template <int L, int UPL, bool BITS>
+__global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 2 : 1)
+    k_pull(PullArgs a) {
   vs::grid_wait();
   HopCtr &hc = a.ctr->hop[a.h];
-  if (hc.strategy != ST_PULL || hc.short_pull) return;
+  if (hc.strategy != ST_PULL || hc.short_pull || (hc.bits != 0) != BITS) return;
+  constexpr int NW = BITS ? 32 : 8;  // warps
+  extern __shared__ uint4 s_bits[];
+  if (BITS)
+    for (uint32_t i = threadIdx.x; i < (a.V + 127) / 128; i += blockDim.x)
+      s_bits[i] = __ldg(reinterpret_cast<const uint4 *>(a.bits) + i);
   constexpr uint32_t G = 32 / L, CH = kChunk<L>;
   __shared__ uint4 s_um[L * UPL];  // what a row can gain: the union of layer h-1, rows still growing
   __shared__ uint4 s_un[L * UPL];  // union of the rows this block wrote
@@ -1122,7 +1167,7 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
   __syncthreads();
   // a row of one sector is loaded as fast as its flag, and a nearly full layer has few rows to skip
   const bool useflag = a.Q > 2 && pc.active_vertices * 10 < 9ull * a.V;
-  const uint32_t *flag = useflag ? a.flagF : nullptr;
+  const uint32_t *flag = BITS ? reinterpret_cast<const uint32_t *>(s_bits) : useflag ? a.flagF : nullptr;
   const uint4 *F = a.F + q0;
   const bool known = a.res_vis && a.Q >= 8;  // resflag 0: the visited row is zero, without reading it
   // rows are often complete only once a good part of all bits is visited; before
@@ -1167,7 +1212,7 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
       bool sat = group_all<L>(covered<L, UPL>(s_um, qn, cov, acc));
       const int64_t beg = a.in.off[pc4.z][v], end = a.in.off[pc4.z][v + 1];
       const uint32_t n = (uint32_t)min((int64_t)pc4.w + a.piece_edges, end - beg);
-      gather_list<L, UPL>(a, F, flag, s_um, qn, a.in.adj[pc4.z] + beg, n, pc4.w + (L < 32 ? g * CH : 0),
+      gather_list<L, UPL, BITS>(a, F, flag, s_um, qn, a.in.adj[pc4.z] + beg, n, pc4.w + (L < 32 ? g * CH : 0),
                           L < 32 ? G * CH : 32, cov, acc, sat);
 #pragma unroll
       for (int o = L; o < 32; o <<= 1)
@@ -1208,7 +1253,7 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
           if (lane == 0) *cnt = np;
         }
       }
-      if (mine) group_epilogue<L, UPL>(a, v, g == 0, q0, qn, s_um, s_un, vv, acc, nb, nv, ns, ro, so, po);
+      if (mine) group_epilogue<L, UPL, NW>(a, v, g == 0, q0, qn, s_um, s_un, vv, acc, nb, nv, ns, ro, so, po);
     } else {
       // the tile's list starts at once: lane i holds those of target v0 + i (a tile of
       // L > 1 has at most 16 targets, so lane i + 1 holds the end too)
@@ -1239,8 +1284,8 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 
           sat = sat || c;
         }
         _Pragma("unroll") for (int l = 0; l < 2; l++) if (l < a.in.n)
-          gather_list<L, UPL>(a, F, flag, s_um, qn, a.in.adj[l] + beg[l], n[l], 0, L < 32 ? CH : 32, vv, acc, sat);
-        group_epilogue<L, UPL>(a, v, valid, q0, qn, s_um, s_un, vv, acc, nb, nv, ns, ro, so, po);
+          gather_list<L, UPL, BITS>(a, F, flag, s_um, qn, a.in.adj[l] + beg[l], n[l], 0, L < 32 ? CH : 32, vv, acc, sat);
+        group_epilogue<L, UPL, NW>(a, v, valid, q0, qn, s_um, s_un, vv, acc, nb, nv, ns, ro, so, po);
       }
     }
     task = __shfl_sync(FULL, nexttask, 0);
@@ -2088,7 +2133,8 @@ __device__ __forceinline__ void slot_build(const uint32_t *__restrict__ flagF, c
 // pair list (deferred) or in their slots (virt), if hop h reads rows; the rows of
 // layer h's buffer that an older layer left, if hop h needs them clean (SPARSE and
 // PUSH write with atomics, a multi-slice PULL in parts; any PULL at hop 1 and later
-// overwrites them itself); the pair counts of the short-row index.
+// overwrites them itself); the pair counts of the short-row index; the row flags of
+// layer h-1 as bits for a dense PULL that wants them.
 struct PrepArgs {
   const uint2 *pairs;
   uint32_t *cnt;
@@ -2098,6 +2144,7 @@ struct PrepArgs {
   uint32_t *flagN;
   Tiny *tiny;
   uint16_t *slots;
+  uint32_t *bits;
   uint32_t V, W, Q, slot_n;
   uint64_t cap;
   const Ctr *ctr;
@@ -2112,6 +2159,12 @@ __global__ void __launch_bounds__(256) k_hop_prep(PrepArgs a) {
   const int s = a.ctr->hop[a.h].strategy;
   if (a.clear && (s == ST_SPARSE || s == ST_PUSH || (s == ST_PULL && a.ctr->multislice)))
     clear_flagged(a.N, a.flagN, a.V, a.Q);
+  if (a.bits && a.ctr->hop[a.h].bits)
+    for (uint32_t v0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; v0 < a.V; v0 += gridDim.x * blockDim.x) {
+      const uint32_t v = v0 + (threadIdx.x & 31);
+      const unsigned m = __ballot_sync(FULL, v < a.V && a.flagF[v]);
+      if ((threadIdx.x & 31) == 0) a.bits[v0 >> 5] = m;
+    }
   if (a.slots && pairs_build(a.ctr, a.h))
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x) a.cnt[v] = 0;
 }
@@ -2342,15 +2395,15 @@ const ShortVariant &pick_short(uint32_t Q) { return kShort[short_tile(Q) == 4 ? 
 
 struct PullVariant {
   int L, UPL;
-  PullFn pull;
+  PullFn pull, bits;
 };
 
-#define VS_VARIANT(L, U) {L, U, k_pull<L, U>}
-const PullVariant kVariants[] = {
-    VS_VARIANT(1, 1),  VS_VARIANT(2, 1),  VS_VARIANT(4, 1),  VS_VARIANT(8, 1), VS_VARIANT(16, 1),
-    VS_VARIANT(32, 1), VS_VARIANT(32, 2), VS_VARIANT(32, 4), VS_VARIANT(32, 8),
-};
+#define VS_VARIANT(L) {L, 1, k_pull<L, 1, false>, k_pull<L, 1, true>}
+#define VS_WIDE(U) {32, U, k_pull<32, U, false>, nullptr}  // L = 32: 1% slower with bits on power laws
+const PullVariant kVariants[] = {VS_VARIANT(1),  VS_VARIANT(2), VS_VARIANT(4), VS_VARIANT(8), VS_VARIANT(16),
+                                 VS_WIDE(1),     VS_WIDE(2),    VS_WIDE(4),    VS_WIDE(8)};
 #undef VS_VARIANT
+#undef VS_WIDE
 
 const PullVariant &pick_variant(uint32_t qslice) {
   for (const auto &v : kVariants)
@@ -2370,6 +2423,7 @@ struct vs_expand_plan {
   uint32_t S = 0, W = 0, Q = 0, qslice = 0, nslices = 1;
   uint64_t *buf[2] = {nullptr, nullptr};
   uint32_t *flag[2] = {nullptr, nullptr};
+  uint32_t *bits = nullptr;  // row flags of the layer a dense PULL reads
   uint64_t *vis = nullptr, *acc = nullptr;
   uint2 *pairs[2] = {nullptr, nullptr};
   unsigned long long *pdeg[2] = {nullptr, nullptr}, *doff = nullptr, *bsum = nullptr;
@@ -2388,7 +2442,7 @@ struct vs_expand_plan {
   size_t ctr_bytes = 0;        // ctr, un and queue are one allocation, zeroed at every run start
   bool use_vis = false, use_acc = false, clear_diag = false;
   bool collect_stats = false;
-  int grid_pull = 0, grid_sparse = 0, grid_v = 0, grid_push = 0, grid_short = 0;
+  int grid_bits = 0, grid_pull = 0, grid_sparse = 0, grid_v = 0, grid_push = 0, grid_short = 0;
   vs_bitmat result{};
   bool has_result = false;
   // tuning knobs of the fixed planner
@@ -2439,13 +2493,24 @@ inline bool short_slots_ok(uint32_t S, uint32_t nslices, double share, uint64_t 
   return share >= 0 && S <= 32768 && nslices == 1 && (share > 1.0 || (W >= 32 && V * 8ull * W > l2_bytes() / 2));
 }
 
+// Whether a plan's dense PULL hops may read row flags as bits.  Whole runs against flags
+// in global memory, power laws and R-MAT graphs of 16K to 1.2M vertices: rows of 3 to 16
+// uint4 gain 3 to 16% from 128K vertices on and lose up to 5% at 16K to 64K (the block's
+// prologue and one launch a hop); rows of one or two gain 2 to 23% at 18M list entries
+// and more and lose 1 to 5% at 4M to 8M; rows of 32 lanes lose 1% on power laws.
+inline bool bits_ok(uint32_t V, uint32_t qslice, bool slots, uint64_t list_edges) {
+  const PullVariant &v = pick_variant(qslice);
+  if (!v.bits || V > BITS_MAX_V || (slots && v.L < 16)) return false;  // (no room to write slots in narrow rows)
+  return v.L <= 2 ? list_edges >= BITS_MIN_EDGES : V >= BITS_MIN_V;
+}
+
 int plan_free(vs_expand_plan *pl) {
   if (!pl) return VS_OK;
   const cudaStream_t st = pl->last_stream;
   void *ptrs[] = {pl->tiny[0], pl->tiny[1], pl->slot[0], pl->slot[1], pl->resflag, pl->pdeg[0], pl->pdeg[1], pl->doff,
                   pl->bsum, pl->hmask, pl->rowk, pl->buf[0], pl->buf[1], pl->flag[0], pl->flag[1], pl->vis, pl->acc,
                   pl->pairs[0], pl->pairs[1], pl->push_list, pl->touched, pl->d_src,
-                  pl->d_tgt, pl->d_dist, pl->ctr, pl->pieces, pl->heavy_rows, pl->heavy_np, pl->heavy_left};
+                  pl->d_tgt, pl->d_dist, pl->ctr, pl->pieces, pl->heavy_rows, pl->heavy_np, pl->heavy_left, pl->bits};
   for (void *p : ptrs)  // stream-ordered after the plan's last run
     if (p) dfree(p, st);
   for (cudaEvent_t e : pl->ev)
@@ -2658,6 +2723,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   } else {
     pl->short_min = 0;
   }
+  if (bits_ok(V, pl->qslice, pl->slot[0] != nullptr, (p->direction == VS_DIR_BOTH && g->directed ? 2 : 1) * g->E)) PL_ALLOC(pl->bits, bits_smem(V) / 4);
 #undef PL_ALLOC
   cudaError_t e = cudaSuccess;
   // every row starts zero; later runs clear only the rows their flags mark
@@ -2722,6 +2788,10 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   const int occ = occupancy_grid(var.pull, 256, 0, 8);
   pl->tile = G;
   while (pl->tile < 16 && (uint64_t)V / pl->tile > 64ull * occ) pl->tile *= 2;
+  if (pl->bits) {
+    cudaFuncSetAttribute(var.bits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bits_smem(BITS_MAX_V));
+    pl->grid_bits = occupancy_grid(var.bits, 1024, bits_smem(V), 1);
+  }
   const uint64_t tasks = pl->npieces + ((uint64_t)V + pl->tile - 1) / pl->tile;
   pl->grid_pull = (int)std::max<uint64_t>(1, std::min<uint64_t>(occ, (tasks + 7) / 8));
   if (pl->slot[0]) {
@@ -2766,7 +2836,9 @@ int vs_expand_plan_footprint(const vs_graph *g, uint32_t S, const vs_expand_para
   const uint64_t multi = std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, std::max<uint64_t>(thr, piece_edges(L))));
   b += 16 * (list_edges / piece_edges(L) + 2 * std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, thr)));
   b += multi * (W * 8 + 4 + 4 * nslices) + (uint64_t)(p->k_max + 1) * (W * 8 + 4 * nslices);
-  if (short_slots_ok(S, nslices, p->short_share, V, (uint32_t)W))
+  const bool slots = short_slots_ok(S, nslices, p->short_share, V, (uint32_t)W);
+  if (bits_ok((uint32_t)V, qs, slots, list_edges)) b += bits_smem((uint32_t)V);
+  if (slots)
     b += 2 * V * (2 * slot_entries((uint32_t)W) + sizeof(Tiny));  // short-row words and slots of both buffers
   *bytes = b;
   return VS_OK;
@@ -2868,6 +2940,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     da.log_features = pl->log_features;
     da.both = p.direction == VS_DIR_BOTH && g->directed;
     da.pair_cap = pl->pair_cap;
+    da.bits_ok = pl->bits != nullptr;
     da.sparse_frac = pl->sparse_frac;
     da.push_frac = pl->push_frac;
     da.picker = pl->picker;
@@ -2896,6 +2969,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     prep.flagN = pl->flag[nbuf];
     prep.tiny = pl->tiny[fb];
     prep.slots = pl->slot[fb];
+    prep.bits = pl->bits;
     prep.V = V;
     prep.W = W;
     prep.Q = Q;
@@ -3006,6 +3080,8 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
                                                 pl->ctr, h);
       vs::launch_next(k_short_index, pl->grid_v, 256, 0, st, prep);
     }
+    a.bits = pl->bits;
+    if (pl->bits && h > 1) vs::launch_next(var.bits, dim3(pl->grid_bits, pl->nslices), 1024, bits_smem(V), st, a);
     vs::launch_next(var.pull, dim3(pl->grid_pull, pl->nslices), 256, 0, st, a);
     if (pl->slot[0]) {
       const ShortVariant &sv = pick_short(Q);

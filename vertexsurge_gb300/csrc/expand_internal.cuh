@@ -22,6 +22,7 @@ struct HopCtr {
   unsigned scan_done;                  // SPARSE: blocks of its degree scan that have finished
   int overflow;                        // SPARSE: pair list overflowed
   int strategy;                        // strategy run at hop h (0 = not run)
+  int bits;                            // dense PULL reads layer h-1's row flags as bits
   int short_pull;                      // PULL reads the short rows of layer h-1 through their slots
   int short_long;                      // ... and most of its new rows will be too long for a slot
   int short_slots;                     // ... reading slots (count in entry 0) instead of tiny words
@@ -69,6 +70,7 @@ struct SeedArgs {
 struct DecideArgs {
   Ctr *ctr;
   int h, path, forced, picker_on, log_features, both;
+  int bits_ok;  // the plan keeps row flags as bits
   int push_ok;  // the plan launches PUSH kernels (the picker may choose PUSH)
   uint32_t S, V, W, k_min, k_max;
   uint64_t E, pair_cap;
@@ -125,6 +127,7 @@ struct PullArgs {
   const uint4 *F;
   uint4 *N, *vis, *acc;
   const uint32_t *flagF;
+  const uint32_t *bits;  // flagF as bits (NULL: not kept)
   uint32_t *flagN;  // 0: empty row; 1: non-zero row in the buffer; 2: non-zero row held in its slot only
   uint32_t V, Q, qslice;
   int multislice, shortest, acc_on;
