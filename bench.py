@@ -489,12 +489,16 @@ def join_inputs(w, n):
     return (batch.zipf_keys(rng, n, w["V"], perm, w["skew"]), batch.zipf_keys(rng, n, w["V"], perm, w["skew"]))
 
 
-def join_bytes(n_build, n_probe):
-    """Algorithmic bytes of a count-only Flat x Flat join of 4-byte keys
-    (the hash join's compulsory bytes, no output): both key columns read, the
-    table cleared (16 B per slot: key and count, capacity the power of two
-    >= 2 N_b, at least 64), one 16-byte insert per build row and at least one
-    32-byte sector per probe."""
+def join_bytes(n_build, n_probe, key_max):
+    """Algorithmic bytes of a count-only Flat x Flat join of 4-byte vertex-id keys, no
+    output.  Keys below max(4M, 4 N_b) are counted in an array: the build keys read
+    twice (their largest, then their counts), the probe keys once, the array cleared
+    and its counts written once.  Others go through the hash table: both key columns
+    read, the table cleared (16 B per slot: key and count, capacity the power of two
+    >= 2 N_b, at least 64), one 16-byte insert per build row and at least one 32-byte
+    sector per probe."""
+    if key_max < max(1 << 22, 4 * n_build):
+        return 8 * n_build + 4 * n_probe + 8 * (key_max + 1)
     cap = 64
     while cap < 2 * n_build:
         cap *= 2
@@ -562,7 +566,7 @@ def run_join(args, w, rank, world, local_rank, reference=False):
         e1.record(stream)
         torch.cuda.synchronize()
         ms = e0.elapsed_time(e1) / args.steps
-        byt = join_bytes(n, n)
+        byt = join_bytes(n, n, int(kb.max()))
         rows.append({"rows_per_side": n, "ms": ms, "Mrows_per_s": 2 * n / ms / 1e3, "count": c, "bytes": byt,
                      "GB_per_s": byt / ms / 1e6, "frac": byt / ms / 1e6 / peak})
         total_ms += ms
@@ -580,7 +584,8 @@ def run_join(args, w, rank, world, local_rank, reference=False):
             "roofline": {"bound": "hbm", "achieved": big["GB_per_s"], "peak": peak, "unit": "GB/s",
                          "frac": big["frac"], "frac_nominal": big["GB_per_s"] / NOMINAL_HBM_GBS,
                          "traffic": None, "peak_source": peak_kind,
-                         "bytes": "4 N_b + 4 N_p + 16 cap + 16 N_b + 32 N_p (largest size)"},
+                         "bytes": "8 N_b + 4 N_p + 8 (largest key + 1) with the counts in an array, else "
+                                  "4 N_b + 4 N_p + 16 cap + 16 N_b + 32 N_p (largest size)"},
             "cpu_baseline": None, "parity": {"sizes": len(rows), "equal": True,
                                              "against": "numpy sum of multiplicity products per key"},
             "e2e": None, "gpu_launches": vs.kernel_launches() - launches0, "clocks": clk}
@@ -857,27 +862,18 @@ def run_gpu(args, w, rank, world, local_rank):
     ms_per_step = ms / args.steps
     value = world * src_edges * args.steps / (ms / 1e3) / 1e9
 
-    # expand A alone with each short-mode kernel (the next target's visited
-    # words and flag loaded ahead, and not: pull kernel bit 2), per-hop
-    # CUDA-event times of the PULL hops
+    # expand A alone, per-hop CUDA-event times of the PULL hops when some ran in short mode
     short_kernels = None
     if any(stA["short_pull"][1:]):
         short_kernels = {}
-        kind0 = int(tA.get("pull_kind", 0))
-        for name, kind in (("preload", kind0 & 3), ("no_preload", (kind0 & 3) | 4)):
-            pA.set_pull_kernel(kind)
-            per_hop = {}
-            for _ in range(3):
-                pA.run(dA, stream=stream)
-            for _ in range(5):
-                pA.run(dA, stream=stream)
-                sth = pA.stats(stream)
-                for h in range(1, sth["hops_run"] + 1):
-                    if sth["strategy"][h] == vs.STRAT_PULL:
-                        per_hop[str(h)] = per_hop.get(str(h), 0.0) + sth["pull_ms"][h] / 5
-            short_kernels[name] = per_hop
-        pA.set_pull_kernel(kind0)
-        pA.run(dA, stream=stream)  # the result the parity check reads comes from the tuned kernel
+        for _ in range(3):
+            pA.run(dA, stream=stream)
+        for _ in range(5):
+            pA.run(dA, stream=stream)
+            sth = pA.stats(stream)
+            for h in range(1, sth["hops_run"] + 1):
+                if sth["strategy"][h] == vs.STRAT_PULL:
+                    short_kernels[str(h)] = short_kernels.get(str(h), 0.0) + sth["pull_ms"][h] / 5
 
     # e2e: one-shot C-ABI calls, sources from pinned host memory, counts read back
     pA.set_tuning(timing=False)

@@ -2,11 +2,9 @@
 
 For one query shape (graph, source count, hop range, path type, direction) it
 times the expand under candidate settings and keeps the fastest:
-  * the PULL kernel shape (vs_expand_plan_set_pull_kernel: occupancy bound and
-    L2 cache policies),
   * the SPARSE threshold of the fixed planner (pair-list edge work below this
     fraction of E runs as SPARSE),
-  * the hub degree bin (in-degree above which a vertex gets a whole CTA),
+  * the hub degree bin (in-degree above which a vertex's list comes in pieces),
   * the source-word group width (words per PULL pass) for very wide rows,
   * whether PULL hops over sparse frontier rows gather the rows' source lists.
 Timing uses CUDA events around whole plan runs on the plan's stream; every
@@ -43,9 +41,10 @@ def _time_runs(plan, src, repeats, stream):
 
 
 def tune(dg, src, k_min, k_max, path="shortest", direction="forward", stream=None, repeats=3,
-         pull_kinds=(0, 1, 2, 3), sparse_fracs=(0.0005, 0.002, 0.005, 0.02), hub_thresholds=(0, 256),
+         pull_kinds=(0,), sparse_fracs=(0.0005, 0.002, 0.005, 0.02), hub_thresholds=(0, 256),
          slice_words=(0,), short_shares=(0.0, -1.0), cache_file: str | None = None) -> dict:
-    """Time the candidates; returns {'pull_kind', 'sparse_frac', 'hub_threshold', 'slice_words',
+    """Time the candidates (the PULL kernel kinds of vs_expand_plan_set_pull_kernel all run
+    the same kernel; a caller may still pass several); returns {'pull_kind', 'sparse_frac', 'hub_threshold', 'slice_words',
     'short_share', 'ms', 'table'} and caches it."""
     import torch
     key = _key(dg, len(src), k_min, k_max, path, direction)
