@@ -351,7 +351,8 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
     // pays 7 to 18 per edge for neighbour and flag (with the row's lanes) and 0.8
     // per word of every active row from L2; short mode 12.5 per edge, 21 per id read
     // from words (10 on a last hop, which keeps no lists), 1.5 per id read from
-    // slots and 350 per target row then searched for bits (none on a last hop),
+    // slots (with 6 more per edge where slots are wider than 32 bytes: 8,192 sources on
+    // the 10M-vertex power law, hop 3 9.96 ms from slots and 7.28 from words) and 350 per target row then searched for bits (none on a last hop),
     // and about twice the dense price for a row too long for a slot.
     bool sp = false, slots = false, lng = false;
     if (s_choice == ST_PULL && a.short_min > 0 && !c->multislice) {
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
       }
       const float t_long = 1.6f * W * longs;
       const float t_words = 12.5f * E + (a.last ? 10.f : 21.f) * ids + t_long;
-      const float t_slots = 12.5f * E + 1.5f * fminf(ids, 15.f * so) + (a.last ? 0.f : 350.f * fminf(V, ids)) + t_long;
+      const float t_slots = (a.W <= 64 ? 12.5f : 18.5f) * E + 1.5f * fminf(ids, 15.f * so) + (a.last ? 0.f : 350.f * fminf(V, ids)) + t_long;
       slots = counted && t_slots < t_words;
       if (a.short_min > 1.0) {
         sp = true;
@@ -735,10 +736,10 @@ __global__ void __launch_bounds__(256, 4) k_sparse(SparseArgs a) {
 // shared-memory row with 32-bit atomics, and only longer rows are gathered
 // whole (see the kernel).  Short rows of a layer with a successor stay in their slots only
 // (flag 2, buffer row zero) unless the layer's rows are read directly;
-// k_materialize writes them out before a hop that reads rows.  Layers
+// k_hop_prep writes them out before a hop that reads rows.  Layers
 // written by SPARSE or the seed get their words and slots from the hop's
-// pair list (k_pairs_*), layers written by PUSH or an overflowed SPARSE hop
-// from their rows (k_slot_build), when the next hop reads them.
+// pair list (k_pairs_slots, k_short_index), layers written by PUSH or an overflowed SPARSE hop
+// from their rows (k_short_index), when the next hop reads them.
 // A tiny word is 0 for an empty row; otherwise its top two bits are a class:
 // 1 = one id in bits 0..14, 2 = two ids in bits 0..14 and 15..29, 3 = the
 // row's bit count (saturated at 0xFFFF) in bits 0..15, its ids in the slot
@@ -1590,14 +1591,17 @@ __device__ __forceinline__ void word_edges(const PullArgs &a, ShortEdges &s, uin
 }
 
 // 32 edges of a slot hop: u the neighbour, its slot's first 32 bytes.
-template <int MODE>
+template <int MODE, bool WIDE>
 __device__ __forceinline__ void slot_edges(const PullArgs &a, ShortEdges &s, uint32_t own, uint32_t u,
                                            const uint4 first, const uint4 second) {
   uint32_t n = first.x & 0xFFFFu;
   if (!__any_sync(FULL, n)) return;
   if (MODE == SH_GEN) s.touched |= __reduce_or_sync(FULL, n ? 1u << own : 0u);
   s.se += n && n < a.slot_n;
-  const bool far = n >= CHUNK_IDS || n >= a.slot_n;
+  // ids up to the end of a second 32 bytes are read here as well; a slot of 64 entries
+  // with more, and rows longer than a slot, are put aside
+  const bool two = WIDE && n >= CHUNK_IDS && n < 2 * CHUNK_IDS && n < a.slot_n;
+  const bool far = !two && (n >= CHUNK_IDS || n >= a.slot_n);
   put_aside(a, s, far, own, u, n);
   if (far) n = 0;
   const uint32_t mx = __reduce_max_sync(FULL, n);
@@ -1609,13 +1613,26 @@ __device__ __forceinline__ void slot_edges(const PullArgs &a, ShortEdges &s, uin
     const uint32_t id = i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu;
     if (i <= n && may_grow(a, id)) or_id(row, id);
   }
+  // (put aside, two slots at a time by the whole warp, rows of 16 to 31 ids took twice
+  // as long: 8,192 sources on the 10M-vertex power law, hop 4 30.5 -> 14.4 ms)
+  if (WIDE && __any_sync(FULL, two)) {
+    uint4 x = make_uint4(0, 0, 0, 0), y = x;
+    if (two) ld_slot(a.slot_in + (size_t)u * (a.slot_n / 8) + 2, x, y);
+    const uint32_t z[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (uint32_t i = 0; i < CHUNK_IDS; i++) {
+      if (CHUNK_IDS + i > mx) break;
+      const uint32_t id = i & 1 ? z[i >> 1] >> 16 : z[i >> 1] & 0xFFFFu;
+      if (two && CHUNK_IDS + i <= n && may_grow(a, id)) or_id(row, id);
+    }
+  }
 }
 
 // The in-lists of the tile's targets, end to end (lane t: length deg of target t,
 // which starts at entry `at` of adj; consecutive lists are consecutive there, a
 // gap is a target that comes in pieces).  Rounds of G x 32 edges with their loads
 // in flight at once; the warps of the SM cover the waits.
-template <int MODE, bool SLOTS, int T>
+template <int MODE, int SLOTS, int T>
 __device__ __forceinline__ void short_edges(const PullArgs &a, ShortEdges &s, const uint32_t *__restrict__ adj,
                                             int64_t at, uint32_t deg, bool gaps) {
   constexpr int G = SLOTS ? 2 : SH_GROUP;
@@ -1657,13 +1674,13 @@ __device__ __forceinline__ void short_edges(const PullArgs &a, ShortEdges &s, co
         if (u[k] != NONE) ld_slot(a.slot_in + (size_t)u[k] * sq, x[k], y[k]);
       }
 #pragma unroll
-      for (int k = 0; k < G; k++) slot_edges<MODE>(a, s, own[k], u[k], x[k], y[k]);
+      for (int k = 0; k < G; k++) slot_edges<MODE, SLOTS == 2>(a, s, own[k], u[k], x[k], y[k]);
     }
     drain<MODE>(a, s, c + 32 * G >= total);
   }
 }
 
-template <int MODE, bool SLOTS, int T>
+template <int MODE, int SLOTS, int T>
 __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
   const uint32_t lane = threadIdx.x & 31, Q = a.Q;
   uint4 *bm = s_short + wb;
@@ -1889,11 +1906,11 @@ inline size_t short_smem(uint32_t Q, uint32_t slot_n) {
 // will mostly be long finishes LIST as GEN; whether it reads words or slots is the
 // device's: of the two kernels of a hop one returns at once (one kernel for both
 // would need the registers of both).
-template <int MODE, bool SLOTS, int T>
+template <int MODE, int SLOTS, int T>
 __global__ void __launch_bounds__(SH_WARPS * 32, 4) k_pull_short(const __grid_constant__ PullArgs a) {
   vs::grid_wait();
   const HopCtr &hc = a.ctr->hop[a.h];
-  if (hc.strategy != ST_PULL || !hc.short_pull || !a.tiny_in || (hc.short_slots != 0) != SLOTS ||
+  if (hc.strategy != ST_PULL || !hc.short_pull || !a.tiny_in || (hc.short_slots != 0) != (SLOTS != 0) ||
       (MODE == SH_LIST && hc.short_long) || (MODE == SH_GEN && a.list_too && !hc.short_long))
     return;
   for (uint32_t q = threadIdx.x; q < a.Q; q += blockDim.x) {
@@ -2381,17 +2398,21 @@ Lists push_lists(const vs_graph *g, int dir) {
 
 using PullFn = void (*)(PullArgs);
 
-// Short-mode kernels of a tile size: words and slots by mode (a slot hop has no LIST).
+// Short-mode kernels of a row width: words and slots by mode (a slot hop has no LIST).
+// Slots of 16 entries have kernels of their own: the second piece of a wider one,
+// never there, cost 4% of a 14 ms run in registers and code.
 struct ShortVariant {
   uint32_t T;
   PullFn words[3], slots[3];
 };
-#define VS_SHORT(T) \
-  {T, {k_pull_short<SH_LIST, false, T>, k_pull_short<SH_LAST, false, T>, k_pull_short<SH_GEN, false, T>}, \
-   {nullptr, k_pull_short<SH_LAST, true, T>, k_pull_short<SH_GEN, true, T>}}
-const ShortVariant kShort[2] = {VS_SHORT(4), VS_SHORT(2)};
+#define VS_SHORT(T, K) \
+  {T, {k_pull_short<SH_LIST, 0, T>, k_pull_short<SH_LAST, 0, T>, k_pull_short<SH_GEN, 0, T>}, \
+   {nullptr, k_pull_short<SH_LAST, K, T>, k_pull_short<SH_GEN, K, T>}}
+const ShortVariant kShort[3] = {VS_SHORT(4, 1), VS_SHORT(4, 2), VS_SHORT(2, 2)};
 #undef VS_SHORT
-const ShortVariant &pick_short(uint32_t Q) { return kShort[short_tile(Q) == 4 ? 0 : 1]; }
+const ShortVariant &pick_short(uint32_t Q, uint32_t slot_n) {
+  return kShort[short_tile(Q) == 2 ? 2 : slot_n > CHUNK_IDS ? 1 : 0];
+}
 
 struct PullVariant {
   int L, UPL;
@@ -2797,7 +2818,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   if (pl->slot[0]) {
     const size_t sm = short_smem(pl->Q, pl->slot_n);
     int occ_short = 0;
-    const ShortVariant &sv = pick_short(pl->Q);
+    const ShortVariant &sv = pick_short(pl->Q, pl->slot_n);
     for (PullFn f : {sv.words[0], sv.words[1], sv.words[2], sv.slots[1], sv.slots[2]}) {
       if (sm > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       occ_short = std::max(occ_short, occupancy_grid(f, SH_WARPS * 32, sm, 8));
@@ -3084,7 +3105,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     if (pl->bits && h > 1) vs::launch_next(var.bits, dim3(pl->grid_bits, pl->nslices), 1024, bits_smem(V), st, a);
     vs::launch_next(var.pull, dim3(pl->grid_pull, pl->nslices), 256, 0, st, a);
     if (pl->slot[0]) {
-      const ShortVariant &sv = pick_short(Q);
+      const ShortVariant &sv = pick_short(Q, pl->slot_n);
       const size_t sm = short_smem(Q, pl->slot_n);
       const bool last = a.last && a.shortest && !a.acc_on;
       a.list_too = !last && a.tiny_out && a.virt_out && !a.acc_on;
