@@ -1166,8 +1166,12 @@ __global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : U
     s_un[q] = make_uint4(0, 0, 0, 0);
   }
   __syncthreads();
-  // a row of one sector is loaded as fast as its flag, and a nearly full layer has few rows to skip
-  const bool useflag = a.Q > 2 && pc.active_vertices * 10 < 9ull * a.V;
+  // a row of one sector is loaded as fast as its flag, and a nearly full layer has few
+  // rows to skip.  On a graph below the bits' size a hop is bound by its chains of loads:
+  // rows of up to four uint4 come without the flag before them, eight at a time (R-MAT of
+  // 4K to 64K vertices, 300 to 500 sources: 6 to 20% of a run, power laws 1 to 12%; wider
+  // rows lose up to 4% at eight uint4 and 13% at sixteen)
+  const bool useflag = a.Q > 2 && pc.active_vertices * 10 < 9ull * a.V && !(L <= 4 && a.V < BITS_MIN_V);
   const uint32_t *flag = BITS ? reinterpret_cast<const uint32_t *>(s_bits) : useflag ? a.flagF : nullptr;
   const uint4 *F = a.F + q0;
   const bool known = a.res_vis && a.Q >= 8;  // resflag 0: the visited row is zero, without reading it
