@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(256) k_isect(Args a) {
           } else if (keep) {
             if (d.kind == DEP_MAT) {
               keep = x < d.rows && ((d.words[(size_t)col[i] * d.wpc + (x >> 6)] >> (x & 63)) & 1ull);
-            } else if (meth[i] == M_BITMAP) {
-              keep = (__ldg(d.hub_bm + (size_t)hs[i] * d.hub_words + (x >> 6)) >> (x & 63)) & 1ull;
+            } else if (meth[i] == M_BITMAP) {  // the walked list may be another graph's, with more vertices
+              keep = x < d.n_u && (__ldg(d.hub_bm + (size_t)hs[i] * d.hub_words + (x >> 6)) >> (x & 63)) & 1ull;
             } else if (d.kind == DEP_SORTED) {
               keep = in_sorted(d.adj, lo[i], hi[i], x);
             } else {
@@ -328,11 +328,12 @@ __device__ __forceinline__ PairTuple pair_tuple(const Args &a, uint64_t t, int l
   return p;
 }
 
-// Candidate x of a walked list in the other list of its tuple.
+// Candidate x of a walked list in the other list of its tuple (of another graph,
+// perhaps: its bitmaps end at its own last vertex).
 __device__ __forceinline__ bool pair_member(const Args &a, int w1, int hs, int64_t olo, int64_t ohi, uint32_t x) {
   if (x >= a.cache_rows) return false;
   const Dep &o = w1 ? a.dep[0] : a.dep[1];
-  return hs >= 0 ? ((__ldg(o.hub_bm + (size_t)hs * o.hub_words + (x >> 6)) >> (x & 63)) & 1ull)
+  return hs >= 0 ? x < o.n_u && ((__ldg(o.hub_bm + (size_t)hs * o.hub_words + (x >> 6)) >> (x & 63)) & 1ull)
                  : in_sorted(o.adj, olo, ohi, x);
 }
 
