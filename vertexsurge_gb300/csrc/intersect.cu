@@ -820,7 +820,8 @@ int grid_for(uint64_t n, int per_block = 256) {
 }
 
 // The hub bitmaps of one list direction of g, built once (the smallest
-// power-of-two degree threshold within the budgets above).
+// power-of-two degree threshold within the budgets above); none are left behind by a
+// call that fails.
 int hub_index(vs_graph *g, bool fwd, cudaStream_t st, const vs_hub_index **out) {
   std::lock_guard<std::mutex> lock(g->hub_mu);
   vs_hub_index &h = g->hub[fwd ? 0 : 1];
@@ -832,14 +833,14 @@ int hub_index(vs_graph *g, bool fwd, cudaStream_t st, const vs_hub_index **out) 
   h.words = (V + 63) / 64;
   const uint64_t per = (uint64_t)h.words * 8;
   const uint64_t cap = std::min<uint64_t>(HUB_BUDGET / std::max<uint64_t>(per, 1), 1u << 20);
+  Scratch sc{st};
   unsigned long long *bins = nullptr;
-  VS_TRY(dalloc_n(&bins, 64, st));
+  VS_TRY(sc.get(&bins, 64));
   VS_CK(cudaMemsetAsync(bins, 0, 64 * 8, st));
   if (V) { k_deg_bins<<<grid_for(V), 256, 0, st>>>(off, V, bins); vs::note_launch(); }
   unsigned long long hb[64];
   VS_CK(cudaMemcpyAsync(hb, bins, sizeof(hb), cudaMemcpyDeviceToHost, st));
   VS_CK(cudaStreamSynchronize(st));
-  dfree(bins, st);
   // bin k holds degrees in [2^k, 2^(k+1)): hubs with degree >= 2^k number sum(hb[k..])
   int k = 0;
   while ((1ull << k) < HUB_MIN_DEG) k++;
@@ -850,27 +851,39 @@ int hub_index(vs_graph *g, bool fwd, cudaStream_t st, const vs_hub_index **out) 
   while (k > 0 && (1ull << (k - 1)) >= LIST_MIN_DEG && n + hb[k - 1] <= cap && (n + hb[k - 1]) * per <= LIST_BUDGET)
     n += hb[--k];
   h.min_deg = (uint32_t)std::min<uint64_t>(1ull << k, 0xffffffffull);
-  h.n = (uint32_t)n;
-  h.built = true;
   if (n == 0 || cap == 0) {
-    h.n = 0;
+    h.built = true;
     return VS_OK;
   }
+  // without room for them the call goes on by binary search, and a later one tries again
   uint32_t *hubs = nullptr;
   unsigned *cnt = nullptr;
-  VS_TRY(dalloc_n(&h.slot, V, st));
-  VS_TRY(dalloc_n(&h.bm, (size_t)n * h.words, st));
-  VS_TRY(dalloc_n(&hubs, n, st));
-  VS_TRY(dalloc_n(&cnt, 1, st));
-  VS_CK(cudaMemsetAsync(cnt, 0, 4, st));
-  VS_CK(cudaMemsetAsync(h.bm, 0, (size_t)n * per, st));
-  { k_hub_slots<<<grid_for(V), 256, 0, st>>>(off, V, h.min_deg, (uint32_t)n, h.slot, hubs, cnt); vs::note_launch(); }
-  { k_hub_fill<<<(unsigned)std::min<uint64_t>(n, (uint64_t)sm_count() * 8), 256, 0, st>>>(off, adj, hubs, (uint32_t)n,
-                                                                                      h.bm, h.words); vs::note_launch(); }
-  VS_CK(cudaGetLastError());
-  VS_CK(cudaStreamSynchronize(st));  // other streams may use the bitmaps next
-  dfree(hubs, st);
-  dfree(cnt, st);
+  int32_t *slot = nullptr;
+  uint64_t *bm = nullptr;
+  int rc = VS_OK;
+  if ((rc = sc.get(&hubs, n)) != VS_OK || (rc = sc.get(&cnt, 1)) != VS_OK || (rc = dalloc_n(&slot, V, st)) != VS_OK ||
+      (rc = dalloc_n(&bm, (size_t)n * h.words, st)) != VS_OK) {
+    dfree(slot, st);
+    return rc == VS_ERR_OOM ? VS_OK : rc;
+  }
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 4, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(bm, 0, (size_t)n * per, st);
+  if (e == cudaSuccess) {
+    { k_hub_slots<<<grid_for(V), 256, 0, st>>>(off, V, h.min_deg, (uint32_t)n, slot, hubs, cnt); vs::note_launch(); }
+    { k_hub_fill<<<(unsigned)std::min<uint64_t>(n, (uint64_t)sm_count() * 8), 256, 0, st>>>(off, adj, hubs, (uint32_t)n, bm,
+                                                                                        h.words); vs::note_launch(); }
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // other streams may use the bitmaps next
+  if (e != cudaSuccess) {
+    dfree(slot, st);
+    dfree(bm, st);
+    return cuda_fail(e, "adjacency bitmaps", __FILE__, __LINE__);
+  }
+  h.slot = slot;
+  h.bm = bm;
+  h.n = (uint32_t)n;
+  h.built = true;
   return VS_OK;
 }
 
