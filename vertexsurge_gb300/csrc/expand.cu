@@ -1711,6 +1711,7 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
       const int64_t beg = a.in.off[pc.z][pc.x] + pc.w, end = a.in.off[pc.z][pc.x + 1];
       const uint32_t n = (uint32_t)min((int64_t)a.piece_edges, end - beg);
       short_edges<SH_GEN, SLOTS, 1>(a, s, a.in.adj[pc.z], beg, lane ? 0u : n, false);
+      __syncwarp();  // every lane's ids are in the bitmap
       bool mine = true;
       if (np > 1) {
         uint4 *sum = a.heavy_rows + (size_t)pc.y * Q;
