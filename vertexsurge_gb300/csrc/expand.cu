@@ -1432,6 +1432,7 @@ template <int MODE> __device__ __forceinline__ unsigned do_aside(const PullArgs 
         }
       }
     }
+    __syncwarp();  // ids are in before the next pair's whole rows are added word by word
   }
   return whole;
 }
