@@ -1898,7 +1898,8 @@ inline void short_layout(PullArgs &a, uint32_t T) {
   a.sh_aside = a.sh_queue + (8 + SH_IDS) / 4;
   a.sh_warp = a.sh_aside + SH_ASIDE / 2;
 }
-// Targets per tile: rows up to 512 bytes eight, wider ones two.
+constexpr uint32_t SHORT_MAX_Q = 256;  // cells of the widest rows (ids of 15 bits)
+// Targets per tile: rows up to 1 KB four, wider ones two.
 inline uint32_t short_tile(uint32_t Q) { return Q <= 64 ? 4 : 2; }
 inline size_t short_smem(uint32_t Q, uint32_t slot_n) {
   PullArgs a;
@@ -2517,7 +2518,7 @@ inline uint32_t slot_entries(uint32_t W) { return W <= 64 ? 16 : W <= 128 ? 32 :
 // of L2, nor for rows below 32 words: a dense hop of 16-word rows took 0.25 ms on
 // the 1M-vertex power law where a short one took 0.38 (unless forced: share > 1).
 inline bool short_slots_ok(uint32_t S, uint32_t nslices, double share, uint64_t V, uint32_t W) {
-  return share >= 0 && S <= 32768 && nslices == 1 && (share > 1.0 || (W >= 32 && V * 8ull * W > l2_bytes() / 2));
+  return share >= 0 && S <= 128 * SHORT_MAX_Q && nslices == 1 && (share > 1.0 || (W >= 32 && V * 8ull * W > l2_bytes() / 2));
 }
 
 // Whether a plan's dense PULL hops may read row flags as bits.  Whole runs against flags
@@ -2826,7 +2827,10 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     int occ_short = 0;
     const ShortVariant &sv = pick_short(pl->Q, pl->slot_n);
     for (PullFn f : {sv.words[0], sv.words[1], sv.words[2], sv.slots[1], sv.slots[2]}) {
-      if (sm > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      // the limit is the kernel's, which plans of other widths share: that of the widest rows
+      if (sm > 48 * 1024)
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)short_smem(SHORT_MAX_Q, slot_entries(2 * SHORT_MAX_Q)));
       occ_short = std::max(occ_short, occupancy_grid(f, SH_WARPS * 32, sm, 8));
     }
     const uint64_t stasks = pl->npieces + ((uint64_t)V + short_tile(pl->Q) - 1) / short_tile(pl->Q);
