@@ -944,33 +944,54 @@ __device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__re
       sat = sat || c;
     }
   } else {
+    // The non-empty rows of 32 entries are numbered through shared memory, so that a
+    // round of R rows is R addresses, loads and ORs without a search for the next bit,
+    // a select and a test per row: 39 -> 21 warp instructions a list entry, which
+    // bounds rows that come from L2 (40K vertices of 60 neighbours, 4,096 sources: 122 ->
+    // 88 us a hop; the 1M-vertex power law's four hops 3.90 -> 3.63 ms).
     constexpr int R = UPL == 1 ? 8 : UPL == 2 ? 4 : 2;  // rows in flight
+    __shared__ uint4 s_id[8][8];
+    uint32_t *ids = reinterpret_cast<uint32_t *>(s_id[threadIdx.x >> 5]);
     for (; j < n && !sat; j += step) {
       uint32_t id = NONE;
       if (j + lane < n) id = __ldg(adj + j + lane);
       if ((BITS || flag) && id != NONE && !has_row<BITS>(flag, id)) id = NONE;
-      unsigned m = __ballot_sync(FULL, id != NONE);
-      while (m) {
+      const unsigned m = __ballot_sync(FULL, id != NONE);
+      const int c = __popc(m);
+      __syncwarp();  // every lane is past the last entries
+      if (id != NONE) ids[__popc(m & lanemask_lt())] = id;
+      __syncwarp();
+      for (int t = 0; t < c; t += R) {
         uint32_t u[R];
 #pragma unroll
-        for (int k = 0; k < R; k++) {  // m is the same on every lane
-          const uint32_t t = __shfl_sync(FULL, id, m ? __ffs(m) - 1 : 0);
-          u[k] = m ? t : NONE;
-          m &= m - 1;
-        }
+        for (int k = 0; k < R; k++) u[k] = ids[t + k];  // R divides 32; those from c on are not used
+        if (t + R <= c) {
 #pragma unroll
-        for (int t = 0; t < UPL; t++) {
-          const uint32_t q = lane + t * 32;
-          uint4 x[R];
+          for (int i = 0; i < UPL; i++) {
+            const uint32_t q = lane + i * 32;
+            if (q < qn) {
+              uint4 x[R];
 #pragma unroll
-          for (int k = 0; k < R; k++) {
-            x[k] = make_uint4(0, 0, 0, 0);
-            if (u[k] != NONE && q < qn) x[k] = __ldg(F + (size_t)u[k] * a.Q + q);
+              for (int k = 0; k < R; k++) x[k] = __ldg(F + (size_t)u[k] * a.Q + q);
+#pragma unroll
+              for (int k = 0; k < R; k++) acc[i] = or4(acc[i], x[k]);
+            }
           }
+        } else {
 #pragma unroll
-          for (int k = 0; k < R; k++) acc[t] = or4(acc[t], x[k]);
+          for (int i = 0; i < UPL; i++) {
+            const uint32_t q = lane + i * 32;
+            uint4 x[R];
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+              x[k] = make_uint4(0, 0, 0, 0);
+              if (t + k < c && q < qn) x[k] = __ldg(F + (size_t)u[k] * a.Q + q);
+            }
+#pragma unroll
+            for (int k = 0; k < R; k++) acc[i] = or4(acc[i], x[k]);
+          }
         }
-        if (group_all<32>(covered<L, UPL>(s_um, qn, vv, acc))) {
+        if ((t + R < c || j + step < n) && group_all<32>(covered<L, UPL>(s_um, qn, vv, acc))) {
           sat = true;
           break;
         }
