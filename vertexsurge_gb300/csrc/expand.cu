@@ -991,7 +991,8 @@ __device__ __forceinline__ void gather_list(const PullArgs &a, const uint4 *__re
             for (int k = 0; k < R; k++) acc[i] = or4(acc[i], x[k]);
           }
         }
-        if ((t + R < c || j + step < n) && group_all<32>(covered<L, UPL>(s_um, qn, vv, acc))) {
+        // whether the row is complete is asked every 8 rows: 60 instructions for a row of 8 uint4 a lane
+        if ((t + R) % 8 == 0 && (t + R < c || j + step < n) && group_all<32>(covered<L, UPL>(s_um, qn, vv, acc))) {
           sat = true;
           break;
         }
@@ -1164,7 +1165,7 @@ __device__ __forceinline__ void group_epilogue(const PullArgs &a, uint32_t v, bo
 // 1,001 sources both ways on R-MAT 20, hops 2 to 5 2.25 -> 2.06 ms; 2,048 sources on the
 // power law, two hops 1.20 -> 1.09 ms.
 template <int L, int UPL, bool BITS>
-__global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : UPL == 2 ? 3 : UPL == 4 ? 2 : 1)
+__global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : UPL == 2 ? 3 : 2)
     k_pull(PullArgs a) {
   vs::grid_wait();
   HopCtr &hc = a.ctr->hop[a.h];
