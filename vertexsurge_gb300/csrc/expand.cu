@@ -1328,9 +1328,9 @@ __global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : U
 // their rows as bitmaps in shared memory.  Their in-lists lie end to end in the
 // CSR and are read as one range, 32 edges at a time whatever the degrees, a lane
 // per edge, the loads of several such rounds in flight at once:
-//   words  most edges of such a layer come from empty rows, so the ids of the
-//          others are queued and OR-ed into the bitmaps 32 at a time, a full
-//          warp whatever target they belong to;
+//   words  a lane per edge ORs its word's ids; where they are also appended to lists
+//          (LIST), and most edges come from empty rows, they are queued and taken 32 at
+//          a time, a full warp whatever target they belong to;
 //   slots  a lane per edge ORs its slot's ids.
 // In-neighbours with 16 ids or more are put aside: those with a slot are done by
 // all lanes, an id each, the others are rows gathered whole.
@@ -1342,7 +1342,7 @@ __global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : U
 //         Long rows, and targets that got a whole row, are done from the bitmap.
 //   LAST  nothing follows the layer: the bitmaps start as the visited rows and
 //         are written back; popcounts before and after give the new bits.
-//   GEN   any other hop (accumulator, kept layer, long new rows): the bitmaps
+//   GEN   any other hop (slots, accumulator, kept layer, long new rows): the bitmaps
 //         start empty and finish_row does every touched target.
 //
 // What bounds it: instructions and latency (about 170 warp instructions a target at
@@ -1459,50 +1459,84 @@ template <int MODE> __device__ __forceinline__ unsigned do_aside(const PullArgs 
   return whole;
 }
 
-// A target from its bitmap row (raw unions, or unions and visited bits): new bits
-// = row & ~visited; visited, accumulator, union, next-layer row, word, slot,
-// flag.  The row is overwritten with the new bits; returns their number.
-__device__ __forceinline__ uint32_t finish_row(const PullArgs &a, uint32_t wb, uint32_t t, uint32_t v) {
-  uint4 *row = s_short + wb + t * a.Q, *s_un = s_short;
+// The new bits of the T targets from v0 on that are in fm, from their bitmap rows (raw
+// unions, or unions and visited bits): row & ~visited, left in the bitmap; visited,
+// accumulator, union.  The targets' visited and accumulator cells are in flight at
+// once: one target after the other cost a chain of three misses each (4,096 sources on
+// the 10M-vertex power law, a hop into an accumulator, 8.4 -> 7.7 ms).  Lane t gets
+// target t's number of new bits.
+template <int T>
+__device__ __forceinline__ uint32_t new_bits(const PullArgs &a, uint32_t wb, unsigned fm, uint32_t v0) {
+  uint4 *rows = s_short + wb, *s_un = s_short;
   const uint4 *hm = a.hmask ? s_short + a.Q : nullptr;
-  uint16_t *list = reinterpret_cast<uint16_t *>(s_short + wb + a.sh_list) + t * a.slot_n;
   const uint32_t lane = threadIdx.x & 31;
   __syncwarp();
-  const uint32_t oldf = a.flagN[v];
-  uint32_t bits = 0;
+  uint32_t bits[T];
+#pragma unroll
+  for (int t = 0; t < T; t++) bits[t] = 0;
   for (uint32_t q = lane; q < a.Q; q += 32) {
-    const size_t idx = (size_t)v * a.Q + q;
-    uint4 x = row[q];
-    if (hm) x = and4(x, hm[q]);
-    if (nz4(x) && a.shortest) {
-      const uint4 vv = a.vis[idx];
-      x = andnot4(x, vv);
-      if (nz4(x)) a.vis[idx] = or4(vv, x);
+    uint4 x[T], y[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+      x[t] = fm >> t & 1u ? rows[t * a.Q + q] : make_uint4(0, 0, 0, 0);
+      if (hm) x[t] = and4(x[t], hm[q]);
     }
-    if (nz4(x)) {
-      bits += popc4(x);
-      if (a.acc_on) {
-        const uint4 o = a.acc[idx];
-        if (nz4(andnot4(x, o))) a.acc[idx] = or4(o, x);
-      }
-      if (!a.last) {
-        const uint4 n = andnot4(x, s_un[q]);
-        unsigned *w = reinterpret_cast<unsigned *>(s_un + q);
-        if (n.x) atomicOr(w, n.x);
-        if (n.y) atomicOr(w + 1, n.y);
-        if (n.z) atomicOr(w + 2, n.z);
-        if (n.w) atomicOr(w + 3, n.w);
+    if (a.shortest) {
+#pragma unroll
+      for (int t = 0; t < T; t++) y[t] = nz4(x[t]) ? a.vis[(size_t)(v0 + t) * a.Q + q] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int t = 0; t < T; t++) {
+        x[t] = andnot4(x[t], y[t]);
+        if (nz4(x[t])) a.vis[(size_t)(v0 + t) * a.Q + q] = or4(y[t], x[t]);
       }
     }
-    row[q] = x;
+    if (a.acc_on) {
+#pragma unroll
+      for (int t = 0; t < T; t++) y[t] = nz4(x[t]) ? a.acc[(size_t)(v0 + t) * a.Q + q] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int t = 0; t < T; t++)
+        if (nz4(andnot4(x[t], y[t]))) a.acc[(size_t)(v0 + t) * a.Q + q] = or4(y[t], x[t]);
+    }
+    uint4 u = x[0];
+#pragma unroll
+    for (int t = 1; t < T; t++) u = or4(u, x[t]);
+    if (!a.last) {
+      const uint4 n = andnot4(u, s_un[q]);
+      unsigned *w = reinterpret_cast<unsigned *>(s_un + q);
+      if (n.x) atomicOr(w, n.x);
+      if (n.y) atomicOr(w + 1, n.y);
+      if (n.z) atomicOr(w + 2, n.z);
+      if (n.w) atomicOr(w + 3, n.w);
+    }
+#pragma unroll
+    for (int t = 0; t < T; t++)
+      if (fm >> t & 1u) {
+        rows[t * a.Q + q] = x[t];
+        bits[t] += popc4(x[t]);
+      }
   }
-  const uint32_t total = __reduce_add_sync(FULL, bits);
+  uint32_t total = 0;
+#pragma unroll
+  for (int t = 0; t < T; t++) {
+    const uint32_t n = __reduce_add_sync(FULL, bits[t]);
+    if (lane == t) total = n;
+  }
+  return total;
+}
+
+// What follows from target t's new bits (in its bitmap row, `total` of them): next-layer
+// row, word, slot, flag (oldf before).
+__device__ __forceinline__ void finish_row(const PullArgs &a, uint32_t wb, uint32_t t, uint32_t v, uint32_t total,
+                                           uint32_t oldf) {
+  uint4 *row = s_short + wb + t * a.Q;
+  uint16_t *list = reinterpret_cast<uint16_t *>(s_short + wb + a.sh_list) + t * a.slot_n;
+  const uint32_t lane = threadIdx.x & 31;
   if (lane == 0 && total && (a.res_vis || a.acc_on)) a.resflag[v] = 1;
   if (a.last) {  // layer k_max is not kept: leave the buffer row and its flag clean
     if (oldf == 1)
       for (uint32_t q = lane; q < a.Q; q += 32) a.N[(size_t)v * a.Q + q] = make_uint4(0, 0, 0, 0);
     if (lane == 0 && oldf) a.flagN[v] = 0;
-    return total;
+    return;
   }
   bool virt = false;
   if (a.tiny_out) {
@@ -1545,7 +1579,6 @@ __device__ __forceinline__ uint32_t finish_row(const PullArgs &a, uint32_t wb, u
     const uint32_t nf = total ? (virt ? 2u : 1u) : 0u;
     if (nf != oldf) a.flagN[v] = nf;
   }
-  return total;
 }
 
 // What a warp carries over the edges of its tile.
@@ -1554,6 +1587,7 @@ struct ShortEdges {
   unsigned whole, touched;      // targets that got a whole row; any id
 };
 
+constexpr int SLOT_LANES = 4;                       // slots of 32 and more ids among 32 edges worth reading in place
 constexpr uint32_t SH_GROUP = 2;                    // word hops: 32-edge items per round
 constexpr uint32_t SH_IDS = 32 + SH_GROUP * 64;     // queued ids at most
 constexpr uint32_t SH_ASIDE = 32 + SH_GROUP * 32;   // in-neighbours put aside at most
@@ -1601,18 +1635,50 @@ template <int MODE> __device__ __forceinline__ void drain(const PullArgs &a, Sho
   }
 }
 
+// ids 1..n of a slot's first 32 bytes into a target's bitmap.
+__device__ __forceinline__ void or_chunk(const PullArgs &a, uint32_t *row, uint32_t n, uint32_t mx, const uint4 x,
+                                         const uint4 y) {
+  const uint32_t w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+  for (uint32_t i = 1; i < CHUNK_IDS; i++) {
+    if (i > mx) break;
+    const uint32_t id = i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu;
+    if (i <= n && may_grow(a, id)) or_id(row, id);
+  }
+}
+
+// The same for the lanes with n ids in vertex u's slot, loaded here.
+__device__ __forceinline__ void or_slot(const PullArgs &a, uint32_t *row, uint32_t n, uint32_t u) {
+  uint4 x = make_uint4(0, 0, 0, 0), y = x;
+  if (n) ld_slot(a.slot_in + (size_t)u * (a.slot_n / 8), x, y);
+  or_chunk(a, row, n, __reduce_max_sync(FULL, n), x, y);
+}
+
 // 32 edges of a word hop: u the neighbour (NONE: no edge), t its word, own the target.
 template <int MODE>
 __device__ __forceinline__ void word_edges(const PullArgs &a, ShortEdges &s, uint32_t own, uint32_t u, Tiny t) {
   if (!__any_sync(FULL, t)) return;
   const uint32_t cls = t >> 30;
   if (MODE == SH_GEN) s.touched |= __reduce_or_sync(FULL, t ? 1u << own : 0u);
-  queue_id(a, s, cls == 1 || cls == 2, own, t & 0x7FFFu);
+  const uint32_t id0 = t & 0x7FFFu, id1 = t >> 15 & 0x7FFFu;
+  const bool one = cls == 1 || cls == 2;
+  uint32_t *row = reinterpret_cast<uint32_t *>(s_short + s.wb + own * a.Q);
+  if (MODE == SH_LIST)
+    queue_id(a, s, one, own, id0);
+  else if (one && may_grow(a, id0))  // no list to append to: into the bitmap at once
+    or_id(row, id0);
   uint32_t n = cls;
   if (__any_sync(FULL, cls > 1)) {
-    queue_id(a, s, cls == 2, own, t >> 15 & 0x7FFFu);
+    if (MODE == SH_LIST)
+      queue_id(a, s, cls == 2, own, id1);
+    else if (cls == 2 && may_grow(a, id1))
+      or_id(row, id1);
     if (cls == 3) n = t & 0xFFFFu;
-    put_aside(a, s, cls == 3, own, u, n);  // 3 to 15 ids: an id per lane too
+    // 3 to 15 ids: each lane its own slot where no list grows, else put aside, an id per
+    // lane of the warp (put aside always, layers of 3 to 5 ids a row took 1.6 times as long)
+    const bool held = MODE != SH_LIST && cls == 3 && n < CHUNK_IDS;
+    put_aside(a, s, cls == 3 && !held, own, u, n);
+    if (MODE != SH_LIST && __any_sync(FULL, held)) or_slot(a, row, held ? n : 0u, u);
   }
   s.se += n && n < a.slot_n;
 }
@@ -1625,34 +1691,33 @@ __device__ __forceinline__ void slot_edges(const PullArgs &a, ShortEdges &s, uin
   if (!__any_sync(FULL, n)) return;
   if (MODE == SH_GEN) s.touched |= __reduce_or_sync(FULL, n ? 1u << own : 0u);
   s.se += n && n < a.slot_n;
-  // ids up to the end of a second 32 bytes are read here as well; a slot of 64 entries
-  // with more, and rows longer than a slot, are put aside
-  const bool two = WIDE && n >= CHUNK_IDS && n < 2 * CHUNK_IDS && n < a.slot_n;
-  const bool far = !two && (n >= CHUNK_IDS || n >= a.slot_n);
+  // a wide slot's further 32 bytes are read here as well; where few lanes have more
+  // than two of them, those lanes' slots, and rows longer than a slot, are put aside
+  bool far = n >= (WIDE ? a.slot_n : CHUNK_IDS);
+  if (WIDE) {
+    const bool many = n >= 2 * CHUNK_IDS && !far;
+    if (__popc(__ballot_sync(FULL, many)) < SLOT_LANES) far = far || many;
+  }
   put_aside(a, s, far, own, u, n);
   if (far) n = 0;
   const uint32_t mx = __reduce_max_sync(FULL, n);
   uint32_t *row = reinterpret_cast<uint32_t *>(s_short + s.wb + own * a.Q);
-  const uint32_t w[8] = {first.x, first.y, first.z, first.w, second.x, second.y, second.z, second.w};
-#pragma unroll
-  for (uint32_t i = 1; i < CHUNK_IDS; i++) {
-    if (i > mx) break;
-    const uint32_t id = i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu;
-    if (i <= n && may_grow(a, id)) or_id(row, id);
-  }
+  or_chunk(a, row, n, mx, first, second);
   // (put aside, two slots at a time by the whole warp, rows of 16 to 31 ids took twice
   // as long: 8,192 sources on the 10M-vertex power law, hop 4 30.5 -> 14.4 ms)
-  if (WIDE && __any_sync(FULL, two)) {
-    uint4 x = make_uint4(0, 0, 0, 0), y = x;
-    if (two) ld_slot(a.slot_in + (size_t)u * (a.slot_n / 8) + 2, x, y);
-    const uint32_t z[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  if (WIDE)
+    for (uint32_t i0 = CHUNK_IDS; i0 <= mx; i0 += CHUNK_IDS) {
+      const bool on = n >= i0;
+      uint4 x = make_uint4(0, 0, 0, 0), y = x;
+      if (on) ld_slot(a.slot_in + (size_t)u * (a.slot_n / 8) + i0 / 8, x, y);
+      const uint32_t z[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
-    for (uint32_t i = 0; i < CHUNK_IDS; i++) {
-      if (CHUNK_IDS + i > mx) break;
-      const uint32_t id = i & 1 ? z[i >> 1] >> 16 : z[i >> 1] & 0xFFFFu;
-      if (two && CHUNK_IDS + i <= n && may_grow(a, id)) or_id(row, id);
+      for (uint32_t i = 0; i < CHUNK_IDS; i++) {
+        if (i0 + i > mx) break;
+        const uint32_t id = i & 1 ? z[i >> 1] >> 16 : z[i >> 1] & 0xFFFFu;
+        if (on && i0 + i <= n && may_grow(a, id)) or_id(row, id);
+      }
     }
-  }
 }
 
 // The in-lists of the tile's targets, end to end (lane t: length deg of target t,
@@ -1726,6 +1791,7 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
     s.whole = s.touched = 0;
     uint32_t v0;
     unsigned fm = 0;  // targets from v0 on to be done from their bitmaps
+    uint32_t oldf = 0, total = 0;  // lane t: target t's flag (1: the buffer row holds an older layer's bits) and new bits
     if (task < a.npieces) {  // part of one long list
       const uint4 pc = __ldg(a.pieces + task);
       const uint32_t np = pc.y == NONE ? 1u : a.heavy_np[pc.y];
@@ -1755,6 +1821,10 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
       }
       v0 = pc.x;
       fm = mine;
+      if (fm) {
+        oldf = a.flagN[v0];
+        total = new_bits<1>(a, wb, 1u, v0);
+      }
     } else {
       v0 = (task - a.npieces) * T;
       const uint32_t v = v0 + lane;
@@ -1807,7 +1877,7 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
         short_edges<MODE, SLOTS, T>(a, s, l ? a.in.adj[1] : a.in.adj[0], beg, deg, gaps);
       }
       __syncwarp();
-      const uint32_t oldf = valid ? a.flagN[v] : 0u;  // 1: the buffer row holds an older layer's bits
+      if (valid) oldf = a.flagN[v];
       bool clean = valid && oldf == 1;                // ... and nothing will be written there
       if (MODE == SH_LAST) {
         const unsigned vm = __ballot_sync(FULL, valid);
@@ -1887,11 +1957,14 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
         z &= z - 1;
         for (uint32_t q = lane; q < Q; q += 32) a.N[(size_t)(v0 + t) * Q + q] = make_uint4(0, 0, 0, 0);
       }
+      if (MODE != SH_LAST && fm) total = new_bits<T>(a, wb, fm, v0);
     }
+    __syncwarp();
     while (fm) {
       const uint32_t t = __ffs(fm) - 1;
       fm &= fm - 1;
-      const uint32_t c = finish_row(a, wb, t, v0 + t);
+      const uint32_t c = __shfl_sync(FULL, total, t);
+      finish_row(a, wb, t, v0 + t, c, __shfl_sync(FULL, oldf, t));
       if (lane == 0 && c) {
         nb += c;
         nv++;
@@ -1962,27 +2035,31 @@ __device__ __forceinline__ void materialize(uint32_t *__restrict__ flagF, uint4 
   const HopCtr &p = ctr->hop[h - 1], &c = ctr->hop[h];
   if (!prev_virt || p.strategy != ST_PULL || (p.short_rows & 0xFFFFFFFFull) == 0) return;
   if (c.strategy == 0 || (c.strategy == ST_PULL && c.short_pull)) return;
-  const int lane = threadIdx.x & 31;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; base < V; base += warps * 32) {
     const uint32_t v = base + lane;
-    unsigned m = __ballot_sync(FULL, v < V && flagF[v] == 2);
+    const bool two = v < V && flagF[v] == 2;
+    unsigned m = __ballot_sync(FULL, two);
+    if (two) flagF[v] = 1;
     while (m) {
-      const int b = __ffs(m) - 1;
-      m &= m - 1;
-      const uint32_t r = base + b;
-      const uint16_t *slot = slots + (size_t)r * slot_n;
-      const uint32_t cnt = slot[0];
-      for (uint32_t q0 = 0; q0 < Q; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        uint32_t w[4] = {0, 0, 0, 0};
-        for (uint32_t i = 1; i <= cnt; i++) {
-          const uint32_t id = slot[i];
-          if (id >> 7 == q) w[(id >> 5) & 3] |= 1u << (id & 31);
-        }
-        if (q < Q) F[(size_t)r * Q + q] = make_uint4(w[0], w[1], w[2], w[3]);
+      // an id per lane into the row, which is zero, four rows' slots in flight at once
+      uint32_t r[4], e[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        r[k] = m ? base + __ffs(m) - 1 : NONE;
+        m &= m - 1;
+        e[k] = r[k] != NONE && lane < slot_n ? slots[(size_t)r[k] * slot_n + lane] : 0u;
       }
-      if (lane == 0) flagF[r] = 1;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t cnt = __shfl_sync(FULL, e[k], 0);  // 0 past the last row
+        uint32_t *row = reinterpret_cast<uint32_t *>(F + (size_t)r[k] * Q);
+        if (lane && lane <= cnt) atomicOr(row + (e[k] >> 5), 1u << (e[k] & 31));
+        if (lane + 32 <= cnt) {
+          const uint32_t id = slots[(size_t)r[k] * slot_n + lane + 32];
+          atomicOr(row + (id >> 5), 1u << (id & 31));
+        }
+      }
     }
   }
 }
@@ -2982,6 +3059,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
   const bool stats = pl->collect_stats || pl->log_features || (pl->picker && p.use_picker);
   for (uint32_t h = 1; h <= p.k_max; h++) {
     const int fb = (h - 1) & 1, nbuf = h & 1;
+    const bool acc_on = pl->use_acc && h >= p.k_min && h <= p.k_max;
     DecideArgs da;
     da.ctr = pl->ctr;
     da.h = h;
@@ -3034,7 +3112,6 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     prep.virt = pl->slot[0] && leave_in_slots(h - 1);
     prep.clear = h > 1;  // hop 1 writes a buffer the run start cleared
     if (h > 1 || pl->slot[0]) vs::launch_next(k_hop_prep, pl->grid_v, 256, 0, st, prep);
-    const bool acc_on = pl->use_acc && h >= p.k_min && h <= p.k_max;
     SparseArgs sp;
     sp.ctr = pl->ctr;
     sp.h = h;
