@@ -346,14 +346,16 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
   }
   if (t == 0) {
     cur.strategy = s_choice;
-    // short mode where the hop costs less, in ps measured on GB300 over 1M- and
-    // 4M-vertex power-law and R-MAT graphs with 512 to 8,192 sources: a dense hop
-    // pays 7 to 18 per edge for neighbour and flag (with the row's lanes) and 0.8
-    // per word of every active row from L2; short mode 12.5 per edge, 21 per id read
-    // from words (10 on a last hop, which keeps no lists), 1.5 per id read from
-    // slots (with 6 more per edge where slots are wider than 32 bytes: 8,192 sources on
-    // the 10M-vertex power law, hop 3 9.96 ms from slots and 7.28 from words) and 350 per target row then searched for bits (none on a last hop),
-    // and about twice the dense price for a row too long for a slot.
+    // short mode where the hop costs less, in ps fitted on GB300 to 1,920 hops of 2,048
+    // to 30,000 sources over power-law, uniform and R-MAT graphs of 100K to 10M vertices,
+    // each hop timed dense, from words and from slots (the rule's choices take 1% longer
+    // than the best of the three; with prices taken at 1M vertices and more they took up
+    // to 2.1 times as long at 200K to 1M).  A dense hop pays 11 to 24 per list entry for
+    // neighbour and flag (with the row's lanes) and 0.88 per word of every active row;
+    // short mode 12.5 per entry, 19 per id read from words (3 on a last hop, which keeps no
+    // lists; 33 where every target is searched for its bits), 1.1 per id read from slots
+    // of 32 bytes (wider ones 0.75, and 14 per entry) and 3.1 per word of the target rows
+    // then searched (none on a last hop), and 0.9 per word of a row too long for a slot.
     bool sp = false, slots = false, lng = false;
     if (s_choice == ST_PULL && a.short_min > 0 && !c->multislice) {
       const bool counted = prev.strategy == ST_PULL;  // ... its layer's words, slots and degrees
@@ -367,18 +369,19 @@ __global__ void __launch_bounds__(256) k_decide(DecideArgs a) {
       } else {
         rows = ids * (act / fmaxf(1.f, (float)prev.new_bits));
       }
-      const float t_long = 1.6f * W * longs;
-      const float t_words = 12.5f * E + (a.last ? 10.f : 21.f) * ids + t_long;
-      const float t_slots = (a.W <= 64 ? 12.5f : 18.5f) * E + 1.5f * fminf(ids, 15.f * so) + (a.last ? 0.f : 350.f * fminf(V, ids)) + t_long;
+      const float t_long = 0.9f * W * longs, held = a.W <= 64 ? 15.f : a.W <= 128 ? 31.f : 63.f;  // ids a slot holds
+      const float t_words = 12.5f * E + (a.last ? 3.f : a.gen ? 33.f : 19.f) * ids + t_long;
+      const float t_slots = (a.W <= 64 ? 12.5f : 14.f) * E + (a.W <= 64 ? 1.1f : 0.75f) * fminf(ids, held * so) +
+                            (a.last ? 0.f : 3.1f * V * W) + t_long;
       slots = counted && t_slots < t_words;
       if (a.short_min > 1.0) {
         sp = true;
-      } else if (!counted || (float)(prev.short_rows & 0xFFFFFFFFull) >= (float)a.short_min * act) {
-        const float flag = act >= 0.9f * V ? 6.f : a.W <= 8 ? 7.f : a.W <= 16 ? 8.f : a.W <= 32 ? 12.f : 18.f;
-        sp = (slots ? t_slots : t_words) < 0.9f * (flag * E + 0.8f * W * rows);
+      } else if (!counted || (double)(prev.short_rows & 0xFFFFFFFFull) >= a.short_min * (double)prev.active_vertices) {
+        const float flag = act >= 0.9f * V ? 11.f : a.W <= 32 ? 16.f : 24.f;
+        sp = (slots ? t_slots : t_words) < 0.8f * (flag * E + 0.88f * W * rows);
       }
       // more than half a slot of ids per target: its new row will often be long
-      lng = ids > 1.2f * V * (a.W <= 64 ? 16 : a.W <= 128 ? 32 : 64);
+      lng = ids > 1.2f * V * (held + 1.f);
     }
     cur.short_pull = sp;
     // row flags as bits where they save loads: below 9 in 10 active vertices for rows of
@@ -3080,6 +3083,7 @@ int vs_expand_plan_run(vs_expand_plan *pl, const uint32_t *sources, const uint32
     da.rowk = pl->use_hmask ? pl->rowk : nullptr;
     da.short_min = pl->short_min;
     da.last = h == p.k_max && pl->use_vis && !pl->use_acc && p.path_type != VS_PATH_FIND_SHORTEST && !pl->layer_out[h];
+    da.gen = !da.last && (acc_on || !leave_in_slots(h));
     da.W = W;
     da.k_min = p.k_min;
     da.k_max = p.k_max;

@@ -78,6 +78,7 @@ struct DecideArgs {
   const void *picker;  // bf16 weights of a vs_picker (NULL = fixed planner)
   const uint32_t *rowk;  // [0] largest row hop limit (NULL: no row limits)
   int last;              // nothing reads layer h and the result is the visited matrix
+  int gen;               // a short-mode hop over words searches every touched target for its bits
   double short_min;      // short-mode PULL needs at least this share of the frontier's rows short (0: off; > 1: always)
 };
 
