@@ -32,14 +32,30 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned long long EMPTY = HT_EMPTY;
 using Table = HashTable;
 
-// An array indexed by vertex-id keys (below, at k_key_max).
+// Rows per vertex-id key, in an array indexed by the key (below, at k_key_max).
 struct Direct {
-  uint32_t *cnt;   // rows per key; with k_direct_rows one plus the key's row
+  uint32_t *cnt;
   uint32_t bound;  // entries of the array
-  uint32_t *ctl;   // [0] largest build key, [1] some key has several rows
+  uint32_t *top;   // largest build key
 };
 
-__device__ __forceinline__ bool direct_ok(const Direct &d) { return d.ctl[0] < d.bound; }
+__device__ __forceinline__ bool direct_ok(const Direct &d) { return *d.top < d.bound; }
+
+// The build side of a join that lists rows (below, at k_join_clear).
+struct Build {
+  Table t;               // keys (hash), rows per slot; off: first of the slot's rows, within its tile of 1,024 slots
+  unsigned long long *tile_off;  // ... and the tile's
+  uint32_t *row;         // by key: one plus a row that holds it
+  uint32_t bound;        // keys the array has room for (0: none)
+  uint32_t *ctl;         // [0] largest key, [1] some key has several rows, [2] [3] blocks of the scans that are done
+  uint64_t n;            // rows
+};
+enum { J_HASH, J_ROWS, J_UNIQUE };
+
+__device__ __forceinline__ int join_mode(const Build &b) {
+  if (!b.bound || b.ctl[0] >= b.bound) return J_HASH;
+  return b.ctl[1] ? J_ROWS : J_UNIQUE;
+}
 
 __device__ __forceinline__ unsigned long long load_key(const void *col, int type, uint64_t i) {
   return type == VS_T_I64 ? (unsigned long long)((const long long *)col)[i]
@@ -48,9 +64,11 @@ __device__ __forceinline__ unsigned long long load_key(const void *col, int type
 
 // Build: count rows per key.  Lanes holding the same key elect one leader
 // that adds the group's size (skewed keys cost one atomic per warp).
-__global__ void k_build(Table t, const void *keycol, int ktype, uint64_t n, uint32_t *slot_of) {
+template <class Slot>
+__device__ __forceinline__ void build_rows(const Table &t, const void *keycol, int ktype, uint64_t lo, uint64_t n,
+                                           uint32_t *slot_of, Slot find) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
+  for (uint64_t i0 = lo + (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
     const uint64_t i = i0 + threadIdx.x;
     const bool valid = i < n;
     const unsigned long long k = valid ? load_key(keycol, ktype, i) : EMPTY - 1;
@@ -60,13 +78,17 @@ __global__ void k_build(Table t, const void *keycol, int ktype, uint64_t n, uint
       const int leader = __ffs(peers) - 1;
       uint64_t slot = 0;
       if ((int)(threadIdx.x & 31) == leader) {
-        slot = ht_insert(t, k);
+        slot = find(k, i);
         atomicAdd(&t.cnt[slot], (unsigned long long)__popc(peers));
       }
       slot = __shfl_sync(peers, slot, leader);
       if (slot_of) slot_of[i] = (uint32_t)slot;
     }
   }
+}
+
+__global__ void k_build(Table t, const void *keycol, int ktype, uint64_t n) {
+  build_rows(t, keycol, ktype, 0, n, nullptr, [&](unsigned long long k, uint64_t) { return ht_insert(t, k); });
 }
 
 // Count-only build: each block first counts its rows' keys in a table of
@@ -120,8 +142,8 @@ __global__ void __launch_bounds__(256) k_build_count(Table t, const void *keycol
 
 // ---------------------------------------------------------------------------
 // Vertex-id keys below a bound of a few times the build rows need no hash: an
-// array indexed by the key holds each key's count (and build row), in L2 where the
-// hash table of 10M keys is 537 MB of HBM.  The largest build key is found on the
+// array indexed by the key holds each key's count, in L2 where the hash table of 10M
+// keys is 537 MB of HBM.  The largest build key is found on the
 // device and every kernel checks it against the bound, so the host waits for
 // nothing; above the bound the count's kernels use the hash table instead.  Count of
 // 10M x 10M Zipf-skewed keys below 10M: 432 -> 117 us, of which counting the build
@@ -139,14 +161,14 @@ __global__ void __launch_bounds__(256) k_key_max(const uint32_t *__restrict__ ke
   if ((threadIdx.x & 31) == 0) atomicMax(ctl, m);
 }
 
-// Clears the part of the arrays that the keys use, or the hash table that takes
-// their place (when there is one).
+// Clears the part of the array that the keys use, or the hash table that takes its
+// place.
 __global__ void __launch_bounds__(256) k_direct_clear(Direct d, Table t) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (direct_ok(d)) {
-    const uint32_t n4 = d.ctl[0] / 4 + 1;  // the bound is a multiple of four
+    const uint32_t n4 = *d.top / 4 + 1;  // the bound is a multiple of four
     for (uint64_t i = i0; i < n4; i += stride) reinterpret_cast<uint4 *>(d.cnt)[i] = make_uint4(0, 0, 0, 0);
-  } else if (t.keys) {
+  } else {
     for (uint64_t i = i0; i <= t.cap; i += stride) {
       t.keys[i] = EMPTY;
       t.cnt[i] = 0;
@@ -198,7 +220,7 @@ __global__ void __launch_bounds__(512) k_direct_count(Direct d, Table t, const u
 // Sum of the counts of the probe keys.
 __global__ void __launch_bounds__(256) k_direct_probe(Direct d, Table t, const uint32_t *__restrict__ keys,
                                                       uint64_t n, unsigned long long *total) {
-  const uint32_t top = d.ctl[0];
+  const uint32_t top = *d.top;
   unsigned long long s = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (!direct_ok(d)) {
@@ -223,32 +245,200 @@ __global__ void __launch_bounds__(256) k_direct_probe(Direct d, Table t, const u
   block_add(s, total);
 }
 
-// Materialising joins whose build keys are unique (a property table): one plus the
-// key's row in place of its count.
-__global__ void __launch_bounds__(256) k_direct_rows(Direct d, const uint32_t *__restrict__ keys, uint64_t n) {
-  if (!direct_ok(d)) return;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    if (__ldcg(d.ctl + 1)) return;  // a repeated key: the general join will run
-    const uint32_t k = __ldg(keys + i);
-    if (atomicExch(&d.cnt[k], (uint32_t)i + 1) != 0) d.ctl[1] = 1;
+// Joins that list rows.  Vertex-id keys below a bound get their slot from an array
+// indexed by the key that holds (one plus) a row with it: the row itself where every key
+// has one (a property table: UNIQUE), else the row's number is the key's slot (ROWS);
+// other keys get it from the hash table.  Which of the three it is the device finds on
+// the way, and kernels that the mode has no use for return at once, so that the host
+// waits once, for the number of rows: told first whether the keys are unique, a join
+// of repeated keys waited some 40 us longer.  4M probe rows against 1M rows of five
+// columns in all: unique keys 376 (hash table) -> 173 us, repeated ones 417 -> 400; 4,000
+// against 1,000 rows of repeated keys 125 -> 98.
+__global__ void __launch_bounds__(256) k_join_clear(Build b) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (join_mode(b) == J_HASH) {
+    for (uint64_t i = i0; i <= b.t.cap; i += stride) {
+      b.t.keys[i] = EMPTY;
+      b.t.cnt[i] = 0;
+    }
+  } else {
+    const uint32_t n4 = b.ctl[0] / 4 + 1;  // the bound is a multiple of four
+    for (uint64_t i = i0; i < n4; i += stride) reinterpret_cast<uint4 *>(b.row)[i] = make_uint4(0, 0, 0, 0);
+    for (uint64_t i = i0; i < b.n; i += stride) b.t.cnt[i] = 0;
   }
 }
 
-// Matching probe rows per tile of FK_ROWS (sums[tile]) and in all.
+// Build rows [i_lo, i_hi) into the array, until a key is met again, or into the hash
+// table.  The first rows come alone, with few blocks: in most tables with repeated keys one
+// is met among them, and the atomics and stores of a full grid that meets one at the same
+// time took 134 us for 1M rows.
+__global__ void __launch_bounds__(256) k_join_build(Build b, const void *keycol, int ktype, uint32_t *slot_of, uint64_t i_lo,
+                                                    uint64_t i_hi) {
+  if (!b.bound || b.ctl[0] >= b.bound) {
+    build_rows(b.t, keycol, ktype, i_lo, i_hi, slot_of, [&](unsigned long long k, uint64_t) { return ht_insert(b.t, k); });
+    return;
+  }
+  const uint32_t *keys = (const uint32_t *)keycol;
+  const unsigned lane = threadIdx.x & 31;
+  for (uint64_t i0 = i_lo + (uint64_t)blockIdx.x * blockDim.x; i0 < i_hi; i0 += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = i0 + threadIdx.x;
+    const bool known = __shfl_sync(FULL, __ldcg(b.ctl + 1), 0);
+    if (known) return;
+    const uint32_t k = i < i_hi ? __ldg(keys + i) : 0u;
+    // a key twice in the warp needs no atomic (hot keys would queue at one address)
+    const unsigned peers = __match_any_sync(FULL, i < i_hi ? (unsigned long long)k : EMPTY - lane);
+    bool again = i < i_hi && (peers & lanemask_lt());
+    if (!__any_sync(FULL, again) && i < i_hi) again = atomicExch(&b.row[k], (uint32_t)i + 1) != 0;
+    if (__any_sync(FULL, again)) {
+      if (lane == 0 && !__ldcg(b.ctl + 1)) b.ctl[1] = 1;
+      return;
+    }
+  }
+}
+
+// Repeated keys: the array completed, and rows per slot.
+__global__ void __launch_bounds__(256) k_join_count(Build b, const uint32_t *__restrict__ keys, uint32_t *slot_of) {
+  if (join_mode(b) != J_ROWS) return;
+  build_rows(b.t, keys, VS_T_VID, 0, b.n, slot_of, [&](unsigned long long k, uint64_t i) {
+    uint32_t r = __ldcg(b.row + k);
+    if (!r) {
+      r = atomicCAS(&b.row[k], 0u, (uint32_t)i + 1);
+      if (!r) r = (uint32_t)i + 1;
+    }
+    return (uint64_t)(r - 1);
+  });
+}
+
+// Exclusive prefix in one launch: out within tiles of 1,024, and by the block that
+// finishes last the tiles' starts.  n_hash elements in HASH mode, n_rows in ROWS mode;
+// element n gets the total.
+__global__ void __launch_bounds__(256) k_join_scan(Build b, const unsigned long long *__restrict__ in,
+                                                   unsigned long long *__restrict__ out, unsigned long long *tile_off,
+                                                   uint64_t n_hash, uint64_t n_rows, uint32_t *done) {
+  const int mode = join_mode(b);
+  if (mode == J_UNIQUE) return;
+  const uint64_t n = mode == J_HASH ? n_hash : n_rows, tiles = n / 1024 + 1;  // element n has a tile too
+  if (blockIdx.x >= tiles) return;
+  __shared__ unsigned long long wt[8];
+  __shared__ bool s_last;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  unsigned long long v[4] = {0, 0, 0, 0};
+  auto scan4 = [&]() {  // v becomes the exclusive prefix over the block's 1,024 values; returns their sum
+    const unsigned long long run = v[0] + v[1] + v[2] + v[3];
+    unsigned long long incl = run;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) wt[w] = incl;
+    __syncthreads();
+    unsigned long long pre = 0, sum = 0;
+    for (int k = 0; k < 8; k++) {
+      if (k < w) pre += wt[k];
+      sum += wt[k];
+    }
+    pre += incl - run;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned long long x = v[k];
+      v[k] = pre;
+      pre += x;
+    }
+    __syncthreads();
+    return sum;
+  };
+  for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint64_t base = tile * 1024 + (uint64_t)t * 4;
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = base + k < n ? in[base + k] : 0ull;
+    const unsigned long long sum = scan4();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (base + k <= n) out[base + k] = v[k];
+    if (t == 0) tile_off[tile] = sum;
+  }
+  __threadfence();
+  __syncthreads();
+  const uint64_t blocks = tiles < gridDim.x ? tiles : gridDim.x;
+  if (t == 0) s_last = atomicAdd(done, 1u) == blocks - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  unsigned long long carry = 0;
+  for (uint64_t b0 = 0; b0 < tiles; b0 += 1024) {
+    const uint64_t base = b0 + (uint64_t)t * 4;
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = base + k < tiles ? __ldcg(tile_off + base + k) : 0ull;
+    const unsigned long long sum = scan4();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (base + k < tiles) tile_off[base + k] = carry + v[k];
+    carry += sum;
+  }
+}
+
+__device__ __forceinline__ unsigned long long start_of(const unsigned long long *__restrict__ off,
+                                                       const unsigned long long *__restrict__ tile_off, uint64_t i) {
+  return off[i] + tile_off[i >> 10];
+}
+
+// Build rows by slot (the counts go down to zero); one lane takes the places of a
+// warp's rows of one slot (300K rows, 38% of one key: 106 -> 32 us).
+__global__ void __launch_bounds__(256) k_join_scatter(Build b, const uint32_t *__restrict__ slot_of,
+                                                      uint32_t *__restrict__ rows_by_key) {
+  if (join_mode(b) == J_UNIQUE) return;
+  const unsigned lane = threadIdx.x & 31;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < b.n; i0 += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = i0 + threadIdx.x;
+    const uint32_t s = i < b.n ? slot_of[i] : 0u;
+    const unsigned peers = __match_any_sync(FULL, i < b.n ? (unsigned long long)s : EMPTY - lane);
+    const int leader = __ffs(peers) - 1;
+    unsigned long long at = 0;
+    if (i < b.n && (int)lane == leader)
+      at = start_of(b.t.off, b.tile_off, s) + atomicAdd(&b.t.cnt[s], 0ull - __popc(peers)) - __popc(peers);
+    at = __shfl_sync(FULL, at, leader);
+    if (i < b.n) rows_by_key[at + __popc(peers & lanemask_lt())] = (uint32_t)i;
+  }
+}
+
+// Probe.  UNIQUE: matching rows per tile of FK_ROWS (sums[tile]); else matches per row
+// and the row's slot.  All of them in *total.
 constexpr int FK_ROWS = 1024;
-__global__ void __launch_bounds__(256) k_fk_count(Direct d, const uint32_t *__restrict__ keys, uint64_t n,
-                                                  unsigned long long *__restrict__ sums, unsigned long long *total) {
-  if (!direct_ok(d) || d.ctl[1]) return;
-  const uint32_t top = d.ctl[0];
-  __shared__ uint32_t part[8];
+__global__ void __launch_bounds__(256) k_join_probe(Build b, const void *keycol, int ktype, uint64_t n,
+                                                    unsigned long long *__restrict__ sums,
+                                                    unsigned long long *__restrict__ pcnt, uint32_t *__restrict__ pslot,
+                                                    unsigned long long *total, int unique_only) {
+  const int mode = join_mode(b);
+  if (unique_only && mode != J_UNIQUE) return;
+  const uint32_t *keys = (const uint32_t *)keycol;
+  const uint32_t top = b.ctl[0];
   unsigned long long all = 0;
-  for (uint64_t b = blockIdx.x; b * FK_ROWS < n; b += gridDim.x) {
+  if (mode != J_UNIQUE) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+      uint64_t slot;
+      if (mode == J_HASH) {
+        slot = ht_find(b.t, load_key(keycol, ktype, i));
+      } else {
+        const uint32_t k = __ldg(keys + i);
+        slot = k <= top ? (uint64_t)__ldg(b.row + k) - 1 : ~0ull;  // 0: no row
+      }
+      unsigned long long c = 0;
+      if (slot != ~0ull) c = start_of(b.t.off, b.tile_off, slot + 1) - start_of(b.t.off, b.tile_off, slot);
+      all += c;
+      pcnt[i] = c;
+      pslot[i] = (uint32_t)(slot == ~0ull ? 0 : slot);
+    }
+    block_add(all, total);
+    return;
+  }
+  __shared__ uint32_t part[8];
+  for (uint64_t tile = blockIdx.x; tile * FK_ROWS < n; tile += gridDim.x) {
     uint32_t c = 0;
 #pragma unroll
     for (int k = 0; k < FK_ROWS / 256; k++) {
-      const uint64_t i = b * FK_ROWS + k * 256 + threadIdx.x;
+      const uint64_t i = tile * FK_ROWS + k * 256 + threadIdx.x;
       const uint32_t x = i < n ? __ldg(keys + i) : 0xffffffffu;
-      c += x <= top && __ldg(d.cnt + x);
+      c += x <= top && __ldg(b.row + x);
     }
     c = __reduce_add_sync(FULL, c);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
@@ -256,7 +446,7 @@ __global__ void __launch_bounds__(256) k_fk_count(Direct d, const uint32_t *__re
     if (threadIdx.x == 0) {
       uint32_t t = 0;
       for (int w = 0; w < 8; w++) t += part[w];
-      sums[b] = t;
+      sums[tile] = t;
       all += t;
     }
     __syncthreads();
@@ -274,27 +464,13 @@ __global__ void k_build_cols(Table t, const uint32_t *col_map, uint32_t cols) {
   }
 }
 
-__global__ void k_scatter(Table t, const uint32_t *slot_of, uint64_t n, uint32_t *rows_by_key) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t s = slot_of[i];
-    rows_by_key[t.off[s] + atomicAdd(&t.cur[s], 1ull)] = (uint32_t)i;
-  }
-}
-
-// Probe: matches per probe row (and the slot), total into *total.
-__global__ void k_probe(Table t, const void *keycol, int ktype, uint64_t n,
-                        unsigned long long *pcnt, uint32_t *pslot, unsigned long long *total) {
+// Probe: sum of the counts of the probe keys.
+__global__ void k_probe(Table t, const void *keycol, int ktype, uint64_t n, unsigned long long *total) {
   unsigned long long s = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t slot = ht_find(t, load_key(keycol, ktype, i));
-    const unsigned long long c = slot == ~0ull ? 0ull : t.cnt[slot];
-    s += c;
-    if (pcnt) {
-      pcnt[i] = c;
-      pslot[i] = (uint32_t)(slot == ~0ull ? 0 : slot);
-    }
+    if (slot != ~0ull) s += t.cnt[slot];
   }
   block_add(s, total);
 }
@@ -394,48 +570,53 @@ struct OutCol {
 struct EmitArgs {
   OutCol col[16];
   int ncols;
-  const unsigned long long *poff;  // n_probe + 1
+  const unsigned long long *poff, *ptile;  // first output row of every probe row, within its tile and the tile's
   const uint32_t *pslot;
   const uint32_t *rows_by_key;
-  Table t;
+  Build b;
   uint64_t n_probe, out_rows;
 };
 
 // Output rows [blk*R, blk*R + R) of every block; thread -> probe row by a
-// binary search of poff inside the block's probe range.
+// binary search of the rows' starts inside the block's probe range.
 constexpr int EMIT_ROWS = 2048;
 
 __global__ void __launch_bounds__(256) k_emit(EmitArgs a) {
   __shared__ uint64_t p_lo, p_hi;
+  __shared__ unsigned long long s_start[EMIT_ROWS];
   const uint64_t o0 = (uint64_t)blockIdx.x * EMIT_ROWS;
   if (o0 >= a.out_rows) return;
   const uint64_t o1 = min(o0 + EMIT_ROWS, a.out_rows);
   if (threadIdx.x == 0) {
-    // largest p with poff[p] <= o0, and with poff[p] <= o1 - 1
+    // largest p that starts at or before o0, and at or before o1 - 1
     uint64_t lo = 0, hi = a.n_probe;
     while (hi - lo > 1) {
       uint64_t mid = (lo + hi) / 2;
-      if (a.poff[mid] <= o0) lo = mid; else hi = mid;
+      if (start_of(a.poff, a.ptile, mid) <= o0) lo = mid; else hi = mid;
     }
     p_lo = lo;
     uint64_t lo2 = lo, hi2 = a.n_probe;
     while (hi2 - lo2 > 1) {
       uint64_t mid = (lo2 + hi2) / 2;
-      if (a.poff[mid] <= o1 - 1) lo2 = mid; else hi2 = mid;
+      if (start_of(a.poff, a.ptile, mid) <= o1 - 1) lo2 = mid; else hi2 = mid;
     }
     p_hi = lo2;
   }
+  __syncthreads();
+  const bool held = p_hi - p_lo < EMIT_ROWS;  // the range's starts fit
+  if (held)
+    for (uint64_t p = p_lo + threadIdx.x; p <= p_hi; p += blockDim.x) s_start[p - p_lo] = start_of(a.poff, a.ptile, p);
   __syncthreads();
   for (uint64_t o = o0 + threadIdx.x; o < o1; o += blockDim.x) {
     uint64_t lo = p_lo, hi = p_hi + 1;
     while (hi - lo > 1) {
       uint64_t mid = (lo + hi) / 2;
-      if (a.poff[mid] <= o) lo = mid; else hi = mid;
+      if ((held ? s_start[mid - p_lo] : start_of(a.poff, a.ptile, mid)) <= o) lo = mid; else hi = mid;
     }
     const uint64_t p = lo;
-    const uint64_t j = o - a.poff[p];
+    const uint64_t j = o - (held ? s_start[p - p_lo] : start_of(a.poff, a.ptile, p));
     const uint32_t s = a.pslot[p];
-    const uint64_t b = a.rows_by_key[a.t.off[s] + j];
+    const uint64_t b = a.rows_by_key[start_of(a.b.t.off, a.b.tile_off, s) + j];
     for (int c = 0; c < a.ncols; c++) {
       const OutCol &oc = a.col[c];
       const uint64_t r = oc.side ? b : p;
@@ -452,9 +633,9 @@ __global__ void __launch_bounds__(256) k_emit(EmitArgs a) {
 // matches and no per-row counts, offsets or slots go through memory.  Bound by random
 // sectors, one for the row and one per build column: the row sits in the key's word
 // itself (a count and a row array: 54 -> 44 us for 4M rows of 20 bytes).
-__global__ void __launch_bounds__(256) k_fk_emit(EmitArgs a, Direct d, const uint32_t *__restrict__ keys,
+__global__ void __launch_bounds__(256) k_fk_emit(EmitArgs a, const uint32_t *__restrict__ keys,
                                                  const unsigned long long *__restrict__ tile_off) {
-  const uint32_t top = d.ctl[0];
+  const uint32_t top = a.b.ctl[0];
   __shared__ uint32_t part[FK_ROWS / 32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint64_t b = blockIdx.x; b * FK_ROWS < a.n_probe; b += gridDim.x) {
@@ -468,7 +649,7 @@ __global__ void __launch_bounds__(256) k_fk_emit(EmitArgs a, Direct d, const uin
       row[k] = i < a.n_probe ? __ldg(keys + i) : 0xffffffffu;
     }
 #pragma unroll
-    for (int k = 0; k < FK_ROWS / 256; k++) row[k] = row[k] <= top ? __ldg(d.cnt + row[k]) : 0u;  // one plus the row
+    for (int k = 0; k < FK_ROWS / 256; k++) row[k] = row[k] <= top ? __ldg(a.b.row + row[k]) : 0u;  // one plus the row
 #pragma unroll
     for (int k = 0; k < FK_ROWS / 256; k++) {
       hit[k] = __ballot_sync(FULL, row[k] != 0);
@@ -503,41 +684,57 @@ __global__ void __launch_bounds__(256) k_fk_emit(EmitArgs a, Direct d, const uin
   }
 }
 
+// One allocation for the arrays of a call: an allocation and its release cost the host
+// about 1.5 us, a small join has ten.
 struct Scratch {
   cudaStream_t st;
-  void *p[16] = {};
-  int n = 0;
-  template <typename T> int get(T **out, size_t count) {
-    int rc = dalloc_n(out, count, st);
-    if (rc == VS_OK) p[n++] = *out;
-    return rc;
+  char *base = nullptr;
+  size_t bytes = 0;
+  explicit Scratch(cudaStream_t s) : st(s) {}
+  template <typename T> size_t add(size_t n) {  // offset of n elements
+    const size_t at = bytes;
+    bytes += (sizeof(T) * (n ? n : 1) + 255) / 256 * 256;
+    return at;
   }
-  ~Scratch() {
-    for (int i = 0; i < n; i++) dfree(p[i], st);
+  int alloc() { return dalloc_n(&base, bytes, st); }
+  template <typename T> T *at(size_t off) const { return reinterpret_cast<T *>(base + off); }
+  void release() {  // the layout stays
+    dfree(base, st);
+    base = nullptr;
   }
+  ~Scratch() { release(); }
 };
 
-int table_alloc(Scratch &sc, uint64_t n_keys, bool with_val, bool with_off, Table *t, bool clear = true) {
-  t->cap = ht_capacity(std::max<uint64_t>(n_keys, 1));
-  VS_TRY(sc.get(&t->keys, t->cap + 1));
-  VS_TRY(sc.get(&t->cnt, t->cap + 1));
-  if (clear) {
-    VS_CK(cudaMemsetAsync(t->keys, 0xff, 8 * (t->cap + 1), sc.st));
-    VS_CK(cudaMemsetAsync(t->cnt, 0, 8 * (t->cap + 1), sc.st));
+// A hash table's arrays within a scratch, and `extra` elements of 8 bytes zeroed with its
+// counters.
+struct TablePart {
+  size_t keys = 0, cnt = 0, zeroed = 0, end = 0, val = 0;
+  bool with_val = false;
+  uint64_t cap = 0;
+  void add(Scratch &sc, uint64_t n_keys, bool val_, size_t extra) {
+    cap = ht_capacity(std::max<uint64_t>(n_keys, 1));
+    with_val = val_;
+    keys = sc.add<uint64_t>(cap + 1);
+    cnt = sc.add<uint64_t>(cap + 1);
+    zeroed = extra ? sc.add<uint64_t>(extra) : sc.bytes;
+    end = sc.bytes;
+    val = val_ ? sc.add<uint32_t>(cap + 1) : 0;
   }
-  t->val = nullptr;
-  t->off = t->cur = nullptr;
-  if (with_val) {
-    VS_TRY(sc.get(&t->val, t->cap + 1));
-    VS_CK(cudaMemsetAsync(t->val, 0xff, 4 * (t->cap + 1), sc.st));
+  Table table(const Scratch &sc) const {
+    Table t{};
+    t.cap = cap;
+    t.keys = sc.at<unsigned long long>(keys);
+    t.cnt = sc.at<unsigned long long>(cnt);
+    if (with_val) t.val = sc.at<uint32_t>(val);
+    return t;
   }
-  if (with_off) {
-    VS_TRY(sc.get(&t->off, t->cap + 2));
-    VS_TRY(sc.get(&t->cur, t->cap + 1));
-    VS_CK(cudaMemsetAsync(t->cur, 0, 8 * (t->cap + 1), sc.st));
+  int clear(const Scratch &sc) const {
+    VS_CK(cudaMemsetAsync(sc.base + keys, 0xff, 8 * (cap + 1), sc.st));
+    VS_CK(cudaMemsetAsync(sc.base + cnt, 0, end - cnt, sc.st));
+    if (with_val) VS_CK(cudaMemsetAsync(sc.base + val, 0xff, 4 * (cap + 1), sc.st));
+    return VS_OK;
   }
-  return VS_OK;
-}
+};
 
 int grid_for(uint64_t n, int per_block = 256) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + per_block - 1) / per_block,
@@ -558,26 +755,13 @@ struct FlatSide {
   uint32_t key;
 };
 
-// Key bound up to which the direct arrays are used.  They take 4 bytes an entry
-// (8 with rows) where a hash table takes 32 to 64 a row, so up to four entries a
-// row they are the smaller of the two; below 4M entries (16 MB, cleared in 5 us, in
-// L2) they win whatever the rows.
-uint32_t direct_bound(uint64_t n_build) {
-  return n_build > (1ull << 28) ? 0u : (uint32_t)std::max<uint64_t>(1u << 22, (4 * n_build + 3) / 4 * 4);
-}
-
-// The direct arrays of the build keys, and a total before their control words (one
-// 16-byte block, read back at once).  VS_ERR_OOM leaves nothing behind.
-int direct_alloc(Scratch &sc, const uint32_t *keys, uint64_t n, uint32_t bound, const Table &t, Direct *d,
-                 unsigned long long **total) {
-  d->bound = bound;
-  VS_TRY(sc.get(total, 2));
-  d->ctl = reinterpret_cast<uint32_t *>(*total + 1);
-  VS_TRY(sc.get(&d->cnt, bound));
-  VS_CK(cudaMemsetAsync(*total, 0, 16, sc.st));
-  { k_key_max<<<std::min(grid_for((n + 3) / 4), 4 * sm_count()), 256, 0, sc.st>>>(keys, n, d->ctl); vs::note_launch(); }
-  { k_direct_clear<<<std::min(grid_for((bound + 3) / 4), 8 * sm_count()), 256, 0, sc.st>>>(*d, t); vs::note_launch(); }
-  return VS_OK;
+// Key bound up to which an array indexed by the key is used: 4 bytes an entry where a
+// hash table takes 32 to 64 a row.  Below 4M entries (16 MB, cleared in 5 us, in L2) it
+// wins whatever the rows.  Above, counts take it up to 4 entries a row, joins that list
+// rows up to 12 (1M rows, keys below 12M: unique 366 -> 184 us, repeated 362 -> 361;
+// keys above, 40M: 6% slower than without asking for the largest key).
+uint32_t direct_bound(uint64_t n_build, uint64_t per_row) {
+  return n_build > (1ull << 27) ? 0u : (uint32_t)std::max<uint64_t>(1u << 22, per_row * n_build / 4 * 4);
 }
 
 // Result schema: a's columns, then b's non-key columns.
@@ -603,30 +787,138 @@ int join_columns(FlatSide a, FlatSide b, bool build_a, int32_t *types, EmitArgs 
   return VS_OK;
 }
 
-// The rows of a join whose build keys fit the direct arrays and are unique (a
-// property table): no slots, scatter or per-row offsets.  *done stays false when
-// they are not; the general join then runs.  4M probe rows x 1M build rows, five
-// columns: 376 -> 167 us.
-int join_unique(Scratch &sc, FlatSide a, FlatSide b, bool build_a, Direct d, const uint32_t *bkeys, uint64_t nb,
-                const uint32_t *pkeys, uint64_t np, unsigned long long *d_total, uint64_t max_rows, vs_flat **out,
-                uint64_t *count, bool *done) {
-  cudaStream_t st = sc.st;
-  const uint64_t tiles = (np + FK_ROWS - 1) / FK_ROWS;
-  unsigned long long *sums, *offs;
-  VS_TRY(sc.get(&sums, tiles));
-  VS_TRY(sc.get(&offs, tiles + 1));
-  const int grid = (int)std::min<uint64_t>(tiles, (uint64_t)sm_count() * 8);
-  { k_direct_rows<<<grid_for(nb), 256, 0, st>>>(d, bkeys, nb); vs::note_launch(); }
-  { k_fk_count<<<grid, 256, 0, st>>>(d, pkeys, np, sums, d_total); vs::note_launch(); }
+// Count of a flat join: of vertex-id keys through the array indexed by the key, or the
+// hash table in its place (chosen on the device), of others through the hash table.
+int count_flat_flat(FlatSide bd, FlatSide pr, uint64_t *count, cudaStream_t st) {
+  const uint64_t nb = bd.f->nrows, np = pr.f->nrows;
+  const uint32_t *bkeys = (const uint32_t *)bd.f->cols[bd.key], *pkeys = (const uint32_t *)pr.f->cols[pr.key];
+  const uint32_t bound = bd.f->types[bd.key] == VS_T_VID && nb && np ? direct_bound(nb, 4) : 0u;
+  Scratch sc{st};
+  TablePart tp;
+  if (bound) {
+    tp.add(sc, nb, false, 0);
+    const size_t o_ctl = sc.add<uint64_t>(2), o_cnt = sc.add<uint32_t>(bound);
+    const int rc = sc.alloc();
+    if (rc != VS_OK && rc != VS_ERR_OOM) return rc;
+    if (rc == VS_OK) {
+      const Table t = tp.table(sc);
+      unsigned long long *d_total = sc.at<unsigned long long>(o_ctl);
+      const Direct d{sc.at<uint32_t>(o_cnt), bound, reinterpret_cast<uint32_t *>(d_total + 1)};
+      VS_CK(cudaMemsetAsync(d_total, 0, 16, st));
+      { k_key_max<<<std::min(grid_for((nb + 3) / 4), 4 * sm_count()), 256, 0, st>>>(bkeys, nb, d.top); vs::note_launch(); }
+      { k_direct_clear<<<std::min(grid_for((bound + 3) / 4), 8 * sm_count()), 256, 0, st>>>(d, t); vs::note_launch(); }
+      { k_direct_count<<<std::min(grid_for(nb, 512), 2 * sm_count()), 512, 0, st>>>(d, t, bkeys, nb); vs::note_launch(); }
+      { k_direct_probe<<<grid_for(np), 256, 0, st>>>(d, t, pkeys, np, d_total); vs::note_launch(); }
+      VS_CK(cudaGetLastError());
+      return read_total(d_total, count, st);
+    }
+    sc.bytes = 0;  // no room for both
+  }
+  tp.add(sc, nb, false, 1);
+  VS_TRY(sc.alloc());
+  VS_TRY(tp.clear(sc));
+  const Table t = tp.table(sc);
+  unsigned long long *d_total = sc.at<unsigned long long>(tp.zeroed);
+  if (nb)
+    { k_build_count<<<std::min(grid_for(nb), 4 * sm_count()), 256, 0, st>>>(t, bkeys, bd.f->types[bd.key], nb); vs::note_launch(); }
+  if (np)
+    { k_probe<<<grid_for(np), 256, 0, st>>>(t, pkeys, pr.f->types[pr.key], np, d_total); vs::note_launch(); }
   VS_CK(cudaGetLastError());
+  return read_total(d_total, count, st);
+}
+
+// Build rows from which a join that lists rows asks whether the keys are unique before it
+// goes on (at `early`).
+constexpr uint64_t ASK_ROWS = 512 << 10;
+
+// Flat x Flat join.  a = deps[0], b = deps[1]; result = a cols + b non-key cols.
+int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, vs_flat **out,
+                   uint64_t *count, cudaStream_t st) {
+  if (a.f->types[a.key] != b.f->types[b.key])
+    return fail(VS_ERR_ARG, "join key types differ (%d vs %d)", a.f->types[a.key], b.f->types[b.key]);
+  // GPU build side: the smaller table (the reference builds on the larger,
+  // join.cpp:39-43; the side only changes the output order)
+  const bool build_a = a.f->nrows < b.f->nrows;
+  const FlatSide &bd = build_a ? a : b, &pr = build_a ? b : a;
+  if (only_count) return count_flat_flat(bd, pr, count, st);
+  const uint64_t nb = bd.f->nrows, np = pr.f->nrows;
+  const int ktype = bd.f->types[bd.key];
+  const void *bkeys = bd.f->cols[bd.key], *pkeys = pr.f->cols[pr.key];
+  Build d{};
+  d.n = nb;
+  d.bound = ktype == VS_T_VID && nb && np ? direct_bound(nb, 12) : 0u;
+  const uint64_t tiles = (np + FK_ROWS - 1) / FK_ROWS;
+  Scratch sc{st};
+  TablePart tp;
+  size_t o_ctl, o_off, o_toff, o_slot, o_rows, o_pcnt, o_poff, o_ptile, o_pslot, o_row;
+  for (;;) {
+    sc.bytes = 0;
+    tp.add(sc, nb, false, 0);
+    o_ctl = sc.add<uint64_t>(3);  // total, then the control words
+    o_off = sc.add<uint64_t>(tp.cap + 2);
+    o_toff = sc.add<uint64_t>((tp.cap + 1) / 1024 + 1);
+    o_slot = sc.add<uint32_t>(nb);
+    o_rows = sc.add<uint32_t>(nb);
+    o_pcnt = sc.add<uint64_t>(np);
+    o_poff = sc.add<uint64_t>(np + 1);
+    o_ptile = sc.add<uint64_t>(np / 1024 + 1);
+    o_pslot = sc.add<uint32_t>(np);
+    o_row = sc.add<uint32_t>(d.bound);
+    const int rc = sc.alloc();
+    if (rc == VS_OK) break;
+    if (rc != VS_ERR_OOM || !d.bound) return rc;
+    d.bound = 0;  // without the array
+  }
+  d.t = tp.table(sc);
+  d.t.off = sc.at<unsigned long long>(o_off);
+  d.tile_off = sc.at<unsigned long long>(o_toff);
+  d.row = sc.at<uint32_t>(o_row);
+  unsigned long long *d_total = sc.at<unsigned long long>(o_ctl), *pcnt = sc.at<unsigned long long>(o_pcnt),
+                     *poff = sc.at<unsigned long long>(o_poff), *ptile = sc.at<unsigned long long>(o_ptile);
+  d.ctl = reinterpret_cast<uint32_t *>(d_total + 1);
+  uint32_t *slot_of = sc.at<uint32_t>(o_slot), *rows_by_key = sc.at<uint32_t>(o_rows), *pslot = sc.at<uint32_t>(o_pslot);
+  unsigned long long *sums = pcnt, *offs = poff;  // UNIQUE: by tile
+  const int cap_grid = 8 * sm_count();
+  VS_CK(cudaMemsetAsync(d_total, 0, 24, st));
+  if (d.bound)
+    { k_key_max<<<std::min(grid_for((nb + 3) / 4), 4 * sm_count()), 256, 0, st>>>((const uint32_t *)bkeys, nb, d.ctl); vs::note_launch(); }
+  { k_join_clear<<<std::min(grid_for(std::max<uint64_t>(tp.cap + 1, d.bound / 4)), cap_grid), 256, 0, st>>>(d); vs::note_launch(); }
+  const uint64_t first = std::min<uint64_t>(nb, d.bound ? 512ull * sm_count() : nb);  // rows
+  if (first) { k_join_build<<<grid_for(first), 256, 0, st>>>(d, bkeys, ktype, slot_of, 0, first); vs::note_launch(); }
+  if (nb > first) { k_join_build<<<grid_for(nb - first), 256, 0, st>>>(d, bkeys, ktype, slot_of, first, nb); vs::note_launch(); }
   struct {
     unsigned long long total;
-    uint32_t top, dup;
-  } h;
-  VS_CK(cudaMemcpyAsync(&h, d_total, 16, cudaMemcpyDeviceToHost, st));
-  VS_CK(cudaStreamSynchronize(st));
-  if (h.top >= d.bound || h.dup) return VS_OK;
-  *done = true;
+    uint32_t top, repeated;
+  } h{};
+  auto probe = [&](int unique_only) {
+    if (np) {
+      k_join_probe<<<grid_for(np), 256, 0, st>>>(d, pkeys, ktype, np, sums, pcnt, pslot, d_total, unique_only);
+      vs::note_launch();
+    }
+  };
+  auto ask = [&]() {  // the rows' number, and the mode
+    VS_CK(cudaGetLastError());
+    VS_CK(cudaMemcpyAsync(&h, d_total, 16, cudaMemcpyDeviceToHost, st));
+    VS_CK(cudaStreamSynchronize(st));
+    return VS_OK;
+  };
+  auto unique = [&]() { return d.bound && h.top < d.bound && !h.repeated; };
+  // a wait more costs a join of repeated keys some 10 us; the kernels that a join of
+  // unique keys does not need cost it as much
+  const bool early = d.bound && nb >= ASK_ROWS;
+  if (early) {
+    probe(1);
+    VS_TRY(ask());
+  }
+  if (!early || !unique()) {
+    if (d.bound) { k_join_count<<<std::min(grid_for(nb), cap_grid), 256, 0, st>>>(d, (const uint32_t *)bkeys, slot_of); vs::note_launch(); }
+    { k_join_scan<<<std::min(grid_for(tp.cap + 1, 1024), cap_grid), 256, 0, st>>>(d, d.t.cnt, d.t.off, d.tile_off, tp.cap + 1,
+                                                                                  nb, d.ctl + 2); vs::note_launch(); }
+    if (nb) { k_join_scatter<<<std::min(grid_for(nb), cap_grid), 256, 0, st>>>(d, slot_of, rows_by_key); vs::note_launch(); }
+    probe(0);
+    { k_join_scan<<<std::min(grid_for(np + 1, 1024), cap_grid), 256, 0, st>>>(d, pcnt, poff, ptile, np, np, d.ctl + 3); vs::note_launch(); }
+    VS_TRY(ask());
+  }
   *count = h.total;
   const uint64_t rows = std::min<uint64_t>(h.total, max_rows);
   int32_t types[16];
@@ -635,10 +927,22 @@ int join_unique(Scratch &sc, FlatSide a, FlatSide b, bool build_a, Direct d, con
   vs_flat *f = nullptr;
   VS_TRY(flat_alloc(ea.ncols, types, rows, st, &f));
   for (int i = 0; i < ea.ncols; i++) ea.col[i].dst = f->cols[i];
+  ea.poff = poff;
+  ea.ptile = ptile;
+  ea.pslot = pslot;
+  ea.rows_by_key = rows_by_key;
+  ea.b = d;
   ea.n_probe = np;
   ea.out_rows = rows;
-  const int rc = rows ? exclusive_scan_u64(sums, offs, tiles, st) : VS_OK;
-  if (rc == VS_OK && rows) { k_fk_emit<<<grid, 256, 0, st>>>(ea, d, pkeys, offs); vs::note_launch(); }
+  int rc = VS_OK;
+  if (rows && unique()) {
+    rc = exclusive_scan_u64(sums, offs, tiles, st);
+    if (rc == VS_OK)
+      { k_fk_emit<<<(int)std::min<uint64_t>(tiles, cap_grid), 256, 0, st>>>(ea, (const uint32_t *)pkeys, offs); vs::note_launch(); }
+  } else if (rows) {
+    k_emit<<<(unsigned)((rows + EMIT_ROWS - 1) / EMIT_ROWS), 256, 0, st>>>(ea);
+    vs::note_launch();
+  }
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (rc != VS_OK || e != cudaSuccess) {
@@ -651,120 +955,18 @@ int join_unique(Scratch &sc, FlatSide a, FlatSide b, bool build_a, Direct d, con
                             : VS_OK;
 }
 
-// Flat x Flat join.  a = deps[0], b = deps[1]; result = a cols + b non-key cols.
-int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, vs_flat **out,
-                   uint64_t *count, cudaStream_t st) {
-  if (a.f->types[a.key] != b.f->types[b.key])
-    return fail(VS_ERR_ARG, "join key types differ (%d vs %d)", a.f->types[a.key], b.f->types[b.key]);
-  // GPU build side: the smaller table (the reference builds on the larger,
-  // join.cpp:39-43; the side only changes the output order)
-  const bool build_a = a.f->nrows < b.f->nrows;
-  const FlatSide &bd = build_a ? a : b, &pr = build_a ? b : a;
-  Scratch sc{st};
-  Table t{};
-  const uint64_t nb = bd.f->nrows, np = pr.f->nrows;
-  const bool vid = bd.f->types[bd.key] == VS_T_VID;
-  const uint32_t *bkeys = (const uint32_t *)bd.f->cols[bd.key], *pkeys = (const uint32_t *)pr.f->cols[pr.key];
-  const uint32_t bound = vid && nb && np ? direct_bound(nb) : 0u;
-  if (bound) {
-    Scratch dsc{st};
-    Direct d;
-    unsigned long long *d_total = nullptr;
-    const int rc = only_count ? table_alloc(sc, nb, false, false, &t, false) : VS_OK;
-    if (rc != VS_OK) return rc;
-    const int dc = direct_alloc(dsc, bkeys, nb, bound, t, &d, &d_total);
-    if (dc != VS_OK && dc != VS_ERR_OOM) return dc;
-    if (dc == VS_OK && only_count) {  // the arrays, or the hash table in their place
-      { k_direct_count<<<std::min(grid_for((nb + 3) / 4, 512), 2 * sm_count()), 512, 0, st>>>(d, t, bkeys, nb); vs::note_launch(); }
-      { k_direct_probe<<<grid_for((np + 3) / 4), 256, 0, st>>>(d, t, pkeys, np, d_total); vs::note_launch(); }
-      VS_CK(cudaGetLastError());
-      return read_total(d_total, count, st);
-    }
-    if (dc == VS_OK) {
-      bool done = false;
-      const int rr = join_unique(dsc, a, b, build_a, d, bkeys, nb, pkeys, np, d_total, max_rows, out, count, &done);
-      if (rr != VS_OK || done) return rr;
-    }
-  }
-  if (bound && only_count) {  // the table is there; no room for the arrays beside it
-    VS_CK(cudaMemsetAsync(t.keys, 0xff, 8 * (t.cap + 1), st));
-    VS_CK(cudaMemsetAsync(t.cnt, 0, 8 * (t.cap + 1), st));
-  } else {
-    VS_TRY(table_alloc(sc, bd.f->nrows, false, !only_count, &t));
-  }
-  uint32_t *slot_of = nullptr;
-  if (!only_count) VS_TRY(sc.get(&slot_of, bd.f->nrows));
-  if (bd.f->nrows && only_count)
-    { k_build_count<<<std::min(grid_for(bd.f->nrows), 4 * sm_count()), 256, 0, st>>>(
-          t, bd.f->cols[bd.key], bd.f->types[bd.key], bd.f->nrows); vs::note_launch(); }
-  else if (bd.f->nrows)
-    { k_build<<<grid_for(bd.f->nrows), 256, 0, st>>>(t, bd.f->cols[bd.key], bd.f->types[bd.key],
-                                                   bd.f->nrows, slot_of); vs::note_launch(); }
-  unsigned long long *d_total;
-  VS_TRY(sc.get(&d_total, 1));
-  VS_CK(cudaMemsetAsync(d_total, 0, 8, st));
-  if (only_count) {
-    if (pr.f->nrows)
-      { k_probe<<<grid_for(pr.f->nrows), 256, 0, st>>>(t, pr.f->cols[pr.key], pr.f->types[pr.key],
-                                                     pr.f->nrows, nullptr, nullptr, d_total); vs::note_launch(); }
-    VS_CK(cudaGetLastError());
-    return read_total(d_total, count, st);
-  }
-  // group build rows by key
-  VS_TRY(exclusive_scan_u64(t.cnt, t.off, t.cap + 1, st));
-  uint32_t *rows_by_key;
-  VS_TRY(sc.get(&rows_by_key, bd.f->nrows));
-  if (bd.f->nrows) { k_scatter<<<grid_for(bd.f->nrows), 256, 0, st>>>(t, slot_of, bd.f->nrows, rows_by_key); vs::note_launch(); }
-  unsigned long long *pcnt, *poff;
-  uint32_t *pslot;
-  VS_TRY(sc.get(&pcnt, pr.f->nrows));
-  VS_TRY(sc.get(&poff, pr.f->nrows + 1));
-  VS_TRY(sc.get(&pslot, pr.f->nrows));
-  if (pr.f->nrows)
-    { k_probe<<<grid_for(pr.f->nrows), 256, 0, st>>>(t, pr.f->cols[pr.key], pr.f->types[pr.key],
-                                                   pr.f->nrows, pcnt, pslot, d_total); vs::note_launch(); }
-  VS_TRY(exclusive_scan_u64(pcnt, poff, pr.f->nrows, st));
-  uint64_t total = 0;
-  VS_TRY(read_total(d_total, &total, st));
-  *count = total;
-  const uint64_t rows = std::min<uint64_t>(total, max_rows);
-  int32_t types[16];
-  EmitArgs ea{};
-  VS_TRY(join_columns(a, b, build_a, types, &ea));
-  const int nc = ea.ncols;
-  vs_flat *f = nullptr;
-  VS_TRY(flat_alloc(nc, types, rows, st, &f));
-  for (int i = 0; i < nc; i++) ea.col[i].dst = f->cols[i];
-  ea.poff = poff;
-  ea.pslot = pslot;
-  ea.rows_by_key = rows_by_key;
-  ea.t = t;
-  ea.n_probe = pr.f->nrows;
-  ea.out_rows = rows;
-  if (rows) { k_emit<<<(unsigned)((rows + EMIT_ROWS - 1) / EMIT_ROWS), 256, 0, st>>>(ea); vs::note_launch(); }
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    vs_flat_free(f);
-    return cuda_fail(e, "hash join", __FILE__, __LINE__);
-  }
-  *out = f;
-  return total > max_rows ? fail(VS_ERR_CAPACITY, "join produced %llu rows, bound %llu",
-                                 (unsigned long long)total, (unsigned long long)max_rows)
-                          : VS_OK;
-}
-
 // Count-only Flat x Mat: the flat side's multiplicities against column popcounts.
 int count_flat_mat(FlatSide f, const vs_bitmat *m, uint64_t *count, cudaStream_t st) {
   if (f.f->types[f.key] != VS_T_VID) return fail(VS_ERR_ARG, "matrix keys are VIDs; flat key is not");
   Scratch sc{st};
-  Table t;
-  VS_TRY(table_alloc(sc, f.f->nrows, false, false, &t));
+  TablePart tp;
+  tp.add(sc, f.f->nrows, false, 1);
+  VS_TRY(sc.alloc());
+  VS_TRY(tp.clear(sc));
+  const Table t = tp.table(sc);
   if (f.f->nrows)
-    { k_build<<<grid_for(f.f->nrows), 256, 0, st>>>(t, f.f->cols[f.key], VS_T_VID, f.f->nrows, nullptr); vs::note_launch(); }
-  unsigned long long *d_total;
-  VS_TRY(sc.get(&d_total, 1));
-  VS_CK(cudaMemsetAsync(d_total, 0, 8, st));
+    { k_build<<<grid_for(f.f->nrows), 256, 0, st>>>(t, f.f->cols[f.key], VS_T_VID, f.f->nrows); vs::note_launch(); }
+  unsigned long long *d_total = sc.at<unsigned long long>(tp.zeroed);
   if (m->cols)
     { k_count_mat<<<grid_for((uint64_t)m->cols * 32), 256, 0, st>>>(t, m->words, m->cols, m->wpc,
                                                                  m->col_map, d_total); vs::note_launch(); }
@@ -774,11 +976,11 @@ int count_flat_mat(FlatSide f, const vs_bitmat *m, uint64_t *count, cudaStream_t
 
 int count_mat_mat(const vs_bitmat *a, const vs_bitmat *b, uint64_t *count, cudaStream_t st) {
   Scratch sc{st};
-  Table t{};
   const bool direct = !a->col_map && !b->col_map;
   if (direct) {
-    unsigned long long *d_total;
-    VS_TRY(sc.get(&d_total, 1));
+    sc.add<uint64_t>(1);
+    VS_TRY(sc.alloc());
+    unsigned long long *d_total = sc.at<unsigned long long>(0);
     VS_CK(cudaMemsetAsync(d_total, 0, 8, st));
     const uint32_t cols = std::min(a->cols, b->cols);
     if (cols)
@@ -788,13 +990,13 @@ int count_mat_mat(const vs_bitmat *a, const vs_bitmat *b, uint64_t *count, cudaS
     VS_CK(cudaGetLastError());
     return read_total(d_total, count, st);
   }
-  {
-    VS_TRY(table_alloc(sc, a->cols, true, false, &t));
-    if (a->cols) { k_build_cols<<<grid_for(a->cols), 256, 0, st>>>(t, a->col_map, a->cols); vs::note_launch(); }
-  }
-  unsigned long long *d_total;
-  VS_TRY(sc.get(&d_total, 1));
-  VS_CK(cudaMemsetAsync(d_total, 0, 8, st));
+  TablePart tp;
+  tp.add(sc, a->cols, true, 1);
+  VS_TRY(sc.alloc());
+  VS_TRY(tp.clear(sc));
+  const Table t = tp.table(sc);
+  if (a->cols) { k_build_cols<<<grid_for(a->cols), 256, 0, st>>>(t, a->col_map, a->cols); vs::note_launch(); }
+  unsigned long long *d_total = sc.at<unsigned long long>(tp.zeroed);
   if (b->cols)
     { k_count_mat_mat<<<grid_for((uint64_t)b->cols * 32), 256, 0, st>>>(
         t, a->words, a->cols, a->wpc, b->words, b->cols, b->wpc, b->col_map, direct ? 1 : 0, d_total); vs::note_launch(); }
@@ -983,8 +1185,8 @@ int vs_hash_join_count_noalloc(const void *keys_a, uint64_t na, const void *keys
   t.cnt = base + (NOALLOC_SLOTS + 1);
   unsigned long long *total = base + 2 * (NOALLOC_SLOTS + 1);
   { k_noalloc_clear<<<grid_for(t.cap + 1), 256, 0, st>>>(t.keys, t.cnt, total, t.cap); vs::note_launch(); }
-  if (nbld) { k_build<<<grid_for(nbld), 256, 0, st>>>(t, bk, key_type, nbld, nullptr); vs::note_launch(); }
-  if (nprb) { k_probe<<<grid_for(nprb), 256, 0, st>>>(t, pk, key_type, nprb, nullptr, nullptr, total); vs::note_launch(); }
+  if (nbld) { k_build<<<grid_for(nbld), 256, 0, st>>>(t, bk, key_type, nbld); vs::note_launch(); }
+  if (nprb) { k_probe<<<grid_for(nprb), 256, 0, st>>>(t, pk, key_type, nprb, total); vs::note_launch(); }
   VS_CK(cudaGetLastError());
   VS_CK(cudaMemcpyAsync(count, total, sizeof(unsigned long long), cudaMemcpyDefault, st));
   VS_CK(cudaStreamSynchronize(st));
