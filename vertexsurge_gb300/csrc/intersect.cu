@@ -88,6 +88,7 @@ struct Args {
   uint64_t mask_cap;             // below 2^32 - 1
   unsigned long long *mask_n;    // words the tasks need, kept or not
   uint32_t *mask_at;             // a task's first word
+  uint32_t tuples;               // of a task, at most PAIR_TUPLES
 };
 
 constexpr int ISECT_CHUNK = 4;  // base tuples a warp takes from the queue at a time
@@ -414,7 +415,8 @@ __global__ void __launch_bounds__(256) k_isect_pair_pieces(Args a, const ulonglo
 }
 
 // Rows of a two-adjacency intersection (triangle listing): counts per tuple, then,
-// with the prefix sums, the rows.  A warp takes PAIR_TUPLES tuples (a task), lane j
+// with the prefix sums, the rows.  A warp takes up to PAIR_TUPLES tuples (a task; fewer
+// where there are not enough for every warp: eight tuples of hubs 710 -> 158 us), lane j
 // loading tuple j's lists, so their dependent loads overlap, and walks each shorter
 // list 64 candidates at a time (two membership loads per lane in flight).  Bound by
 // the latency of those loads.  The counting pass keeps a bit per candidate, from
@@ -444,11 +446,11 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
   unsigned long long tot = 0;
   for (;;) {
     unsigned long long t0 = 0;
-    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)PAIR_TUPLES);
+    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)a.tuples);
     t0 = __shfl_sync(FULLMASK, t0, 0);
     if (t0 >= a.nbase) break;
     const uint64_t t = t0 + lane;
-    const bool mine = lane < PAIR_TUPLES && t < a.nbase;
+    const bool mine = lane < a.tuples && t < a.nbase;
     PairTuple p{0, 0, 0, 0, 0, -1};
     unsigned long long pos = 0;
     if (mine) {
@@ -467,7 +469,7 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
       at = __shfl_sync(FULLMASK, at, PAIR_TUPLES - 1);
       if (at + __shfl_sync(FULLMASK, end, PAIR_TUPLES - 1) <= a.mask_cap) {
         mo = (uint32_t)(at + end - nw);
-        if (lane == 0) a.mask_at[t0 / PAIR_TUPLES] = (uint32_t)at;
+        if (lane == 0) a.mask_at[t0 / a.tuples] = (uint32_t)at;
       }
     }
     unsigned long long found = 0;  // lane j: matches of tuple j
@@ -531,10 +533,10 @@ __global__ void __launch_bounds__(256) k_isect_pair_emit(Args a) {
   const int lane = threadIdx.x & 31;
   for (;;) {
     unsigned long long t0 = 0;
-    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)PAIR_TUPLES);
+    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)a.tuples);
     t0 = __shfl_sync(FULLMASK, t0, 0);
     if (t0 >= a.nbase) break;
-    const uint64_t tn = t0 + PAIR_TUPLES < a.nbase ? t0 + PAIR_TUPLES : a.nbase;
+    const uint64_t tn = t0 + a.tuples < a.nbase ? t0 + a.tuples : a.nbase;
     unsigned long long out = a.toff[t0];
     const unsigned long long out_end = a.toff[tn] < a.max_rows ? a.toff[tn] : a.max_rows;
     if (out >= out_end) continue;
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(256) k_isect_pair_emit(Args a) {
     const uint32_t start = lane < PAIR_TUPLES ? end - nw : end;
     const uint32_t words = __shfl_sync(FULLMASK, end, PAIR_TUPLES - 1);
     const uint32_t *walk = (p.w1 ? a.dep[1] : a.dep[0]).adj + p.wlo - (int64_t)start * 32;
-    const uint32_t *mask = a.mask + a.mask_at[t0 / PAIR_TUPLES];
+    const uint32_t *mask = a.mask + a.mask_at[t0 / a.tuples];
     for (uint32_t w0 = 0; w0 < words && out < out_end; w0 += 32) {
       const uint32_t w = w0 + lane, m = w < words ? __ldg(mask + w) : 0u;
       int own = 0;  // the last tuple whose words start at or before w
@@ -1067,6 +1069,7 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
   }
   a.tcnt = tcnt;
   a.total = d_total;
+  a.tuples = 1;
   a.emit = 0;
   const int grid = grid_for(a.nbase * 32);
   VS_TRY(sc.get(&a.next, 1));
@@ -1105,10 +1108,11 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
     }
   } else if (a.nbase) {
     if (pair) {
+      while (a.tuples < PAIR_TUPLES && a.nbase >= 64ull * sm_count() * a.tuples) a.tuples *= 2;  // 32 warps an SM, twice
       // bits of the candidates for the emitting pass: room for 512 a tuple (64 bytes of
       // scratch, 256 MB in all), none when memory is short
       a.mask_cap = std::min<uint64_t>(16 * a.nbase, 1ull << 26);
-      if (sc.get(&a.mask, a.mask_cap) != VS_OK || sc.get(&a.mask_at, a.nbase / PAIR_TUPLES + 1) != VS_OK) {
+      if (sc.get(&a.mask, a.mask_cap) != VS_OK || sc.get(&a.mask_at, a.nbase / a.tuples + 1) != VS_OK) {
         cudaGetLastError();
         a.mask = nullptr;
       }
