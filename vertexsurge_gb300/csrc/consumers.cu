@@ -47,32 +47,34 @@ struct Scratch {
 };
 
 // ---- column popcounts --------------------------------------------------------
-// G = min(32, pow2 >= uint4 per column) lanes per column, 4 columns per group in
-// flight at once: bound by reading the matrix.
+// G = min(32, pow2 >= uint4 per column) lanes per column, K columns per group in
+// flight at once: bound by reading the matrix.  K is 4, or 1 where that leaves warps
+// without a column (64 columns of 1M rows: 134 -> 74 us).
+template <int K>
 __global__ void __launch_bounds__(256) k_col_counts(const uint4 *__restrict__ w, uint32_t Q, uint32_t cols, uint32_t G,
                                                     const uint32_t *__restrict__ colnz, uint32_t *__restrict__ cnt) {
   const uint32_t lane = threadIdx.x & 31, gl = lane & (G - 1), g = lane / G, gpw = 32 / G;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const uint64_t warps = (uint64_t)gridDim.x * blockDim.x / 32;
   // warp-uniform loop: every lane reaches the group shuffles
-  for (uint64_t base = warp * gpw * 4; base < cols; base += warps * gpw * 4) {
-    uint32_t s[4];
-    bool look[4];
+  for (uint64_t base = warp * gpw * K; base < cols; base += warps * gpw * K) {
+    uint32_t s[K];
+    bool look[K];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < K; k++) {
       const uint64_t c = base + k * gpw + g;
       look[k] = c < cols && (!colnz || __ldg(colnz + c));
       s[k] = 0;
     }
     for (uint32_t q = gl; q < Q; q += G) {
-      uint4 x[4];
+      uint4 x[K];
 #pragma unroll
-      for (int k = 0; k < 4; k++) x[k] = look[k] ? __ldg(w + (base + k * gpw + g) * Q + q) : make_uint4(0, 0, 0, 0);
+      for (int k = 0; k < K; k++) x[k] = look[k] ? __ldg(w + (base + k * gpw + g) * Q + q) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int k = 0; k < 4; k++) s[k] += popc4(x[k]);
+      for (int k = 0; k < K; k++) s[k] += popc4(x[k]);
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < K; k++) {
       if (G == 32)
         s[k] = __reduce_add_sync(0xffffffffu, s[k]);
       else
@@ -199,8 +201,13 @@ int column_counts(const vs_bitmat *m, Scratch &sc, uint32_t **cnt) {
   uint32_t G = 1;
   while (G < 32 && G < m->wpc / 2) G <<= 1;
   if (m->cols)
-    { k_col_counts<<<grid_for(((uint64_t)m->cols * G + 3) / 4), 256, 0, sc.st>>>(
-          reinterpret_cast<const uint4 *>(m->words), m->wpc / 2, m->cols, G, m->colnz, *cnt); vs::note_launch(); }
+    {
+      const bool few = (uint64_t)m->cols * G < 4ull * 32 * 32 * sm_count();  // 32 warps an SM
+      (few ? k_col_counts<1> : k_col_counts<4>)<<<grid_for(few ? (uint64_t)m->cols * G : ((uint64_t)m->cols * G + 3) / 4), 256,
+                                                  0, sc.st>>>(reinterpret_cast<const uint4 *>(m->words), m->wpc / 2, m->cols, G,
+                                                              m->colnz, *cnt);
+      vs::note_launch();
+    }
   VS_CK(cudaGetLastError());
   return VS_OK;
 }
