@@ -73,9 +73,13 @@ __global__ void __launch_bounds__(256) k_transpose(const uint64_t *__restrict__ 
       s_in[(q * 4 + 3) * TP_IN + c] = x.w;
     }
     __syncthreads();
+    // blocks that hold part of the matrix (whole output uint4: the words past the last
+    // column are zeros)
+    const uint32_t nw = min((uint32_t)TPW, (in_rows - tr * TP + 31) / 32), ng = min((uint32_t)TPW, (in_cols - tc * TP + 127) / 128 * 4);
 #pragma unroll 4
     for (uint32_t b = warp; b < TPW * TPW; b += 8) {  // 32 x 32 blocks: word w of columns 32g..32g+31
       const uint32_t w = b / TPW, g = b % TPW;
+      if (w >= nw || g >= ng) continue;
       uint32_t x = s_in[w * TP_IN + g * 32 + lane];
       x = __byte_perm(x, __shfl_xor_sync(FULL, x, 16), sel16);
       x = __byte_perm(x, __shfl_xor_sync(FULL, x, 8), sel8);
