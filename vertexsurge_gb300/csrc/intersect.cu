@@ -811,6 +811,13 @@ struct Scratch {
     if (rc == VS_OK) p[n++] = *out;
     return rc;
   }
+  void drop(void *x) {  // give one back early
+    for (int i = 0; i < n; i++)
+      if (p[i] == x) {
+        dfree(x, st);
+        p[i] = nullptr;
+      }
+  }
   ~Scratch() {
     for (int i = 0; i < n; i++) dfree(p[i], st);
   }
@@ -1144,7 +1151,13 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
   for (uint32_t c = 0; c < bf->ncols; c++) types[c] = bf->types[c];
   types[bf->ncols] = VS_T_VID;
   vs_flat *f = nullptr;
-  VS_TRY(flat_alloc(bf->ncols + 1, types, rows, st, &f));
+  int rf = flat_alloc(bf->ncols + 1, types, rows, st, &f);
+  if (rf == VS_ERR_OOM && a.mask) {  // the candidates' bits hold the room: they are tested again
+    sc.drop(a.mask);
+    a.mask = nullptr;
+    rf = flat_alloc(bf->ncols + 1, types, rows, st, &f);
+  }
+  VS_TRY(rf);
   a.nbcols = (int)bf->ncols;
   for (uint32_t c = 0; c < bf->ncols; c++) {
     a.col[c].dst = f->cols[c];
