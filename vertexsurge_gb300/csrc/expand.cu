@@ -2966,7 +2966,9 @@ int vs_expand_plan_footprint(const vs_graph *g, uint32_t S, const vs_expand_para
   const uint32_t nslices = (uint32_t)((W / 2 + qs - 1) / qs);
   const int L = pick_variant(qs).L;
   const uint64_t thr = p->hub_threshold ? std::min(p->hub_threshold, 1u << 16) : heavy_default(L);
-  const uint64_t multi = std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, std::max<uint64_t>(thr, piece_edges(L))));
+  // (of two lists one each may already be two pieces, whatever their length)
+  const bool two = p->direction == VS_DIR_BOTH && g->directed;
+  const uint64_t multi = std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, std::max<uint64_t>(thr, two ? 0 : piece_edges(L))));
   b += 16 * (list_edges / piece_edges(L) + 2 * std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, thr)));
   b += multi * (W * 8 + 4 + 4 * nslices) + (uint64_t)(p->k_max + 1) * (W * 8 + 4 * nslices);
   const bool slots = short_slots_ok(S, nslices, p->short_share, V, (uint32_t)W);
