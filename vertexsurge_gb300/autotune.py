@@ -43,9 +43,10 @@ def _time_runs(plan, src, repeats, stream):
 def tune(dg, src, k_min, k_max, path="shortest", direction="forward", stream=None, repeats=3,
          pull_kinds=(0,), sparse_fracs=(0.0005, 0.002, 0.005, 0.02), hub_thresholds=(0, 256),
          slice_words=(0,), short_shares=(0.0, -1.0), cache_file: str | None = None) -> dict:
-    """Time the candidates (the PULL kernel kinds of vs_expand_plan_set_pull_kernel all run
-    the same kernel; a caller may still pass several); returns {'pull_kind', 'sparse_frac', 'hub_threshold', 'slice_words',
-    'short_share', 'ms', 'table'} and caches it."""
+    """Time the candidates; returns {'pull_kind', 'sparse_frac', 'hub_threshold', 'slice_words',
+    'short_share', 'ms', 'table'} and caches it.  The PULL kernel kinds of
+    vs_expand_plan_set_pull_kernel all run the same kernel: they share a time, and the first
+    one passed is the setting's."""
     import torch
     key = _key(dg, len(src), k_min, k_max, path, direction)
     if key in _CACHE:
@@ -67,11 +68,11 @@ def tune(dg, src, k_min, k_max, path="shortest", direction="forward", stream=Non
                 try:
                     for pk in pull_kinds:
                         plan.set_pull_kernel(pk)
-                        for sf in sparse_fracs:
-                            plan.set_tuning(sparse_frac=sf)
-                            ms = _time_runs(plan, dsrc, repeats, stream)
-                            table.append({"pull_kind": pk, "sparse_frac": sf, "hub_threshold": hub,
-                                          "slice_words": sw, "short_share": rb, "ms": ms})
+                    for sf in sparse_fracs:
+                        plan.set_tuning(sparse_frac=sf)
+                        ms = _time_runs(plan, dsrc, repeats, stream)
+                        table += [{"pull_kind": pk, "sparse_frac": sf, "hub_threshold": hub,
+                                   "slice_words": sw, "short_share": rb, "ms": ms} for pk in pull_kinds]
                 finally:
                     plan.free()
     best = min(table, key=lambda r: r["ms"])

@@ -2682,7 +2682,7 @@ PlanCache &plan_cache() {
 bool same_params(const vs_expand_params &a, const vs_expand_params &b) {
   return a.k_min == b.k_min && a.k_max == b.k_max && a.path_type == b.path_type && a.direction == b.direction &&
          a.strategy == b.strategy && a.use_picker == b.use_picker && a.hub_threshold == b.hub_threshold &&
-         a.slice_words == b.slice_words && a.pair_capacity == b.pair_capacity && a.pull_kernel == b.pull_kernel &&
+         a.slice_words == b.slice_words && a.pair_capacity == b.pair_capacity &&  // (pull_kernel has no effect)
          a.sparse_frac == b.sparse_frac && a.short_share == b.short_share;
 }
 
