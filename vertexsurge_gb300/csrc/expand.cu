@@ -838,6 +838,9 @@ template <int L> constexpr int kChunk = L == 1 ? 8 : 32;
 // longest list, so narrow rows (many groups) cut earlier.
 inline uint32_t piece_edges(int L) { return L <= 8 ? 512 : 256; }
 inline uint32_t heavy_default(int L) { return L <= 8 ? 64 : 256; }
+// Lists up to here are walked whole when the caller asks for it: four of them still
+// number their entries in 32 bits.
+constexpr uint32_t HEAVY_MAX = 1u << 28;
 
 // Whether `p` holds on every lane of this lane's group.
 template <int L> __device__ __forceinline__ bool group_all(bool p) {
@@ -2869,7 +2872,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   }
   // heavy targets of the pull direction set and their pieces
   const PullVariant &var = pick_variant(pl->qslice);
-  pl->heavy_threshold = p->hub_threshold ? std::min(p->hub_threshold, 1u << 16) : heavy_default(var.L);
+  pl->heavy_threshold = p->hub_threshold ? std::min(p->hub_threshold, HEAVY_MAX) : heavy_default(var.L);
   {
     Lists in = pull_lists(g, p->direction);
     unsigned *dn = nullptr;
@@ -2965,7 +2968,7 @@ int vs_expand_plan_footprint(const vs_graph *g, uint32_t S, const vs_expand_para
   qs = std::max<uint32_t>(1, std::min<uint32_t>(qs, 256));
   const uint32_t nslices = (uint32_t)((W / 2 + qs - 1) / qs);
   const int L = pick_variant(qs).L;
-  const uint64_t thr = p->hub_threshold ? std::min(p->hub_threshold, 1u << 16) : heavy_default(L);
+  const uint64_t thr = p->hub_threshold ? std::min(p->hub_threshold, HEAVY_MAX) : heavy_default(L);
   // (of two lists one each may already be two pieces, whatever their length)
   const bool two = p->direction == VS_DIR_BOTH && g->directed;
   const uint64_t multi = std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, std::max<uint64_t>(thr, two ? 0 : piece_edges(L))));
