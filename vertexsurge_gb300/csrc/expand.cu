@@ -2643,7 +2643,7 @@ int plan_free(vs_expand_plan *pl) {
   void *ptrs[] = {pl->tiny[0], pl->tiny[1], pl->slot[0], pl->slot[1], pl->resflag, pl->pdeg[0], pl->pdeg[1], pl->doff,
                   pl->bsum, pl->hmask, pl->rowk, pl->buf[0], pl->buf[1], pl->flag[0], pl->flag[1], pl->vis, pl->acc,
                   pl->pairs[0], pl->pairs[1], pl->push_list, pl->touched, pl->d_src,
-                  pl->d_tgt, pl->d_dist, pl->ctr, pl->pieces, pl->heavy_rows, pl->heavy_np, pl->heavy_left, pl->bits};
+                  pl->d_tgt, pl->d_dist, pl->ctr, pl->pieces, pl->bits};
   for (void *p : ptrs)  // stream-ordered after the plan's last run
     if (p) dfree(p, st);
   for (cudaEvent_t e : pl->ev)
@@ -2875,13 +2875,12 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
   pl->heavy_threshold = p->hub_threshold ? std::min(p->hub_threshold, HEAVY_MAX) : heavy_default(var.L);
   {
     Lists in = pull_lists(g, p->direction);
-    unsigned *dn = nullptr;
-    uint32_t *heavy = nullptr;
-    if ((rc = dalloc_n(&heavy, V, st)) != VS_OK || (rc = dalloc_n(&dn, 8, st)) != VS_OK) {
-      dfree(heavy, st);
+    unsigned *dn = nullptr;  // counters, then the heavy targets
+    if ((rc = dalloc_n(&dn, 8 + (size_t)V, st)) != VS_OK) {
       plan_free(pl);
       return rc;
     }
+    uint32_t *heavy = dn + 8;
     cudaMemsetAsync(dn, 0, 8 * sizeof(unsigned), st);
     const uint32_t pe = piece_edges(var.L);
     { k_hubs<<<sm_count() * 4, 256, 0, st>>>(in, V, pl->heavy_threshold, pe, heavy, dn); vs::note_launch(); }
@@ -2891,23 +2890,22 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     pl->nheavy = hn[0];
     pl->npieces = hn[1];
     const size_t nmulti = hn[2];
-    if (e == cudaSuccess && pl->nheavy) {
-      if ((rc = dalloc_n(&pl->pieces, pl->npieces, st)) != VS_OK ||
-          (rc = dalloc_n(&pl->heavy_rows, nmulti * pl->Q, st)) != VS_OK ||
-          (rc = dalloc_n(&pl->heavy_np, nmulti, st)) != VS_OK ||
-          (rc = dalloc_n(&pl->heavy_left, nmulti * pl->nslices, st)) != VS_OK) {
-        dfree(heavy, st);
+    if (e == cudaSuccess && pl->nheavy) {  // one allocation: pieces, unions, counts
+      const size_t rows = nmulti * pl->Q;
+      if ((rc = dalloc_n(&pl->pieces, pl->npieces + rows + (nmulti * (1 + pl->nslices) + 3) / 4, st)) != VS_OK) {
         dfree(dn, st);
         plan_free(pl);
         return rc;
       }
-      e = cudaMemsetAsync(pl->heavy_rows, 0, nmulti * pl->Q * 16, st);
+      pl->heavy_rows = pl->pieces + pl->npieces;
+      pl->heavy_np = reinterpret_cast<uint32_t *>(pl->heavy_rows + rows);
+      pl->heavy_left = pl->heavy_np + nmulti;
+      e = cudaMemsetAsync(pl->heavy_rows, 0, rows * 16, st);
+      // (a first run on another stream waits for this one)
       { k_hub_pieces<<<sm_count() * 4, 256, 0, st>>>(in, heavy, pl->nheavy, pe, pl->pieces, dn + 3, pl->heavy_np,
                                                      pl->heavy_left, pl->nslices); vs::note_launch(); }
       if (e == cudaSuccess) e = cudaGetLastError();
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // runs may be on any stream
     }
-    dfree(heavy, st);
     dfree(dn, st);
     if (e != cudaSuccess) {
       plan_free(pl);
