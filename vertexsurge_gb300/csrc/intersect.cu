@@ -61,6 +61,7 @@ struct Dep {
   const int32_t *hub_slot;
   const uint64_t *hub_bm;
   uint32_t hub_words;
+  uint32_t limit;  // new vertices below this: its graph's, and the caller's bound
 };
 
 struct OutCol {
@@ -88,7 +89,7 @@ struct Args {
   uint64_t mask_cap;             // below 2^32 - 1
   unsigned long long *mask_n;    // words the tasks need, kept or not
   uint32_t *mask_at;             // a task's first word
-  uint32_t tuples;               // of a task, at most PAIR_TUPLES
+  int shift;                     // a task has 1 << shift tuples, at most PAIR_TUPLES
 };
 
 constexpr int ISECT_CHUNK = 4;  // base tuples a warp takes from the queue at a time
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(256) k_isect(Args a) {
             if (d.kind == DEP_MAT) {
               keep = x < d.rows && ((d.words[(size_t)col[i] * d.wpc + (x >> 6)] >> (x & 63)) & 1ull);
             } else if (meth[i] == M_BITMAP) {  // the walked list may be another graph's, with more vertices
-              keep = x < d.n_u && (__ldg(d.hub_bm + (size_t)hs[i] * d.hub_words + (x >> 6)) >> (x & 63)) & 1ull;
+              keep = x < d.limit && (__ldg(d.hub_bm + (size_t)hs[i] * d.hub_words + (x >> 6)) >> (x & 63)) & 1ull;
             } else if (d.kind == DEP_SORTED) {
               keep = in_sorted(d.adj, lo[i], hi[i], x);
             } else {
@@ -332,9 +333,9 @@ __device__ __forceinline__ PairTuple pair_tuple(const Args &a, uint64_t t, int l
 // Candidate x of a walked list in the other list of its tuple (of another graph,
 // perhaps: its bitmaps end at its own last vertex).
 __device__ __forceinline__ bool pair_member(const Args &a, int w1, int hs, int64_t olo, int64_t ohi, uint32_t x) {
-  if (x >= a.cache_rows) return false;
   const Dep &o = w1 ? a.dep[0] : a.dep[1];
-  return hs >= 0 ? x < o.n_u && ((__ldg(o.hub_bm + (size_t)hs * o.hub_words + (x >> 6)) >> (x & 63)) & 1ull)
+  if (x >= o.limit) return false;
+  return hs >= 0 ? ((__ldg(o.hub_bm + (size_t)hs * o.hub_words + (x >> 6)) >> (x & 63)) & 1ull)
                  : in_sorted(o.adj, olo, ohi, x);
 }
 
@@ -446,11 +447,11 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
   unsigned long long tot = 0;
   for (;;) {
     unsigned long long t0 = 0;
-    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)a.tuples);
+    if (lane == 0) t0 = atomicAdd(a.next, 1ull << a.shift);
     t0 = __shfl_sync(FULLMASK, t0, 0);
     if (t0 >= a.nbase) break;
     const uint64_t t = t0 + lane;
-    const bool mine = lane < a.tuples && t < a.nbase;
+    const bool mine = lane < 1 << a.shift && t < a.nbase;
     PairTuple p{0, 0, 0, 0, 0, -1};
     unsigned long long pos = 0;
     if (mine) {
@@ -469,7 +470,7 @@ template <bool EMIT> __global__ void __launch_bounds__(256) k_isect_pair_rows(Ar
       at = __shfl_sync(FULLMASK, at, PAIR_TUPLES - 1);
       if (at + __shfl_sync(FULLMASK, end, PAIR_TUPLES - 1) <= a.mask_cap) {
         mo = (uint32_t)(at + end - nw);
-        if (lane == 0) a.mask_at[t0 / a.tuples] = (uint32_t)at;
+        if (lane == 0) a.mask_at[t0 >> a.shift] = (uint32_t)at;
       }
     }
     unsigned long long found = 0;  // lane j: matches of tuple j
@@ -533,10 +534,10 @@ __global__ void __launch_bounds__(256) k_isect_pair_emit(Args a) {
   const int lane = threadIdx.x & 31;
   for (;;) {
     unsigned long long t0 = 0;
-    if (lane == 0) t0 = atomicAdd(a.next, (unsigned long long)a.tuples);
+    if (lane == 0) t0 = atomicAdd(a.next, 1ull << a.shift);
     t0 = __shfl_sync(FULLMASK, t0, 0);
     if (t0 >= a.nbase) break;
-    const uint64_t tn = t0 + a.tuples < a.nbase ? t0 + a.tuples : a.nbase;
+    const uint64_t tn = min(t0 + (1ull << a.shift), (unsigned long long)a.nbase);
     unsigned long long out = a.toff[t0];
     const unsigned long long out_end = a.toff[tn] < a.max_rows ? a.toff[tn] : a.max_rows;
     if (out >= out_end) continue;
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(256) k_isect_pair_emit(Args a) {
     const uint32_t start = lane < PAIR_TUPLES ? end - nw : end;
     const uint32_t words = __shfl_sync(FULLMASK, end, PAIR_TUPLES - 1);
     const uint32_t *walk = (p.w1 ? a.dep[1] : a.dep[0]).adj + p.wlo - (int64_t)start * 32;
-    const uint32_t *mask = a.mask + a.mask_at[t0 / a.tuples];
+    const uint32_t *mask = a.mask + a.mask_at[t0 >> a.shift];
     for (uint32_t w0 = 0; w0 < words && out < out_end; w0 += 32) {
       const uint32_t w = w0 + lane, m = w < words ? __ldg(mask + w) : 0u;
       int own = 0;  // the last tuple whose words start at or before w
@@ -1047,6 +1048,7 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
   bool hubs = false;
   for (uint32_t i = 0; i < ndeps; i++)
     if (deps[i].graph) {
+      a.dep[i].limit = (uint32_t)std::min<uint64_t>(a.cache_rows, a.dep[i].n_u);
       fg = deps[i].graph;
       hubs |= a.dep[i].hub_slot != nullptr;
     }
@@ -1076,7 +1078,7 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
   }
   a.tcnt = tcnt;
   a.total = d_total;
-  a.tuples = 1;
+  a.shift = 0;
   a.emit = 0;
   const int grid = grid_for(a.nbase * 32);
   VS_TRY(sc.get(&a.next, 1));
@@ -1115,11 +1117,11 @@ int vs_mintersect_ex(vs_table_ref base, const vs_isect_dep *deps, uint32_t ndeps
     }
   } else if (a.nbase) {
     if (pair) {
-      while (a.tuples < PAIR_TUPLES && a.nbase >= 64ull * sm_count() * a.tuples) a.tuples *= 2;  // 32 warps an SM, twice
+      while (1 << a.shift < PAIR_TUPLES && a.nbase >> a.shift >= 64ull * sm_count()) a.shift++;  // 32 warps an SM, twice
       // bits of the candidates for the emitting pass: room for 512 a tuple (64 bytes of
       // scratch, 256 MB in all), none when memory is short
       a.mask_cap = std::min<uint64_t>(16 * a.nbase, 1ull << 26);
-      if (sc.get(&a.mask, a.mask_cap) != VS_OK || sc.get(&a.mask_at, a.nbase / a.tuples + 1) != VS_OK) {
+      if (sc.get(&a.mask, a.mask_cap) != VS_OK || sc.get(&a.mask_at, (a.nbase >> a.shift) + 1) != VS_OK) {
         cudaGetLastError();
         a.mask = nullptr;
       }
