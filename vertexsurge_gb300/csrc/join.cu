@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(256) k_direct_probe(Direct d, Table t, const u
 // of repeated keys waited some 40 us longer.  4M probe rows against 1M rows of five
 // columns in all: unique keys 376 (hash table) -> 173 us, repeated ones 417 -> 400; 4,000
 // against 1,000 rows of repeated keys 125 -> 98.
-__global__ void __launch_bounds__(256) k_join_clear(Build b) {
+__global__ void __launch_bounds__(256) k_join_clear(Build b, int counts) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (join_mode(b) == J_HASH) {
     for (uint64_t i = i0; i <= b.t.cap; i += stride) {
@@ -264,7 +264,8 @@ __global__ void __launch_bounds__(256) k_join_clear(Build b) {
   } else {
     const uint32_t n4 = b.ctl[0] / 4 + 1;  // the bound is a multiple of four
     for (uint64_t i = i0; i < n4; i += stride) reinterpret_cast<uint4 *>(b.row)[i] = make_uint4(0, 0, 0, 0);
-    for (uint64_t i = i0; i < b.n; i += stride) b.t.cnt[i] = 0;
+    if (counts)
+      for (uint64_t i = i0; i < b.n; i += stride) b.t.cnt[i] = 0;
   }
 }
 
@@ -879,10 +880,13 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
   uint32_t *slot_of = sc.at<uint32_t>(o_slot), *rows_by_key = sc.at<uint32_t>(o_rows), *pslot = sc.at<uint32_t>(o_pslot);
   unsigned long long *sums = pcnt, *offs = poff;  // UNIQUE: by tile
   const int cap_grid = 8 * sm_count();
+  // a wait more costs a join of repeated keys some 10 us; the kernels that a join of
+  // unique keys does not need cost it as much
+  const bool early = d.bound && nb >= ASK_ROWS;
   VS_CK(cudaMemsetAsync(d_total, 0, 24, st));
   if (d.bound)
     { k_key_max<<<std::min(grid_for((nb + 3) / 4), 4 * sm_count()), 256, 0, st>>>((const uint32_t *)bkeys, nb, d.ctl); vs::note_launch(); }
-  { k_join_clear<<<std::min(grid_for(std::max<uint64_t>(tp.cap + 1, d.bound / 4)), cap_grid), 256, 0, st>>>(d); vs::note_launch(); }
+  { k_join_clear<<<std::min(grid_for(std::max<uint64_t>(tp.cap + 1, d.bound / 4)), cap_grid), 256, 0, st>>>(d, !early); vs::note_launch(); }
   const uint64_t first = std::min<uint64_t>(nb, d.bound ? 512ull * sm_count() : nb);  // rows
   if (first) { k_join_build<<<grid_for(first), 256, 0, st>>>(d, bkeys, ktype, slot_of, 0, first); vs::note_launch(); }
   if (nb > first) { k_join_build<<<grid_for(nb - first), 256, 0, st>>>(d, bkeys, ktype, slot_of, first, nb); vs::note_launch(); }
@@ -903,14 +907,12 @@ int join_flat_flat(FlatSide a, FlatSide b, bool only_count, uint64_t max_rows, v
     return VS_OK;
   };
   auto unique = [&]() { return d.bound && h.top < d.bound && !h.repeated; };
-  // a wait more costs a join of repeated keys some 10 us; the kernels that a join of
-  // unique keys does not need cost it as much
-  const bool early = d.bound && nb >= ASK_ROWS;
   if (early) {
     probe(1);
     VS_TRY(ask());
   }
   if (!early || !unique()) {
+    if (early && h.top < d.bound) VS_CK(cudaMemsetAsync(d.t.cnt, 0, 8 * nb, st));  // its slots, not cleared yet
     if (d.bound) { k_join_count<<<std::min(grid_for(nb), cap_grid), 256, 0, st>>>(d, (const uint32_t *)bkeys, slot_of); vs::note_launch(); }
     { k_join_scan<<<std::min(grid_for(tp.cap + 1, 1024), cap_grid), 256, 0, st>>>(d, d.t.cnt, d.t.off, d.tile_off, tp.cap + 1,
                                                                                   nb, d.ctl + 2); vs::note_launch(); }
