@@ -2837,7 +2837,7 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     PL_ALLOC(pl->d_tgt, S);
     PL_ALLOC(pl->d_dist, S);
   }
-  {  // counters, layer unions and task queues in one block: one memset clears them
+  {  // counters, layer unions and task queues in one block, which a run's first kernel clears
     const size_t c = (sizeof(Ctr) + 15) / 16 * 16, u = (size_t)(p->k_max + 1) * pl->Q * 16;
     pl->ctr_bytes = (c + u + (size_t)(p->k_max + 1) * pl->nslices * 4 + 15) / 16 * 16;
     char *base = nullptr;
@@ -2893,13 +2893,13 @@ int vs_expand_plan_create(vs_graph *g, uint32_t S, const vs_expand_params *p,
     pl->npieces = hn[1];
     const size_t nmulti = hn[2];
     if (e == cudaSuccess && pl->nheavy) {  // one allocation: pieces, unions, counts
-      const size_t rows = nmulti * pl->Q;
-      if ((rc = dalloc_n(&pl->pieces, pl->npieces + rows + (nmulti * (1 + pl->nslices) + 3) / 4, st)) != VS_OK) {
+      const size_t rows = nmulti * pl->Q, first = ((size_t)pl->npieces + 15) / 16 * 16;  // rows of whole lines
+      if ((rc = dalloc_n(&pl->pieces, first + rows + (nmulti * (1 + pl->nslices) + 3) / 4, st)) != VS_OK) {
         dfree(dn, st);
         plan_free(pl);
         return rc;
       }
-      pl->heavy_rows = pl->pieces + pl->npieces;
+      pl->heavy_rows = pl->pieces + first;
       pl->heavy_np = reinterpret_cast<uint32_t *>(pl->heavy_rows + rows);
       pl->heavy_left = pl->heavy_np + nmulti;
       e = cudaMemsetAsync(pl->heavy_rows, 0, rows * 16, st);
@@ -2972,7 +2972,7 @@ int vs_expand_plan_footprint(const vs_graph *g, uint32_t S, const vs_expand_para
   // (of two lists one each may already be two pieces, whatever their length)
   const bool two = p->direction == VS_DIR_BOTH && g->directed;
   const uint64_t multi = std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, std::max<uint64_t>(thr, two ? 0 : piece_edges(L))));
-  b += 16 * (list_edges / piece_edges(L) + 2 * std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, thr)));
+  b += 16 * (16 + list_edges / piece_edges(L) + 2 * std::min<uint64_t>(V, list_edges / std::max<uint64_t>(1, thr)));
   b += multi * (W * 8 + 4 + 4 * nslices) + (uint64_t)(p->k_max + 1) * (W * 8 + 4 * nslices);
   const bool slots = short_slots_ok(S, nslices, p->short_share, V, (uint32_t)W);
   if (bits_ok((uint32_t)V, qs, slots, list_edges)) b += bits_smem((uint32_t)V);
