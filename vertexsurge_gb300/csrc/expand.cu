@@ -1831,7 +1831,7 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
       fm = mine;
       if (fm) {
         oldf = a.flagN[v0];
-        total = new_bits<1>(a, wb, 1u, v0);
+        if (MODE != SH_LIST) total = new_bits<1>(a, wb, 1u, v0);
       }
     } else {
       v0 = (task - a.npieces) * T;
@@ -1965,13 +1965,14 @@ __device__ __forceinline__ void pull_short_run(const PullArgs &a, uint32_t wb) {
         z &= z - 1;
         for (uint32_t q = lane; q < Q; q += 32) a.N[(size_t)(v0 + t) * Q + q] = make_uint4(0, 0, 0, 0);
       }
-      if (MODE != SH_LAST && fm) total = new_bits<T>(a, wb, fm, v0);
+      if (MODE == SH_GEN && fm) total = new_bits<T>(a, wb, fm, v0);
     }
     __syncwarp();
     while (fm) {
       const uint32_t t = __ffs(fm) - 1;
       fm &= fm - 1;
-      const uint32_t c = __shfl_sync(FULL, total, t);
+      if (MODE == SH_LIST) total = new_bits<1>(a, wb + t * Q, 1u, v0 + t);  // few: one at a time keeps the registers
+      const uint32_t c = __shfl_sync(FULL, total, MODE == SH_LIST ? 0 : t);
       finish_row(a, wb, t, v0 + t, c, __shfl_sync(FULL, oldf, t));
       if (lane == 0 && c) {
         nb += c;
