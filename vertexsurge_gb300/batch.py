@@ -84,9 +84,10 @@ class Batch:
 
     lanes > 1 runs the waves on that many concurrent branches of the captured
     graph, wave w on lane w mod lanes, each lane with its own expand plan and
-    stream: while one wave is in a hop that leaves SMs idle (pair-list hops,
-    decide and clear kernels, the tail of a PULL hop) another wave's kernels
-    fill them."""
+    stream: another wave's kernels may run while one wave is in a hop that leaves
+    SMs idle (pair-list hops, the tail of a PULL hop).  The kernels of a run are placed
+    before the previous one ends and hold their SMs' slots, so a second lane gains
+    little; `tune_wave_rows` times both."""
 
     def __init__(self, dg, queries: list, wave_rows: int, stream, path="shortest", direction="forward",
                  setting: dict | None = None, picker=None, lanes: int = 1):

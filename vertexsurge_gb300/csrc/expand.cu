@@ -1351,16 +1351,16 @@ __global__ void __launch_bounds__(BITS ? 1024 : 256, BITS ? 1 : UPL == 1 ? 4 : U
 //   GEN   any other hop (slots, accumulator, kept layer, long new rows): the bitmaps
 //         start empty and finish_row does every touched target.
 //
-// What bounds it: instructions and latency (about 170 warp instructions a target at
-// 28 edges, IPC 1.5 of 4 with 32 warps on the SM), not DRAM (15 to 25% of the copy
-// rate).  So no call in a kernel's loops (around one, 40 registers went to local
+// What bounds it: instructions and latency (2M-vertex power law, 28 edges a target,
+// 2,048 sources: 200 warp instructions a target where lists are kept, 490 where every
+// target was searched, 0.75 issued a cycle and scheduler), not DRAM.  So no call in a kernel's loops (around one, 40 registers went to local
 // memory that L1 could not hold: 2.2 times slower), words and slots in kernels of
 // their own (together they spill), four targets a tile (eight halve what is left of
 // L1: 7.85 -> 12.2 ms on the 10M-vertex slot hop).  Against a warp per target with
 // its row in registers, 4,096 sources: 1M-vertex power law, the hop after SPARSE 545
 // (a dense hop; short mode did not pay) -> 345 us; backward lists, 2,048 sources 645 +
-// a CTA per hub 409 -> 755 us; 10M vertices, third hop 5.56 -> 5.01 ms, last hop 7.88
-// -> 7.85 ms.
+// a CTA per hub 409 -> 755 us; 10M vertices, third hop 5.56 -> 5.0 ms, last hop 7.88
+// -> 7.7 ms.
 enum { SH_LIST = 0, SH_LAST = 1, SH_GEN = 2 };
 constexpr int SH_WARPS = 8;
 
